@@ -208,3 +208,79 @@ def tolerance(case):
         return {"rel": 1e-5}
     # against 64-bit sums: 2.1e-4, the rounding to fp16
     return {"rel": 8e-4}
+
+
+def _dense_columns(bW, alpha, q_bias, n0, n1):
+    """Columns n0..n1 of the dense weight in 64 bits, [K, n1 - n0]: bit k % 32 of word k / 32 is the sign of weight k."""
+    kw, q, _ = bW.shape
+    G = alpha.shape[0]
+    shift = torch.arange(32, device=bW.device, dtype=torch.int32).view(1, 32, 1)
+    w = 0.0
+    for b in range(q):
+        sign = ((bW[:, b, None, n0:n1] >> shift) & 1).double().mul_(2).sub_(1).view(G, kw * 32 // G, n1 - n0)
+        w = w + sign * alpha[:, b, None, n0:n1].double()
+    if q_bias is not None:
+        w = w + q_bias[:, None, n0:n1].double()
+    return w.view(kw * 32, n1 - n0)
+
+
+def _product(x, bW, alpha, q_bias):
+    """x [m, K] times the weight in 64 bits, a few thousand columns at a time."""
+    N = bW.shape[2]
+    step = max(1, (1 << 26) // (bW.shape[0] * 32))
+    return torch.cat([x.double() @ _dense_columns(bW, alpha, q_bias, n, min(N, n + step)) for n in range(0, N, step)], dim=1)
+
+
+def _exact_scales(w, q, g, rounds):
+    """The quantiser's scales in 64 bits, [G, q, N]: greedy start, then per round the scales from the normal equations
+    by q steps of conjugate gradient (1e-6 in both denominators) and every weight to the nearest level."""
+    N, K = w.shape
+    w = w.double().view(-1, g)
+    c, i = torch.arange(2**q, device=w.device)[:, None], torch.arange(q, device=w.device)[None, :]
+    signs = torch.where(((c >> (q - 1 - i)) & 1) == 1, -1.0, 1.0).double()
+    r, B, alpha = w.clone(), [], []
+    for _ in range(q):
+        B.append(torch.sign(r))
+        alpha.append(r.abs().mean(dim=1))
+        r = r - B[-1] * alpha[-1][:, None]
+    B, alpha = torch.stack(B, dim=2), torch.stack(alpha, dim=1)
+    for _ in range(rounds if q > 1 else 0):
+        A = B.transpose(1, 2) @ B
+        r = (B.transpose(1, 2) @ w[:, :, None] - A @ alpha[:, :, None])[:, :, 0]
+        p, new = r, (r * r).sum(1)
+        for _ in range(q):
+            old, Ap = new, (A @ p[:, :, None])[:, :, 0]
+            a = (old / ((p * Ap).sum(1) + 1e-6))[:, None]
+            alpha, r = alpha + a * p, r - a * Ap
+            new = (r * r).sum(1)
+            p = r + (new / (old + 1e-6))[:, None] * p
+        alpha = alpha.abs().sort(dim=1, descending=True).values
+        level, order = (alpha @ signs.T).sort(dim=1, stable=True)
+        at = torch.searchsorted((level[:, 1:] + level[:, :-1]) / 2, w, right=True)
+        B = signs[torch.gather(order, 1, at)]
+    return alpha.view(N, K // g, q).permute(1, 2, 0)
+
+
+def exact(case, seed):
+    """The outputs of run in 64 bits.  The converter's are whole numbers and roundings that are compared bit for bit, the
+    quantiser's packed words are choices between levels: both have no such value."""
+    kind, gen = case["kind"], _gen(seed)
+    if kind in ("matmul", "linear"):
+        N, K, q, g, m = (case[k] for k in ("N", "K", "q", "g", "m"))
+        container = _layer(gen, N, K, q, g, case["bias"])
+        x = torch.randn((m, K), device="cuda", generator=gen).half()
+        y = _product(x, *container)
+        return y.view(1, m, N) if kind == "linear" else y
+    if kind == "stack":
+        h, f, q, g = case["hidden"], case["ffn"], case["q"], case["g"]
+        x = torch.randn(h, device="cuda", generator=gen).half()[None]
+        for _ in range(case["layers"]):
+            # the first `hidden` values of the first product stand in for the attention result
+            for N, K in ((3 * h, h), (h, h), (f, h), (h, f)):
+                bW, scales = _planes(gen, N, K, q), _scales(gen, (K // g, q, N), 1.0 / math.sqrt(K * q))
+                x = _product(x[:, :K], bW, scales, None)
+        return x[0]
+    if kind == "quantize":
+        w = torch.randn((case["N"], case["K"]), device="cuda", generator=gen) * 0.02
+        return None, _exact_scales(w, case["q"], case["g"], case["rounds"])
+    return None
