@@ -231,6 +231,318 @@ bcq_quantize_kernel(const BqParams p) {
     }
 }
 
+// ---- groups up to 512 wide, up to four planes ----
+// Same arithmetic, several groups to a warp.  LG lanes share one group and hold E weights each (LG * E >= g), so the
+// conjugate gradient, whose arithmetic every lane of a group repeats, and the log2(LG) shuffles of a sum are paid once
+// for 32 / LG groups.  Per round the group writes one table entry per level, in ascending order of the levels: the level's
+// signs as floats and its Gram contributions (1 per pair of planes whose signs differ) packed in 10-bit fields, three
+// pairs to a word.  A weight then costs its q comparisons, one table read, q multiply-adds (B^T w) and one integer add
+// (B^T B) per word of pairs, and the sums of the next round are complete when the weights of this one are placed.
+// Bound by instruction issue, not by memory: the weights are read once.  Measured, N = K = 4096, q = 3, g = 128, 15
+// rounds: 395 us; bcq_quantize_kernel, which gives every group a whole warp, takes 3291 us.
+// Element e of a group: (i * LG + lane) * 4 + c for register 4 i + c, so that four consecutive weights are one 128-bit
+// load and eight consecutive lanes hold the 32 weights of a packed word.
+constexpr int kBqTileWarps = 8;
+constexpr int kBqTileMaxG = 512;              // 32 lanes of 16 weights; a field of pair counts holds up to 1023
+constexpr int kBqTileMaxQ = 4;                // the levels' signs are one 128-bit table entry
+
+template <int LG>
+__device__ __forceinline__ float group_sum_f(float v) {
+#pragma unroll
+    for (int o = LG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+template <int LG>
+__device__ __forceinline__ uint32_t group_sum_u(uint32_t v) {
+#pragma unroll
+    for (int o = LG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+template <int E, int LG, int Q>
+__global__ void __launch_bounds__(kBqTileWarps * 32)
+bcq_quantize_tile_kernel(const BqParams p) {
+    constexpr int GPW = 32 / LG;                           // groups per warp
+    constexpr int NLEV = 1 << Q;
+    constexpr int PAIRS = Q * (Q - 1) / 2;
+    constexpr int PW = (PAIRS + 2) / 3;                    // words of packed pair counts
+    __shared__ float s_level[kBqTileWarps][GPW][NLEV];     // unsorted, then ascending
+    __shared__ __align__(16) float s_sign[kBqTileWarps][GPW][NLEV][4];
+    __shared__ uint32_t s_pair[kBqTileWarps][GPW][NLEV][PW > 0 ? PW : 1];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int l = lane % LG, sub = lane / LG;
+    const int G = p.K / p.g, g = p.g;
+    const long long groups = (long long)p.N * G;
+    const long long first = ((long long)blockIdx.x * kBqTileWarps + wib) * GPW;
+    if (first >= groups) return;                           // whole warps leave together
+    // groups of consecutive rows share a warp: their packed words are neighbours
+    const bool live = first + sub < groups;                // a group beyond the end repeats the warp's first one
+    const long long grp = live ? first + sub : first;
+    const int gi = (int)(grp / p.N), n = (int)(grp % p.N);
+    const float* wg = p.w + (size_t)n * p.K + (size_t)gi * g;
+
+    float wv[E];
+    uint32_t valid = 0u;                                   // bit e: register e holds a weight
+    if (g % 4 == 0 && (reinterpret_cast<uintptr_t>(p.w) & 15) == 0) {        // then so are K and every group's start
+#pragma unroll
+        for (int i = 0; i < E / 4; i++) {
+            const int at = (i * LG + l) * 4;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (at < g) {
+                v = __ldg(reinterpret_cast<const float4*>(wg + at));
+                valid |= 15u << (4 * i);
+            }
+            wv[4 * i] = v.x; wv[4 * i + 1] = v.y; wv[4 * i + 2] = v.z; wv[4 * i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int at = ((e >> 2) * LG + l) * 4 + (e & 3);
+            wv[e] = at < g ? wg[at] : 0.f;
+            valid |= (at < g ? 1u : 0u) << e;
+        }
+    }
+
+    float alpha[Q], btw[Q];
+    uint32_t pos[Q], nz[Q];                                // per plane: sign is +1 / sign is not 0, bit e for register e
+    float A[Q][Q];                                         // B^T B
+    // ---- greedy ----
+    {
+        float r[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) r[e] = wv[e];
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            float s = 0.f, t = 0.f;
+#pragma unroll
+            for (int e = 0; e < E; e++) s += fabsf(r[e]);                    // padding elements are 0
+            float a = group_sum_f<LG>(s) / (float)g;
+            if (a != a) a = 0.f;
+            alpha[i] = a;
+            pos[i] = nz[i] = 0u;
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const float b = r[e] > 0.f ? 1.f : (r[e] < 0.f ? -1.f : 0.f);
+                if (b > 0.f) pos[i] |= 1u << e;
+                if (b != 0.f) nz[i] |= 1u << e;
+                t += b * wv[e];
+                r[e] -= b * a;
+            }
+            // padding never counts: its weight is 0, and its code is masked out
+            pos[i] &= valid;
+            nz[i] &= valid;
+            btw[i] = group_sum_f<LG>(t);
+        }
+#pragma unroll
+        for (int i = 0; i < Q; i++)
+#pragma unroll
+            for (int j = i; j < Q; j++) {
+                const uint32_t both = nz[i] & nz[j];
+                const int c = __popc(both) - 2 * __popc((pos[i] ^ pos[j]) & both);
+                A[i][j] = A[j][i] = (float)(int)group_sum_u<LG>((uint32_t)c);
+            }
+    }
+
+    // ---- alternating refinement ----
+    const uint32_t pad = (uint32_t)(E - __popc(valid));
+    for (int round = 0; Q > 1 && round < p.rounds; round++) {
+        // Q steps of conjugate gradient from the current alpha
+        {
+            float x[Q], r[Q], pp[Q], Ap[Q];
+            float rtr_new = 0.f;
+#pragma unroll
+            for (int i = 0; i < Q; i++) {
+                x[i] = alpha[i];
+                float s = 0.f;
+#pragma unroll
+                for (int j = 0; j < Q; j++) s += A[i][j] * alpha[j];
+                r[i] = btw[i] - s;
+                pp[i] = r[i];
+                rtr_new += r[i] * r[i];
+            }
+#pragma unroll
+            for (int it = 0; it < Q; it++) {
+                const float rtr = rtr_new;
+                float pAp = 0.f;
+#pragma unroll
+                for (int i = 0; i < Q; i++) {
+                    float s = 0.f;
+#pragma unroll
+                    for (int j = 0; j < Q; j++) s += A[i][j] * pp[j];
+                    Ap[i] = s;
+                    pAp += pp[i] * s;
+                }
+                const float a = rtr / (pAp + 1e-6f);
+                rtr_new = 0.f;
+#pragma unroll
+                for (int i = 0; i < Q; i++) {
+                    x[i] += a * pp[i];
+                    r[i] -= a * Ap[i];
+                    rtr_new += r[i] * r[i];
+                }
+                const float beta = rtr_new / (rtr + 1e-6f);
+#pragma unroll
+                for (int i = 0; i < Q; i++) pp[i] = r[i] + beta * pp[i];
+            }
+            // |alpha| descending (insertion sort)
+#pragma unroll
+            for (int i = 0; i < Q; i++) alpha[i] = fabsf(x[i]);
+#pragma unroll
+            for (int i = 1; i < Q; i++) {
+#pragma unroll
+                for (int j = i; j > 0; j--)
+                    if (alpha[j] > alpha[j - 1]) { const float t = alpha[j]; alpha[j] = alpha[j - 1]; alpha[j - 1] = t; }
+            }
+        }
+        // the levels, in ascending order, ties by index: level c has sign -1 on plane i iff bit Q-1-i of c is set
+        constexpr int LPL = (NLEV + LG - 1) / LG;          // levels per lane
+        float lv[LPL];
+        __syncwarp();                                      // the previous round's tables have been read
+#pragma unroll
+        for (int u = 0; u < LPL; u++) {
+            const int c = l + u * LG;
+            float v = 0.f;
+#pragma unroll
+            for (int i = 0; i < Q; i++) v += ((c >> (Q - 1 - i)) & 1) ? -alpha[i] : alpha[i];
+            lv[u] = v;
+            if (c < NLEV) s_level[wib][sub][c] = v;
+        }
+        __syncwarp();
+        int rank[LPL];
+#pragma unroll
+        for (int u = 0; u < LPL; u++) rank[u] = 0;
+#pragma unroll
+        for (int d = 0; d < NLEV; d++) {
+            const float o = s_level[wib][sub][d];
+#pragma unroll
+            for (int u = 0; u < LPL; u++) rank[u] += (o < lv[u] || (o == lv[u] && d < l + u * LG)) ? 1 : 0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < LPL; u++) {
+            const int c = l + u * LG;
+            if (c >= NLEV) continue;
+            s_level[wib][sub][rank[u]] = lv[u];
+            float sg[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) sg[i] = i < Q ? (((c >> (Q - 1 - i)) & 1) ? -1.f : 1.f) : 0.f;
+            *reinterpret_cast<float4*>(s_sign[wib][sub][rank[u]]) = make_float4(sg[0], sg[1], sg[2], sg[3]);
+            uint32_t pk[PW > 0 ? PW : 1] = {};
+            int t = 0;
+#pragma unroll
+            for (int i = 0; i < Q; i++)
+#pragma unroll
+                for (int j = i + 1; j < Q; j++, t++) pk[t / 3] |= (uint32_t)(((c >> (Q - 1 - i)) ^ (c >> (Q - 1 - j))) & 1) << (10 * (t % 3));
+#pragma unroll
+            for (int i = 0; i < PW; i++) s_pair[wib][sub][rank[u]][i] = pk[i];
+        }
+        __syncwarp();
+        // every weight to its nearest level: bisection on the midpoints, `w < mid` goes left
+        float mid[NLEV - 1];
+#pragma unroll
+        for (int c = 0; c + 1 < NLEV; c++) mid[c] = (s_level[wib][sub][c] + s_level[wib][sub][c + 1]) / 2.f;
+        const bool last = round + 1 == p.rounds;
+        auto place = [&](float w) {
+            int at = 0;
+            float m = mid[NLEV / 2 - 1];
+#pragma unroll
+            for (int s = NLEV / 2; s > 0; s >>= 1) {
+                at = w < m ? at : at + s;
+                if (s > 1) {
+                    // the midpoint of the half that is left: at + s / 2 - 1, out of registers
+                    float next = mid[s / 2 - 1];
+#pragma unroll
+                    for (int c = s; c < NLEV; c += s) next = at == c ? mid[c + s / 2 - 1] : next;
+                    m = next;
+                }
+            }
+            return at;
+        };
+        if (!last) {
+            uint32_t pk[PW > 0 ? PW : 1] = {};
+#pragma unroll
+            for (int i = 0; i < Q; i++) btw[i] = 0.f;
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const int at = place(wv[e]);
+                const float4 sg = *reinterpret_cast<const float4*>(s_sign[wib][sub][at]);
+                const float sv[4] = {sg.x, sg.y, sg.z, sg.w};
+#pragma unroll
+                for (int i = 0; i < Q; i++) btw[i] = fmaf(sv[i], wv[e], btw[i]);
+#pragma unroll
+                for (int i = 0; i < PW; i++) pk[i] += s_pair[wib][sub][at][i];
+            }
+            // padding registers hold 0 and were placed with it: their pairs come off again
+            if (pad) {
+                const int at = place(0.f);
+#pragma unroll
+                for (int i = 0; i < PW; i++) pk[i] -= pad * s_pair[wib][sub][at][i];
+            }
+#pragma unroll
+            for (int i = 0; i < Q; i++) {
+                btw[i] = group_sum_f<LG>(btw[i]);
+                A[i][i] = (float)g;
+            }
+#pragma unroll
+            for (int i = 0; i < PW; i++) pk[i] = group_sum_u<LG>(pk[i]);
+            int t = 0;
+#pragma unroll
+            for (int i = 0; i < Q; i++)
+#pragma unroll
+                for (int j = i + 1; j < Q; j++, t++)
+                    A[i][j] = A[j][i] = (float)(g - 2 * (int)((pk[t / 3] >> (10 * (t % 3))) & 1023u));
+        } else {
+#pragma unroll
+            for (int i = 0; i < Q; i++) { pos[i] = 0u; nz[i] = valid; }
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const float4 sg = *reinterpret_cast<const float4*>(s_sign[wib][sub][place(wv[e])]);
+                const float sv[4] = {sg.x, sg.y, sg.z, sg.w};
+#pragma unroll
+                for (int i = 0; i < Q; i++) pos[i] |= (sv[i] > 0.f ? 1u : 0u) << e;
+            }
+#pragma unroll
+            for (int i = 0; i < Q; i++) pos[i] &= valid;
+        }
+    }
+
+    // ---- outputs ----
+    if (live && l == 0) {
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            if (p.alpha_py) p.alpha_py[((size_t)n * G + gi) * Q + i] = alpha[i];
+            if (p.alpha_k) p.alpha_k[((size_t)gi * Q + i) * p.N + n] = __float2half_rn(alpha[i]);
+        }
+    }
+    if (live && p.binary_py) {
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int at = ((e >> 2) * LG + l) * 4 + (e & 3);
+            if (at < g) {
+                signed char* dst = p.binary_py + (((size_t)n * G + gi) * g + at) * Q;
+#pragma unroll
+                for (int i = 0; i < Q; i++) dst[i] = (signed char)(((nz[i] >> e) & 1u) ? (((pos[i] >> e) & 1u) ? 1 : -1) : 0);
+            }
+        }
+    }
+    if (p.bW) {                                            // g % 32 == 0: whole words; a zero code packs as -1
+        constexpr int NIB = LG >= 8 ? 1 : 8 / LG;          // nibbles of one word in the same lane
+        constexpr int WL = LG >= 8 ? 8 : LG;               // lanes that share a word
+#pragma unroll
+        for (int i = 0; i < E / 4; i += NIB)
+#pragma unroll
+            for (int b = 0; b < Q; b++) {
+                uint32_t word = 0u;
+#pragma unroll
+                for (int k = 0; k < NIB; k++) word |= ((pos[b] >> (4 * (i + k))) & 15u) << (4 * (k * LG + l % WL));
+#pragma unroll
+                for (int o = WL / 2; o > 0; o >>= 1) word |= __shfl_xor_sync(0xffffffffu, word, o);
+                const int kw = (i * LG + l) / 8;           // word of the group
+                if (live && l % WL == 0 && kw * 32 < g) p.bW[((size_t)(gi * (g / 32) + kw) * Q + b) * p.N + n] = word;
+            }
+    }
+}
+
 // ---- groups wider than 1024 (the reference's default is one group per row): one CTA per (row, group) ----
 // Same arithmetic; the codes live in shared memory (2 bytes per weight), the weights are re-read from global memory
 // (L2) twice per round, sums go through warp shuffles and a shared-memory stage, and warp 0 solves for alpha and

@@ -70,6 +70,29 @@ def test_device_quantiser_matches_oracle(N, K, g, q, rounds):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,K,g,q,rounds", [
+    # groups up to 512 wide and up to four planes share a warp: every lane count, full and ragged lanes, a group count that
+    # is no multiple of a warp's, widths that are no multiple of 4, no refinement at all, weights that are exactly 0
+    (5, 192, 64, 3, 4), (7, 96, 32, 2, 3), (3, 512, 512, 4, 5), (9, 400, 400, 3, 3), (11, 200, 50, 3, 3), (13, 129, 43, 4, 2),
+    (6, 384, 192, 2, 15), (33, 256, 128, 1, 3), (4, 260, 65, 4, 0), (1, 128, 128, 3, 1)])
+def test_device_quantiser_several_groups_per_warp(N, K, g, q, rounds):
+    import torch
+    import lutgemm_b200 as L
+    rng = np.random.default_rng(N * K + q)
+    w = (rng.normal(0, 0.02, (N, K))).astype(np.float32)
+    w[:, ::17] = 0.0
+    _, B_ref, alpha_ref = bq.quantize(w, q, rounds, g)
+    _, B, alpha = L.bcq_quantize(w, q, rounds, g)
+    _compare(alpha, B, alpha_ref, B_ref.astype(np.int8), w)
+    if g % 32 == 0:
+        # the container layout holds the same codes (+1 = set bit) and the same scales
+        bW, alpha_k = L.bcq_quantize_device(torch.from_numpy(w).cuda(), q, rounds=rounds, group_size=g)
+        bits = (B.reshape(N, K // 32, 32, q) > 0).astype(np.uint64) << np.arange(32, dtype=np.uint64)[:, None]
+        assert np.array_equal(bW.cpu().numpy().view(np.uint32), bits.sum(2).transpose(1, 2, 0).astype(np.uint32))
+        assert np.array_equal(alpha_k.cpu().numpy(), alpha.transpose(1, 2, 0).astype(np.float16))
+
+
+@pytest.mark.gpu
 def test_device_quantiser_feeds_the_matmul():
     """Quantise on the device straight into the container layout, multiply, compare with x W_hat^T from the oracle."""
     import torch
