@@ -19,6 +19,7 @@
 #include "gemv_tma2.cuh"
 #include "gemv_seq.cuh"
 #include "gemm_tc.cuh"
+#include "gemm_hl.cuh"
 #include "gemm_i8.cuh"
 #include "bcq_quantize.cuh"
 #include "gptq3.cuh"
@@ -579,6 +580,153 @@ int gemm_tc_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
     return LUTGEMM_ERR_BITS;
 }
 
+// ---- split-operand kernel (gemm_hl.cuh): plan, launch ----
+// fp32 workspace rows (of N columns) that a batch of m can ask for: split-k is only planned while the output has fewer
+// than about one tile of 128 x 256 per SM, which bounds it to some 20 MB.
+int hl_rows_for(int N, int m) {
+    const int T = (N + lg::kHlCols - 1) / lg::kHlCols;
+    const int cap = lg::kHlRows * (sm_count() / T + 1);
+    const int rows = m < cap ? m : cap;
+    return rows > tc_rows_for(m) ? rows : tc_rows_for(m);
+}
+
+// One CTA per SM: an item is 128 columns x 256 rows, and an item may be cut into two halves of 128 rows or into k-ranges.
+// Cost model in cycles: a block of 64 k takes the tensor pipe 4 cycles per row (two passes; 2 with one) and the expansion
+// at least kHlExpCycles whatever the rows; a CTA's start, first loads and epilogue add kHlCtaCycles, a split's reductions
+// and last-arriver pass kHlSplitCycles.  The plan with the smallest estimate is taken: whole items, halves, whole items
+// with a last partial wave of halves, each with 1 to 8 k-ranges.
+constexpr int kHlExpCycles = 560, kHlCtaCycles = 7000, kHlSplitCycles = 4000;
+void hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) {
+    const int sms = sm_count();
+    const int T = (w->N + lg::kHlCols - 1) / lg::kHlCols, RT = (m + lg::kHlRows - 1) / lg::kHlRows;
+    const long long items = (long long)T * RT;
+    const int blocks = (w->K + lg::kHlStepK - 1) / lg::kHlStepK;
+    const int per_row = (w->q == 1 && !w->q_bias) ? 2 : 4;
+    auto block_cost = [&](int rows) { const int t = per_row * ((rows + 15) / 16 * 16); return t > kHlExpCycles ? t : kHlExpCycles; };
+    const int whole_rows = m < lg::kHlRows ? m : lg::kHlRows, half_rows = m < 128 ? m : 128;
+    const long long units = m <= 128 ? items : (long long)T * ((m + 127) / 128);       // halves that have rows
+    p->col_tiles = T;
+    p->splits = 1;
+    p->blocks_per_split = blocks;
+    p->full_items = (int)items;
+    double best = 1e300;
+    auto consider = [&](long long full, long long halves, int c) {
+        const int bps = (blocks + c - 1) / c;
+        const int real = (blocks + bps - 1) / bps;
+        const long long nf = full * real, nh = halves * real;
+        const double extra = kHlCtaCycles + (real > 1 ? kHlSplitCycles : 0);
+        const double t = (double)((nf + sms - 1) / sms) * (extra + (double)bps * block_cost(whole_rows)) +
+                         (double)((nh + sms - 1) / sms) * (extra + (double)bps * block_cost(half_rows));
+        if (t < best * 0.98) {
+            best = t;
+            p->full_items = (int)full; p->splits = real; p->blocks_per_split = bps;
+        }
+    };
+    const long long tail_full = items / sms * sms;
+    for (int c = 1; c <= 8 && c <= blocks; c++) {
+        if (c > 1 && (!may_split || items >= sms)) break;
+        consider(items, 0, c);
+        if (m > 128) {
+            consider(0, units, c);
+            if (c == 1 && tail_full > 0 && tail_full < items) consider(tail_full, 2 * (items - tail_full), 1);
+        }
+    }
+}
+
+// From this many rows on the split-operand kernel is the faster one (see gemm_hl.cuh).
+constexpr int kHlFromRows = 129;
+bool gemm_hl_ok(const lutgemm_weight* w, int m) { return w->tc_ok && w->q <= 4 && m >= kHlFromRows; }
+
+// fp32 rows of the workspace for at least `rows` rows of w's width, growing the container's own workspace when that is
+// possible now (it synchronises the device: not inside a stream capture).  *have false: not available.
+int hl_have_rows(lutgemm_weight* w, lutgemm_workspace* ws, int rows, cudaStream_t st, bool* have) {
+    *have = (long long)ws->tc_rows * ws->n_cap >= (long long)rows * w->N;
+    if (*have || ws != &w->own) return LUTGEMM_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone) return LUTGEMM_OK;
+    if (ws->tc_partial) LG_CUDA(cudaFree(ws->tc_partial));
+    ws->tc_partial = nullptr;
+    ws->tc_rows = 0;
+    LG_CUDA(cudaMalloc(&ws->tc_partial, (size_t)rows * w->N * sizeof(float)));
+    LG_CUDA(cudaMemset(ws->tc_partial, 0, (size_t)rows * w->N * sizeof(float)));
+    ws->tc_rows = rows;
+    *have = true;
+    return LUTGEMM_OK;
+}
+
+template <int Q>
+int launch_gemm_hl_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::HlParams& p, dim3 grid, cudaStream_t st) {
+    static bool configured[64][2] = {};   // the attribute is per device
+    const bool bias = w->q_bias != nullptr;
+    auto kern = bias ? lg::gemm_hl_kernel<Q, true> : lg::gemm_hl_kernel<Q, false>;
+    int dev = 0;
+    LG_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !configured[dev][bias]) {
+        LG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lg::kSmemLimit));
+        if (dev < 64) configured[dev][bias] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(lg::kHlThreads);
+    cfg.dynamicSmemBytes = (size_t)lg::kSmemLimit;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_pdl.load() ? 1 : 0;
+    LG_CUDA(cudaLaunchKernelEx(&cfg, kern, tmX, p));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    LG_CUDA(cudaGetLastError());
+    return LUTGEMM_OK;
+}
+
+// Rows [0, m) through the split-operand kernel, one launch (gemm_hl_ok holds).
+int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __half* y16, float* y32, int m, cudaStream_t st) {
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return LUTGEMM_ERR_CUDA;
+    // what a call without reserved scratch is told does not depend on the kernel: the plane kernel's rule, for its first launch
+    int unused_split = 1, unused_steps = 0;
+    int rc = tc_split(w, ws, m < 128 ? m : 128, st, &unused_split, &unused_steps);
+    if (rc != LUTGEMM_OK) return rc;
+    lg::HlParams p = {};
+    hl_plan(w, m, !ordered_for(ws), &p);
+    if (p.splits > 1) {
+        bool have = false;
+        rc = hl_have_rows(w, ws, m, st, &have);
+        if (rc != LUTGEMM_OK) return rc;
+        if (!have) hl_plan(w, m, false, &p);
+    }
+    p.box_rows = m < lg::kHlBoxRows ? (m + 15) / 16 * 16 : lg::kHlBoxRows;
+    p.x_slot_bytes = (m <= lg::kHlBoxRows || p.full_items == 0 ? 1 : 2) * p.box_rows * 128;
+    p.x_slots = lg::kHlXBudget / p.x_slot_bytes;
+    if (p.x_slots > lg::kHlMaxSlots) p.x_slots = lg::kHlMaxSlots;
+    CUtensorMap tmX;
+    {
+        cuuint64_t dims[2] = {(cuuint64_t)w->K, (cuuint64_t)m};
+        cuuint64_t strides[1] = {(cuuint64_t)w->K * 2};
+        cuuint32_t box[2] = {64, (cuuint32_t)p.box_rows};
+        cuuint32_t es[2] = {1, 1};
+        if (enc(&tmX, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(x), dims, strides, box, es,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return LUTGEMM_ERR_CUDA;
+    }
+    p.bW = w->bW; p.alpha = w->alpha; p.q_bias = w->q_bias;
+    p.partial = ws->tc_partial; p.counters = ws->counters; p.status = ws->status;
+    p.y16 = y16; p.y32 = y32;
+    p.N = w->N; p.K = w->K; p.G = w->G; p.g = w->g; p.m = m;
+    const long long items = (long long)p.col_tiles * ((m + lg::kHlRows - 1) / lg::kHlRows);
+    dim3 grid((unsigned)(p.full_items + 2 * (items - p.full_items)), p.splits);
+    switch (w->q) {
+        case 1: return launch_gemm_hl_q<1>(w, tmX, p, grid, st);
+        case 2: return launch_gemm_hl_q<2>(w, tmX, p, grid, st);
+        case 3: return launch_gemm_hl_q<3>(w, tmX, p, grid, st);
+        case 4: return launch_gemm_hl_q<4>(w, tmX, p, grid, st);
+    }
+    return LUTGEMM_ERR_BITS;
+}
+
 template <int Q>
 int launch_gemm_i8_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::I8Params& p, dim3 grid, cudaStream_t st) {
     static bool configured[64][2] = {};   // the attribute is per device
@@ -698,6 +846,7 @@ int matmul_impl(__half* y16, float* y32, const void* in, lutgemm_weight_t w, int
         }
         return LUTGEMM_OK;
     }
+    if (gemm_hl_ok(w, m)) return gemm_hl_rows(w, ws, x, y16, y32, m, st);
     // batched: 128 rows per tensor-core launch
     for (int r0 = 0; r0 < m; r0 += 128) {
         const int rows = (m - r0 < 128) ? (m - r0) : 128;
@@ -967,7 +1116,7 @@ int lutgemm_weight_reserve_batch(lutgemm_weight_t w, int m) {
     if (!w) return LUTGEMM_ERR_NULL;
     if (m < 1 || m > kMaxBatch) return LUTGEMM_ERR_BATCH;
     lutgemm_workspace* ws = &w->own;
-    const int rows = tc_rows_for(m);
+    const int rows = hl_rows_for(w->N, m);
     if (m >= 2 && ws->tc_rows < rows) {
         if (ws->tc_partial) LG_CUDA(cudaFree(ws->tc_partial));
         ws->tc_partial = nullptr; ws->tc_rows = 0;

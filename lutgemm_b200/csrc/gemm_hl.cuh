@@ -1,0 +1,428 @@
+// Batched BCQ matmul with the planes folded into one split operand, on the 5th-generation tensor cores, sm_100a.
+//
+// gemm_tc.cuh multiplies every bit plane by itself: q (or q + 1 with q_bias) tensor-core passes over the activations.
+// Inside a scale group a weight takes only 2^q values, W = q_bias + sum_b +-alpha_b, so here each column's values are
+// computed once per group in fp32, split as hi + lo (two fp16 numbers, lo = fp16(W - hi)) and the packed bits only
+// choose between them: two passes whatever q is, and no rounding of the weight beyond 2^-22 of it.  So that lo never
+// falls into fp16's subnormals (and hi never overflows) a CTA scales every column by a power of two taken from the
+// largest scale of that column in the CTA's k-range, and takes it out again in the epilogue.  (One plane without q_bias
+// is exact as it is: one pass, no lo.)
+//
+//   CTA = 128 output columns x up to 256 activation rows x a k-range, walked in blocks of 64 k.
+//   16 expansion warps: warp (quarter lq of the columns, sub) takes the blocks j with j mod 4 == sub.  Lane = column.  The
+//   packed words and scales come straight from global memory, one block of this warp (four of the CTA) ahead.  The
+//   lane writes the 2^q (hi, lo) pairs of its column to its own bank of a table in shared memory (no other lane reads
+//   them: no synchronisation, no bank conflicts), turns the q words into one code per byte (a bit transpose of shifts
+//   and LOP3s), looks 64 weights up (one PRMT makes a code byte and the lane's bank an address) and stores them with
+//   tcgen05.st as the A operand in tensor memory.
+//   One lane issues tcgen05.mma.kind::f16: M = 128 columns, N = rows, K = 16, A (hi, then lo) in tensor memory, the
+//   activations [rows][64 k] (TMA, 128-byte swizzle) in shared memory, one fp32 accumulator.
+//
+// Tensor memory: 256 accumulator columns, then four operand stages of 64 columns (hi 32, lo 32), one per `sub`.
+//
+// All mbarrier waits are bounded, as in gemm_tc.cuh.
+#pragma once
+#include "gemm_tc.cuh"
+
+namespace lg {
+
+constexpr int kHlCols = 128;                  // output columns per CTA
+constexpr int kHlStepK = 64;                  // k per block
+constexpr int kHlRows = 256;                  // most activation rows per CTA
+constexpr int kHlBoxRows = 128;               // rows per TMA box of the activations (fewer when the call has fewer)
+constexpr int kHlExpWarps = 16, kHlMmaWarp = 0, kHlTmaWarp = 1, kHlFirstExpWarp = 2;
+constexpr int kHlThreads = (kHlFirstExpWarp + kHlExpWarps) * 32;      // 576
+constexpr int kHlStages = 4;                  // operand stages in tensor memory, one per `sub`
+constexpr uint32_t kHlACol = 256;             // first operand column
+constexpr int kHlMaxSlots = 8;                // activation ring
+constexpr int kHlTableBytes = kHlExpWarps * 16 * 128;                 // offset 0: [pair of warps][16 values][2 warps][32 lanes] x 4 B
+constexpr int kHlScaleOff = kHlTableBytes;                            // [128] largest |scale| (fp16 bits) per column
+constexpr int kHlBarOff = kHlScaleOff + kHlCols * 4;
+constexpr int kHlXOff = kHlTableBytes + 1024;                         // multiple of 1024: swizzle atoms
+constexpr int kHlXBudget = kSmemLimit - kHlXOff;                      // also the epilogue's transposes (16 x 16 x 33 floats)
+
+struct HlParams {
+    const uint32_t* bW;      // [K/32][q][N]
+    const __half* alpha;     // [G][q][N]
+    const __half* q_bias;    // [G][N] or nullptr
+    float* partial;          // [m][N] fp32, zero between launches (split-k only)
+    unsigned* counters;      // one per output tile, zero between launches
+    int* status;
+    __half* y16;             // [m][N] or nullptr
+    float* y32;              // [m][N] or nullptr
+    int N, K, G, g, m;
+    int col_tiles;           // tiles of 128 columns
+    int full_items;          // items (column tile, 256 rows) that one CTA takes whole; the rest go as two halves of 128 rows
+    int splits;              // k-ranges per item; a range is blocks_per_split blocks of 64 k
+    int blocks_per_split;
+    int box_rows;            // rows of a TMA box: 128, or m rounded up to 16 when that is less
+    int x_slot_bytes, x_slots;
+};
+
+// (hi, lo) of two values, hi in the low half of an entry
+__device__ __forceinline__ void hl_pack_pair(float v0, float v1, uint32_t& e0, uint32_t& e1) {
+    const __half2 hi = __floats2half2_rn(v0, v1);
+    const float2 f = __half22float2(hi);
+    const __half2 lo = __floats2half2_rn(v0 - f.x, v1 - f.y);
+    const uint32_t h = *reinterpret_cast<const uint32_t*>(&hi), l = *reinterpret_cast<const uint32_t*>(&lo);
+    e0 = prmt_b32(h, l, 0x5410u);
+    e1 = prmt_b32(h, l, 0x7632u);
+}
+
+// Q: number of bit planes (1..4); BIAS: container has q_bias.  tmX: 2-D map {K, m} of fp16, box {64, box_rows}, 128-byte swizzle.
+template <int Q, bool BIAS>
+__global__ void __launch_bounds__(kHlThreads, 1)
+gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
+    constexpr int NV = 1 << Q;
+    constexpr int PASSES = (Q == 1 && !BIAS) ? 1 : 2;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const uint32_t smem_base = smem_u32(smem);
+    const uint32_t bar_xfull = smem_base + kHlBarOff;             // kHlMaxSlots each
+    const uint32_t bar_xempty = bar_xfull + 8 * kHlMaxSlots;
+    const uint32_t bar_afull = bar_xempty + 8 * kHlMaxSlots;      // kHlStages each
+    const uint32_t bar_aempty = bar_afull + 8 * kHlStages;
+    const uint32_t bar_acc = bar_aempty + 8 * kHlStages;
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + kHlBarOff + 16 * kHlMaxSlots + 16 * kHlStages + 16);
+    int* s_flag = reinterpret_cast<int*>(s_tmem + 1);
+    unsigned* s_max = reinterpret_cast<unsigned*>(smem + kHlScaleOff);
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int N = p.N;
+    // this CTA's item: 256 rows, or a half of one
+    int item = blockIdx.x, half_row = 0, rows_cap = kHlRows;
+    if (item >= p.full_items) {
+        const int h = item - p.full_items;
+        item = p.full_items + (h >> 1);
+        half_row = (h & 1) * (kHlRows / 2);
+        rows_cap = kHlRows / 2;
+    }
+    const int n0 = (item % p.col_tiles) * kHlCols;
+    const int row0 = (item / p.col_tiles) * kHlRows + half_row;
+    if (row0 >= p.m) return;                                      // the second half of a last, short item
+    const int rows = min(rows_cap, p.m - row0);
+    const int n_mma = (rows + 15) & ~15;
+    const int blocks_total = (p.K + kHlStepK - 1) / kHlStepK;
+    const int blk_begin = blockIdx.y * p.blocks_per_split;
+    const int nblk = min(blocks_total, blk_begin + p.blocks_per_split) - blk_begin;      // >= 1 by the plan
+
+    if (tid == 0) {
+        for (int s = 0; s < kHlMaxSlots; s++) {
+            mbar_init(bar_xfull + 8 * s, 1);
+            mbar_init(bar_xempty + 8 * s, 1);
+        }
+        for (int s = 0; s < kHlStages; s++) {
+            mbar_init(bar_afull + 8 * s, 4);                      // the four column quarters
+            mbar_init(bar_aempty + 8 * s, 1);
+        }
+        mbar_init(bar_acc, 1);
+        mbar_fence_init();
+    }
+    if (tid < kHlCols) s_max[tid] = 0u;
+    if (warp == kHlMmaWarp) {
+        tmem_alloc(smem_u32(s_tmem), kTcTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *s_tmem;
+    bool timed_out = false;
+    // the packed planes and scales are never written by a kernel: their stream starts while the previous kernel drains
+    pdl_launch_dependents();
+
+    const int lq = warp & 3;                                      // TMEM lane quarter this warp may access
+    const int ew = warp - kHlFirstExpWarp, sub = ew >> 2;
+    const int col_l = lq * 32 + lane, col = n0 + col_l;
+    float unscale = 1.f;
+    if (warp >= kHlFirstExpWarp) {
+        // ---------------- expansion ----------------
+        const bool col_ok = col < N;
+        const size_t row_w = (size_t)Q * N;                       // words per k-word row, scales per group
+        uint32_t w[2][Q];
+        unsigned short av[2][Q], bv[2];
+        // this lane's next block: its words, its group (advanced by 4 blocks = 256 k without a division)
+        const uint32_t* wptr = p.bW + (size_t)(blk_begin + sub) * 2 * row_w + col;
+        int knext = (blk_begin + sub) * kHlStepK;
+        const int kend = min(p.K, (blk_begin + nblk) * kHlStepK);
+        int grp = knext / p.g, grem = knext % p.g;
+        const int ginc = (4 * kHlStepK) / p.g, grinc = (4 * kHlStepK) % p.g;
+        auto fetch = [&]() {
+            const bool ok = col_ok && knext < kend, ok1 = col_ok && knext + 32 < kend;
+            const unsigned short* a0 = reinterpret_cast<const unsigned short*>(p.alpha) + (size_t)grp * row_w + col;
+            const unsigned short* q0 = reinterpret_cast<const unsigned short*>(p.q_bias) + (BIAS ? (size_t)grp * N + col : 0);
+#pragma unroll
+            for (int b = 0; b < Q; b++) {
+                w[0][b] = ok ? __ldg(wptr + (size_t)b * N) : 0u;
+                w[1][b] = ok1 ? __ldg(wptr + row_w + (size_t)b * N) : 0u;
+                av[0][b] = ok ? __ldg(a0 + (size_t)b * N) : (unsigned short)0;
+            }
+            if (BIAS) bv[0] = ok ? __ldg(q0) : (unsigned short)0;
+            if (p.g < kHlStepK) {                                 // g == 32: the second word has scales of its own
+#pragma unroll
+                for (int b = 0; b < Q; b++) av[1][b] = ok1 ? __ldg(a0 + row_w + (size_t)b * N) : (unsigned short)0;
+                if (BIAS) bv[1] = ok1 ? __ldg(q0 + N) : (unsigned short)0;
+            }
+            wptr += 8 * row_w;
+            knext += 4 * kHlStepK;
+            grp += ginc;
+            grem += grinc;
+            if (grem >= p.g) { grem -= p.g; grp++; }
+        };
+        fetch();
+        // largest |scale| per column over this k-range: 16 threads x 8 columns per row of scales
+        {
+            const int grp0 = blk_begin * kHlStepK / p.g;
+            const int grp1 = min(p.G, (kend + p.g - 1) / p.g);
+            const int et = tid - kHlFirstExpWarp * 32, c8 = (et & 15) * 8;
+            uint32_t mx[4] = {0u, 0u, 0u, 0u};
+            if (n0 + c8 < N) {                                    // N % 8 == 0: whole chunks
+                const int a_rows = (grp1 - grp0) * Q, all = a_rows + (BIAS ? grp1 - grp0 : 0);
+#pragma unroll 4
+                for (int r = et >> 4; r < all; r += kHlExpWarps * 2) {
+                    const __half* src = r < a_rows ? p.alpha + ((size_t)grp0 * Q + r) * N : p.q_bias + (size_t)(grp0 + r - a_rows) * N;
+                    const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + n0 + c8));
+                    const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int i = 0; i < 4; i++) mx[i] = __vmaxu2(mx[i], vv[i] & 0x7fff7fffu);      // |fp16| orders like its bits
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) mx[i] = __vmaxu2(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 16));
+            if (lane < 16) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    atomicMax(s_max + c8 + 2 * i, mx[i] & 0xffffu);
+                    atomicMax(s_max + c8 + 2 * i + 1, mx[i] >> 16);
+                }
+            }
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(kHlExpWarps * 32) : "memory");
+        // |W| <= (Q + 1) max < 2^(e + 4) with e = exponent of max: the scale 2^(11 - e) keeps |W| below 2^15.  All
+        // zero, or not finite: 1 (the column's result is not finite either).
+        float scale = 1.f;
+        {
+            const unsigned mbits = s_max[col_l];
+            if (mbits != 0u && mbits < 0x7c00u) {
+                const int e = (int)(__float_as_uint(__half2float(__ushort_as_half((unsigned short)mbits))) >> 23) - 127;
+                scale = __uint_as_float((uint32_t)(127 + 11 - e) << 23);
+                unscale = __uint_as_float((uint32_t)(127 - 11 + e) << 23);
+            }
+        }
+        // table entry of code c at (pair << 12) + (c << 8) + bank: the code byte carries the pair in its high nibble
+        const uint32_t bank = (uint32_t)lane * 4u + (uint32_t)(ew & 1) * 128u;
+        const uint32_t pair4 = (uint32_t)(ew >> 1) * 0x10101010u;
+        unsigned char* tab = smem + (ew >> 1) * 4096 + bank;
+        const uint32_t t_dst = tmem_base + ((uint32_t)(lq * 32) << 16) + kHlACol + (uint32_t)sub * 64u;
+        int round = 0;
+        for (int j = sub; j < nblk; j += kHlStages, round++) {
+            uint32_t cw[2][Q];
+            float a[2][Q], qb[2] = {0.f, 0.f};
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+#pragma unroll
+                for (int b = 0; b < Q; b++) cw[u][b] = w[u][b];
+                if (u == 0 || p.g < kHlStepK) {
+#pragma unroll
+                    for (int b = 0; b < Q; b++) a[u][b] = __half2float(__ushort_as_half(av[u][b])) * scale;
+                    if (BIAS) qb[u] = __half2float(__ushort_as_half(bv[u])) * scale;
+                }
+            }
+            fetch();
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (u == 0 || p.g < kHlStepK) {
+                    // the column's 2^Q values: bit b of the code set = +alpha_b
+                    float bound = fabsf(qb[u]);
+#pragma unroll
+                    for (int b = 0; b < Q; b++) bound += fabsf(a[u][b]);
+                    float v[NV];
+                    v[0] = qb[u];
+#pragma unroll
+                    for (int b = Q - 1; b >= 0; b--) {            // v[c] for c a multiple of 2^b, halving the stride
+#pragma unroll
+                        for (int c = 0; c < NV; c += 2 << b) {
+                            const float s = v[c];
+                            v[c] = s - a[u][b];
+                            v[c + (1 << b)] = s + a[u][b];
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < NV; c += 2) {
+                        uint32_t e0, e1;
+                        hl_pack_pair(v[c], v[c + 1], e0, e1);
+                        *reinterpret_cast<uint32_t*>(tab + c * 256) = e0;
+                        *reinterpret_cast<uint32_t*>(tab + (c + 1) * 256) = e1;
+                    }
+                    if (!(bound <= 65504.f)) {                    // an infinite or NaN scale: the value itself, lo = 0
+#pragma unroll 1
+                        for (int c = 0; c < NV; c++) {
+                            uint32_t* e = reinterpret_cast<uint32_t*>(tab + c * 256);
+                            if ((*e & 0x7c00u) == 0x7c00u) *e &= 0xffffu;
+                        }
+                    }
+                }
+                // q words of 32 bits -> nibble words (code of weight 4 i + r = nibble i of n[r]) -> one code per byte
+                uint32_t lo4[4], hi4[4];
+                {
+                    const uint32_t w0 = cw[u][0], w1 = Q > 1 ? cw[u][Q > 1 ? 1 : 0] : 0u;
+                    const uint32_t w2 = Q > 2 ? cw[u][Q > 2 ? 2 : 0] : 0u, w3 = Q > 3 ? cw[u][Q > 3 ? 3 : 0] : 0u;
+                    const uint32_t e01 = (w0 & 0x55555555u) | ((w1 << 1) & 0xaaaaaaaau), o01 = ((w0 >> 1) & 0x55555555u) | (w1 & 0xaaaaaaaau);
+                    const uint32_t e23 = (w2 & 0x55555555u) | ((w3 << 1) & 0xaaaaaaaau), o23 = ((w2 >> 1) & 0x55555555u) | (w3 & 0xaaaaaaaau);
+                    uint32_t n[4];
+                    n[0] = (e01 & 0x33333333u) | ((e23 << 2) & 0xccccccccu);
+                    n[1] = (o01 & 0x33333333u) | ((o23 << 2) & 0xccccccccu);
+                    n[2] = ((e01 >> 2) & 0x33333333u) | (e23 & 0xccccccccu);
+                    n[3] = ((o01 >> 2) & 0x33333333u) | (o23 & 0xccccccccu);
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        lo4[r] = (n[r] & 0x0f0f0f0fu) | pair4;
+                        hi4[r] = ((n[r] >> 4) & 0x0f0f0f0fu) | pair4;
+                    }
+                }
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    uint32_t e[4];
+#pragma unroll
+                    for (int r = 0; r < 4; r++)
+                        e[r] = *reinterpret_cast<const uint32_t*>(smem + prmt_b32((i & 1) ? hi4[r] : lo4[r], bank, 0x6504u | (uint32_t)((i >> 1) << 4)));
+                    hi[2 * i] = prmt_b32(e[0], e[1], 0x5410u);
+                    hi[2 * i + 1] = prmt_b32(e[2], e[3], 0x5410u);
+                    if (PASSES == 2) {
+                        lo[2 * i] = prmt_b32(e[0], e[1], 0x7632u);
+                        lo[2 * i + 1] = prmt_b32(e[2], e[3], 0x7632u);
+                    }
+                }
+                if (u == 0 && round > 0) {                        // the stage is touched only here: the work above overlaps its last MMAs
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar_aempty + 8 * sub, (round - 1) & 1))) { timed_out = true; break; }
+                    tc_fence_after_sync();
+                }
+                tmem_st_x16(t_dst + (uint32_t)u * 16u, hi);
+                if (PASSES == 2) tmem_st_x16(t_dst + 32u + (uint32_t)u * 16u, lo);
+            }
+            if (timed_out) break;
+            tmem_st_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_afull + 8 * sub);
+        }
+    } else if (warp == kHlTmaWarp) {
+        // ---------------- TMA: activation blocks [rows][64 k] (the whole warp walks the loop, lane 0 issues) ----------------
+        if (lane == 0) tma_prefetch_descriptor(&tmX);
+        pdl_wait_prior_grids();                                   // the activations may come from the previous kernel
+        const int boxes = (rows + p.box_rows - 1) / p.box_rows;
+        const uint32_t box_bytes = (uint32_t)p.box_rows * 128u;
+        int xs = 0, round = 0;
+        for (int j = 0; j < nblk; j++) {
+            if (round > 0) {
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar_xempty + 8 * xs, (round - 1) & 1))) { timed_out = true; break; }
+            }
+            if (lane == 0) {
+                const uint32_t dst = smem_base + kHlXOff + xs * p.x_slot_bytes;
+                mbar_arrive_expect_tx(bar_xfull + 8 * xs, boxes * box_bytes);      // rows and k beyond the end are zero-filled and counted
+                for (int i = 0; i < boxes; i++)
+                    tma_load_2d(dst + i * box_bytes, &tmX, (blk_begin + j) * kHlStepK, row0 + i * p.box_rows, bar_xfull + 8 * xs);
+            }
+            __syncwarp();
+            if (++xs == p.x_slots) { xs = 0; round++; }
+        }
+    } else {
+        // ---------------- MMA issue ----------------
+        const uint32_t idesc = umma_idesc_f16_f32(n_mma);
+        const uint64_t dx0 = umma_desc_k_sw128(smem_base + kHlXOff);
+        int xs = 0, xround = 0;
+        for (int j = 0; j < nblk; j++) {
+            const int st = j & (kHlStages - 1);
+            const uint32_t ap = (uint32_t)(j / kHlStages) & 1u;
+            if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar_xfull + 8 * xs, xround & 1) && mbar_wait_bounded(bar_afull + 8 * st, ap))) {
+                timed_out = true;
+                break;
+            }
+            tc_fence_after_sync();
+            if (lane == 0) {
+                const uint32_t a_t = tmem_base + kHlACol + (uint32_t)st * 64u;
+                const uint64_t dx = dx0 + (uint64_t)((xs * p.x_slot_bytes) >> 4);
+#pragma unroll
+                for (int ps = 0; ps < PASSES; ps++)
+#pragma unroll
+                    for (int k16 = 0; k16 < 4; k16++)
+                        umma_f16_ts(tmem_base, a_t + (uint32_t)(ps * 32 + k16 * 8), dx + (uint64_t)(k16 * 2), idesc,
+                                    (j | ps | k16) ? 1u : 0u);
+                umma_commit(bar_aempty + 8 * st);
+                umma_commit(bar_xempty + 8 * xs);
+            }
+            __syncwarp();
+            if (++xs == p.x_slots) { xs = 0; xround++; }
+        }
+        if (lane == 0) umma_commit(bar_acc);
+        __syncwarp();
+    }
+    pdl_wait_prior_grids();                  // before any store to global memory
+    if (timed_out) atomicExch(p.status, kStatusTcTimeout);
+
+    // ---------------- epilogue: TMEM lane = output column, TMEM column = activation row ----------------
+    const bool split = p.splits > 1;
+    if (warp >= kHlFirstExpWarp) {
+        const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar_acc, 0));
+        if (!ok) atomicExch(p.status, kStatusTcTimeout);
+        tc_fence_after_sync();
+        const uint32_t t_src = tmem_base + ((uint32_t)(lq * 32) << 16);
+        // the activation ring is idle: every load has been consumed when the accumulators are complete
+        float* scratch = reinterpret_cast<float*>(smem + kHlXOff) + ew * (16 * 33);
+        for (int c = sub; 16 * c < rows && ok; c += 4) {          // 16 activation rows per tcgen05.ld; warp-uniform
+            uint32_t r[16];
+            tmem_ld_x16(t_src + 16u * (uint32_t)c, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) * unscale);
+            tc_store_block(scratch, r, lane, row0 + 16 * c, n0 + lq * 32, row0 + rows, N, split, p.partial, p.y16, p.y32);
+        }
+        tc_fence_before_sync();
+    }
+    if (split) __threadfence();
+    __syncthreads();
+    if (warp == kHlMmaWarp) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, kTcTmemCols);
+    }
+    if (!split) return;
+
+    // ---------------- split-k: the last CTA of the tile converts the reduced sums and zeroes the workspace ----------------
+    if (tid == 0) {
+        const unsigned prev = atomicAdd(p.counters + blockIdx.x, 1u);
+        *s_flag = (prev == (unsigned)p.splits - 1u);
+    }
+    __syncthreads();
+    if (!*s_flag) return;
+    __threadfence();
+    const int nvec = rows * (kHlCols / 4);
+    for (int base = tid; base < nvec; base += 4 * kHlThreads) {
+        float4 v[4];
+        size_t off[4];
+        bool live[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int idx = base + u * kHlThreads;
+            const int c = n0 + 4 * (idx % (kHlCols / 4));
+            live[u] = idx < nvec && c < N;
+            off[u] = (size_t)(row0 + idx / (kHlCols / 4)) * (size_t)N + c;
+            if (live[u]) v[u] = __ldcg(reinterpret_cast<const float4*>(p.partial + off[u]));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (!live[u]) continue;
+            __stcg(reinterpret_cast<float4*>(p.partial + off[u]), make_float4(0.f, 0.f, 0.f, 0.f));
+            if (p.y32) *reinterpret_cast<float4*>(p.y32 + off[u]) = v[u];
+            if (p.y16) {
+                __half2 lo = __floats2half2_rn(v[u].x, v[u].y), hi = __floats2half2_rn(v[u].z, v[u].w);
+                uint2 o;
+                o.x = *reinterpret_cast<uint32_t*>(&lo);
+                o.y = *reinterpret_cast<uint32_t*>(&hi);
+                *reinterpret_cast<uint2*>(p.y16 + off[u]) = o;
+            }
+        }
+    }
+    if (tid == 0) p.counters[blockIdx.x] = 0u;
+}
+
+}  // namespace lg
