@@ -267,6 +267,21 @@ def test_device_packer_and_converter_bit_exact():
     assert np.array_equal(qb_d.cpu().numpy(), qb_h.astype(np.float16))
 
 
+@pytest.mark.parametrize("N,K,q,g,shift", [(32, 128, 4, 128, 0), (33, 160, 1, 32, 0), (7, 32, 8, 32, 0), (95, 2080, 3, 32, 0),
+                                           (64, 1152, 5, 384, 0), (40, 256, 2, 64, 1), (31, 96, 6, 96, 3), (50, 1056, 7, 32, 0)])
+def test_device_converter_ragged_rows_words_and_alignment(N, K, q, g, shift):
+    """Rows that are no multiple of a warp's 32, k that is no multiple of its 128, codes that start off a 16-byte boundary."""
+    scale, zero, code = synth.uniform_layer(N, K, q, g, seed=N + K)
+    buf = torch.empty(code.size + shift, dtype=torch.int32, device="cuda")
+    d_code = buf[shift:].view(code.shape)
+    d_code.copy_(torch.from_numpy(code))
+    got = L.uniform_to_bcq_device(torch.from_numpy(scale).cuda(), torch.from_numpy(zero).cuda(), d_code, q)
+    bW, alpha, q_bias = L.uniform_to_bcq(scale, zero, code, q)
+    assert np.array_equal(got[0].cpu().numpy().view(np.uint32), bW)
+    assert np.array_equal(got[1].cpu().numpy(), alpha.astype(np.float16))
+    assert np.array_equal(got[2].cpu().numpy(), q_bias.astype(np.float16))
+
+
 def test_host_call_with_page_locked_buffers_reads_fresh_inputs():
     """The host-buffer call with page-locked buffers reused across calls: every call must see what the host wrote just
     before it, and pageable buffers must give the same numbers."""
