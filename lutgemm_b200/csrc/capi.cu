@@ -633,9 +633,15 @@ void hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) {
     }
 }
 
-// From this many rows on the split-operand kernel is the faster one (see gemm_hl.cuh).
-constexpr int kHlFromRows = 129;
-bool gemm_hl_ok(const lutgemm_weight* w, int m) { return w->tc_ok && w->q <= 4 && m >= kHlFromRows; }
+// From which row count the split-operand kernel is the faster one: it always takes two tensor-core passes, gemm_tc one
+// per plane and one for q_bias.  Measured, us (gemm_tc / split operand), g = 128: 2 passes, 8192 x 8192, 96 rows 33.3 / 33.8,
+// 128 rows 39.1 / 35.7; 3 passes, 8192 x 8192, 32 rows 31.6 / 32.0, 64 rows 36.7 / 32.4; 4 passes, 12288 x 4096, 32 rows
+// 28.0 / 30.0, 64 rows 33.7 / 31.0, 96 rows 40.5 / 32.3; 5 passes, 28672 x 8192, 4 rows 160 / 116.
+bool gemm_hl_ok(const lutgemm_weight* w, int m) {
+    const int passes = w->q + (w->q_bias ? 1 : 0);
+    const int from = passes >= 5 ? 4 : passes >= 3 ? 64 : passes == 2 ? 97 : 129;
+    return w->tc_ok && w->q <= 4 && m >= from;
+}
 
 // fp32 rows of the workspace for at least `rows` rows of w's width, growing the container's own workspace when that is
 // possible now (it synchronises the device: not inside a stream capture).  *have false: not available.
@@ -846,7 +852,7 @@ int matmul_impl(__half* y16, float* y32, const void* in, lutgemm_weight_t w, int
         }
         return LUTGEMM_OK;
     }
-    if (gemm_hl_ok(w, m)) return gemm_hl_rows(w, ws, x, y16, y32, m, st);
+    if (gemm_hl_ok(w, m) && !gemm_i8_ok(w, m)) return gemm_hl_rows(w, ws, x, y16, y32, m, st);
     // batched: 128 rows per tensor-core launch
     for (int r0 = 0; r0 < m; r0 += 128) {
         const int rows = (m - r0 < 128) ? (m - r0) : 128;

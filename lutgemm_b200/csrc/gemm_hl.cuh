@@ -20,6 +20,10 @@
 //
 // Tensor memory: 256 accumulator columns, then four operand stages of 64 columns (hi 32, lo 32), one per `sub`.
 //
+// At 256 rows a block of 64 k takes the tensor pipe 1024 cycles and shared memory about as long (the activations are read
+// once for hi and once for lo: 64 KB, beside 32 KB arriving and 40 KB of table traffic, at 128 bytes a cycle); the expansion
+// issues for about 700 cycles at q = 4 with q_bias and bounds the kernel below 200 rows.  Measured, us, 8192 x 8192, q = 4 +
+// q_bias, 2048 rows: 424 (1296 as 16 launches of gemm_tc).  28672 x 8192, q = 4 + q_bias, 4 rows: 116 (160).
 // All mbarrier waits are bounded, as in gemm_tc.cuh.
 #pragma once
 #include "gemm_tc.cuh"
@@ -59,6 +63,29 @@ struct HlParams {
     int x_slot_bytes, x_slots;
 };
 
+// One lane of a converged warp: 1 there, 0 elsewhere.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e;
+}
+// umma_f16_ts / umma_commit under a predicate, for a warp that stays converged.
+__device__ __forceinline__ void umma_f16_ts_if(uint32_t on, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                               uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p, q;\n"
+        "setp.ne.b32 q, %5, 0;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(on) : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t on, uint32_t bar) {
+    asm volatile(
+        "{\n.reg .pred q;\n"
+        "setp.ne.b32 q, %1, 0;\n"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar), "r"(on) : "memory");
+}
+
 // (hi, lo) of two values, hi in the low half of an entry
 __device__ __forceinline__ void hl_pack_pair(float v0, float v1, uint32_t& e0, uint32_t& e1) {
     const __half2 hi = __floats2half2_rn(v0, v1);
@@ -86,7 +113,9 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
     int* s_flag = reinterpret_cast<int*>(s_tmem + 1);
     unsigned* s_max = reinterpret_cast<unsigned*>(smem + kHlScaleOff);
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // the warp number through a shuffle: the compiler then knows it to be the same in every lane, and what depends on it
+    // only (rows of words and scales, groups, block counts) is computed once per warp in uniform registers
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int N = p.N;
     // this CTA's item: 256 rows, or a half of one
     int item = blockIdx.x, half_row = 0, rows_cap = kHlRows;
@@ -125,7 +154,7 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = *s_tmem;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *s_tmem, 0);
     bool timed_out = false;
     // the packed planes and scales are never written by a kernel: their stream starts while the previous kernel drains
     pdl_launch_dependents();
@@ -136,33 +165,39 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
     float unscale = 1.f;
     if (warp >= kHlFirstExpWarp) {
         // ---------------- expansion ----------------
-        const bool col_ok = col < N;
         const size_t row_w = (size_t)Q * N;                       // words per k-word row, scales per group
         uint32_t w[2][Q];
         unsigned short av[2][Q], bv[2];
-        // this lane's next block: its words, its group (advanced by 4 blocks = 256 k without a division)
-        const uint32_t* wptr = p.bW + (size_t)(blk_begin + sub) * 2 * row_w + col;
+        // This warp's next block: its words, its group (advanced by 4 blocks = 256 k without a division).  Loads are not
+        // predicated: a column beyond N reads column N - 1 (its accumulators are never stored), a word beyond K the block's
+        // first word with that word's scales (the activations there are zero), a block beyond the range nothing at all.
+        const unsigned col_c = (unsigned)min(col, N - 1);
+        const uint32_t* wrow = p.bW + (size_t)(blk_begin + sub) * 2 * row_w;
         int knext = (blk_begin + sub) * kHlStepK;
         const int kend = min(p.K, (blk_begin + nblk) * kHlStepK);
         int grp = knext / p.g, grem = knext % p.g;
         const int ginc = (4 * kHlStepK) / p.g, grinc = (4 * kHlStepK) % p.g;
         auto fetch = [&]() {
-            const bool ok = col_ok && knext < kend, ok1 = col_ok && knext + 32 < kend;
-            const unsigned short* a0 = reinterpret_cast<const unsigned short*>(p.alpha) + (size_t)grp * row_w + col;
-            const unsigned short* q0 = reinterpret_cast<const unsigned short*>(p.q_bias) + (BIAS ? (size_t)grp * N + col : 0);
+            if (knext < kend) {                                   // warp-uniform
+                const bool second = knext + 32 < kend;
+                const uint32_t* wrow1 = second ? wrow + row_w : wrow;
+                const unsigned short* arow = reinterpret_cast<const unsigned short*>(p.alpha) + (size_t)grp * row_w;
 #pragma unroll
-            for (int b = 0; b < Q; b++) {
-                w[0][b] = ok ? __ldg(wptr + (size_t)b * N) : 0u;
-                w[1][b] = ok1 ? __ldg(wptr + row_w + (size_t)b * N) : 0u;
-                av[0][b] = ok ? __ldg(a0 + (size_t)b * N) : (unsigned short)0;
-            }
-            if (BIAS) bv[0] = ok ? __ldg(q0) : (unsigned short)0;
-            if (p.g < kHlStepK) {                                 // g == 32: the second word has scales of its own
+                for (int b = 0; b < Q; b++) {
+                    w[0][b] = __ldg(wrow + (size_t)b * N + col_c);
+                    w[1][b] = __ldg(wrow1 + (size_t)b * N + col_c);
+                    av[0][b] = __ldg(arow + (size_t)b * N + col_c);
+                }
+                if (BIAS) bv[0] = __ldg(reinterpret_cast<const unsigned short*>(p.q_bias) + (size_t)grp * N + col_c);
+                if (p.g < kHlStepK) {                             // g == 32: the second word has scales of its own
+                    const int g1 = grp + (second ? 1 : 0);
+                    const unsigned short* arow1 = reinterpret_cast<const unsigned short*>(p.alpha) + (size_t)g1 * row_w;
 #pragma unroll
-                for (int b = 0; b < Q; b++) av[1][b] = ok1 ? __ldg(a0 + row_w + (size_t)b * N) : (unsigned short)0;
-                if (BIAS) bv[1] = ok1 ? __ldg(q0 + N) : (unsigned short)0;
+                    for (int b = 0; b < Q; b++) av[1][b] = __ldg(arow1 + (size_t)b * N + col_c);
+                    if (BIAS) bv[1] = __ldg(reinterpret_cast<const unsigned short*>(p.q_bias) + (size_t)g1 * N + col_c);
+                }
             }
-            wptr += 8 * row_w;
+            wrow += 8 * row_w;
             knext += 4 * kHlStepK;
             grp += ginc;
             grem += grinc;
@@ -235,23 +270,29 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
                     float bound = fabsf(qb[u]);
 #pragma unroll
                     for (int b = 0; b < Q; b++) bound += fabsf(a[u][b]);
-                    float v[NV];
-                    v[0] = qb[u];
+                    // without q_bias the values of c and of its complement are each other's negatives
+                    constexpr int NC = BIAS || Q == 1 ? NV : NV / 2;
+                    float v[NC];
+                    v[0] = BIAS || Q == 1 ? qb[u] : -a[u][Q - 1];
 #pragma unroll
-                    for (int b = Q - 1; b >= 0; b--) {            // v[c] for c a multiple of 2^b, halving the stride
+                    for (int b = (BIAS || Q == 1 ? Q : Q - 1) - 1; b >= 0; b--) {      // v[c] for c a multiple of 2^b, halving the stride
 #pragma unroll
-                        for (int c = 0; c < NV; c += 2 << b) {
+                        for (int c = 0; c < NC; c += 2 << b) {
                             const float s = v[c];
                             v[c] = s - a[u][b];
                             v[c + (1 << b)] = s + a[u][b];
                         }
                     }
 #pragma unroll
-                    for (int c = 0; c < NV; c += 2) {
+                    for (int c = 0; c < NC; c += 2) {
                         uint32_t e0, e1;
                         hl_pack_pair(v[c], v[c + 1], e0, e1);
                         *reinterpret_cast<uint32_t*>(tab + c * 256) = e0;
                         *reinterpret_cast<uint32_t*>(tab + (c + 1) * 256) = e1;
+                        if (NC < NV) {
+                            *reinterpret_cast<uint32_t*>(tab + (NV - 1 - c) * 256) = e0 ^ 0x80008000u;
+                            *reinterpret_cast<uint32_t*>(tab + (NV - 2 - c) * 256) = e1 ^ 0x80008000u;
+                        }
                     }
                     if (!(bound <= 65504.f)) {                    // an infinite or NaN scale: the value itself, lo = 0
 #pragma unroll 1
@@ -328,8 +369,12 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
         }
     } else {
         // ---------------- MMA issue ----------------
+        // The whole warp walks straight through and one elected lane's predicate guards the instructions: their operands
+        // stay in uniform registers.  Inside an `if (lane == 0)` every tcgen05.mma took ~120 cycles to issue, whatever
+        // its N: more than it runs up to 240 rows (8192 x 8192, q = 2, 128 rows: 47.5 us against 37.6).
         const uint32_t idesc = umma_idesc_f16_f32(n_mma);
         const uint64_t dx0 = umma_desc_k_sw128(smem_base + kHlXOff);
+        const uint32_t elected = elect_one();
         int xs = 0, xround = 0;
         for (int j = 0; j < nblk; j++) {
             const int st = j & (kHlStages - 1);
@@ -339,22 +384,19 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
                 break;
             }
             tc_fence_after_sync();
-            if (lane == 0) {
-                const uint32_t a_t = tmem_base + kHlACol + (uint32_t)st * 64u;
-                const uint64_t dx = dx0 + (uint64_t)((xs * p.x_slot_bytes) >> 4);
+            const uint32_t a_t = tmem_base + kHlACol + (uint32_t)st * 64u;
+            const uint64_t dx = dx0 + (uint64_t)((xs * p.x_slot_bytes) >> 4);
 #pragma unroll
-                for (int ps = 0; ps < PASSES; ps++)
+            for (int ps = 0; ps < PASSES; ps++)
 #pragma unroll
-                    for (int k16 = 0; k16 < 4; k16++)
-                        umma_f16_ts(tmem_base, a_t + (uint32_t)(ps * 32 + k16 * 8), dx + (uint64_t)(k16 * 2), idesc,
-                                    (j | ps | k16) ? 1u : 0u);
-                umma_commit(bar_aempty + 8 * st);
-                umma_commit(bar_xempty + 8 * xs);
-            }
-            __syncwarp();
+                for (int k16 = 0; k16 < 4; k16++)
+                    umma_f16_ts_if(elected, tmem_base, a_t + (uint32_t)(ps * 32 + k16 * 8), dx + (uint64_t)(k16 * 2), idesc,
+                                   (j | ps | k16) ? 1u : 0u);
+            umma_commit_if(elected, bar_aempty + 8 * st);
+            umma_commit_if(elected, bar_xempty + 8 * xs);
             if (++xs == p.x_slots) { xs = 0; xround++; }
         }
-        if (lane == 0) umma_commit(bar_acc);
+        umma_commit_if(elected, bar_acc);
         __syncwarp();
     }
     pdl_wait_prior_grids();                  // before any store to global memory
