@@ -1726,10 +1726,13 @@ int lutgemm_uniform_to_bcq_device(const float* d_scale, const float* d_zero, con
     if (!d_scale || !d_zero || !d_code || !d_bW || !d_alpha || !d_q_bias) return LUTGEMM_ERR_NULL;
     if (N < 1 || G < 1 || g < 32 || g % 32 != 0) return LUTGEMM_ERR_SHAPE;
     if (q < 1 || q > 8) return LUTGEMM_ERR_BITS;
-    dim3 grid((N + 255) / 256, (unsigned)((size_t)G * g / 32));
-    if (grid.y > 65535) return LUTGEMM_ERR_TOO_LARGE;
-    lg::uniform_to_bcq_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_scale, d_zero, d_code, N, G, g, q, d_bW,
-                                                                      (__half*)d_alpha, (__half*)d_q_bias);
+    const size_t k_words = (size_t)G * g / 32;
+    if (k_words > 65535) return LUTGEMM_ERR_TOO_LARGE;
+    const dim3 grid((N + 31) / 32, (unsigned)((k_words + 4 * lg::kU2bWarps - 1) / (4 * lg::kU2bWarps)));
+    auto kern = q == 1 ? lg::uniform_to_bcq_kernel<1> : q == 2 ? lg::uniform_to_bcq_kernel<2> : q == 3 ? lg::uniform_to_bcq_kernel<3>
+              : q == 4 ? lg::uniform_to_bcq_kernel<4> : q == 5 ? lg::uniform_to_bcq_kernel<5> : q == 6 ? lg::uniform_to_bcq_kernel<6>
+              : q == 7 ? lg::uniform_to_bcq_kernel<7> : lg::uniform_to_bcq_kernel<8>;
+    kern<<<grid, lg::kU2bWarps * 32, 0, (cudaStream_t)stream>>>(d_scale, d_zero, d_code, N, G, g, d_bW, (__half*)d_alpha, (__half*)d_q_bias);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     LG_CUDA(cudaGetLastError());
     return LUTGEMM_OK;
