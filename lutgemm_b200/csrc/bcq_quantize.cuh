@@ -240,8 +240,9 @@ bcq_quantize_kernel(const BqParams p) {
 // (B^T B) per word of pairs, and the sums of the next round are complete when the weights of this one are placed.
 // Bound by instruction issue, not by memory: the weights are read once.  Measured, N = K = 4096, q = 3, g = 128, 15
 // rounds: 395 us; bcq_quantize_kernel, which gives every group a whole warp, takes 3291 us.
-// Element e of a group: (i * LG + lane) * 4 + c for register 4 i + c, so that four consecutive weights are one 128-bit
-// load and eight consecutive lanes hold the 32 weights of a packed word.
+// Sums are added in the order of bcq_quantize_kernel, whose lane L holds weights L, L + 32, ...: a lane here stands for
+// NJ = 32 / LG of those lanes (lane, lane + LG, ...), keeps their partial sums apart and adds them first, which is that
+// kernel's shuffle over distances 16 .. LG.  So both give the same bits, and which one a group takes does not show.
 constexpr int kBqTileWarps = 8;
 constexpr int kBqTileMaxG = 512;              // 32 lanes of 16 weights; a field of pair counts holds up to 1023
 constexpr int kBqTileMaxQ = 4;                // the levels' signs are one 128-bit table entry
@@ -259,9 +260,21 @@ __device__ __forceinline__ uint32_t group_sum_u(uint32_t v) {
     return v;
 }
 
-template <int E, int LG, int Q>
+// Partial sums of the NJ lanes that a lane stands for, then the shuffles.
+template <int LG>
+__device__ __forceinline__ float tile_sum_f(float (&v)[32 / LG]) {
+#pragma unroll
+    for (int d = 16 / LG; d > 0; d >>= 1)
+#pragma unroll
+        for (int j = 0; j < d; j++) v[j] += v[j + d];
+    return group_sum_f<LG>(v[0]);
+}
+
+template <int LG, int Q>
 __global__ void __launch_bounds__(kBqTileWarps * 32)
 bcq_quantize_tile_kernel(const BqParams p) {
+    constexpr int E = 16;                                  // weights per lane: register e is weight (e % EE) * 32 + LG * (e / EE) + l
+    constexpr int NJ = 32 / LG, EE = E / NJ;
     constexpr int GPW = 32 / LG;                           // groups per warp
     constexpr int NLEV = 1 << Q;
     constexpr int PAIRS = Q * (Q - 1) / 2;
@@ -283,24 +296,11 @@ bcq_quantize_tile_kernel(const BqParams p) {
 
     float wv[E];
     uint32_t valid = 0u;                                   // bit e: register e holds a weight
-    if (g % 4 == 0 && (reinterpret_cast<uintptr_t>(p.w) & 15) == 0) {        // then so are K and every group's start
 #pragma unroll
-        for (int i = 0; i < E / 4; i++) {
-            const int at = (i * LG + l) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (at < g) {
-                v = __ldg(reinterpret_cast<const float4*>(wg + at));
-                valid |= 15u << (4 * i);
-            }
-            wv[4 * i] = v.x; wv[4 * i + 1] = v.y; wv[4 * i + 2] = v.z; wv[4 * i + 3] = v.w;
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-            const int at = ((e >> 2) * LG + l) * 4 + (e & 3);
-            wv[e] = at < g ? wg[at] : 0.f;
-            valid |= (at < g ? 1u : 0u) << e;
-        }
+    for (int e = 0; e < E; e++) {
+        const int at = (e % EE) * 32 + LG * (e / EE) + l;
+        wv[e] = at < g ? __ldg(wg + at) : 0.f;
+        valid |= (at < g ? 1u : 0u) << e;
     }
 
     float alpha[Q], btw[Q];
@@ -313,10 +313,10 @@ bcq_quantize_tile_kernel(const BqParams p) {
         for (int e = 0; e < E; e++) r[e] = wv[e];
 #pragma unroll
         for (int i = 0; i < Q; i++) {
-            float s = 0.f, t = 0.f;
+            float s[NJ] = {}, t[NJ] = {};
 #pragma unroll
-            for (int e = 0; e < E; e++) s += fabsf(r[e]);                    // padding elements are 0
-            float a = group_sum_f<LG>(s) / (float)g;
+            for (int e = 0; e < E; e++) s[e / EE] += fabsf(r[e]);            // padding elements are 0
+            float a = tile_sum_f<LG>(s) / (float)g;
             if (a != a) a = 0.f;
             alpha[i] = a;
             pos[i] = nz[i] = 0u;
@@ -325,13 +325,13 @@ bcq_quantize_tile_kernel(const BqParams p) {
                 const float b = r[e] > 0.f ? 1.f : (r[e] < 0.f ? -1.f : 0.f);
                 if (b > 0.f) pos[i] |= 1u << e;
                 if (b != 0.f) nz[i] |= 1u << e;
-                t += b * wv[e];
+                t[e / EE] += b * wv[e];
                 r[e] -= b * a;
             }
             // padding never counts: its weight is 0, and its code is masked out
             pos[i] &= valid;
             nz[i] &= valid;
-            btw[i] = group_sum_f<LG>(t);
+            btw[i] = tile_sum_f<LG>(t);
         }
 #pragma unroll
         for (int i = 0; i < Q; i++)
@@ -460,15 +460,14 @@ bcq_quantize_tile_kernel(const BqParams p) {
         };
         if (!last) {
             uint32_t pk[PW > 0 ? PW : 1] = {};
-#pragma unroll
-            for (int i = 0; i < Q; i++) btw[i] = 0.f;
+            float part[Q][NJ] = {};
 #pragma unroll
             for (int e = 0; e < E; e++) {
                 const int at = place(wv[e]);
                 const float4 sg = *reinterpret_cast<const float4*>(s_sign[wib][sub][at]);
                 const float sv[4] = {sg.x, sg.y, sg.z, sg.w};
 #pragma unroll
-                for (int i = 0; i < Q; i++) btw[i] = fmaf(sv[i], wv[e], btw[i]);
+                for (int i = 0; i < Q; i++) part[i][e / EE] = fmaf(sv[i], wv[e], part[i][e / EE]);
 #pragma unroll
                 for (int i = 0; i < PW; i++) pk[i] += s_pair[wib][sub][at][i];
             }
@@ -480,7 +479,7 @@ bcq_quantize_tile_kernel(const BqParams p) {
             }
 #pragma unroll
             for (int i = 0; i < Q; i++) {
-                btw[i] = group_sum_f<LG>(btw[i]);
+                btw[i] = tile_sum_f<LG>(part[i]);
                 A[i][i] = (float)g;
             }
 #pragma unroll
@@ -517,7 +516,7 @@ bcq_quantize_tile_kernel(const BqParams p) {
     if (live && p.binary_py) {
 #pragma unroll
         for (int e = 0; e < E; e++) {
-            const int at = ((e >> 2) * LG + l) * 4 + (e & 3);
+            const int at = (e % EE) * 32 + LG * (e / EE) + l;
             if (at < g) {
                 signed char* dst = p.binary_py + (((size_t)n * G + gi) * g + at) * Q;
 #pragma unroll
@@ -526,19 +525,16 @@ bcq_quantize_tile_kernel(const BqParams p) {
         }
     }
     if (p.bW) {                                            // g % 32 == 0: whole words; a zero code packs as -1
-        constexpr int NIB = LG >= 8 ? 1 : 8 / LG;          // nibbles of one word in the same lane
-        constexpr int WL = LG >= 8 ? 8 : LG;               // lanes that share a word
 #pragma unroll
-        for (int i = 0; i < E / 4; i += NIB)
+        for (int kw = 0; kw < EE; kw++)                    // word of the group: registers kw, kw + EE, ... of all its lanes
 #pragma unroll
             for (int b = 0; b < Q; b++) {
                 uint32_t word = 0u;
 #pragma unroll
-                for (int k = 0; k < NIB; k++) word |= ((pos[b] >> (4 * (i + k))) & 15u) << (4 * (k * LG + l % WL));
+                for (int j = 0; j < NJ; j++) word |= ((pos[b] >> (j * EE + kw)) & 1u) << (LG * j + l);
 #pragma unroll
-                for (int o = WL / 2; o > 0; o >>= 1) word |= __shfl_xor_sync(0xffffffffu, word, o);
-                const int kw = (i * LG + l) / 8;           // word of the group
-                if (live && l % WL == 0 && kw * 32 < g) p.bW[((size_t)(gi * (g / 32) + kw) * Q + b) * p.N + n] = word;
+                for (int o = LG / 2; o > 0; o >>= 1) word |= __shfl_xor_sync(0xffffffffu, word, o);
+                if (live && l == kw % LG && kw * 32 < g) p.bW[((size_t)(gi * (g / 32) + kw) * Q + b) * p.N + n] = word;
             }
     }
 }

@@ -930,10 +930,10 @@ void launch_bcq_tile(const lg::BqParams& p, long long groups, cudaStream_t st) {
     const long long per_cta = (long long)lg::kBqTileWarps * (32 / lanes);
     const unsigned ctas = (unsigned)((groups + per_cta - 1) / per_cta);
     const dim3 block(lg::kBqTileWarps * 32);
-    if (lanes == 4) lg::bcq_quantize_tile_kernel<16, 4, Q><<<ctas, block, 0, st>>>(p);
-    else if (lanes == 8) lg::bcq_quantize_tile_kernel<16, 8, Q><<<ctas, block, 0, st>>>(p);
-    else if (lanes == 16) lg::bcq_quantize_tile_kernel<16, 16, Q><<<ctas, block, 0, st>>>(p);
-    else lg::bcq_quantize_tile_kernel<16, 32, Q><<<ctas, block, 0, st>>>(p);
+    if (lanes == 4) lg::bcq_quantize_tile_kernel<4, Q><<<ctas, block, 0, st>>>(p);
+    else if (lanes == 8) lg::bcq_quantize_tile_kernel<8, Q><<<ctas, block, 0, st>>>(p);
+    else if (lanes == 16) lg::bcq_quantize_tile_kernel<16, Q><<<ctas, block, 0, st>>>(p);
+    else lg::bcq_quantize_tile_kernel<32, Q><<<ctas, block, 0, st>>>(p);
 }
 
 template <int WPG, bool BIAS>
