@@ -20,6 +20,7 @@
 #include "gemv_seq.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_hl.cuh"
+#include "gemm_frag.cuh"
 #include "gemm_i8.cuh"
 #include "bcq_quantize.cuh"
 #include "gptq3.cuh"
@@ -654,7 +655,7 @@ int hl_have_rows(lutgemm_weight* w, lutgemm_workspace* ws, int rows, cudaStream_
     ws->tc_partial = nullptr;
     ws->tc_rows = 0;
     LG_CUDA(cudaMalloc(&ws->tc_partial, (size_t)rows * w->N * sizeof(float)));
-    LG_CUDA(cudaMemset(ws->tc_partial, 0, (size_t)rows * w->N * sizeof(float)));
+    LG_CUDA(cudaMemsetAsync(ws->tc_partial, 0, (size_t)rows * w->N * sizeof(float), st));     // before the kernel that follows
     ws->tc_rows = rows;
     *have = true;
     return LUTGEMM_OK;
@@ -733,6 +734,76 @@ int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
     return LUTGEMM_ERR_BITS;
 }
 
+// ---- register-operand kernel (gemm_frag.cuh): plan, launch ----
+// One CTA per SM and one wave: the slabs of k first (a slab is what the warps of a CTA hold activations for), then as many
+// column ranges as still fit.  Cost in units of 4096 weights: the longest warp's share, plus what a column tile's sum and a
+// slab's start cost.
+bool frag_plan(const lutgemm_weight* w, int m, lg::FrParams* p, dim3* grid) {
+    if (w->N % 4 != 0 || m > lg::kFrMaxRows) return false;
+    const int gw = w->g % 128 == 0 ? 4 : w->g % 64 == 0 ? 2 : 1;
+    p->depth = lg::fr_depth(gw, m <= 8 ? 1 : 2, w->q, w->q_bias != nullptr);
+    if (p->depth < 2) return false;
+    const int ks = m <= 8 ? 2 : 1, P = w->q + (w->q_bias ? 1 : 0);
+    const int steps = (w->K + 127) / 128, tiles = (w->N + lg::kFrCols - 1) / lg::kFrCols, sms = sm_count();
+    double best = 1e300;
+    for (int kw = 16; kw >= 2; kw /= 2) {
+        const int slabs = (steps + kw * ks - 1) / (kw * ks);
+        const int sps = (steps + slabs - 1) / slabs;
+        int ranges = sms / slabs;
+        if (ranges < 1) ranges = 1;
+        const int tpc = (tiles + ranges - 1) / ranges;
+        ranges = (tiles + tpc - 1) / tpc;
+        const int cw = lg::kFrWarps / kw, rounds = (tpc + cw - 1) / cw, wsteps = (sps + kw - 1) / kw;
+        const double waves = (double)(((long long)slabs * ranges + sms - 1) / sms);
+        const double t = waves * (12.0 + rounds * (wsteps * P + 1.0)) + (slabs > 1 ? 8.0 : 0.0);
+        if (t < best) {
+            best = t;
+            p->kw = kw; p->steps_per_slab = sps; p->tiles_per_cta = tpc;
+            *grid = dim3(ranges, slabs);
+        }
+    }
+    return grid->y <= 65535;
+}
+
+template <int MT, int GW>
+int launch_gemm_frag(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, cudaStream_t st) {
+    static bool configured[64][2] = {};   // the attribute is per device
+    const bool bias = w->q_bias != nullptr;
+    auto kern = bias ? lg::gemm_frag_kernel<MT, GW, true> : lg::gemm_frag_kernel<MT, GW, false>;
+    int dev = 0;
+    LG_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !configured[dev][bias]) {
+        LG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lg::kFrSmemBytes));
+        if (dev < 64) configured[dev][bias] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(lg::kFrThreads);
+    cfg.dynamicSmemBytes = (size_t)lg::kFrSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_pdl.load() ? 1 : 0;
+    LG_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    LG_CUDA(cudaGetLastError());
+    return LUTGEMM_OK;
+}
+
+int gemm_frag_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, lg::FrParams p, dim3 grid, const __half* x, __half* y16,
+                   float* y32, int m, cudaStream_t st) {
+    p.bW = w->bW; p.alpha = w->alpha; p.q_bias = w->q_bias; p.x = x;
+    p.partial = ws->tc_partial; p.counters = ws->counters;
+    p.y16 = y16; p.y32 = y32;
+    p.N = w->N; p.K = w->K; p.q = w->q; p.g = w->g; p.m = m;
+    p.ones = 0x3c003c00u; p.twos = 0x40004000u; p.fours = 0x44004400u;
+    if (w->g % 128 == 0) return m <= 8 ? launch_gemm_frag<1, 4>(w, p, grid, st) : launch_gemm_frag<2, 4>(w, p, grid, st);
+    if (w->g % 64 == 0) return m <= 8 ? launch_gemm_frag<1, 2>(w, p, grid, st) : launch_gemm_frag<2, 2>(w, p, grid, st);
+    return m <= 8 ? launch_gemm_frag<1, 1>(w, p, grid, st) : launch_gemm_frag<2, 1>(w, p, grid, st);
+}
+
 template <int Q>
 int launch_gemm_i8_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::I8Params& p, dim3 grid, cudaStream_t st) {
     static bool configured[64][2] = {};   // the attribute is per device
@@ -801,6 +872,49 @@ int gemm_i8_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
     return LUTGEMM_ERR_BITS;
 }
 
+// Batches that the register-operand kernel is the fastest for.  Measured, us, register operand against what ran instead,
+// g = 128: 8192 x 8192, q = 2, 2 rows 17.6 / 13.1 (two-row LUT kernel), 3 rows 17.8 / 21.5 (that and one LUT row); q = 3, 4 rows
+// 22.2 / 28.7, 8 rows 23.8 / 28.9, 16 rows 32.9 / 29.8 (gemm_tc); q = 1, 8 rows 14.8 / 16.0; 12288 x 4096, q = 4, 8 rows
+// 20.1 / 25.7, 16 rows 34.4 / 26.3; 2048 x 2048, q = 4, 4 rows 4.7 / 8.1; 28672 x 8192, q = 4 + q_bias, 4 rows 82.6 / 116.5
+// (gemm_hl).  Containers that the tcgen05 kernels refuse (N % 8 != 0, or a group size that neither divides nor is a multiple
+// of 128) take it for every batch, 16 rows at a time: what is left for them is one matvec per row.
+bool frag_wanted(const lutgemm_weight* w, const lutgemm_workspace* ws, int m) {
+    if (m < 2 || w->N % 4 != 0 || ordered_for(ws) || gemm_i8_ok(w, m)) return false;
+    if (m < kBatchedFromRows && g_variant.load() != 0) return false;       // the caller asked for a matvec kernel by name
+    if (m == 2) return !gemv_pair_ok(w, ws);
+    return m <= 8 || !w->tc_ok;
+}
+
+// *taken false and LUTGEMM_OK: no plan, or no scratch that could be had now; the caller goes on as without this kernel.
+int frag_rows_if_ready(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __half* y16, float* y32, int m,
+                       cudaStream_t st, bool* taken) {
+    *taken = false;
+    lg::FrParams p[2] = {};
+    dim3 grid[2];
+    const int whole = m / lg::kFrMaxRows, rest = m % lg::kFrMaxRows;       // launches of 16 rows, and one of the rest
+    if (whole && !frag_plan(w, lg::kFrMaxRows, &p[0], &grid[0])) return LUTGEMM_OK;
+    if (rest && !frag_plan(w, rest, &p[1], &grid[1])) return LUTGEMM_OK;
+    if (m >= kBatchedFromRows && w->tc_ok) {
+        // what a call without reserved scratch is told does not depend on the kernel: the plane kernel's rule
+        int unused_split = 1, unused_steps = 0;
+        const int rc = tc_split(w, ws, m < 128 ? m : 128, st, &unused_split, &unused_steps);
+        if (rc != LUTGEMM_OK) return rc;
+    }
+    if ((whole && grid[0].y > 1) || (rest && grid[1].y > 1)) {
+        bool have = false;
+        const int rc = hl_have_rows(w, ws, whole ? lg::kFrMaxRows : m, st, &have);
+        if (rc != LUTGEMM_OK || !have) return rc;
+    }
+    *taken = true;
+    for (int r0 = 0; r0 < m; r0 += lg::kFrMaxRows) {
+        const int rows = m - r0 < lg::kFrMaxRows ? m - r0 : lg::kFrMaxRows, i = rows == lg::kFrMaxRows ? 0 : 1;
+        const int rc = gemm_frag_rows(w, ws, p[i], grid[i], x + (size_t)r0 * w->K, y16 ? y16 + (size_t)r0 * w->N : nullptr,
+                                      y32 ? y32 + (size_t)r0 * w->N : nullptr, rows, st);
+        if (rc != LUTGEMM_OK) return rc;
+    }
+    return LUTGEMM_OK;
+}
+
 // ---- scratch for lutgemm_matvec_static_scratch: lives in the library image, never allocated ----
 constexpr int kStaticMaxN = 65536;                       // widest output the static entry point takes
 constexpr size_t kStaticRowBytes = (size_t)kStaticMaxN * sizeof(float);
@@ -835,10 +949,15 @@ int matmul_impl(__half* y16, float* y32, const void* in, lutgemm_weight_t w, int
     if (ws->n_cap < w->N || ws->slabs < (w->K + lg::kSlab2 - 1) / lg::kSlab2) return LUTGEMM_ERR_TOO_LARGE;
     cudaStream_t st = (cudaStream_t)stream;
     const __half* x = (const __half*)in;
+    const int batched_mode = g_batched.load();
+    if (batched_mode != 0 && frag_wanted(w, ws, m)) {
+        bool taken = false;
+        const int rc = frag_rows_if_ready(w, ws, x, y16, y32, m, st, &taken);
+        if (taken || rc != LUTGEMM_OK) return rc;
+    }
     // Up to three rows one LUT matvec per row is cheaper than the tensor-core kernel, whose cost is nearly
     // independent of m up to 64 rows (measured: 8192^2, q = 2: m x 10.2 us against 29 us; 12288^2, q = 3:
     // m x 17.6 us against 64 us).
-    const int batched_mode = g_batched.load();
     if (m == 1 || batched_mode == 0 || (batched_mode == 1 && m < kBatchedFromRows) || !w->tc_ok) {
         const bool pairs = gemv_pair_ok(w, ws);
         for (int r = 0; r < m;) {

@@ -1,0 +1,406 @@
+// BCQ matmul for a handful of rows (up to 16) on the warp-level tensor instruction, sm_100a.
+//
+// With few rows the tcgen05 kernels are bound by what is not proportional to the rows: expanding every weight and passing
+// it through tensor memory.  mma.sync takes its A operand from registers, so here a packed word becomes operand
+// registers in the lane that loaded it and nothing of the expansion is ever stored:
+//
+//   A warp takes 32 output columns x 128 k, all planes, at a time (a "unit").  Lane (r = lane / 4, t = lane % 4) holds,
+//   per plane, the packed words of columns 4 r .. 4 r + 3 at k-word t (one 128-bit load); columns 4 r, 4 r + 1 are rows
+//   r, r + 8 of a first 16 x 16 operand tile, 4 r + 2, 4 r + 3 of a second.  The order of k inside a product is free as
+//   long as both operands agree: bits (j, j + 16) of a word are the two halves of one operand register.  The activations of
+//   the same k are the B operand, in registers for the whole kernel: a warp keeps its k-range and walks over the columns.
+//   One LOP3 makes an operand register of a word whose bits lie at one of four places of the fp16 format: 15 (sign: -1 or
+//   +1), 14 (exponent: 0 or 2), 10 (exponent: 2 or 4), 9 (mantissa: 4 or 6).  The two values differ by 2 each time, so the
+//   sign's product is that of the operand less (1 + the lower value) times the activation: a sum over the group that does
+//   not depend on the weights and is what the fp32 accumulator starts from.  16 bit positions then need 5 shifts, not 15.
+//   The accumulator of a plane and scale group is multiplied by alpha in fp32; q_bias takes the group's sum of activations.
+//   Units come through a ring in shared memory that belongs to one warp (cp.async, no barriers).  The warps that
+//   split k add up through shared memory once per 32 columns, k-ranges of different CTAs through fp32 reductions in L2.
+//
+// GW: packed words per scale group inside a unit: 4 (group size a multiple of 128), 2 (of 64), 1 (of 32).  With fewer
+// than four, the four lanes t of a product share the words of one group (each takes NJ = 4 GW of the 16 bit positions).
+// MT: tiles of 8 activation rows (1 or 2).  KS: units along k that a warp keeps activations for (2 for 8 rows, 1 for 16).
+//
+// Bound by instruction issue and its latencies: per plane and 4096 weights 64 LOP3, 20 shifts and 16 MT mma.sync, on 16 warps
+// that 128 registers a thread allow; plus some 10 us at 8192 x 8192 that do not grow with the planes (activations, column
+// sums, k-ranges).  Measured, 28672 x 8192, q = 4 + q_bias, 4 rows: 82.6 us = 1.65 TB/s (160 with gemm_tc, 116 with gemm_hl;
+// 121 with one shift per bit position and a plane at a time).
+#pragma once
+#include "gemv_tma.cuh"
+
+namespace lg {
+
+constexpr int kFrWarps = 16;
+constexpr int kFrThreads = kFrWarps * 32;
+constexpr int kFrCols = 32;                   // columns per unit
+constexpr int kFrMaxRows = 16;
+constexpr int kFrRedStride = 12;              // floats between the rows of a reduction block: conflict-free stores
+constexpr int kFrMaxDepth = 6;
+constexpr int kFrSmemBytes = kSmemLimit;
+__host__ __device__ constexpr int fr_unit_bytes(int gw, int q, bool bias) { return q * 512 + (q + (bias ? 1 : 0)) * (4 / gw) * 64; }
+__host__ __device__ constexpr int fr_red_floats(int mt) { return 4 * mt * 8 * kFrRedStride; }     // per warp
+// units of a warp's ring (at least 2 are needed)
+__host__ __device__ constexpr int fr_depth(int gw, int mt, int q, bool bias) {
+    const int per_warp = (kFrSmemBytes - 16 - 2 * kFrWarps * fr_red_floats(mt) * 4) / kFrWarps;
+    const int d = per_warp / fr_unit_bytes(gw, q, bias);
+    return d > kFrMaxDepth ? kFrMaxDepth : d;
+}
+
+struct FrParams {
+    const uint32_t* bW;      // [K/32][q][N]
+    const __half* alpha;     // [G][q][N]
+    const __half* q_bias;    // [G][N] or nullptr
+    const __half* x;         // [m][K]
+    float* partial;          // [m][N] fp32, zero between launches (more than one slab)
+    unsigned* counters;      // [gridDim.x], zero between launches
+    __half* y16;             // [m][N] or nullptr
+    float* y32;              // [m][N] or nullptr
+    int N, K, q, g, m;
+    int kw;                  // warps that split a slab's k: 2, 4, 8 or 16; the other factor of 16 splits the columns
+    int steps_per_slab;      // 128-k steps of a slab, at most kw * KS
+    int tiles_per_cta;       // 32-column tiles per CTA
+    int depth;               // units of a warp's ring
+    // fp16 pairs of 1, 2 and 4: as arguments they stay in registers; as literals the compiler made them anew for every LOP3
+    uint32_t ones, twos, fours;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(live ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// D += A B, m16n8k16, fp16 in, fp32 accumulation
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// Where bit position pos of a half goes (shift left by fr_shift) and what it becomes there: class 0 the sign, 1 to 3 as above.
+__host__ __device__ constexpr int fr_shift(int pos) {
+    return pos >= 14 || pos == 10 || pos == 9 ? 0 : pos >= 12 || pos == 8 || pos == 7 ? 2 : pos == 11 || pos == 6 || pos == 5 ? 4
+           : pos >= 3 ? 6 : pos >= 1 ? 8 : 10;
+}
+__host__ __device__ constexpr int fr_class(int pos) {
+    const int at = pos + fr_shift(pos);
+    return at == 15 ? 0 : at == 14 ? 1 : at == 10 ? 2 : 3;
+}
+// minus (1 + the lower value) of the class, fp16 pair
+__host__ __device__ constexpr uint32_t fr_offset(int pos) {
+    return fr_class(pos) == 0 ? 0u : fr_class(pos) == 1 ? 0xbc00bc00u : fr_class(pos) == 2 ? 0xc200c200u : 0xc500c500u;
+}
+template <int LUT>
+__device__ __forceinline__ uint32_t lop3(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(d) : "r"(a), "r"(b), "r"(c), "n"(LUT));
+    return d;
+}
+// operand register of bit position POS (of both halves)
+template <int POS>
+__device__ __forceinline__ uint32_t fr_operand(uint32_t word, uint32_t ones, uint32_t twos, uint32_t fours) {
+    const uint32_t w = word << fr_shift(POS);
+    constexpr int cls = fr_class(POS);
+    if constexpr (cls == 0) return lop3<0xae>(w, 0x80008000u, ones);              // (~w & mask) | 1: set -> +1, clear -> -1
+    else if constexpr (cls == 1) return w & 0x40004000u;                            // 0 or 2
+    else if constexpr (cls == 2) return lop3<0xea>(w, 0x04000400u, twos);         // (w & mask) | 2: 2 or 4
+    else return lop3<0xea>(w, 0x02000200u, fours);                                 // (w & mask) | 4: 4 or 6
+}
+// One plane of one scale group: both operand tiles times MT x 8 rows.  Product S: positions FIRST + 2 S, FIRST + 2 S + 1.
+template <int S, int COUNT, int FIRST, int MT>
+__device__ __forceinline__ void fr_products(float (&d0)[MT][4], float (&d1)[MT][4], const uint32_t (&w)[4],
+                                            const uint32_t (&bx)[COUNT][MT][2], uint32_t ones, uint32_t twos, uint32_t fours) {
+    if constexpr (S < COUNT) {
+        constexpr int P0 = FIRST + 2 * S, P1 = P0 + 1;
+        const uint32_t a0[4] = {fr_operand<P0>(w[0], ones, twos, fours), fr_operand<P0>(w[1], ones, twos, fours),
+                                fr_operand<P1>(w[0], ones, twos, fours), fr_operand<P1>(w[1], ones, twos, fours)};
+        const uint32_t a1[4] = {fr_operand<P0>(w[2], ones, twos, fours), fr_operand<P0>(w[3], ones, twos, fours),
+                                fr_operand<P1>(w[2], ones, twos, fours), fr_operand<P1>(w[3], ones, twos, fours)};
+#pragma unroll
+        for (int nt = 0; nt < MT; nt++) {
+            mma_16816(d0[nt], a0, bx[S][nt]);
+            mma_16816(d1[nt], a1, bx[S][nt]);
+        }
+        fr_products<S + 1, COUNT, FIRST, MT>(d0, d1, w, bx, ones, twos, fours);
+    }
+}
+// What those accumulators start from: the offsets' products.
+template <int S, int COUNT, int FIRST, int MT>
+__device__ __forceinline__ void fr_start(float (&d)[MT][4], const uint32_t (&bx)[COUNT][MT][2]) {
+    if constexpr (S < COUNT) {
+        constexpr uint32_t o0 = fr_offset(FIRST + 2 * S), o1 = fr_offset(FIRST + 2 * S + 1);
+        const uint32_t a[4] = {o0, o0, o1, o1};
+#pragma unroll
+        for (int nt = 0; nt < MT; nt++) mma_16816(d[nt], a, bx[S][nt]);
+        fr_start<S + 1, COUNT, FIRST, MT>(d, bx);
+    }
+}
+
+template <int MT, int GW, bool BIAS>
+__global__ void __launch_bounds__(kFrThreads, 1)
+gemm_frag_kernel(const FrParams p) {
+    constexpr int KS = MT == 1 ? 2 : 1;
+    constexpr int NG = 4 / GW;                // scale groups of a unit
+    constexpr int NJ = 4 * GW;                // bit positions (of 16) that a lane takes of its word
+    constexpr int FIRST = 16 - NJ;            // the lane's positions after its words are shifted up: FIRST .. 15
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int r = lane >> 2, t = lane & 3;
+    const int kw_log = 31 - __clz(p.kw), kw_mask = p.kw - 1;
+    const int wk = warp & kw_mask, wc = warp >> kw_log, cw = kFrWarps >> kw_log;
+    const int N = p.N, K = p.K, q = p.q;
+    const uint32_t ones = p.ones, twos = p.twos, fours = p.fours;
+    const int P = q + (BIAS ? 1 : 0);
+    const int a_off = q * 512, ub = a_off + P * NG * 64;          // a unit: words of the planes, then scales [plane][group][32 columns]
+    unsigned char* ring = smem + warp * (p.depth * ub);
+    const uint32_t ring_u = smem_u32(ring);
+    float* red = reinterpret_cast<float*>(smem + kFrSmemBytes - 16 - 2 * kFrWarps * fr_red_floats(MT) * 4);      // [parity][warp][fr_red_floats]
+    int* s_flag = reinterpret_cast<int*>(smem + kFrSmemBytes - 16);
+
+    const int words = K / 32;
+    const int steps_total = (words + 3) / 4;
+    const int slab0 = blockIdx.y * p.steps_per_slab, slab1 = min(steps_total, slab0 + p.steps_per_slab);
+    int nsteps = 0;                           // this warp's steps: slab0 + wk + i kw
+#pragma unroll
+    for (int i = 0; i < KS; i++) nsteps += (slab0 + wk + i * p.kw < slab1) ? 1 : 0;
+    const int tiles = (N + kFrCols - 1) / kFrCols;
+    const int tile0 = blockIdx.x * p.tiles_per_cta, tile1 = min(tiles, tile0 + p.tiles_per_cta);
+
+    // ---- the warp's stream of units: (tile, step) ----
+    int ftile = nsteps ? tile0 + wc : tile1, fi = 0, fslot = 0;
+    const int nalpha = P * NG * 8;            // 8-byte pieces of scales
+    auto fetch = [&]() {
+        if (ftile < tile1) {
+            const int step = slab0 + wk + fi * p.kw;
+            const uint32_t dst = ring_u + fslot * ub;
+            {
+                const int kw = 4 * step + (lane >> 3), col = ftile * kFrCols + 4 * (lane & 7);
+                const bool ok = col < N && kw < words;            // N % 4 == 0: whole quads
+                const uint32_t* src = ok ? p.bW + (size_t)kw * q * N + col : p.bW;
+                const size_t inc = ok ? (size_t)N : 0;
+#pragma unroll 4
+                for (int b = 0; b < q; b++) {
+                    cp_async16(dst + b * 512 + lane * 16, src, ok);
+                    src += inc;
+                }
+            }
+            for (int at = lane; at < nalpha; at += 32) {
+                const int b = at / (NG * 8), gi = (at >> 3) % NG, col = ftile * kFrCols + 4 * (at & 7);
+                const int k = 128 * step + 32 * GW * gi;
+                const bool ok = col < N && k < K;
+                const size_t grp = ok ? (size_t)((unsigned)k / (unsigned)p.g) : 0;
+                const __half* src = (!BIAS || b < q) ? p.alpha + (grp * q + b) * N + col : p.q_bias + grp * N + col;
+                cp_async8(dst + a_off + at * 8, ok ? src : p.alpha, ok);
+            }
+            if (++fslot == p.depth) fslot = 0;
+            if (++fi == nsteps) {
+                fi = 0;
+                ftile += cw;
+            }
+        }
+        cp_async_commit();                    // one group per unit, empty ones at the end: the wait below counts groups
+    };
+    auto wait_unit = [&]() {                  // all but the last depth - 2 groups
+        switch (p.depth) {
+            case 2: cp_async_wait<0>(); break;
+            case 3: cp_async_wait<1>(); break;
+            case 4: cp_async_wait<2>(); break;
+            case 5: cp_async_wait<3>(); break;
+            default: cp_async_wait<4>(); break;
+        }
+        __syncwarp();                         // every lane's copies of this unit have landed, every lane has read the previous one
+    };
+    // packed words and scales are never written by a kernel: the stream starts while the previous kernel drains
+    pdl_launch_dependents();
+#pragma unroll 1
+    for (int i = 0; i < p.depth - 1; i++) fetch();
+    pdl_wait_prior_grids();                   // the activations may come from the previous kernel
+
+    // ---- activations of this warp's k-range, in operand order ----
+    uint32_t bx[KS][NG][NJ / 2][MT][2];
+    float start[KS][NG][MT][2];               // what the accumulators of rows 8 nt + 2 t, + 1 start from
+    float sx[KS][NG][MT][2];                  // BIAS: sums of the group's activations for those rows
+#pragma unroll
+    for (int i = 0; i < KS; i++)
+#pragma unroll
+        for (int gi = 0; gi < NG; gi++) {
+            const int kw = 4 * (slab0 + wk + i * p.kw) + gi * GW + ((t * GW) >> 2);
+            const int j0 = (t * GW % 4) * 4;  // this lane's first bit position
+#pragma unroll
+            for (int nt = 0; nt < MT; nt++) {
+                uint32_t lo[NJ / 2] = {}, hi[NJ / 2] = {};        // activations j0 .. j0 + NJ - 1 of the word, and those + 16
+                const int row = 8 * nt + r;
+                if (i < nsteps && kw < words && row < p.m) {
+                    const __half* src = p.x + (size_t)row * K + 32 * kw + j0;
+                    if constexpr (NJ >= 8) {
+#pragma unroll
+                        for (int v = 0; v < NJ / 8; v++) {
+                            const uint4 a = __ldcg(reinterpret_cast<const uint4*>(src) + v), b = __ldcg(reinterpret_cast<const uint4*>(src + 16) + v);
+                            lo[4 * v] = a.x; lo[4 * v + 1] = a.y; lo[4 * v + 2] = a.z; lo[4 * v + 3] = a.w;
+                            hi[4 * v] = b.x; hi[4 * v + 1] = b.y; hi[4 * v + 2] = b.z; hi[4 * v + 3] = b.w;
+                        }
+                    } else {
+                        const uint2 a = __ldcg(reinterpret_cast<const uint2*>(src)), b = __ldcg(reinterpret_cast<const uint2*>(src + 16));
+                        lo[0] = a.x; lo[1] = a.y;
+                        hi[0] = b.x; hi[1] = b.y;
+                    }
+                }
+#pragma unroll
+                for (int s = 0; s < NJ / 2; s++) {
+                    bx[i][gi][s][nt][0] = prmt_b32(lo[s], hi[s], 0x5410u);       // k of bits 2 s, 2 s + 16
+                    bx[i][gi][s][nt][1] = prmt_b32(lo[s], hi[s], 0x7632u);       // k of bits 2 s + 1, 2 s + 17
+                }
+            }
+            float d[MT][4];
+#pragma unroll
+            for (int nt = 0; nt < MT; nt++) d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f;
+            fr_start<0, NJ / 2, FIRST, MT>(d, bx[i][gi]);
+#pragma unroll
+            for (int nt = 0; nt < MT; nt++) {
+                start[i][gi][nt][0] = d[nt][0];
+                start[i][gi][nt][1] = d[nt][1];
+                if (BIAS) {
+                    const uint32_t one[4] = {ones, ones, ones, ones};
+                    float e[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int s = 0; s < NJ / 2; s++) mma_16816(e, one, bx[i][gi][s][nt]);
+                    sx[i][gi][nt][0] = e[0];
+                    sx[i][gi][nt][1] = e[1];
+                }
+            }
+        }
+
+    // ---- columns ----
+    const int my_tiles = (tile1 - tile0 + cw - 1) >> (4 - kw_log);      // every warp of the CTA walks as many: the barriers match
+    int slot = 0, parity = 0;
+#pragma unroll 1
+    for (int ti = 0; ti < my_tiles; ti++) {
+        const int tile = tile0 + wc + ti * cw;
+        float acc[4][MT][2];
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+#pragma unroll
+            for (int nt = 0; nt < MT; nt++) acc[c][nt][0] = acc[c][nt][1] = 0.f;
+        if (tile < tile1) {
+#pragma unroll
+            for (int i = 0; i < KS; i++) {
+                if (i >= nsteps) continue;
+                wait_unit();
+                fetch();
+                const unsigned char* u = ring + slot * ub;
+                if (++slot == p.depth) slot = 0;
+#pragma unroll 1
+                for (int b = 0; b < q; b++) {
+#pragma unroll
+                    for (int gi = 0; gi < NG; gi++) {
+                        const uint2 av = *reinterpret_cast<const uint2*>(u + a_off + (b * NG + gi) * 64 + r * 8);
+                        const float2 a01 = half2_bits_to_float2(av.x), a23 = half2_bits_to_float2(av.y);
+                        const uint4 wv = *reinterpret_cast<const uint4*>(u + b * 512 + (gi * GW + ((t * GW) >> 2)) * 128 + r * 16);
+                        uint32_t w[4] = {wv.x, wv.y, wv.z, wv.w};
+                        if (GW < 4) {         // this lane's NJ positions to the top of each half
+#pragma unroll
+                            for (int c = 0; c < 4; c++) w[c] <<= FIRST - (t * GW % 4) * 4;
+                        }
+                        float d0[MT][4], d1[MT][4];
+#pragma unroll
+                        for (int nt = 0; nt < MT; nt++)
+#pragma unroll
+                            for (int e = 0; e < 4; e++) d0[nt][e] = d1[nt][e] = start[i][gi][nt][e & 1];
+                        fr_products<0, NJ / 2, FIRST, MT>(d0, d1, w, bx[i][gi], ones, twos, fours);
+#pragma unroll
+                        for (int nt = 0; nt < MT; nt++)
+#pragma unroll
+                            for (int e = 0; e < 2; e++) {
+                                acc[0][nt][e] = fmaf(a01.x, d0[nt][e], acc[0][nt][e]);
+                                acc[1][nt][e] = fmaf(a01.y, d0[nt][2 + e], acc[1][nt][e]);
+                                acc[2][nt][e] = fmaf(a23.x, d1[nt][e], acc[2][nt][e]);
+                                acc[3][nt][e] = fmaf(a23.y, d1[nt][2 + e], acc[3][nt][e]);
+                            }
+                    }
+                }
+                if (BIAS) {
+#pragma unroll
+                    for (int gi = 0; gi < NG; gi++) {
+                        const uint2 av = *reinterpret_cast<const uint2*>(u + a_off + (q * NG + gi) * 64 + r * 8);
+                        const float2 a01 = half2_bits_to_float2(av.x), a23 = half2_bits_to_float2(av.y);
+#pragma unroll
+                        for (int nt = 0; nt < MT; nt++)
+#pragma unroll
+                            for (int e = 0; e < 2; e++) {
+                                acc[0][nt][e] = fmaf(a01.x, sx[i][gi][nt][e], acc[0][nt][e]);
+                                acc[1][nt][e] = fmaf(a01.y, sx[i][gi][nt][e], acc[1][nt][e]);
+                                acc[2][nt][e] = fmaf(a23.x, sx[i][gi][nt][e], acc[2][nt][e]);
+                                acc[3][nt][e] = fmaf(a23.y, sx[i][gi][nt][e], acc[3][nt][e]);
+                            }
+                    }
+                }
+            }
+        }
+        // ---- add the kw warps of this column group: block [column c of the quad][row][r] per warp ----
+        {
+            float* mine = red + (parity * kFrWarps + warp) * fr_red_floats(MT);
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+#pragma unroll
+                for (int nt = 0; nt < MT; nt++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++)
+                        mine[((c * MT + nt) * 8 + 2 * t + e) * kFrRedStride + r] = acc[c][nt][e];
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + wc), "r"(p.kw * 32) : "memory");
+            // 64 MT (row, column quad) sums by two warps per 8 rows, other warps each time
+            const int turn = (wk - ti * 2 * MT) & kw_mask;
+            for (int o = turn * 32 + lane; o < 64 * MT && tile < tile1; o += p.kw * 32) {
+                const int row = o >> 3, rr = o & 7, nt = row >> 3, m8 = row & 7;
+                const int col = tile * kFrCols + 4 * rr;
+                if (row >= p.m || col >= N) continue;
+                const float* src = red + (parity * kFrWarps + wc * p.kw) * fr_red_floats(MT) + (nt * 8 + m8) * kFrRedStride + rr;
+                float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+                for (int v = 0; v < p.kw; v++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) s[c] += src[v * fr_red_floats(MT) + c * MT * 8 * kFrRedStride];
+                const size_t off = (size_t)row * N + col;
+                const float4 f = make_float4(s[0], s[1], s[2], s[3]);
+                if (gridDim.y > 1) {
+                    red_add_v4(p.partial + off, f);
+                } else {
+                    if (p.y32) *reinterpret_cast<float4*>(p.y32 + off) = f;
+                    if (p.y16) {
+                        __half2 lo = __floats2half2_rn(f.x, f.y), hi = __floats2half2_rn(f.z, f.w);
+                        *reinterpret_cast<uint2*>(p.y16 + off) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+                    }
+                }
+            }
+            parity ^= 1;
+        }
+    }
+    if (gridDim.y == 1) return;
+
+    // ---- slabs: the last CTA of the column range converts the reduced sums and zeroes the workspace ----
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        const unsigned prev = atomicAdd(p.counters + blockIdx.x, 1u);
+        *s_flag = (prev == gridDim.y - 1u);
+    }
+    __syncthreads();
+    if (!*s_flag) return;
+    __threadfence();
+    const int c0 = tile0 * kFrCols, quads = (min(N, tile1 * kFrCols) - c0) / 4;
+    for (int idx = tid; idx < quads * p.m; idx += kFrThreads) {
+        const size_t off = (size_t)(idx / quads) * N + c0 + 4 * (idx % quads);
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.partial + off));
+        __stcg(reinterpret_cast<float4*>(p.partial + off), make_float4(0.f, 0.f, 0.f, 0.f));
+        if (p.y32) *reinterpret_cast<float4*>(p.y32 + off) = v;
+        if (p.y16) {
+            __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+            *reinterpret_cast<uint2*>(p.y16 + off) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+        }
+    }
+    if (tid == 0) p.counters[blockIdx.x] = 0u;
+}
+
+}  // namespace lg

@@ -1,0 +1,98 @@
+"""The batched kernels that fold planes or keep operands in registers, at the edges of their tiles, against 64-bit sums."""
+import numpy as np
+import pytest
+
+import lutgemm_b200 as L
+from lutgemm_b200 import synth
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _run(N, K, q, g, bias, m, column_scales=False, ordered=False):
+    bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + K + m, with_bias=bias)
+    if column_scales:
+        # columns whose scales lie far apart, down to fp16's subnormals and up to its largest values
+        s = 2.0 ** np.random.default_rng(m).integers(-18, 18, N)
+        alpha = np.clip(alpha * s, 0, 60000.0 / (q + 1)).astype(np.float16).astype(np.float32)
+        q_bias = None if q_bias is None else np.clip(q_bias * s, -9000.0, 9000.0).astype(np.float16).astype(np.float32)
+    x = synth.activations(m, K, seed=m)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g, q_bias).reserve_batch(m)
+    if ordered:
+        w.set_ordered(1)
+    xd = torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
+    y32 = torch.empty((m, N), dtype=torch.float32, device="cuda")
+    y16 = torch.empty((m, N), dtype=torch.float16, device="cuda")
+    for _ in range(2):                                    # the second call finds the workspace as the first one left it
+        L.matmul_f32(y32, xd, w, m)
+        L.matmul(y16, xd, w, m)
+    a16, b16 = alpha.astype(np.float16), None if q_bias is None else q_bias.astype(np.float16)
+    ref = oracle.bcq_matmul_f64(x, bW, a16, b16, g)
+    # Products are exact, sums are fp32: every addition errs by at most 2^-23 of the largest partial sum, which is at most
+    # 11 |x| |scale| summed (an operand of up to 6 and its offset of up to 5 for a sign).  K / 16 additions per pass.
+    mag = np.abs(a16.astype(np.float64)).sum(1) + (0 if b16 is None else np.abs(b16.astype(np.float64)))       # [G, N]
+    size = np.abs(x.astype(np.float64)).reshape(m, K // g, g).sum(2) @ mag
+    bound = (2 * K / 16 + 64) * 2.0 ** -23 * 11 * size + 1e-30
+    err = np.abs(y32.cpu().numpy().astype(np.float64) - ref)
+    assert (err <= bound).all(), (err / bound).max()
+    # one rounding to fp16 on top: half a unit in the last place, at least half the subnormal step
+    with np.errstate(over="ignore"):
+        lim = bound + np.maximum(np.abs(ref) * 2.0 ** -11, 2.0 ** -25)
+    got = y16.cpu().numpy().astype(np.float64)
+    finite = np.abs(ref) + lim < 65504
+    assert (np.abs(got - ref)[finite] <= lim[finite] * 1.0001).all()
+    w.close()
+
+
+# 128-column tiles, 64-k blocks, 16-row steps, 128- and 256-row items, one and several scale groups per block, a last block
+# of one word, groups wider than what a warp walks in one stride
+@pytest.mark.parametrize("N,K,q,g,bias,m", [
+    (8, 32, 4, 32, True, 17), (136, 96, 4, 32, True, 31), (128, 64, 3, 64, False, 64), (264, 2048, 2, 128, False, 129),
+    (264, 576, 1, 64, True, 130), (1000, 1152, 4, 384, True, 257), (2056, 256, 2, 256, True, 300), (512, 512, 1, 128, False, 144),
+    (120, 4096, 3, 1024, True, 100), (4096, 160, 4, 32, False, 513)])
+def test_split_operand_kernel(N, K, q, g, bias, m):
+    _run(N, K, q, g, bias, m)
+
+
+@pytest.mark.parametrize("q,bias,m", [(4, True, 40), (2, False, 150), (1, False, 200), (3, True, 256)])
+def test_split_operand_kernel_scales_far_apart(q, bias, m):
+    _run(264, 1024, q, 128, bias, m, column_scales=True)
+
+
+def test_split_operand_kernel_ordered_is_reproducible_and_right():
+    _run(264, 2048, 4, 128, True, 140, ordered=True)
+
+
+# 32-column units with ragged last quads and tiles, one to 8 planes, the three kinds of scale group, words beyond K, one and
+# two tiles of 8 rows, one and several k-ranges; the last two go 16 rows at a time
+@pytest.mark.parametrize("N,K,q,g,bias,m", [
+    (4, 32, 1, 32, False, 3), (12, 96, 2, 32, True, 4), (100, 160, 3, 160, False, 5), (36, 4128, 3, 96, True, 2),
+    (33 * 4, 1024, 4, 128, True, 8), (5000, 256, 2, 64, False, 7), (264, 8192, 3, 512, False, 3), (40, 2048, 8, 128, True, 6),
+    (64, 20480, 5, 64, True, 4), (2052, 4128, 3, 96, False, 16), (20, 384, 7, 192, True, 9), (28, 640, 2, 32, False, 35)])
+def test_register_operand_kernel(N, K, q, g, bias, m):
+    _run(N, K, q, g, bias, m)
+
+
+@pytest.mark.parametrize("q,g,bias,m", [(4, 128, True, 8), (3, 64, False, 3), (2, 32, True, 5)])
+def test_register_operand_kernel_scales_far_apart(q, g, bias, m):
+    _run(260, 1024, q, g, bias, m, column_scales=True)
+
+
+def test_three_rows_without_reserved_scratch_inside_a_capture():
+    """A first call of three rows inside a stream capture cannot allocate scratch: it still runs, one or two rows at a time."""
+    N, K, q, g = 512, 8192, 3, 128
+    bW, alpha, _ = synth.bcq_layer(N, K, q, g, seed=5)
+    x = synth.activations(3, K, seed=6)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g)
+    xd = torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
+    y = torch.zeros((3, N), dtype=torch.float32, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        L.matmul_f32(y, xd, w, 3)
+    graph.replay()
+    torch.cuda.synchronize()
+    ref = oracle.bcq_matmul_f64(x, bW, alpha.astype(np.float16), None, g)
+    assert np.linalg.norm(y.cpu().numpy() - ref) <= 1e-5 * np.linalg.norm(ref)
+    w.close()
