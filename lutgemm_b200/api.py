@@ -27,14 +27,16 @@ def _ptr(a):
         assert a.flags["C_CONTIGUOUS"]
         return a.ctypes.data_as(C.c_void_p)
     assert a.is_contiguous()
-    return C.c_void_p(a.data_ptr())
+    return a.data_ptr()
 
 
 def _stream_ptr(stream):
+    """The stream's handle as a plain integer (the prototypes make a pointer of it).  Without a stream, the current one of
+    the current device, asked for as a number: building the Stream object costs more than the rest of a small call."""
     if stream is None:
         import torch
-        stream = torch.cuda.current_stream()
-    return C.c_void_p(stream.cuda_stream)
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return stream.cuda_stream
 
 
 class nQWeight_fp16:
