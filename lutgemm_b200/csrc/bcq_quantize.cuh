@@ -239,7 +239,7 @@ bcq_quantize_kernel(const BqParams p) {
 // pairs to a word.  A weight then costs its q comparisons, one table read, q multiply-adds (B^T w) and one integer add
 // (B^T B) per word of pairs, and the sums of the next round are complete when the weights of this one are placed.
 // Bound by instruction issue, not by memory: the weights are read once.  Measured, N = K = 4096, q = 3, g = 128, 15
-// rounds: 395 us; bcq_quantize_kernel, which gives every group a whole warp, takes 3291 us.
+// rounds: 426 us; bcq_quantize_kernel, which gives every group a whole warp, takes 3291 us.
 // Sums are added in the order of bcq_quantize_kernel, whose lane L holds weights L, L + 32, ...: a lane here stands for
 // NJ = 32 / LG of those lanes (lane, lane + LG, ...), keeps their partial sums apart and adds them first, which is that
 // kernel's shuffle over distances 16 .. LG.  So both give the same bits, and which one a group takes does not show.

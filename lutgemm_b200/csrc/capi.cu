@@ -1985,7 +1985,7 @@ int lutgemm_bcq_quantize_device(const float* d_w, int N, int K, int q, int group
     const long long ctas = (groups + lg::kBqWarps - 1) / lg::kBqWarps;
     if (ctas > 0x7fffffffLL) return LUTGEMM_ERR_TOO_LARGE;
     cudaStream_t st = (cudaStream_t)stream;
-    // The tiled kernel is 8 times as fast wherever it applies; more planes or wider groups take a warp or a CTA per group.
+    // The tiled kernel is 7 to 8 times as fast wherever it was measured (426 / 3292 us at q = 3, g = 128); more planes or wider groups take a warp or a CTA per group.
     if (q <= lg::kBqTileMaxQ && g <= lg::kBqTileMaxG) {
         if (q == 1) launch_bcq_tile<1>(p, groups, st);
         else if (q == 2) launch_bcq_tile<2>(p, groups, st);
