@@ -385,9 +385,11 @@ int lutgemm_set_ordered_reduction(int enabled);
  * two at a time by a two-table kernel that reads the weights once for both; 0: one row per launch.  The pair
  * kernel is used only with the default reductions (not in ordered mode) and the default matvec variant. */
 int lutgemm_set_row_pairs(int enabled);
-/* 1 (default): m >= 4 runs the tensor-core (tcgen05) kernel, 128 rows per launch, smaller batches one LUT
- * matvec per row; 0: always one LUT matvec per row; 2: tensor-core kernel from m = 2.  All compute the same
- * function. */
+/* 1 (default): m >= 4 runs a tensor-core kernel (mma.sync with the weights in registers up to 8 rows; beyond, tcgen05 plane
+ * by plane, 128 rows per launch, or with the planes folded into one split operand, whichever is faster for the row and
+ * plane count), m = 3 and batches on containers that the tcgen05 kernels do not take the mma.sync kernel where scratch is
+ * reserved for them, else the LUT matvec; 0: always one LUT matvec per row; 2: tensor-core kernel from m = 2.  All
+ * compute the same function. */
 int lutgemm_set_batched_path(int mode);
 /* 0 (default): every batch on the tensor-core path takes the fp16 kernel (operand = +-alpha in fp16, exact products).
  * 1: a batch of up to 16 rows on a container of up to 4 planes runs the integer kernel (tcgen05.mma.kind::i8): the packed

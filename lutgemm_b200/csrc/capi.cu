@@ -901,9 +901,14 @@ int frag_rows_if_ready(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x
         if (rc != LUTGEMM_OK) return rc;
     }
     if ((whole && grid[0].y > 1) || (rest && grid[1].y > 1)) {
-        bool have = false;
-        const int rc = hl_have_rows(w, ws, whole ? lg::kFrMaxRows : m, st, &have);
-        if (rc != LUTGEMM_OK || !have) return rc;
+        const int rows = whole ? lg::kFrMaxRows : m;
+        bool have = (long long)ws->tc_rows * ws->n_cap >= (long long)rows * w->N;
+        // calls that never allocated before (fewer than four rows, containers without a tcgen05 kernel) still do not
+        if (!have && m >= kBatchedFromRows && w->tc_ok) {
+            const int rc = hl_have_rows(w, ws, rows, st, &have);
+            if (rc != LUTGEMM_OK) return rc;
+        }
+        if (!have) return LUTGEMM_OK;
     }
     *taken = true;
     for (int r0 = 0; r0 < m; r0 += lg::kFrMaxRows) {
@@ -1985,7 +1990,7 @@ int lutgemm_bcq_quantize_device(const float* d_w, int N, int K, int q, int group
     const long long ctas = (groups + lg::kBqWarps - 1) / lg::kBqWarps;
     if (ctas > 0x7fffffffLL) return LUTGEMM_ERR_TOO_LARGE;
     cudaStream_t st = (cudaStream_t)stream;
-    // The tiled kernel is 7 to 8 times as fast wherever it was measured (426 / 3292 us at q = 3, g = 128); more planes or wider groups take a warp or a CTA per group.
+    // The tiled kernel is 7 to 8 times as fast wherever it was measured (406 / 3292 us at q = 3, g = 128); more planes or wider groups take a warp or a CTA per group.
     if (q <= lg::kBqTileMaxQ && g <= lg::kBqTileMaxG) {
         if (q == 1) launch_bcq_tile<1>(p, groups, st);
         else if (q == 2) launch_bcq_tile<2>(p, groups, st);
