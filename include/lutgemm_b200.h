@@ -387,8 +387,8 @@ int lutgemm_set_ordered_reduction(int enabled);
 int lutgemm_set_row_pairs(int enabled);
 /* 1 (default): m >= 4 runs a tensor-core kernel (mma.sync with the weights in registers up to 8 rows; beyond, tcgen05 plane
  * by plane, 128 rows per launch, or with the planes folded into one split operand, whichever is faster for the row and
- * plane count), m = 3 and batches on containers that the tcgen05 kernels do not take the mma.sync kernel where scratch is
- * reserved for them, else the LUT matvec; 0: always one LUT matvec per row; 2: tensor-core kernel from m = 2.  All
+ * plane count), batches (m >= 3) on containers that the tcgen05 kernels do not take the mma.sync kernel where scratch is
+ * reserved for them, smaller ones the LUT matvec; 0: always one LUT matvec per row; 2: tensor-core kernel from m = 2.  All
  * compute the same function. */
 int lutgemm_set_batched_path(int mode);
 /* 0 (default): every batch on the tensor-core path takes the fp16 kernel (operand = +-alpha in fp16, exact products).

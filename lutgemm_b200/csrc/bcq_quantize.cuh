@@ -271,7 +271,7 @@ __device__ __forceinline__ float tile_sum_f(float (&v)[32 / LG]) {
 }
 
 template <int LG, int Q>
-__global__ void __launch_bounds__(kBqTileWarps * 32, Q == 2 ? 6 : 1)
+__global__ void __launch_bounds__(kBqTileWarps * 32, Q == 2 ? 6 : 4)
 bcq_quantize_tile_kernel(const BqParams p) {
     constexpr int E = 16;                                  // weights per lane: register e is weight (e % EE) * 32 + LG * (e / EE) + l
     constexpr int NJ = 32 / LG, EE = E / NJ;

@@ -873,7 +873,8 @@ int gemm_i8_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 }
 
 // Batches that the register-operand kernel is the fastest for.  Measured, us, register operand against what ran instead,
-// g = 128: 8192 x 8192, q = 2, 2 rows 17.6 / 13.1 (two-row LUT kernel), 3 rows 17.8 / 21.5 (that and one LUT row); q = 3, 4 rows
+// g = 128: 8192 x 8192, q = 2, 2 rows 17.6 / 13.1 (two-row LUT kernel), 3 rows 17.8 / 21.5 (that and one LUT row; on
+// larger weights these two are the faster: 256 / 207); q = 3, 4 rows
 // 22.2 / 28.7, 8 rows 23.8 / 28.9, 16 rows 32.9 / 29.8 (gemm_tc); q = 1, 8 rows 14.8 / 16.0; 12288 x 4096, q = 4, 8 rows
 // 20.1 / 25.7, 16 rows 34.4 / 26.3; 2048 x 2048, q = 4, 4 rows 4.7 / 8.1; 28672 x 8192, q = 4 + q_bias, 4 rows 82.6 / 116.5
 // (gemm_hl).  Containers that the tcgen05 kernels refuse (N % 8 != 0, or a group size that neither divides nor is a multiple
@@ -881,7 +882,8 @@ int gemm_i8_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 bool frag_wanted(const lutgemm_weight* w, const lutgemm_workspace* ws, int m) {
     if (m < 2 || w->N % 4 != 0 || ordered_for(ws) || gemm_i8_ok(w, m)) return false;
     if (m < kBatchedFromRows && g_variant.load() != 0) return false;       // the caller asked for a matvec kernel by name
-    if (m == 2) return !gemv_pair_ok(w, ws);
+    if (m == 2) return false;
+    if (m == 3) return !gemv_pair_ok(w, ws);
     return m <= 8 || !w->tc_ok;
 }
 
