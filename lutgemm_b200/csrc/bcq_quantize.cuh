@@ -243,7 +243,7 @@ bcq_quantize_kernel(const BqParams p) {
 // Sums are added in the order of bcq_quantize_kernel, whose lane L holds weights L, L + 32, ...: a lane here stands for
 // NJ = 32 / LG of those lanes (lane, lane + LG, ...), keeps their partial sums apart and adds them first, which is that
 // kernel's shuffle over distances 16 .. LG.  So both give the same bits, and which one a group takes does not show.
-constexpr int kBqTileWarps = 4;               // 8: 423 us at q = 3, 270 at q = 2, g = 64; 4: 406 and 254 (236 with registers for 6 CTAs)
+constexpr int kBqTileWarps = 4;               // 8: 423 us at q = 3, 270 at q = 2, g = 64; 4: 406 and 254
 constexpr int kBqTileMaxG = 512;              // 32 lanes of 16 weights; a field of pair counts holds up to 1023
 constexpr int kBqTileMaxQ = 4;                // the levels' signs are one 128-bit table entry
 
@@ -271,7 +271,7 @@ __device__ __forceinline__ float tile_sum_f(float (&v)[32 / LG]) {
 }
 
 template <int LG, int Q>
-__global__ void __launch_bounds__(kBqTileWarps * 32, Q == 2 ? 6 : 4)
+__global__ void __launch_bounds__(kBqTileWarps * 32)
 bcq_quantize_tile_kernel(const BqParams p) {
     constexpr int E = 16;                                  // weights per lane: register e is weight (e % EE) * 32 + LG * (e / EE) + l
     constexpr int NJ = 32 / LG, EE = E / NJ;

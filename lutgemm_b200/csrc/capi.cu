@@ -641,7 +641,8 @@ void hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) {
 bool gemm_hl_ok(const lutgemm_weight* w, int m) {
     const int passes = w->q + (w->q_bias ? 1 : 0);
     const int from = passes >= 5 ? 4 : passes >= 3 ? 64 : passes == 2 ? 97 : 129;
-    return w->tc_ok && w->q <= 4 && m >= from;
+    // with g = 32 every block builds two tables: up to 128 rows, where the expansion bounds it, that goes to gemm_tc
+    return w->tc_ok && w->q <= 4 && m >= from && (m > 128 || w->g >= lg::kHlStepK);
 }
 
 // fp32 rows of the workspace for at least `rows` rows of w's width, growing the container's own workspace when that is
@@ -877,14 +878,15 @@ int gemm_i8_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 // larger weights these two are the faster: 256 / 207); q = 3, 4 rows
 // 22.2 / 28.7, 8 rows 23.8 / 28.9, 16 rows 32.9 / 29.8 (gemm_tc); q = 1, 8 rows 14.8 / 16.0; 12288 x 4096, q = 4, 8 rows
 // 20.1 / 25.7, 16 rows 34.4 / 26.3; 2048 x 2048, q = 4, 4 rows 4.7 / 8.1; 28672 x 8192, q = 4 + q_bias, 4 rows 82.6 / 116.5
-// (gemm_hl).  Containers that the tcgen05 kernels refuse (N % 8 != 0, or a group size that neither divides nor is a multiple
+// (gemm_hl); g = 64, 28672 x 8192, q = 4, 4 rows 90.7 / 113.2, 8 rows 95.5 / 114.0; g = 32 (four scales to a unit) 8 rows
+// 118.9 / 114.1, which is why it stays with gemm_tc.  Containers that the tcgen05 kernels refuse (N % 8 != 0, or a group size that neither divides nor is a multiple
 // of 128) take it for every batch, 16 rows at a time: what is left for them is one matvec per row.
 bool frag_wanted(const lutgemm_weight* w, const lutgemm_workspace* ws, int m) {
     if (m < 2 || w->N % 4 != 0 || ordered_for(ws) || gemm_i8_ok(w, m)) return false;
     if (m < kBatchedFromRows && g_variant.load() != 0) return false;       // the caller asked for a matvec kernel by name
     if (m == 2) return false;
     if (m == 3) return !gemv_pair_ok(w, ws);
-    return m <= 8 || !w->tc_ok;
+    return !w->tc_ok || (m <= 8 && w->g % 64 == 0);
 }
 
 // *taken false and LUTGEMM_OK: no plan, or no scratch that could be had now; the caller goes on as without this kernel.
