@@ -89,7 +89,9 @@ int lutgemm_weight_describe(lutgemm_weight_t w, lutgemm_weight_desc* desc);
  * stream; to run one container from several streams at a time give every stream a workspace of its own
  * (lutgemm_matmul_ws below).  A first batched call (m >= 4) on a container that was not told its batch size
  * (lutgemm_weight_reserve_batch) allocates the batched path's fp32 rows, which synchronises the device; inside a
- * stream capture that call fails with LUTGEMM_ERR_BATCH instead. */
+ * stream capture that call fails with LUTGEMM_ERR_BATCH instead.  With rows for 128 (reserved, or once allocated) no later
+ * call allocates, whatever its batch.  Rows that are replaced by more of them stay allocated until the container is
+ * destroyed: a captured graph may still use them. */
 int lutgemm_matmul(void* out_fp16, const void* in_fp16, lutgemm_weight_t w, int m, void* stream);
 
 /* Same computation with the result left in fp32 (no final fp16 rounding). */
@@ -109,6 +111,10 @@ int lutgemm_matmul_wx(void* out_fp16, lutgemm_weight_t w, const void* in_fp16, i
  * call it once after creation, before capturing a CUDA graph that holds a batched call.  No reference counterpart
  * (its scratch is a process-wide singleton grown inside the call, lutGEMM/src/cuda/tmpWeight.hpp:28-35). */
 int lutgemm_weight_reserve_batch(lutgemm_weight_t w, int m);
+
+/* The batched path's fp32 rows of the container's own workspace: device address and bytes in use now (NULL and 0 when none
+ * are allocated), and the bytes of earlier, smaller blocks that are kept until the container is destroyed. */
+int lutgemm_weight_scratch(lutgemm_weight_t w, void** rows, size_t* bytes, size_t* bytes_kept);
 
 /* An explicit split-k workspace: partial rows, arrival counters, a status word and the batched path's fp32 rows for
  * containers up to max_n output features, max_k input features and batches up to max_m.  One workspace serves one

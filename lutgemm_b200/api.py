@@ -101,6 +101,13 @@ class nQWeight_fp16:
         capi.check(capi.lib().lutgemm_weight_reserve_batch(self.handle, int(m)), "reserve_batch")
         return self
 
+    def scratch(self):
+        """(address, bytes, bytes kept) of the batched path's fp32 rows: in use now, and of earlier blocks that captured
+        graphs may still use."""
+        rows, size, kept = C.c_void_p(), C.c_size_t(), C.c_size_t()
+        capi.check(capi.lib().lutgemm_weight_scratch(self.handle, C.byref(rows), C.byref(size), C.byref(kept)), "weight_scratch")
+        return rows.value or 0, size.value, kept.value
+
     def set_ordered(self, mode):
         """Split-k mode of calls on this container's own workspace: 0, 1, or -1 = the process-wide setting."""
         capi.check(capi.lib().lutgemm_weight_set_ordered(self.handle, int(mode)), "weight_set_ordered")

@@ -25,6 +25,14 @@
 #include "bcq_quantize.cuh"
 #include "gptq3.cuh"
 
+// A scratch block that has been replaced by a larger one.  A captured graph may hold its address, so it is given back only
+// with its workspace.
+struct lutgemm_retired_block {
+    void* ptr;
+    size_t bytes;
+    lutgemm_retired_block* next;
+};
+
 // Split-k scratch of the matmul kernels: everything a call writes besides its output.  One per container by
 // default; lutgemm_workspace_create makes more, so that several streams can use one container at a time.
 struct lutgemm_workspace {
@@ -34,6 +42,7 @@ struct lutgemm_workspace {
     int* status = nullptr;       // device word set by a kernel whose bounded wait ran out
     float* tc_partial = nullptr; // fp32 split-k rows of the batched (tensor-core) path, [tc_rows][n_cap], kept zeroed
     int tc_rows = 0;
+    lutgemm_retired_block* retired = nullptr;   // earlier tc_partial blocks
     int n_cap = 0, slabs = 0;    // widest N and most 512-k slabs this workspace serves
     // transposed copies for the (output, nqW, input, n) overload: input [n][K] and output [n][N] fp16
     void* t_in = nullptr;
@@ -233,6 +242,11 @@ void free_workspace_buffers(lutgemm_workspace* ws) {
     if (ws->tc_partial) cudaFree(ws->tc_partial);
     if (ws->t_in) cudaFree(ws->t_in);
     if (ws->t_out) cudaFree(ws->t_out);
+    while (lutgemm_retired_block* r = ws->retired) {
+        ws->retired = r->next;
+        cudaFree(r->ptr);
+        delete r;
+    }
     ws->partial = ws->partial2 = ws->tc_partial = nullptr;
     ws->counters = nullptr;
     ws->status = nullptr;
@@ -251,6 +265,37 @@ inline int ordered_for(const lutgemm_workspace* ws) {
 int tc_rows_for(int m) {
     const int rows = m > 128 ? 128 : m;
     return (rows + 15) / 16 * 16;
+}
+
+// A larger block of fp32 rows (of n_cap columns), zeroed on st; `rows` if they can be had, else at least `rows_min`.  The old
+// block stays allocated: graphs captured with it keep reducing into it.  Growth at least doubles (up to rows_max), so the
+// blocks that are kept are together smaller than the one in use.
+int grow_tc_rows(lutgemm_workspace* ws, int rows, int rows_min, int rows_max, cudaStream_t st) {
+    const size_t row_bytes = (size_t)ws->n_cap * sizeof(float);
+    const int doubled = 2 * ws->tc_rows < rows_max ? 2 * ws->tc_rows : rows_max;
+    int take = doubled > rows ? doubled : rows;
+    float* block = nullptr;
+    cudaError_t e;
+    while ((e = cudaMalloc(&block, take * row_bytes)) != cudaSuccess && take > rows_min) {
+        (void)cudaGetLastError();
+        take = take > rows ? rows : rows_min;
+    }
+    LG_CUDA(e);
+    lutgemm_retired_block* old = ws->tc_partial ? new (std::nothrow) lutgemm_retired_block : nullptr;
+    e = cudaMemsetAsync(block, 0, take * row_bytes, st);
+    if (e != cudaSuccess || (ws->tc_partial && !old)) {
+        delete old;
+        cudaFree(block);
+        LG_CUDA(e);
+        return LUTGEMM_ERR_TOO_LARGE;
+    }
+    if (old) {
+        *old = {ws->tc_partial, ws->tc_rows * row_bytes, ws->retired};
+        ws->retired = old;
+    }
+    ws->tc_partial = block;
+    ws->tc_rows = take;
+    return LUTGEMM_OK;
 }
 
 int fill_workspace(lutgemm_workspace* ws, int N, int K, int batch_rows) {
@@ -502,9 +547,12 @@ int launch_gemm_tc_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::
     return LUTGEMM_OK;
 }
 
+int hl_rows_for(int N, int m);
+
 // Split-k plan of a batched launch (256-column tiles x k-ranges of whole 128-k steps) and, when it splits, the fp32
-// reduction rows of the workspace.
-int tc_split(lutgemm_weight* w, lutgemm_workspace* ws, int m, cudaStream_t st, int* splitk_out, int* steps_per_cta_out) {
+// reduction rows of the workspace: at least m, and `rows` where they have to be allocated anyway (for the kernels that ask
+// for this plan only to follow its rule on scratch).
+int tc_split(lutgemm_weight* w, lutgemm_workspace* ws, int m, int rows, cudaStream_t st, int* splitk_out, int* steps_per_cta_out) {
     const int tiles = (w->N + lg::kTcTileN - 1) / lg::kTcTileN;
     const int steps_total = (w->K + lg::kTcStepK - 1) / lg::kTcStepK;
     // split-k factor: fill whole waves of one CTA per SM; among equally full choices take the smallest
@@ -526,13 +574,9 @@ int tc_split(lutgemm_weight* w, lutgemm_workspace* ws, int m, cudaStream_t st, i
         if (ws != &w->own) return LUTGEMM_ERR_TOO_LARGE;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone) return LUTGEMM_ERR_BATCH;
-        if (ws->tc_partial) LG_CUDA(cudaFree(ws->tc_partial));
-        ws->tc_partial = nullptr;
-        ws->tc_rows = 0;
-        const int rows = tc_rows_for(m);
-        LG_CUDA(cudaMalloc(&ws->tc_partial, (size_t)rows * w->N * sizeof(float)));
-        LG_CUDA(cudaMemset(ws->tc_partial, 0, (size_t)rows * w->N * sizeof(float)));
-        ws->tc_rows = rows;
+        const int need = tc_rows_for(m);
+        const int rc = grow_tc_rows(ws, rows > need ? rows : need, need, hl_rows_for(w->N, kMaxBatch), st);
+        if (rc != LUTGEMM_OK) return rc;
     }
     *splitk_out = splitk;
     *steps_per_cta_out = steps_per_cta;
@@ -560,7 +604,7 @@ int gemm_tc_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
     }
     int splitk = 1;
     {
-        int rc = tc_split(w, ws, m, st, &splitk, &p.steps_per_cta);
+        int rc = tc_split(w, ws, m, m, st, &splitk, &p.steps_per_cta);
         if (rc != LUTGEMM_OK) return rc;
     }
     const int tiles = (w->N + lg::kTcTileN - 1) / lg::kTcTileN;
@@ -645,21 +689,9 @@ bool gemm_hl_ok(const lutgemm_weight* w, int m) {
     return w->tc_ok && w->q <= 4 && m >= from && (m > 128 || w->g >= lg::kHlStepK);
 }
 
-// fp32 rows of the workspace for at least `rows` rows of w's width, growing the container's own workspace when that is
-// possible now (it synchronises the device: not inside a stream capture).  *have false: not available.
-int hl_have_rows(lutgemm_weight* w, lutgemm_workspace* ws, int rows, cudaStream_t st, bool* have) {
-    *have = (long long)ws->tc_rows * ws->n_cap >= (long long)rows * w->N;
-    if (*have || ws != &w->own) return LUTGEMM_OK;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone) return LUTGEMM_OK;
-    if (ws->tc_partial) LG_CUDA(cudaFree(ws->tc_partial));
-    ws->tc_partial = nullptr;
-    ws->tc_rows = 0;
-    LG_CUDA(cudaMalloc(&ws->tc_partial, (size_t)rows * w->N * sizeof(float)));
-    LG_CUDA(cudaMemsetAsync(ws->tc_partial, 0, (size_t)rows * w->N * sizeof(float), st));     // before the kernel that follows
-    ws->tc_rows = rows;
-    *have = true;
-    return LUTGEMM_OK;
+// Whether the workspace has at least `rows` fp32 rows of w's width.
+bool have_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, int rows) {
+    return (long long)ws->tc_rows * ws->n_cap >= (long long)rows * w->N;
 }
 
 template <int Q>
@@ -693,18 +725,13 @@ int launch_gemm_hl_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::
 int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __half* y16, float* y32, int m, cudaStream_t st) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return LUTGEMM_ERR_CUDA;
-    // what a call without reserved scratch is told does not depend on the kernel: the plane kernel's rule, for its first launch
+    // Scratch is allocated, and what a call without reserved scratch is told is decided, by the plane kernel's rule for its
+    // first launch, whatever kernel runs: a container with scratch for 128 rows never allocates again in a call.
     int unused_split = 1, unused_steps = 0;
-    int rc = tc_split(w, ws, m < 128 ? m : 128, st, &unused_split, &unused_steps);
+    const int rc = tc_split(w, ws, m < 128 ? m : 128, hl_rows_for(w->N, m), st, &unused_split, &unused_steps);
     if (rc != LUTGEMM_OK) return rc;
     lg::HlParams p = {};
-    hl_plan(w, m, !ordered_for(ws), &p);
-    if (p.splits > 1) {
-        bool have = false;
-        rc = hl_have_rows(w, ws, m, st, &have);
-        if (rc != LUTGEMM_OK) return rc;
-        if (!have) hl_plan(w, m, false, &p);
-    }
+    hl_plan(w, m, !ordered_for(ws) && have_rows(w, ws, m), &p);
     p.box_rows = m < lg::kHlBoxRows ? (m + 15) / 16 * 16 : lg::kHlBoxRows;
     p.x_slot_bytes = (m <= lg::kHlBoxRows || p.full_items == 0 ? 1 : 2) * p.box_rows * 128;
     p.x_slots = lg::kHlXBudget / p.x_slot_bytes;
@@ -858,7 +885,7 @@ int gemm_i8_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
             return LUTGEMM_ERR_CUDA;
     }
     int splitk = 1;
-    int rc = tc_split(w, ws, m, st, &splitk, &p.steps_per_cta);
+    int rc = tc_split(w, ws, m, m, st, &splitk, &p.steps_per_cta);
     if (rc != LUTGEMM_OK) return rc;
     p.partial = ws->tc_partial; p.counters = ws->counters; p.status = ws->status;
     p.y16 = y16; p.y32 = y32;
@@ -901,19 +928,10 @@ int frag_rows_if_ready(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x
     if (m >= kBatchedFromRows && w->tc_ok) {
         // what a call without reserved scratch is told does not depend on the kernel: the plane kernel's rule
         int unused_split = 1, unused_steps = 0;
-        const int rc = tc_split(w, ws, m < 128 ? m : 128, st, &unused_split, &unused_steps);
+        const int rc = tc_split(w, ws, m < 128 ? m : 128, m, st, &unused_split, &unused_steps);
         if (rc != LUTGEMM_OK) return rc;
     }
-    if ((whole && grid[0].y > 1) || (rest && grid[1].y > 1)) {
-        const int rows = whole ? lg::kFrMaxRows : m;
-        bool have = (long long)ws->tc_rows * ws->n_cap >= (long long)rows * w->N;
-        // calls that never allocated before (fewer than four rows, containers without a tcgen05 kernel) still do not
-        if (!have && m >= kBatchedFromRows && w->tc_ok) {
-            const int rc = hl_have_rows(w, ws, rows, st, &have);
-            if (rc != LUTGEMM_OK) return rc;
-        }
-        if (!have) return LUTGEMM_OK;
-    }
+    if (((whole && grid[0].y > 1) || (rest && grid[1].y > 1)) && !have_rows(w, ws, whole ? lg::kFrMaxRows : m)) return LUTGEMM_OK;
     *taken = true;
     for (int r0 = 0; r0 < m; r0 += lg::kFrMaxRows) {
         const int rows = m - r0 < lg::kFrMaxRows ? m - r0 : lg::kFrMaxRows, i = rows == lg::kFrMaxRows ? 0 : 1;
@@ -1251,17 +1269,26 @@ int lutgemm_weight_reserve_batch(lutgemm_weight_t w, int m) {
     if (m < 1 || m > kMaxBatch) return LUTGEMM_ERR_BATCH;
     lutgemm_workspace* ws = &w->own;
     const int rows = hl_rows_for(w->N, m);
+    int rc = LUTGEMM_OK;
     if (m >= 2 && ws->tc_rows < rows) {
-        if (ws->tc_partial) LG_CUDA(cudaFree(ws->tc_partial));
-        ws->tc_partial = nullptr; ws->tc_rows = 0;
-        LG_CUDA(cudaMalloc(&ws->tc_partial, (size_t)rows * w->N * sizeof(float)));
-        LG_CUDA(cudaMemset(ws->tc_partial, 0, (size_t)rows * w->N * sizeof(float)));
-        ws->tc_rows = rows;
+        rc = grow_tc_rows(ws, rows, rows, hl_rows_for(w->N, kMaxBatch), nullptr);
+        if (rc != LUTGEMM_OK) return rc;
+        LG_CUDA(cudaStreamSynchronize(nullptr));       // zeroed before a call on a stream that does not wait for this one
     }
     // transposed copies of the (output, nqW, input, n) overload
-    int rc = grow(&ws->t_in, &ws->t_in_bytes, (size_t)m * w->K * sizeof(__half), nullptr);
+    rc = grow(&ws->t_in, &ws->t_in_bytes, (size_t)m * w->K * sizeof(__half), nullptr);
     if (rc == LUTGEMM_OK) rc = grow(&ws->t_out, &ws->t_out_bytes, (size_t)m * w->N * sizeof(__half), nullptr);
     return rc;
+}
+
+int lutgemm_weight_scratch(lutgemm_weight_t w, void** rows, size_t* bytes, size_t* bytes_kept) {
+    if (!w || !rows || !bytes || !bytes_kept) return LUTGEMM_ERR_NULL;
+    const lutgemm_workspace* ws = &w->own;
+    *rows = ws->tc_partial;
+    *bytes = (size_t)ws->tc_rows * ws->n_cap * sizeof(float);
+    *bytes_kept = 0;
+    for (const lutgemm_retired_block* r = ws->retired; r; r = r->next) *bytes_kept += r->bytes;
+    return LUTGEMM_OK;
 }
 
 int lutgemm_matmul_wx(void* out, lutgemm_weight_t w, const void* in, int n, void* stream) {

@@ -1,0 +1,116 @@
+"""The batched path's fp32 rows: a block that a captured graph may hold is never given back while its container lives."""
+import numpy as np
+import pytest
+
+import lutgemm_b200 as L
+from lutgemm_b200 import synth
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+# several k-ranges for 16, 128 and 256 rows, so that each of these calls reduces into the rows
+N, K, Q, G = 1024, 4096, 4, 128
+
+
+def _container():
+    bW, alpha, _ = synth.bcq_layer(N, K, Q, G, seed=11)
+    return L.nQWeight_fp16(bW, alpha, K, N, Q, False, K // G), bW, alpha.astype(np.float16)
+
+
+def _device(x):
+    return torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
+
+
+def _close(y, x, bW, alpha):
+    ref = oracle.bcq_matmul_f64(x, bW, alpha, None, G)
+    assert np.linalg.norm(y - ref) <= 8e-4 * np.linalg.norm(ref)      # the rounding to fp16, as in perf/cases.py
+
+
+def _capture(w, x, m):
+    """The graph of one call, its output and its input (which has to live as long as the graph)."""
+    xd = _device(x)
+    y = torch.zeros((m, N), dtype=torch.float16, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        L.matmul(y, xd, w, m)
+    return graph, y, xd
+
+
+def _eager(w, bW, alpha, m, seed):
+    x = synth.activations(m, K, seed=seed)
+    y = torch.empty((m, N), dtype=torch.float16, device="cuda")
+    L.matmul(y, _device(x), w, m)
+    _close(y.cpu().numpy(), x, bW, alpha)
+
+
+@pytest.mark.parametrize("m", [16, 128])
+def test_a_larger_call_leaves_the_rows_of_a_captured_one(m):
+    w, bW, alpha = _container()
+    w.reserve_batch(128)
+    before = w.scratch()
+    x = synth.activations(m, K, seed=m)
+    graph, y, xd = _capture(w, x, m)
+    for rows in (256, 300):
+        _eager(w, bW, alpha, rows, rows)
+        assert w.scratch() == before
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        _close(y.cpu().numpy(), x, bW, alpha)
+    del graph
+    w.close()
+
+
+def test_growth_keeps_the_earlier_rows():
+    """Calls on a container that nothing was reserved for, and a later reservation: more rows, the earlier ones kept."""
+    w, bW, alpha = _container()
+    assert w.scratch() == (0, 0, 0)
+    graphs, blocks = [], set()
+    for m in (16, 40, 128):
+        _eager(w, bW, alpha, m, m)
+        x = synth.activations(m, K, seed=m + 1)
+        graphs.append((*_capture(w, x, m), x))
+        blocks.add(w.scratch()[:2])
+    w.reserve_batch(1024)
+    address, size, kept = w.scratch()
+    assert size >= max(b for _, b in blocks) and kept <= size
+    assert kept == sum(b for a, b in blocks if a != address)
+    assert len({a for a, _ in blocks}) >= 2               # the sizes above do make it grow
+    _eager(w, bW, alpha, 512, 7)
+    for graph, y, xd, x in graphs:
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        _close(y.cpu().numpy(), x, bW, alpha)
+    del graphs, graph
+    w.close()
+
+
+def test_host_call_replays_after_larger_calls_and_reservations():
+    """matmul_host keeps the last call as a graph: it stays right when other calls and reservations come between."""
+    w, bW, alpha = _container()
+    x = synth.activations(128, K, seed=3)
+    out = np.empty((128, N), np.float16)                  # the same buffers each time: the recorded graph is what runs
+    _close(L.matmul_host(out, x, w, 128), x, bW, alpha)
+    before = w.scratch()
+    _eager(w, bW, alpha, 256, 5)
+    assert w.scratch() == before
+    out.fill(0)
+    _close(L.matmul_host(out, x, w, 128), x, bW, alpha)
+    w.reserve_batch(512)
+    assert w.scratch()[2] == before[1]
+    out.fill(0)
+    _close(L.matmul_host(out, x, w, 128), x, bW, alpha)
+    w.close()
+
+
+def test_rising_batches_do_not_allocate_once_128_rows_are_there():
+    w, bW, alpha = _container()
+    _eager(w, bW, alpha, 128, 1)
+    before = w.scratch()
+    for m in (129, 300, 301, 1100):
+        _eager(w, bW, alpha, m, m)
+        assert w.scratch() == before
+    w.close()
