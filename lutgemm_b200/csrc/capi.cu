@@ -636,18 +636,25 @@ int hl_rows_for(int N, int m) {
 }
 
 // One CTA per SM: an item is 128 columns x 256 rows, and an item may be cut into two halves of 128 rows or into k-ranges.
-// Cost model in cycles: a block of 64 k takes the tensor pipe 4 cycles per row (two passes; 2 with one) and the expansion
-// at least kHlExpCycles whatever the rows; a CTA's start, first loads and epilogue add kHlCtaCycles, a split's reductions
-// and last-arriver pass kHlSplitCycles.  The plan with the smallest estimate is taken: whole items, halves, whole items
+// Cost model in cycles: a block of 64 k takes the tensor pipe and shared memory kHlRowCycles per row and pass, and the
+// expansion kHlExpCycles whatever the rows, more with more table entries; a CTA's start, first loads and epilogue add
+// kHlCtaCycles; a split adds kHlSplitCycles and, per row, the reductions in L2 and the last arriver's pass (shared among the
+// k-ranges), which a part-filled wave does faster.  Fitted to 804 timed calls (1024 x 8192 to 28672 x 4096, q = 1 to 4, 16 to
+// 2048 rows, split and not; the estimate's spread is 7 %).  A split that cost 4000 cycles whatever its rows gave 8192 x 2048,
+// q = 1, 256 rows two k-ranges: 21.2 us (14.5 unsplit), and 11008 x 4096, q = 4, 256 rows three: 54.3 (44.5).  Of 942 calls
+// at 14 widths 214 got faster by more than 3 % and 17 slower, the most 5120 x 5120, q = 2, 400 rows: 51.7 (46.4).
+// The plan with the smallest estimate is taken: whole items, halves, whole items
 // with a last partial wave of halves, each with 1 to 8 k-ranges.
-constexpr int kHlExpCycles = 560, kHlCtaCycles = 7000, kHlSplitCycles = 4000;
+constexpr double kHlRowCycles = 2.18, kHlExpCycles = 630, kHlEntryCycles = 8.5, kHlBiasCycles = 14.5;
+constexpr double kHlCtaCycles = 6300, kHlSplitCycles = 4400, kHlSplitRowCycles = 30;
 void hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) {
     const int sms = sm_count();
     const int T = (w->N + lg::kHlCols - 1) / lg::kHlCols, RT = (m + lg::kHlRows - 1) / lg::kHlRows;
     const long long items = (long long)T * RT;
     const int blocks = (w->K + lg::kHlStepK - 1) / lg::kHlStepK;
-    const int per_row = (w->q == 1 && !w->q_bias) ? 2 : 4;
-    auto block_cost = [&](int rows) { const int t = per_row * ((rows + 15) / 16 * 16); return t > kHlExpCycles ? t : kHlExpCycles; };
+    const double per_row = (w->q == 1 && !w->q_bias ? 1 : 2) * kHlRowCycles;
+    const double expansion = kHlExpCycles + kHlEntryCycles * ((1 << w->q) - 2) + (w->q_bias ? kHlBiasCycles : 0);
+    auto block_cost = [&](int rows) { const double t = per_row * ((rows + 15) / 16 * 16); return t > expansion ? t : expansion; };
     const int whole_rows = m < lg::kHlRows ? m : lg::kHlRows, half_rows = m < 128 ? m : 128;
     const long long units = m <= 128 ? items : (long long)T * ((m + 127) / 128);       // halves that have rows
     p->col_tiles = T;
@@ -659,9 +666,13 @@ void hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) {
         const int bps = (blocks + c - 1) / c;
         const int real = (blocks + bps - 1) / bps;
         const long long nf = full * real, nh = halves * real;
-        const double extra = kHlCtaCycles + (real > 1 ? kHlSplitCycles : 0);
-        const double t = (double)((nf + sms - 1) / sms) * (extra + (double)bps * block_cost(whole_rows)) +
-                         (double)((nh + sms - 1) / sms) * (extra + (double)bps * block_cost(half_rows));
+        // n CTAs of `rows` rows, wave after wave
+        auto waves = [&](long long n, int rows) {
+            const double busy = (double)(n < sms ? n : sms) / sms;
+            const double split = real > 1 ? kHlSplitCycles + kHlSplitRowCycles * rows * (1 + 1.8 / real) * (1 + 2 * busy) / 3 : 0.0;
+            return (double)((n + sms - 1) / sms) * (kHlCtaCycles + split + bps * block_cost(rows));
+        };
+        const double t = waves(nf, whole_rows) + waves(nh, half_rows);
         if (t < best * 0.98) {
             best = t;
             p->full_items = (int)full; p->splits = real; p->blocks_per_split = bps;
