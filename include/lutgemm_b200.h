@@ -120,7 +120,9 @@ int lutgemm_weight_scratch(lutgemm_weight_t w, void** rows, size_t* bytes, size_
  * containers up to max_n output features, max_k input features and batches up to max_m.  One workspace serves one
  * stream at a time; two streams may run the SAME container concurrently when each passes its own workspace.
  * lutgemm_matmul_ws / _f32_ws are lutgemm_matmul / _f32 on that workspace (NULL = the container's own) and never
- * allocate: a container or batch beyond the workspace's sizes is refused with LUTGEMM_ERR_TOO_LARGE.
+ * allocate: a container or batch beyond the workspace's sizes is refused with LUTGEMM_ERR_TOO_LARGE.  The fp32 rows are what
+ * the same calls would use of a container's own workspace: min(max_m, 128) x max_n floats, and with max_m above 128 up to
+ * 128 x 256 floats per SM (19 MB) where that is more.
  * lutgemm_workspace_status synchronises and reads the workspace's status word (see lutgemm_weight_device_status).
  * No reference counterpart: the reference runs on the legacy default stream only. */
 typedef struct lutgemm_workspace* lutgemm_workspace_t;
@@ -375,6 +377,9 @@ const char* lutgemm_status_string(int status);
 int lutgemm_last_cuda_error(void);
 /* How many kernels this library has launched in this process (all threads). */
 unsigned long long lutgemm_kernel_launch_count(void);
+/* The matmul kernel that this thread launched last ("" if none yet) and, where the pointers are not NULL, its grid; of the
+ * batched kernels grid_y is the number of k-ranges.  The text is static. */
+const char* lutgemm_last_launch(int* grid_x, int* grid_y);
 /* Tuning knob: columns per CTA of the LUT matvec (0 = automatic).  Process-wide. */
 int lutgemm_set_gemv_ntile(int columns);
 /* Tuning knob: 0 = bulk-copy (TMA) fed matvec kernel (default), 1 = register-streaming kernel.

@@ -206,6 +206,14 @@ def matmul_host(output_np, input_np, nqW, m):
     return output_np
 
 
+def last_launch():
+    """(kernel, grid x, grid y) of the matmul kernel that this thread launched last; of the batched kernels grid y is the
+    number of k-ranges."""
+    gx, gy = C.c_int(), C.c_int()
+    name = capi.lib().lutgemm_last_launch(C.byref(gx), C.byref(gy)).decode()
+    return name, gx.value, gy.value
+
+
 def dequantize_gpu(nqW, d_fW, algo=0, stream=None):
     capi.check(capi.lib().lutgemm_dequantize(nqW.handle, _ptr(d_fW), _stream_ptr(stream)), "dequantize_gpu")
     return d_fW

@@ -28,7 +28,7 @@ SYMBOLS = (
     "lutgemm_from_python_layout", "lutgemm_packer_pack", "lutgemm_packer_unpack",
     "lutgemm_packer_pack_device", "lutgemm_packer_unpack_device", "lutgemm_from_python_layout_device",
     "lutgemm_bcq_quantize", "lutgemm_bcq_quantize_device", "lutgemm_matmul_gptq",
-    "lutgemm_status_string", "lutgemm_last_cuda_error", "lutgemm_kernel_launch_count", "lutgemm_set_gemv_ntile",
+    "lutgemm_status_string", "lutgemm_last_cuda_error", "lutgemm_kernel_launch_count", "lutgemm_last_launch", "lutgemm_set_gemv_ntile",
     "lutgemm_set_gemv_variant", "lutgemm_set_dependent_launch", "lutgemm_set_batched_path", "lutgemm_set_batched_int8", "lutgemm_set_ordered_reduction", "lutgemm_set_row_pairs", "lutgemm_weight_device_status",
 )
 
@@ -137,6 +137,8 @@ def lib():
     L.lutgemm_status_string.restype = C.c_char_p
     L.lutgemm_last_cuda_error.restype = ip
     L.lutgemm_kernel_launch_count.restype = C.c_ulonglong
+    L.lutgemm_last_launch.argtypes = [C.POINTER(ip), C.POINTER(ip)]
+    L.lutgemm_last_launch.restype = C.c_char_p
     L.lutgemm_set_gemv_ntile.argtypes = [ip]
     L.lutgemm_set_gemv_variant.argtypes = [ip]
     L.lutgemm_set_dependent_launch.argtypes = [ip]
@@ -147,7 +149,7 @@ def lib():
     L.lutgemm_weight_device_status.argtypes = [vp, C.POINTER(ip)]
     for name in SYMBOLS:
         fn = getattr(L, name)
-        if name not in ("lutgemm_status_string", "lutgemm_kernel_launch_count"):
+        if name not in ("lutgemm_status_string", "lutgemm_kernel_launch_count", "lutgemm_last_launch"):
             fn.restype = ip
     _LIB = L
     return L

@@ -112,6 +112,9 @@ struct lutgemm_sequence {
 namespace {
 
 thread_local int g_last_cuda = 0;
+// the matmul kernel that this thread launched last (lutgemm_last_launch)
+thread_local const char* g_last_kernel = "";
+thread_local dim3 g_last_grid = dim3(0, 0, 0);
 std::atomic<unsigned long long> g_launches{0};
 std::atomic<int> g_ntile_override{0};
 std::atomic<int> g_pdl{1};
@@ -124,6 +127,11 @@ std::atomic<int> g_variant{0};   // 0: bulk-copy fed kernel (default); 1: regist
 inline int ordered_for(const lutgemm_workspace* ws);
 constexpr int kMaxCounters = 4096;
 constexpr int kMaxBatch = 65536;
+inline void note_launch(const char* kernel, dim3 grid) {
+    g_last_kernel = kernel;
+    g_last_grid = grid;
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+}
 constexpr int kBatchedFromRows = 4;      // m >= 4 goes to the tensor-core kernel
 
 #define LG_CUDA(call)                                  \
@@ -267,6 +275,20 @@ int tc_rows_for(int m) {
     return (rows + 15) / 16 * 16;
 }
 
+int sm_count();
+
+// Rows of N columns for an explicit workspace that serves every width up to N and batches up to m.  The split-operand kernel
+// asks for rows of its call's width (hl_rows_for): the most elements over all widths, in tiles of 128 columns.
+int workspace_rows_for(int N, int m) {
+    long long elements = (long long)tc_rows_for(m) * N;
+    for (int t = 1; t <= (N + lg::kHlCols - 1) / lg::kHlCols && t < sm_count(); t++) {
+        const int rows = lg::kHlRows * ((sm_count() - 1) / t), n = t * lg::kHlCols < N ? t * lg::kHlCols : N;
+        const long long e = (long long)(m < rows ? m : rows) * n;
+        if (e > elements) elements = e;
+    }
+    return (int)((elements + N - 1) / N);
+}
+
 // A larger block of fp32 rows (of n_cap columns), zeroed on st; `rows` if they can be had, else at least `rows_min`.  The old
 // block stays allocated: graphs captured with it keep reducing into it.  Growth at least doubles (up to rows_max), so the
 // blocks that are kept are together smaller than the one in use.
@@ -310,7 +332,7 @@ int fill_workspace(lutgemm_workspace* ws, int N, int K, int batch_rows) {
     LG_CUDA(cudaMalloc(&ws->status, sizeof(int)));
     LG_CUDA(cudaMemset(ws->status, 0, sizeof(int)));
     if (batch_rows > 0) {
-        const int rows = tc_rows_for(batch_rows);
+        const int rows = workspace_rows_for(N, batch_rows);
         LG_CUDA(cudaMalloc(&ws->tc_partial, (size_t)rows * N * sizeof(float)));
         LG_CUDA(cudaMemset(ws->tc_partial, 0, (size_t)rows * N * sizeof(float)));
         ws->tc_rows = rows;
@@ -390,7 +412,7 @@ int launch_gemv_tma(const lutgemm_weight* w, const lg::Gemv2Params& p, dim3 grid
     cfg.attrs = attr;
     cfg.numAttrs = g_pdl.load() ? 1 : 0;
     LG_CUDA(cudaLaunchKernelEx(&cfg, kern, w->tmW, w->tmA, p));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    note_launch("gemv_tma_kernel", grid);
     LG_CUDA(cudaGetLastError());
     return LUTGEMM_OK;
 }
@@ -416,7 +438,7 @@ int launch_gemv_reg(const lg::Gemv2Params& p, dim3 grid, bool bias, cudaStream_t
     cfg.attrs = attr;
     cfg.numAttrs = g_pdl.load() ? 1 : 0;
     LG_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    note_launch("gemv_reg_kernel", grid);
     LG_CUDA(cudaGetLastError());
     return LUTGEMM_OK;
 }
@@ -466,7 +488,7 @@ int launch_gemv_tma2(const lutgemm_weight* w, const lg::Gemv22Params& p, dim3 gr
     cfg.attrs = attr;
     cfg.numAttrs = g_pdl.load() ? 1 : 0;
     LG_CUDA(cudaLaunchKernelEx(&cfg, kern, w->tmW, w->tmA, p));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    note_launch("gemv_tma2_kernel", grid);
     LG_CUDA(cudaGetLastError());
     return LUTGEMM_OK;
 }
@@ -515,7 +537,7 @@ int gemv_row(const lutgemm_weight* w, const lutgemm_workspace* ws, const __half*
     }
     dim3 grid((w->N + 127) / 128);
     lg::gemv_generic_kernel<<<grid, 128, 0, st>>>(w->bW, w->alpha, w->q_bias, x, y16, y32, w->N, w->K, w->q, w->g);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    note_launch("gemv_generic_kernel", grid);
     LG_CUDA(cudaGetLastError());
     return LUTGEMM_OK;
 }
@@ -542,7 +564,7 @@ int launch_gemm_tc_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::
     cfg.attrs = attr;
     cfg.numAttrs = g_pdl.load() ? 1 : 0;
     LG_CUDA(cudaLaunchKernelEx(&cfg, kern, tmX, w->tmWtc, w->tmAtc, w->tmQtc, p));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    note_launch("gemm_tc_kernel", grid);
     LG_CUDA(cudaGetLastError());
     return LUTGEMM_OK;
 }
@@ -644,10 +666,10 @@ int hl_rows_for(int N, int m) {
 // q = 1, 256 rows two k-ranges: 21.2 us (14.5 unsplit), and 11008 x 4096, q = 4, 256 rows three: 54.3 (44.5).  Of 942 calls
 // at 14 widths 214 got faster by more than 3 % and 17 slower, the most 5120 x 5120, q = 2, 400 rows: 51.7 (46.4).
 // The plan with the smallest estimate is taken: whole items, halves, whole items
-// with a last partial wave of halves, each with 1 to 8 k-ranges.
+// with a last partial wave of halves, each with 1 to 8 k-ranges.  Returns the estimate.
 constexpr double kHlRowCycles = 2.18, kHlExpCycles = 630, kHlEntryCycles = 8.5, kHlBiasCycles = 14.5;
 constexpr double kHlCtaCycles = 6300, kHlSplitCycles = 4400, kHlSplitRowCycles = 30;
-void hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) {
+double hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) {
     const int sms = sm_count();
     const int T = (w->N + lg::kHlCols - 1) / lg::kHlCols, RT = (m + lg::kHlRows - 1) / lg::kHlRows;
     const long long items = (long long)T * RT;
@@ -687,6 +709,7 @@ void hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) {
             if (c == 1 && tail_full > 0 && tail_full < items) consider(tail_full, 2 * (items - tail_full), 1);
         }
     }
+    return best;
 }
 
 // From which row count the split-operand kernel is the faster one: it always takes two tensor-core passes, gemm_tc one
@@ -700,10 +723,8 @@ bool gemm_hl_ok(const lutgemm_weight* w, int m) {
     return w->tc_ok && w->q <= 4 && m >= from && (m > 128 || w->g >= lg::kHlStepK);
 }
 
-// Whether the workspace has at least `rows` fp32 rows of w's width.
-bool have_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, int rows) {
-    return (long long)ws->tc_rows * ws->n_cap >= (long long)rows * w->N;
-}
+// fp32 rows of w's width that the workspace has.
+long long rows_there(const lutgemm_weight* w, const lutgemm_workspace* ws) { return (long long)ws->tc_rows * ws->n_cap / w->N; }
 
 template <int Q>
 int launch_gemm_hl_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::HlParams& p, dim3 grid, cudaStream_t st) {
@@ -727,22 +748,18 @@ int launch_gemm_hl_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::
     cfg.attrs = attr;
     cfg.numAttrs = g_pdl.load() ? 1 : 0;
     LG_CUDA(cudaLaunchKernelEx(&cfg, kern, tmX, p));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    note_launch("gemm_hl_kernel", grid);
     LG_CUDA(cudaGetLastError());
     return LUTGEMM_OK;
 }
 
-// Rows [0, m) through the split-operand kernel, one launch (gemm_hl_ok holds).
-int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __half* y16, float* y32, int m, cudaStream_t st) {
+// Rows [0, m) through the split-operand kernel, one launch.
+int gemm_hl_launch(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __half* y16, float* y32, int m, bool may_split,
+                   cudaStream_t st) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return LUTGEMM_ERR_CUDA;
-    // Scratch is allocated, and what a call without reserved scratch is told is decided, by the plane kernel's rule for its
-    // first launch, whatever kernel runs: a container with scratch for 128 rows never allocates again in a call.
-    int unused_split = 1, unused_steps = 0;
-    const int rc = tc_split(w, ws, m < 128 ? m : 128, hl_rows_for(w->N, m), st, &unused_split, &unused_steps);
-    if (rc != LUTGEMM_OK) return rc;
     lg::HlParams p = {};
-    hl_plan(w, m, !ordered_for(ws) && have_rows(w, ws, m), &p);
+    hl_plan(w, m, may_split, &p);
     p.box_rows = m < lg::kHlBoxRows ? (m + 15) / 16 * 16 : lg::kHlBoxRows;
     p.x_slot_bytes = (m <= lg::kHlBoxRows || p.full_items == 0 ? 1 : 2) * p.box_rows * 128;
     p.x_slots = lg::kHlXBudget / p.x_slot_bytes;
@@ -771,6 +788,39 @@ int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
         case 4: return launch_gemm_hl_q<4>(w, tmX, p, grid, st);
     }
     return LUTGEMM_ERR_BITS;
+}
+
+// Rows [0, m), gemm_hl_ok(w, m) holds: one launch, which may split k when the workspace has fp32 rows for all of m.  When it
+// has fewer (a captured call above the reserved batch, a small explicit workspace), either one launch without k-ranges or as
+// many rows at a time as there are; a piece that gemm_tc is the faster for goes there.  Pieces are taken where the model puts
+// them below 0.78 of the one launch: measured at 128 rows a piece, 1024 x 8192, q = 4 + q_bias, 300 rows 38.0 / 59.0 us, 4096 x
+// 11008, q = 1, 256 rows 41.9 / 59.7; above that line 1536 x 4096, q = 1, 256 rows 28.7 / 24.2.
+int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __half* y16, float* y32, int m, cudaStream_t st) {
+    // Scratch is allocated, and what a call without reserved scratch is told is decided, by the plane kernel's rule for its
+    // first launch, whatever kernel runs: a container with scratch for 128 rows never allocates again in a call.
+    int unused_split = 1, unused_steps = 0;
+    int rc = tc_split(w, ws, m < 128 ? m : 128, hl_rows_for(w->N, m), st, &unused_split, &unused_steps);
+    if (rc != LUTGEMM_OK) return rc;
+    const bool ordered = ordered_for(ws);
+    const long long there = rows_there(w, ws);
+    const int piece = there < hl_rows_for(w->N, m) ? (int)(there / 128 * 128) : m;
+    if (!ordered && piece >= 128 && piece < m) {
+        lg::HlParams p = {};
+        double pieces = (m / piece) * hl_plan(w, piece, true, &p);
+        if (m % piece) pieces += hl_plan(w, m % piece, true, &p);
+        if (pieces < 0.78 * hl_plan(w, m, false, &p)) {
+            for (int r0 = 0; r0 < m; r0 += piece) {
+                const int rows = m - r0 < piece ? m - r0 : piece;
+                const __half* xr = x + (size_t)r0 * w->K;
+                __half* y16r = y16 ? y16 + (size_t)r0 * w->N : nullptr;
+                float* y32r = y32 ? y32 + (size_t)r0 * w->N : nullptr;
+                rc = gemm_hl_ok(w, rows) ? gemm_hl_launch(w, ws, xr, y16r, y32r, rows, true, st) : gemm_tc_rows(w, ws, xr, y16r, y32r, rows, st);
+                if (rc != LUTGEMM_OK) return rc;
+            }
+            return LUTGEMM_OK;
+        }
+    }
+    return gemm_hl_launch(w, ws, x, y16, y32, m, !ordered && there >= m, st);
 }
 
 // ---- register-operand kernel (gemm_frag.cuh): plan, launch ----
@@ -826,7 +876,7 @@ int launch_gemm_frag(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, 
     cfg.attrs = attr;
     cfg.numAttrs = g_pdl.load() ? 1 : 0;
     LG_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    note_launch("gemm_frag_kernel", grid);
     LG_CUDA(cudaGetLastError());
     return LUTGEMM_OK;
 }
@@ -865,7 +915,7 @@ int launch_gemm_i8_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::
     cfg.attrs = attr;
     cfg.numAttrs = g_pdl.load() ? 1 : 0;
     LG_CUDA(cudaLaunchKernelEx(&cfg, kern, tmX, w->tmWtc, w->tmAtc, w->tmQtc, p));
-    g_launches.fetch_add(1, std::memory_order_relaxed);
+    note_launch("gemm_i8_kernel", grid);
     LG_CUDA(cudaGetLastError());
     return LUTGEMM_OK;
 }
@@ -942,7 +992,7 @@ int frag_rows_if_ready(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x
         const int rc = tc_split(w, ws, m < 128 ? m : 128, m, st, &unused_split, &unused_steps);
         if (rc != LUTGEMM_OK) return rc;
     }
-    if (((whole && grid[0].y > 1) || (rest && grid[1].y > 1)) && !have_rows(w, ws, whole ? lg::kFrMaxRows : m)) return LUTGEMM_OK;
+    if (((whole && grid[0].y > 1) || (rest && grid[1].y > 1)) && rows_there(w, ws) < (whole ? lg::kFrMaxRows : m)) return LUTGEMM_OK;
     *taken = true;
     for (int r0 = 0; r0 < m; r0 += lg::kFrMaxRows) {
         const int rows = m - r0 < lg::kFrMaxRows ? m - r0 : lg::kFrMaxRows, i = rows == lg::kFrMaxRows ? 0 : 1;
@@ -2142,6 +2192,12 @@ int lutgemm_set_dependent_launch(int enabled) {
 }
 
 int lutgemm_last_cuda_error(void) { return g_last_cuda; }
+const char* lutgemm_last_launch(int* grid_x, int* grid_y) {
+    if (grid_x) *grid_x = (int)g_last_grid.x;
+    if (grid_y) *grid_y = (int)g_last_grid.y;
+    return g_last_kernel;
+}
+
 unsigned long long lutgemm_kernel_launch_count(void) { return g_launches.load(); }
 int lutgemm_set_gemv_ntile(int columns) {
     if (columns < 0) return LUTGEMM_ERR_SHAPE;

@@ -114,3 +114,43 @@ def test_rising_batches_do_not_allocate_once_128_rows_are_there():
         _eager(w, bW, alpha, m, m)
         assert w.scratch() == before
     w.close()
+
+
+@pytest.mark.parametrize("m", [16, 130, 256, 512])
+@pytest.mark.parametrize("max_n", [N, 5 * N])
+def test_explicit_workspace_runs_the_plan_of_the_containers_own(m, max_n):
+    """A workspace of the same batch has the rows for the same k-ranges, for its own width and for narrower containers."""
+    w, bW, alpha = _container()
+    w.reserve_batch(m)
+    x = synth.activations(m, K, seed=m)
+    y = torch.empty((m, N), dtype=torch.float16, device="cuda")
+    L.matmul(y, _device(x), w, m)
+    own = L.last_launch()
+    assert own[2] > 1                                     # k-ranges: the shape is one that needs the rows
+    ws = L.Workspace(max_n, K, m)
+    for _ in range(2):                                    # the second call finds the workspace as the first one left it
+        y.zero_()
+        L.matmul(y, _device(x), w, m, workspace=ws)
+        assert L.last_launch() == own
+        _close(y.cpu().numpy(), x, bW, alpha)
+    assert ws.status() == 0
+    ws.close()
+    w.close()
+
+
+@pytest.mark.parametrize("q,m", [(1, 256), (2, 130), (4, 300), (4, 129), (1, 513)])
+def test_captured_call_above_the_reserved_rows(q, m):
+    """Fewer rows than the call's: some rows at a time or no k-ranges, the outputs the same, and nothing allocated."""
+    bW, alpha, _ = synth.bcq_layer(N, K, q, G, seed=q)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // G).reserve_batch(128)
+    before = w.scratch()
+    x = synth.activations(m, K, seed=m)
+    graph, y, xd = _capture(w, x, m)
+    for _ in range(2):
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        _close(y.cpu().numpy(), x, bW, alpha.astype(np.float16))
+    assert w.scratch() == before
+    del graph
+    w.close()
