@@ -69,6 +69,7 @@ struct lutgemm_weight {
     // q_bias box {256, groups per 128 k} (valid when tc_ok)
     CUtensorMap tmWtc, tmAtc, tmQtc;
     bool tc_ok = false;
+    int hl_split_rows = 0;     // largest batch that the split-operand kernel's plan cuts into k-ranges
     // staging for lutgemm_matmul_host
     void* h_stage_in = nullptr;
     void* d_stage_in = nullptr;
@@ -278,7 +279,7 @@ int tc_rows_for(int m) {
 int sm_count();
 
 // Rows of N columns for an explicit workspace that serves every width up to N and batches up to m.  The split-operand kernel
-// asks for rows of its call's width (hl_rows_for): the most elements over all widths, in tiles of 128 columns.
+// asks for rows of its call's width (hl_split_rows_of): the most elements over all widths, in tiles of 128 columns.
 int workspace_rows_for(int N, int m) {
     long long elements = (long long)tc_rows_for(m) * N;
     for (int t = 1; t <= (N + lg::kHlCols - 1) / lg::kHlCols && t < sm_count(); t++) {
@@ -569,7 +570,11 @@ int launch_gemm_tc_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::
     return LUTGEMM_OK;
 }
 
-int hl_rows_for(int N, int m);
+// fp32 rows for a batch of m: the plane kernel's, and for a batch that the split-operand kernel cuts into k-ranges all of them.
+int batch_rows_for(const lutgemm_weight* w, int m) {
+    const int rows = m < w->hl_split_rows ? m : w->hl_split_rows;
+    return rows > tc_rows_for(m) ? rows : tc_rows_for(m);
+}
 
 // Split-k plan of a batched launch (256-column tiles x k-ranges of whole 128-k steps) and, when it splits, the fp32
 // reduction rows of the workspace: at least m, and `rows` where they have to be allocated anyway (for the kernels that ask
@@ -597,7 +602,7 @@ int tc_split(lutgemm_weight* w, lutgemm_workspace* ws, int m, int rows, cudaStre
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone) return LUTGEMM_ERR_BATCH;
         const int need = tc_rows_for(m);
-        const int rc = grow_tc_rows(ws, rows > need ? rows : need, need, hl_rows_for(w->N, kMaxBatch), st);
+        const int rc = grow_tc_rows(ws, rows > need ? rows : need, need, batch_rows_for(w, kMaxBatch), st);
         if (rc != LUTGEMM_OK) return rc;
     }
     *splitk_out = splitk;
@@ -648,15 +653,6 @@ int gemm_tc_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 }
 
 // ---- split-operand kernel (gemm_hl.cuh): plan, launch ----
-// fp32 workspace rows (of N columns) that a batch of m can ask for: split-k is only planned while the output has fewer
-// than about one tile of 128 x 256 per SM, which bounds it to some 20 MB.
-int hl_rows_for(int N, int m) {
-    const int T = (N + lg::kHlCols - 1) / lg::kHlCols;
-    const int cap = lg::kHlRows * (sm_count() / T + 1);
-    const int rows = m < cap ? m : cap;
-    return rows > tc_rows_for(m) ? rows : tc_rows_for(m);
-}
-
 // One CTA per SM: an item is 128 columns x 256 rows, and an item may be cut into two halves of 128 rows or into k-ranges.
 // Cost model in cycles: a block of 64 k takes the tensor pipe and shared memory kHlRowCycles per row and pass, and the
 // expansion kHlExpCycles whatever the rows, more with more table entries; a CTA's start, first loads and epilogue add
@@ -710,6 +706,26 @@ double hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) 
         }
     }
     return best;
+}
+
+// Largest batch (in steps of 16 rows) that the plan cuts into k-ranges; 0 for containers that the kernel does not take.  k is
+// split only while there are fewer items than SMs, which bounds the rows (148 SMs: 256 at 8192 x 8192, 8.4 MB of fp32; 256 or
+// 512 at 4096 x 4096; none from 18944 columns on; at most some 13 MB).
+int hl_split_rows_of(const lutgemm_weight* w) {
+    if (!w->tc_ok || w->q > 4) return 0;
+    const int T = (w->N + lg::kHlCols - 1) / lg::kHlCols;
+    const int cap = lg::kHlRows * ((sm_count() - 1) / T);
+    lg::HlParams p = {};
+    auto splits = [&](int m) {
+        hl_plan(w, m, true, &p);
+        return p.splits > 1;
+    };
+    int coarse = cap;
+    while (coarse > 0 && !splits(coarse)) coarse -= 128;
+    int rows = coarse;
+    for (int m = coarse + 16; m < coarse + 128 && m < cap; m += 16)
+        if (splits(m)) rows = m;
+    return rows;
 }
 
 // From which row count the split-operand kernel is the faster one: it always takes two tensor-core passes, gemm_tc one
@@ -799,11 +815,11 @@ int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
     // Scratch is allocated, and what a call without reserved scratch is told is decided, by the plane kernel's rule for its
     // first launch, whatever kernel runs: a container with scratch for 128 rows never allocates again in a call.
     int unused_split = 1, unused_steps = 0;
-    int rc = tc_split(w, ws, m < 128 ? m : 128, hl_rows_for(w->N, m), st, &unused_split, &unused_steps);
+    int rc = tc_split(w, ws, m < 128 ? m : 128, batch_rows_for(w, m), st, &unused_split, &unused_steps);
     if (rc != LUTGEMM_OK) return rc;
     const bool ordered = ordered_for(ws);
     const long long there = rows_there(w, ws);
-    const int piece = there < hl_rows_for(w->N, m) ? (int)(there / 128 * 128) : m;
+    const int piece = there < batch_rows_for(w, m) ? (int)(there / 128 * 128) : m;
     if (!ordered && piece >= 128 && piece < m) {
         lg::HlParams p = {};
         double pieces = (m / piece) * hl_plan(w, piece, true, &p);
@@ -1120,6 +1136,7 @@ int finish_create(lutgemm_weight* w, lutgemm_weight_t* out) {
         lutgemm_weight_destroy(w);
         return rc;
     }
+    w->hl_split_rows = hl_split_rows_of(w);
     *out = w;
     return LUTGEMM_OK;
 }
@@ -1329,10 +1346,10 @@ int lutgemm_weight_reserve_batch(lutgemm_weight_t w, int m) {
     if (!w) return LUTGEMM_ERR_NULL;
     if (m < 1 || m > kMaxBatch) return LUTGEMM_ERR_BATCH;
     lutgemm_workspace* ws = &w->own;
-    const int rows = hl_rows_for(w->N, m);
+    const int rows = batch_rows_for(w, m);
     int rc = LUTGEMM_OK;
     if (m >= 2 && ws->tc_rows < rows) {
-        rc = grow_tc_rows(ws, rows, rows, hl_rows_for(w->N, kMaxBatch), nullptr);
+        rc = grow_tc_rows(ws, rows, rows, batch_rows_for(w, kMaxBatch), nullptr);
         if (rc != LUTGEMM_OK) return rc;
         LG_CUDA(cudaStreamSynchronize(nullptr));       // zeroed before a call on a stream that does not wait for this one
     }

@@ -154,3 +154,34 @@ def test_captured_call_above_the_reserved_rows(q, m):
     assert w.scratch() == before
     del graph
     w.close()
+
+
+@pytest.mark.parametrize("n,k,q,rows", [(24576, 512, 1, 128), (24576, 512, 4, 128), (1000, 1024, 5, 128), (1004, 1024, 3, 128),
+                                        (8192, 8192, 4, 512)])
+def test_reserved_rows_are_bounded_by_what_a_plan_can_ask_for(n, k, q, rows):
+    """Wide outputs never split beyond 128 rows, five planes and containers without a tensor-core kernel neither."""
+    bW, alpha, _ = synth.bcq_layer(n, k, q, 128, seed=q)
+    w = L.nQWeight_fp16(bW, alpha, k, n, q, False, k // 128).reserve_batch(2048)
+    assert w.scratch()[1] <= rows * n * 4
+    w.close()
+
+
+@pytest.mark.parametrize("q", [1, 3])
+def test_reserved_rows_are_enough_for_every_plan(q):
+    """Every batch up to the reserved one runs the plan that it has with far more rows than any call can use."""
+    n, k = 2048, 2048
+    bW, alpha, _ = synth.bcq_layer(n, k, q, 128, seed=q)
+    w = L.nQWeight_fp16(bW, alpha, k, n, q, False, k // 128).reserve_batch(2048)
+    plenty = L.Workspace(64 * n, k, 2048)
+    x = _device(synth.activations(2048, k, seed=1))
+    y = torch.empty((2048, n), dtype=torch.float16, device="cuda")
+    split = 0
+    for m in [*range(100, 700, 37), 256, 512, 768, 1024, 1500, 2048]:
+        L.matmul(y, x, w, m, workspace=plenty)
+        free = L.last_launch()
+        L.matmul(y, x, w, m)
+        assert L.last_launch() == free, m
+        split += m > 128 and free[2] > 1
+    assert split > 0
+    plenty.close()
+    w.close()
