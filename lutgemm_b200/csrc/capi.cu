@@ -791,7 +791,7 @@ int gemm_hl_launch(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return LUTGEMM_ERR_CUDA;
     }
-    p.bW = w->bW; p.alpha = w->alpha; p.q_bias = w->q_bias;
+    p.bW = w->bW; p.alpha = w->alpha; p.q_bias = w->q_bias; p.x = x;
     p.partial = ws->tc_partial; p.counters = ws->counters; p.status = ws->status;
     p.y16 = y16; p.y32 = y32;
     p.N = w->N; p.K = w->K; p.G = w->G; p.g = w->g; p.m = m;

@@ -3,10 +3,13 @@
 // gemm_tc.cuh multiplies every bit plane by itself: q (or q + 1 with q_bias) tensor-core passes over the activations.
 // Inside a scale group a weight takes only 2^q values, W = q_bias + sum_b +-alpha_b, so here each column's values are
 // computed once per group in fp32, split as hi + lo (two fp16 numbers, lo = fp16(W - hi)) and the packed bits only
-// choose between them: two passes whatever q is, and no rounding of the weight beyond 2^-22 of it.  So that lo never
-// falls into fp16's subnormals (and hi never overflows) a CTA scales every column by a power of two taken from the
-// largest scale of that column in the CTA's k-range, and takes it out again in the epilogue.  (One plane without q_bias
-// is exact as it is: one pass, no lo.)
+// choose between them: two passes whatever q is, and no rounding of the weight beyond 2^-22 of it.  So that hi never
+// overflows a CTA scales every column by a power of two taken from the largest scale of that column in the CTA's k-range,
+// and takes it out again in the epilogue.  Every W is a multiple of the last place of its group's smallest scale, at least
+// 2^-24: scaled up, or left as it is (largest scale below 8192), lo's last place is no coarser than that and nothing is lost
+// to fp16's subnormals.  Scaled down it may be, where a column has a scale of 8192 or more and one so small that its last
+// place falls below 2^-24: the epilogue computes such a column anew, product by product.  (One plane without q_bias is exact
+// as it is: one pass, no lo.)
 //
 //   CTA = 128 output columns x up to 256 activation rows x a k-range, walked in blocks of 64 k.
 //   16 expansion warps: warp (quarter lq of the columns, sub) takes the blocks j with j mod 4 == sub.  Lane = column.  The
@@ -49,6 +52,7 @@ struct HlParams {
     const uint32_t* bW;      // [K/32][q][N]
     const __half* alpha;     // [G][q][N]
     const __half* q_bias;    // [G][N] or nullptr
+    const __half* x;         // [m][K], what tmX describes
     float* partial;          // [m][N] fp32, zero between launches (split-k only)
     unsigned* counters;      // one per output tile, zero between launches
     int* status;
@@ -96,10 +100,43 @@ __device__ __forceinline__ void hl_pack_pair(float v0, float v1, uint32_t& e0, u
     e1 = prmt_b32(h, l, 0x7632u);
 }
 
+// Groups that the k-range [k0, k1) touches in this column: is the last place of some scale, times 2^(12 - e) with e the
+// exponent of the column's largest (`max_bits`, 8192 or more), below 2^-24?
+template <int Q, bool BIAS>
+__device__ __noinline__ bool hl_has_tiny_scale(const HlParams& p, int col, int k0, int k1, unsigned max_bits) {
+    unsigned least = 0x7c00u;
+    for (int grp = k0 / p.g; grp * p.g < k1; grp++)
+        for (int b = 0; b < Q + (BIAS ? 1 : 0); b++) {
+            const __half* src = b < Q ? p.alpha + ((size_t)grp * Q + b) * p.N : p.q_bias + (size_t)grp * p.N;
+            const unsigned bits = __half_as_ushort(src[col]) & 0x7fffu;
+            if (bits != 0u && bits < least) least = bits;
+        }
+    return (max_bits >> 10) - max(1u, least >> 10) > 26u;
+}
+// One output as the planes give it: products of +-alpha_b (and q_bias) with the activation, which are exact, summed in
+// fp32, 32 k of a plane at a time.  Lane = column; every lane reads the same activations.
+template <int Q, bool BIAS>
+__device__ __noinline__ float hl_by_product(const HlParams& p, int row, int col, int k0, int k1) {
+    const __half* x = p.x + (size_t)row * p.K;
+    float sum = 0.f;
+    for (int k = k0; k < k1; k += 32) {
+        const size_t grp = k / p.g;
+        for (int b = 0; b < Q + (BIAS ? 1 : 0); b++) {
+            const uint32_t w = b < Q ? __ldg(p.bW + ((size_t)(k >> 5) * Q + b) * p.N + col) : 0xffffffffu;
+            const float a = __half2float(b < Q ? p.alpha[(grp * Q + b) * p.N + col] : p.q_bias[grp * p.N + col]);
+            float s = 0.f;
+#pragma unroll 8
+            for (int i = 0; i < 32; i++) s = fmaf((w >> i) & 1u ? a : -a, __half2float(x[k + i]), s);
+            sum += s;
+        }
+    }
+    return sum;
+}
+
 // Q: number of bit planes (1..4); BIAS: container has q_bias.  tmX: 2-D map {K, m} of fp16, box {64, box_rows}, 128-byte swizzle.
 template <int Q, bool BIAS>
 __global__ void __launch_bounds__(kHlThreads, 1)
-gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
+gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ HlParams p) {
     constexpr int NV = 1 << Q;
     constexpr int PASSES = (Q == 1 && !BIAS) ? 1 : 2;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -232,15 +269,15 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
             }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kHlExpWarps * 32) : "memory");
-        // |W| <= (Q + 1) max < 2^(e + 4) with e = exponent of max: the scale 2^(11 - e) keeps |W| below 2^15.  All
-        // zero, or not finite: 1 (the column's result is not finite either).
+        // |W| <= (Q + 1) max < 5 * 2^(e + 1) with e = exponent of max: the scale 2^(12 - e) keeps |W| below 40960.  One
+        // pass needs none (W = +-alpha).  All zero, or not finite: 1 (the column's result is not finite either).
         float scale = 1.f;
         {
             const unsigned mbits = s_max[col_l];
-            if (mbits != 0u && mbits < 0x7c00u) {
+            if (PASSES == 2 && mbits != 0u && mbits < 0x7c00u) {
                 const int e = (int)(__float_as_uint(__half2float(__ushort_as_half((unsigned short)mbits))) >> 23) - 127;
-                scale = __uint_as_float((uint32_t)(127 + 11 - e) << 23);
-                unscale = __uint_as_float((uint32_t)(127 - 11 + e) << 23);
+                scale = __uint_as_float((uint32_t)(127 + 12 - e) << 23);
+                unscale = __uint_as_float((uint32_t)(127 - 12 + e) << 23);
             }
         }
         // table entry of code c at (pair << 12) + (c << 8) + bank: the code byte carries the pair in its high nibble
@@ -411,12 +448,31 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const HlParams p) {
         const uint32_t t_src = tmem_base + ((uint32_t)(lq * 32) << 16);
         // the activation ring is idle: every load has been consumed when the accumulators are complete
         float* scratch = reinterpret_cast<float*>(smem + kHlXOff) + ew * (16 * 33);
+        // columns that the split operand does not hold exactly (not finite: nothing to be exact about)
+        const int k0 = blk_begin * kHlStepK, k1 = min(p.K, (blk_begin + nblk) * kHlStepK), col_c = min(col, N - 1);
+        bool wide = false;
+        if (PASSES == 2) {
+            const unsigned max_bits = s_max[col_l];
+            if (max_bits >= 0x7000u && max_bits < 0x7c00u) wide = hl_has_tiny_scale<Q, BIAS>(p, col_c, k0, k1, max_bits);
+        }
+        const bool any_wide = __any_sync(0xffffffffu, wide);
         for (int c = sub; 16 * c < rows && ok; c += 4) {          // 16 activation rows per tcgen05.ld; warp-uniform
             uint32_t r[16];
             tmem_ld_x16(t_src + 16u * (uint32_t)c, r);
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) * unscale);
+            if (PASSES == 2 && any_wide) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) scratch[i * 33 + lane] = __uint_as_float(r[i]);
+#pragma unroll 1
+                for (int i = 0; i < 16 && 16 * c + i < rows; i++) {
+                    const float v = hl_by_product<Q, BIAS>(p, row0 + 16 * c + i, col_c, k0, k1);
+                    if (wide) scratch[i * 33 + lane] = v;
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i++) r[i] = __float_as_uint(scratch[i * 33 + lane]);
+            }
             tc_store_block(scratch, r, lane, row0 + 16 * c, n0 + lq * 32, row0 + rows, N, split, p.partial, p.y16, p.y32);
         }
         tc_fence_before_sync();

@@ -96,3 +96,50 @@ def test_three_rows_without_reserved_scratch_inside_a_capture():
     ref = oracle.bcq_matmul_f64(x, bW, alpha.astype(np.float16), None, g)
     assert np.linalg.norm(y.cpu().numpy() - ref) <= 1e-5 * np.linalg.norm(ref)
     w.close()
+
+
+def _far_apart_in_a_column(N, K, q, g, bias, m):
+    """Scales whose exponents differ from group to group of one column from one end of fp16 to the other; activations are zero
+    wherever some column's scales are large, so that what the outputs consist of are the products with the small ones."""
+    rng = np.random.default_rng(N + K + q)
+    bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + K + m, with_bias=bias)
+    G = K // g
+    large = np.arange(G) % 2 == 0
+    e = np.where(large[:, None], 30000.0 / (q + 1), 2.0 ** rng.integers(-22, -15, (G, 1))) * np.ones((G, N))
+    # two columns of each eight have no scale of 8192 or more, one neither large nor small ones
+    e[:, 5::8] = np.where(large[:, None], 2.0 ** -3, e[:, 5::8])
+    e[:, 6::8] = np.where(large[:, None], 2.0 ** 10, e[:, 6::8])
+    e[:, 7::8] = 1.0
+    draw = lambda shape: np.abs(rng.normal(1.0, 0.3, shape)) + 0.01
+    alpha = (draw((G, q, N)) * e[:, None, :])
+    alpha[large, 0, ::8] = 40000.0
+    alpha = alpha.astype(np.float16).astype(np.float32)
+    if bias:
+        q_bias = (draw((G, N)) * e * np.where(rng.random((G, N)) < 0.5, -1, 1)).astype(np.float16).astype(np.float32)
+    x = synth.activations(m, K, seed=m)
+    x.reshape(m, G, g)[:, large, :] = 0
+    return bW, alpha, q_bias, x
+
+
+@pytest.mark.parametrize("N,K,q,g,bias,m", [
+    (264, 1024, 4, 64, True, 64), (264, 1024, 2, 64, False, 130), (136, 2048, 1, 128, False, 200), (128, 512, 1, 32, True, 257),
+    (1032, 4096, 3, 256, True, 129)])
+def test_split_operand_kernel_scales_far_apart_within_a_column(N, K, q, g, bias, m):
+    bW, alpha, q_bias, x = _far_apart_in_a_column(N, K, q, g, bias, m)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g, q_bias).reserve_batch(m)
+    xd = torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
+    y = torch.empty((m, N), dtype=torch.float32, device="cuda")
+    L.matmul_f32(y, xd, w, m)
+    assert L.last_launch()[0] == "gemm_hl_kernel"
+    a16, b16 = alpha.astype(np.float16), None if q_bias is None else q_bias.astype(np.float16)
+    ref = oracle.bcq_matmul_f64(x, bW, a16, b16, g)
+    mag = np.abs(a16.astype(np.float64)).sum(1) + (0 if b16 is None else np.abs(b16.astype(np.float64)))
+    size = np.abs(x.astype(np.float64)).reshape(m, K // g, g).sum(2) @ mag
+    # fp32 sums as in _run, with weights (2^-22) instead of products with offsets
+    bound = ((2 * K / 16 + 64) * 2.0 ** -23 + 2.0 ** -22) * size + 1e-30
+    err = np.abs(y.cpu().numpy().astype(np.float64) - ref)
+    assert (err <= bound).all(), (err / bound).max()
+    # the same per column in the 2-norm, where partial sums of terms of either sign are no larger than the whole (1.5: the
+    # spread over 64 rows or more)
+    assert (np.linalg.norm(err, axis=0) <= 1.5 * ((2 * K / 16 + 64) * 2.0 ** -23 + 2.0 ** -22) * np.linalg.norm(ref, axis=0)).all()
+    w.close()
