@@ -8,7 +8,8 @@
 // and takes it out again in the epilogue.  Every W is a multiple of the last place of its group's smallest scale, at least
 // 2^-24: scaled up, or left as it is (largest scale below 8192), lo's last place is no coarser than that and nothing is lost
 // to fp16's subnormals.  Scaled down it may be, where a column has a scale of 8192 or more and one so small that its last
-// place falls below 2^-24: the epilogue computes such a column anew, product by product.  (One plane without q_bias is exact
+// place falls below 2^-24: the epilogue computes such a column anew, product by product.  It does the same for what is not
+// finite in a row with an infinite activation: hi * inf + lo * inf has not the planes' signs.  (One plane without q_bias is exact
 // as it is: one pass, no lo.)
 //
 //   CTA = 128 output columns x up to 256 activation rows x a k-range, walked in blocks of 64 k.
@@ -112,6 +113,18 @@ __device__ __noinline__ bool hl_has_tiny_scale(const HlParams& p, int col, int k
             if (bits != 0u && bits < least) least = bits;
         }
     return (max_bits >> 10) - max(1u, least >> 10) > 26u;
+}
+// Whether this row's activations in [k0, k1) have an infinity, a NaN.  Called by a whole warp.
+__device__ __noinline__ void hl_row_class(const HlParams& p, int row, int k0, int k1, int lane, bool* inf, bool* nan) {
+    unsigned most = 0u;
+    bool any_inf = false;
+    for (int k = k0 + lane; k < k1; k += 32) {
+        const unsigned bits = __half_as_ushort(p.x[(size_t)row * p.K + k]) & 0x7fffu;
+        any_inf |= bits == 0x7c00u;
+        most = max(most, bits);
+    }
+    *inf = __any_sync(0xffffffffu, any_inf);
+    *nan = __any_sync(0xffffffffu, most > 0x7c00u);
 }
 // One output as the planes give it: products of +-alpha_b (and q_bias) with the activation, which are exact, summed in
 // fp32, 32 k of a plane at a time.  Lane = column; every lane reads the same activations.
@@ -270,12 +283,13 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kHlExpWarps * 32) : "memory");
         // |W| <= (Q + 1) max < 5 * 2^(e + 1) with e = exponent of max: the scale 2^(12 - e) keeps |W| below 40960.  One
-        // pass needs none (W = +-alpha).  All zero, or not finite: 1 (the column's result is not finite either).
+        // pass needs none (W = +-alpha).  All zero: 1.  Not finite: the column's result is not finite either, and the
+        // scale for e = 15 keeps the finite weights beside it finite.
         float scale = 1.f;
         {
             const unsigned mbits = s_max[col_l];
-            if (PASSES == 2 && mbits != 0u && mbits < 0x7c00u) {
-                const int e = (int)(__float_as_uint(__half2float(__ushort_as_half((unsigned short)mbits))) >> 23) - 127;
+            if (PASSES == 2 && mbits != 0u) {
+                const int e = mbits >= 0x7c00u ? 15 : (int)(__float_as_uint(__half2float(__ushort_as_half((unsigned short)mbits))) >> 23) - 127;
                 scale = __uint_as_float((uint32_t)(127 + 12 - e) << 23);
                 unscale = __uint_as_float((uint32_t)(127 - 12 + e) << 23);
             }
@@ -462,13 +476,20 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) * unscale);
-            if (PASSES == 2 && any_wide) {
+            unsigned redo = wide ? 0xffffu : 0u;
+#pragma unroll
+            for (int i = 0; i < 16; i++) redo |= (r[i] & 0x7f800000u) == 0x7f800000u ? 1u << i : 0u;
+            if (PASSES == 2 && __any_sync(0xffffffffu, redo != 0u)) {
 #pragma unroll
                 for (int i = 0; i < 16; i++) scratch[i * 33 + lane] = __uint_as_float(r[i]);
 #pragma unroll 1
                 for (int i = 0; i < 16 && 16 * c + i < rows; i++) {
+                    if (!__any_sync(0xffffffffu, (redo >> i) & 1u)) continue;
+                    bool inf, nan;
+                    hl_row_class(p, row0 + 16 * c + i, k0, k1, lane, &inf, &nan);
+                    if (nan || !(inf || any_wide)) continue;      // NaN: so is the row; finite: a scale is not, and that is right
                     const float v = hl_by_product<Q, BIAS>(p, row0 + 16 * c + i, col_c, k0, k1);
-                    if (wide) scratch[i * 33 + lane] = v;
+                    if (((redo >> i) & 1u) && (inf || wide)) scratch[i * 33 + lane] = v;
                 }
 #pragma unroll
                 for (int i = 0; i < 16; i++) r[i] = __float_as_uint(scratch[i * 33 + lane]);

@@ -143,3 +143,52 @@ def test_split_operand_kernel_scales_far_apart_within_a_column(N, K, q, g, bias,
     # spread over 64 rows or more)
     assert (np.linalg.norm(err, axis=0) <= 1.5 * ((2 * K / 16 + 64) * 2.0 ** -23 + 2.0 ** -22) * np.linalg.norm(ref, axis=0)).all()
     w.close()
+
+
+def _not_finite(N, K, q, g, bias, m, kernel):
+    """Rows with an infinite activation give what the planes give, +-alpha_b * x summed: an infinity where all planes of
+    that weight agree in sign, else NaN; NaN rows are NaN, and the other rows do not notice."""
+    bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + K + m, with_bias=bias)
+    alpha = np.maximum(alpha, 2.0 ** -10)                 # 0 * inf would be NaN in every column
+    x = synth.activations(m, K, seed=m)
+    clean = x.copy()
+    x[0, K // 3] = np.inf
+    x[2, K - 1] = -np.inf
+    x[m - 1, 0], x[m - 1, K // 2] = np.inf, -np.inf
+    x[1, K // 2] = np.nan
+    touched = [0, 1, 2, m - 1]
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g, q_bias).reserve_batch(m)
+    xd = torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
+    y = torch.empty((m, N), dtype=torch.float32, device="cuda")
+    a16, b16 = alpha.astype(np.float16), None if q_bias is None else q_bias.astype(np.float16)
+    ref = oracle.bcq_matmul_f64(clean, bW, a16, b16, g)
+    ref[1] = np.nan
+    bits = np.unpackbits(bW.view(np.uint8).reshape(K // 32, q, N, 4), axis=-1, bitorder="little")       # [K / 32, q, N, 32]
+    for r in (0, 2, m - 1):
+        terms = []
+        for k in np.flatnonzero(np.isinf(x[r])):
+            planes = np.where(bits[k // 32, :, :, k % 32] == 1, 1.0, -1.0) * a16[k // g].astype(np.float64)
+            if b16 is not None:
+                planes = np.concatenate([planes, b16[k // g].astype(np.float64)[None]])
+            terms.append(planes * np.float64(x[r, k]))
+        with np.errstate(invalid="ignore"):
+            ref[r] = np.concatenate(terms).sum(0)
+    for _ in range(2):
+        L.matmul_f32(y, xd, w, m)
+        assert L.last_launch()[0] == kernel
+        got = y.cpu().numpy()
+        for r in touched:
+            assert np.array_equal(got[r], ref[r].astype(np.float32), equal_nan=True), r
+        rest = [r for r in range(m) if r not in touched]
+        assert np.linalg.norm(got[rest] - ref[rest]) <= 1e-5 * np.linalg.norm(ref[rest])
+    w.close()
+
+
+@pytest.mark.parametrize("N,K,q,g,bias,m", [(264, 1024, 4, 128, True, 40), (136, 2048, 2, 64, False, 130), (128, 512, 1, 32, True, 257),
+                                            (128, 512, 1, 128, False, 144), (1032, 1024, 3, 256, False, 66)])
+def test_split_operand_kernel_activations_not_finite(N, K, q, g, bias, m):
+    _not_finite(N, K, q, g, bias, m, "gemm_hl_kernel")
+
+
+def test_plane_kernel_activations_not_finite():
+    _not_finite(264, 1024, 2, 128, False, 20, "gemm_tc_kernel")
