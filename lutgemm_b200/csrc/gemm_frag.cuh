@@ -13,6 +13,7 @@
 //   +1), 14 (exponent: 0 or 2), 10 (exponent: 2 or 4), 9 (mantissa: 4 or 6).  The two values differ by 2 each time, so the
 //   sign's product is that of the operand less (1 + the lower value) times the activation: a sum over the group that does
 //   not depend on the weights and is what the fp32 accumulator starts from.  16 bit positions then need 5 shifts, not 15.
+//   (inf - inf: a row with an activation that is not finite is left out and computed product by product at the end.)
 //   The accumulator of a plane and scale group is multiplied by alpha in fp32; q_bias takes the group's sum of activations.
 //   Units come through a ring in shared memory that belongs to one warp (cp.async, no barriers).  The warps that
 //   split k add up through shared memory once per 32 columns, k-ranges of different CTAs through fp32 reductions in L2.
@@ -37,11 +38,12 @@ constexpr int kFrMaxRows = 16;
 constexpr int kFrRedStride = 12;              // floats between the rows of a reduction block: conflict-free stores
 constexpr int kFrMaxDepth = 6;
 constexpr int kFrSmemBytes = kSmemLimit;
+constexpr int kFrTailBytes = 64;              // a flag, 16 bits of rows per warp
 __host__ __device__ constexpr int fr_unit_bytes(int gw, int q, bool bias) { return q * 512 + (q + (bias ? 1 : 0)) * (4 / gw) * 64; }
 __host__ __device__ constexpr int fr_red_floats(int mt) { return 4 * mt * 8 * kFrRedStride; }     // per warp
 // units of a warp's ring (at least 2 are needed)
 __host__ __device__ constexpr int fr_depth(int gw, int mt, int q, bool bias) {
-    const int per_warp = (kFrSmemBytes - 16 - 2 * kFrWarps * fr_red_floats(mt) * 4) / kFrWarps;
+    const int per_warp = (kFrSmemBytes - kFrTailBytes - 2 * kFrWarps * fr_red_floats(mt) * 4) / kFrWarps;
     const int d = per_warp / fr_unit_bytes(gw, q, bias);
     return d > kFrMaxDepth ? kFrMaxDepth : d;
 }
@@ -139,9 +141,59 @@ __device__ __forceinline__ void fr_start(float (&d)[MT][4], const uint32_t (&bx)
     }
 }
 
+// A slab's sums of four columns: the output itself, or its share when k is cut into several slabs.
+__device__ __forceinline__ void fr_store(const FrParams& p, size_t off, float4 f) {
+    if (gridDim.y > 1) {
+        red_add_v4(p.partial + off, f);
+        return;
+    }
+    if (p.y32) *reinterpret_cast<float4*>(p.y32 + off) = f;
+    if (p.y16) {
+        __half2 lo = __floats2half2_rn(f.x, f.y), hi = __floats2half2_rn(f.z, f.w);
+        *reinterpret_cast<uint2*>(p.y16 + off) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    }
+}
+
+// Rows whose activations in this slab are not all finite (`rows`, a bit each): their sums over k-words [kw0, kw1) for columns
+// [c0, c1), by all threads of the CTA, as the planes give them: products of +-alpha_b (and q_bias) with the activation,
+// summed in fp32, 32 k of a plane at a time.
+template <bool BIAS>
+__device__ __noinline__ void fr_by_product(const FrParams& p, unsigned rows, int c0, int c1, int kw0, int kw1) {
+    const int N = p.N, quads = (c1 - c0) / 4;
+    for (int row = 0; row < p.m; row++) {
+        if (!((rows >> row) & 1u)) continue;
+        for (int at = threadIdx.x; at < quads; at += kFrThreads) {
+            const int col = c0 + 4 * at;
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int kw = kw0; kw < kw1; kw++) {
+                const size_t grp = (size_t)(32 * kw / p.g);
+                const __half* x = p.x + (size_t)row * p.K + 32 * kw;
+                for (int b = 0; b < p.q + (BIAS ? 1 : 0); b++) {
+                    const bool plane = !BIAS || b < p.q;
+                    const uint4 w = plane ? __ldg(reinterpret_cast<const uint4*>(p.bW + ((size_t)kw * p.q + b) * N + col))
+                                          : make_uint4(~0u, ~0u, ~0u, ~0u);
+                    const uint2 av = __ldg(reinterpret_cast<const uint2*>((plane ? p.alpha + (grp * p.q + b) * N : p.q_bias + grp * N) + col));
+                    const float2 a01 = half2_bits_to_float2(av.x), a23 = half2_bits_to_float2(av.y);
+                    float s[4] = {0.f, 0.f, 0.f, 0.f};
+                    for (int i = 0; i < 32; i++) {
+                        const float v = __half2float(x[i]);
+                        s[0] = fmaf((w.x >> i) & 1u ? a01.x : -a01.x, v, s[0]);
+                        s[1] = fmaf((w.y >> i) & 1u ? a01.y : -a01.y, v, s[1]);
+                        s[2] = fmaf((w.z >> i) & 1u ? a23.x : -a23.x, v, s[2]);
+                        s[3] = fmaf((w.w >> i) & 1u ? a23.y : -a23.y, v, s[3]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; c++) sum[c] += s[c];
+                }
+            }
+            fr_store(p, (size_t)row * N + col, make_float4(sum[0], sum[1], sum[2], sum[3]));
+        }
+    }
+}
+
 template <int MT, int GW, bool BIAS>
 __global__ void __launch_bounds__(kFrThreads, 1)
-gemm_frag_kernel(const FrParams p) {
+gemm_frag_kernel(const __grid_constant__ FrParams p) {
     constexpr int KS = MT == 1 ? 2 : 1;
     constexpr int NG = 4 / GW;                // scale groups of a unit
     constexpr int NJ = 4 * GW;                // bit positions (of 16) that a lane takes of its word
@@ -157,8 +209,9 @@ gemm_frag_kernel(const FrParams p) {
     const int a_off = q * 512, ub = a_off + P * NG * 64;          // a unit: words of the planes, then scales [plane][group][32 columns]
     unsigned char* ring = smem + warp * (p.depth * ub);
     const uint32_t ring_u = smem_u32(ring);
-    float* red = reinterpret_cast<float*>(smem + kFrSmemBytes - 16 - 2 * kFrWarps * fr_red_floats(MT) * 4);      // [parity][warp][fr_red_floats]
-    int* s_flag = reinterpret_cast<int*>(smem + kFrSmemBytes - 16);
+    float* red = reinterpret_cast<float*>(smem + kFrSmemBytes - kFrTailBytes - 2 * kFrWarps * fr_red_floats(MT) * 4);      // [parity][warp][fr_red_floats]
+    int* s_flag = reinterpret_cast<int*>(smem + kFrSmemBytes - kFrTailBytes);
+    unsigned short* s_open = reinterpret_cast<unsigned short*>(s_flag + 1);       // per warp: rows with an activation that is not finite
 
     const int words = K / 32;
     const int steps_total = (words + 3) / 4;
@@ -223,6 +276,7 @@ gemm_frag_kernel(const FrParams p) {
     uint32_t bx[KS][NG][NJ / 2][MT][2];
     float start[KS][NG][MT][2];               // what the accumulators of rows 8 nt + 2 t, + 1 start from
     float sx[KS][NG][MT][2];                  // BIAS: sums of the group's activations for those rows
+    unsigned open = 0u;                       // rows with an activation that is not finite: nor is, then, what they start from
 #pragma unroll
     for (int i = 0; i < KS; i++)
 #pragma unroll
@@ -262,6 +316,8 @@ gemm_frag_kernel(const FrParams p) {
             for (int nt = 0; nt < MT; nt++) {
                 start[i][gi][nt][0] = d[nt][0];
                 start[i][gi][nt][1] = d[nt][1];
+#pragma unroll
+                for (int e = 0; e < 2; e++) open |= fabsf(d[nt][e]) <= 3.402823466e38f ? 0u : 1u << (8 * nt + 2 * t + e);
                 if (BIAS) {
                     const uint32_t one[4] = {ones, ones, ones, ones};
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
@@ -272,6 +328,10 @@ gemm_frag_kernel(const FrParams p) {
                 }
             }
         }
+
+    open = __reduce_or_sync(0xffffffffu, open);
+    if (lane == 0) s_open[warp] = (unsigned short)open;
+    unsigned by_product = 0u;                 // rows left to fr_by_product
 
     // ---- columns ----
     const int my_tiles = (tile1 - tile0 + cw - 1) >> (4 - kw_log);      // every warp of the CTA walks as many: the barriers match
@@ -352,31 +412,24 @@ gemm_frag_kernel(const FrParams p) {
             asm volatile("bar.sync %0, %1;" ::"r"(1 + wc), "r"(p.kw * 32) : "memory");
             // 64 MT (row, column quad) sums by two warps per 8 rows, other warps each time
             const int turn = (wk - ti * 2 * MT) & kw_mask;
+            // the warps of this barrier hold all of the slab's activations: every column group finds the same rows
+            if (ti == 0) by_product = __reduce_or_sync(0xffffffffu, s_open[wc * p.kw + (lane & kw_mask)]);
             for (int o = turn * 32 + lane; o < 64 * MT && tile < tile1; o += p.kw * 32) {
                 const int row = o >> 3, rr = o & 7, nt = row >> 3, m8 = row & 7;
                 const int col = tile * kFrCols + 4 * rr;
-                if (row >= p.m || col >= N) continue;
+                if (row >= p.m || col >= N || ((by_product >> row) & 1u)) continue;
                 const float* src = red + (parity * kFrWarps + wc * p.kw) * fr_red_floats(MT) + (nt * 8 + m8) * kFrRedStride + rr;
                 float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
                 for (int v = 0; v < p.kw; v++)
 #pragma unroll
                     for (int c = 0; c < 4; c++) s[c] += src[v * fr_red_floats(MT) + c * MT * 8 * kFrRedStride];
-                const size_t off = (size_t)row * N + col;
-                const float4 f = make_float4(s[0], s[1], s[2], s[3]);
-                if (gridDim.y > 1) {
-                    red_add_v4(p.partial + off, f);
-                } else {
-                    if (p.y32) *reinterpret_cast<float4*>(p.y32 + off) = f;
-                    if (p.y16) {
-                        __half2 lo = __floats2half2_rn(f.x, f.y), hi = __floats2half2_rn(f.z, f.w);
-                        *reinterpret_cast<uint2*>(p.y16 + off) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-                    }
-                }
+                fr_store(p, (size_t)row * N + col, make_float4(s[0], s[1], s[2], s[3]));
             }
             parity ^= 1;
         }
     }
+    if (by_product) fr_by_product<BIAS>(p, by_product, tile0 * kFrCols, min(N, tile1 * kFrCols), 4 * slab0, min(words, 4 * slab1));
     if (gridDim.y == 1) return;
 
     // ---- slabs: the last CTA of the column range converts the reduced sums and zeroes the workspace ----

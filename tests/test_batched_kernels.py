@@ -192,3 +192,9 @@ def test_split_operand_kernel_activations_not_finite(N, K, q, g, bias, m):
 
 def test_plane_kernel_activations_not_finite():
     _not_finite(264, 1024, 2, 128, False, 20, "gemm_tc_kernel")
+
+
+@pytest.mark.parametrize("N,K,q,g,bias,m", [(132, 1024, 1, 128, False, 8), (1000, 2048, 3, 64, True, 5), (100, 160, 2, 32, False, 9),
+                                            (36, 4128, 3, 96, True, 18), (264, 8192, 2, 512, False, 4)])
+def test_register_operand_kernel_activations_not_finite(N, K, q, g, bias, m):
+    _not_finite(N, K, q, g, bias, m, "gemm_frag_kernel")
