@@ -84,14 +84,6 @@ def parse():
     return ap.parse_args()
 
 
-def batched_kernel(m, q, bias=False, ordered=False):
-    """The kernel that lutgemm_matmul takes for m >= 4 rows (a group size that divides, or is a multiple of, 128)."""
-    passes = q + (1 if bias else 0)
-    if m <= 8 and not ordered:
-        return "gemm_frag_kernel"
-    return "gemm_hl_kernel" if q <= 4 and m >= (4 if passes >= 5 else 64 if passes >= 3 else 97 if passes == 2 else 129) else "gemm_tc_kernel"
-
-
 def workload_name(a):
     return f"bcq_gemv m={a.m} n={a.n} k={a.k} q={a.q} g={a.g}" + (" +q_bias" if a.bias else "")
 
@@ -611,7 +603,7 @@ def batched_numbers(local):
     import lutgemm_b200 as L
     n = k = 8192
     q, g, rot = 2, 64, 8
-    out = {"workload": f"bcq_gemm n={n} k={k} q={q} g={g}", "kernels": {"m2": "gemv_tma2_kernel", "m16": batched_kernel(16, q), "m128": batched_kernel(128, q)}}
+    out = {"workload": f"bcq_gemm n={n} k={k} q={q} g={g}", "kernels": {}}
     ws = []
     for i in range(rot):
         bW, alpha, _ = synth.bcq_layer(n, k, q, g, seed=synth.seed_for("bench", n, k, q, i))
@@ -625,6 +617,7 @@ def batched_numbers(local):
                 L.matmul(y, x, w, m)
         for _ in range(3):
             step()
+        out["kernels"][f"m{m}"] = L.last_launch()[0]
         torch.cuda.synchronize()
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
@@ -688,7 +681,6 @@ def run_ours(a):
     lib.lutgemm_set_dependent_launch(0 if a.no_pdl else 1)
     lib.lutgemm_set_batched_int8(1 if a.int8 else 0)
     lib.lutgemm_set_ordered_reduction(1 if a.ordered else 0)
-    kernel_name = (("gemv_tma_kernel" if a.m == 1 else "gemv_tma2_kernel") if a.variant == 0 else "gemv_reg_kernel") if a.m < 4 else ("gemm_i8_kernel" if a.int8 and a.m <= 16 and a.q <= 4 else batched_kernel(a.m, a.q, a.bias, a.ordered))
 
     B = synth.algorithmic_bytes(a.n, a.k, a.q, a.g, a.m, a.bias)
     rot = max(1, a.rot)
@@ -712,6 +704,7 @@ def run_ours(a):
 
     for _ in range(max(3, a.warmup)):
         step()
+    kernel_name = L.last_launch()[0]
     barrier()
     # One step (ROT matvecs) is captured once into a CUDA graph and replayed, so that the timed
     # region measures the device, not the Python launch path.

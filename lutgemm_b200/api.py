@@ -32,10 +32,12 @@ def _ptr(a):
 
 def _stream_ptr(stream):
     """The stream's handle as a plain integer (the prototypes make a pointer of it).  Without a stream, the current one of
-    the current device, asked for as a number: building the Stream object costs more than the rest of a small call."""
+    the current device, asked for as a number where this torch has that call (it is not a public one): building the Stream
+    object costs more than the rest of a small call."""
     if stream is None:
         import torch
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        return raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream
     return stream.cuda_stream
 
 

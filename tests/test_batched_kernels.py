@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-def _run(N, K, q, g, bias, m, column_scales=False, ordered=False):
+def _run(kernel, N, K, q, g, bias, m, column_scales=False, ordered=False):
+    """Two calls against 64-bit sums; `kernel` is the one that has to have run them."""
     bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + K + m, with_bias=bias)
     if column_scales:
         # columns whose scales lie far apart, down to fp16's subnormals and up to its largest values
@@ -24,18 +25,31 @@ def _run(N, K, q, g, bias, m, column_scales=False, ordered=False):
     xd = torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
     y32 = torch.empty((m, N), dtype=torch.float32, device="cuda")
     y16 = torch.empty((m, N), dtype=torch.float16, device="cuda")
+    first = None
     for _ in range(2):                                    # the second call finds the workspace as the first one left it
         L.matmul_f32(y32, xd, w, m)
+        assert L.last_launch()[0] == kernel
         L.matmul(y16, xd, w, m)
+        assert L.last_launch()[0] == kernel
+        if ordered:
+            assert first is None or torch.equal(first, y32)
+            first = y32.clone()
     a16, b16 = alpha.astype(np.float16), None if q_bias is None else q_bias.astype(np.float16)
     ref = oracle.bcq_matmul_f64(x, bW, a16, b16, g)
     # Products are exact, sums are fp32: every addition errs by at most 2^-23 of the largest partial sum, which is at most
-    # 11 |x| |scale| summed (an operand of up to 6 and its offset of up to 5 for a sign).  K / 16 additions per pass.
+    # |x| |scale| summed; 11 times that with the register operand (up to 6, and its offset of up to 5, for a sign).  K / 16
+    # additions per pass.  The split operand's weight is off by up to 2^-22 of it.
+    grow = 11 if kernel == "gemm_frag_kernel" else 1
+    unit = grow * (2 * K / 16 + 64) * 2.0 ** -23 + 2.0 ** -22
     mag = np.abs(a16.astype(np.float64)).sum(1) + (0 if b16 is None else np.abs(b16.astype(np.float64)))       # [G, N]
     size = np.abs(x.astype(np.float64)).reshape(m, K // g, g).sum(2) @ mag
-    bound = (2 * K / 16 + 64) * 2.0 ** -23 * 11 * size + 1e-30
+    bound = unit * size + 1e-30
     err = np.abs(y32.cpu().numpy().astype(np.float64) - ref)
     assert (err <= bound).all(), (err / bound).max()
+    # Per column in the 2-norm, where partial sums of terms of either sign are no larger than the whole (1.5: the spread over
+    # 64 rows or more).  A split operand without its low half (2e-4 with these weights) is 6 times beyond this.
+    if m >= 64 and 512 <= K <= 1152:
+        assert (np.linalg.norm(err, axis=0) <= 1.5 * unit * np.linalg.norm(ref, axis=0)).all()
     # one rounding to fp16 on top: half a unit in the last place, at least half the subnormal step
     with np.errstate(over="ignore"):
         lim = bound + np.maximum(np.abs(ref) * 2.0 ** -11, 2.0 ** -25)
@@ -46,55 +60,69 @@ def _run(N, K, q, g, bias, m, column_scales=False, ordered=False):
 
 
 # 128-column tiles, 64-k blocks, 16-row steps, 128- and 256-row items, one and several scale groups per block, a last block
-# of one word, groups wider than what a warp walks in one stride
+# of one word (with one and two scale groups to a block), groups wider than what a warp walks in one stride
 @pytest.mark.parametrize("N,K,q,g,bias,m", [
-    (8, 32, 4, 32, True, 17), (136, 96, 4, 32, True, 31), (128, 64, 3, 64, False, 64), (264, 2048, 2, 128, False, 129),
+    (8, 32, 4, 32, True, 130), (136, 96, 4, 32, True, 140), (264, 160, 3, 32, True, 300), (128, 64, 3, 64, False, 64), (520, 1024, 2, 32, True, 131), (264, 2048, 2, 128, False, 129),
     (264, 576, 1, 64, True, 130), (1000, 1152, 4, 384, True, 257), (2056, 256, 2, 256, True, 300), (512, 512, 1, 128, False, 144),
     (120, 4096, 3, 1024, True, 100), (4096, 160, 4, 32, False, 513)])
 def test_split_operand_kernel(N, K, q, g, bias, m):
-    _run(N, K, q, g, bias, m)
+    _run("gemm_hl_kernel", N, K, q, g, bias, m)
 
 
 @pytest.mark.parametrize("q,bias,m", [(4, True, 40), (2, False, 150), (1, False, 200), (3, True, 256)])
 def test_split_operand_kernel_scales_far_apart(q, bias, m):
-    _run(264, 1024, q, 128, bias, m, column_scales=True)
+    _run("gemm_hl_kernel", 264, 1024, q, 128, bias, m, column_scales=True)
 
 
 def test_split_operand_kernel_ordered_is_reproducible_and_right():
-    _run(264, 2048, 4, 128, True, 140, ordered=True)
+    _run("gemm_hl_kernel", 264, 2048, 4, 128, True, 140, ordered=True)
+
+
+# narrow groups up to 128 rows, where a block of 64 k holds several scale groups
+@pytest.mark.parametrize("N,K,q,g,bias,m", [(8, 32, 4, 32, True, 17), (136, 96, 4, 32, True, 31), (264, 512, 2, 32, False, 4)])
+def test_plane_kernel_narrow_groups(N, K, q, g, bias, m):
+    _run("gemm_tc_kernel", N, K, q, g, bias, m)
 
 
 # 32-column units with ragged last quads and tiles, one to 8 planes, the three kinds of scale group, words beyond K, one and
 # two tiles of 8 rows, one and several k-ranges; the last two go 16 rows at a time
 @pytest.mark.parametrize("N,K,q,g,bias,m", [
-    (4, 32, 1, 32, False, 3), (12, 96, 2, 32, True, 4), (100, 160, 3, 160, False, 5), (36, 4128, 3, 96, True, 2),
+    (4, 32, 1, 32, False, 3), (12, 96, 2, 32, True, 4), (100, 160, 3, 160, False, 5), (36, 4128, 3, 96, True, 3),
     (33 * 4, 1024, 4, 128, True, 8), (5000, 256, 2, 64, False, 7), (264, 8192, 3, 512, False, 4), (40, 2048, 8, 128, True, 6),
-    (64, 20480, 5, 64, True, 4), (2052, 4128, 3, 96, False, 16), (20, 384, 7, 192, True, 9), (28, 640, 2, 32, False, 35)])
+    (64, 20480, 5, 64, True, 4), (2052, 4128, 3, 96, False, 16), (20, 384, 7, 192, True, 7), (28, 640, 2, 32, False, 35)])
 def test_register_operand_kernel(N, K, q, g, bias, m):
-    _run(N, K, q, g, bias, m)
+    _run("gemm_frag_kernel", N, K, q, g, bias, m)
 
 
 @pytest.mark.parametrize("q,g,bias,m", [(4, 128, True, 8), (3, 64, False, 4), (2, 32, True, 5)])
 def test_register_operand_kernel_scales_far_apart(q, g, bias, m):
-    _run(260, 1024, q, g, bias, m, column_scales=True)
+    _run("gemm_frag_kernel", 260, 1024, q, g, bias, m, column_scales=True)
 
 
 def test_three_rows_without_reserved_scratch_inside_a_capture():
-    """A first call of three rows inside a stream capture cannot allocate scratch: it still runs, one or two rows at a time."""
-    N, K, q, g = 512, 8192, 3, 128
+    """A first call of three rows inside a stream capture cannot allocate scratch: a container whose register-operand plan
+    has several k-ranges still runs it, one row at a time, and with that kernel once scratch is reserved."""
+    N, K, q, g = 516, 8160, 3, 96
     bW, alpha, _ = synth.bcq_layer(N, K, q, g, seed=5)
     x = synth.activations(3, K, seed=6)
     w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g)
     xd = torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
     y = torch.zeros((3, N), dtype=torch.float32, device="cuda")
+    ref = oracle.bcq_matmul_f64(x, bW, alpha.astype(np.float16), None, g)
     graph = torch.cuda.CUDAGraph()
     torch.cuda.synchronize()
     with torch.cuda.graph(graph):
         L.matmul_f32(y, xd, w, 3)
+    assert L.last_launch()[0] == "gemv_reg_kernel"
     graph.replay()
     torch.cuda.synchronize()
-    ref = oracle.bcq_matmul_f64(x, bW, alpha.astype(np.float16), None, g)
     assert np.linalg.norm(y.cpu().numpy() - ref) <= 1e-5 * np.linalg.norm(ref)
+    assert w.scratch() == (0, 0, 0)
+    w.reserve_batch(3)
+    L.matmul_f32(y.zero_(), xd, w, 3)
+    assert L.last_launch()[0] == "gemm_frag_kernel" and L.last_launch()[2] > 1
+    assert np.linalg.norm(y.cpu().numpy() - ref) <= 1e-5 * np.linalg.norm(ref)
+    del graph
     w.close()
 
 
