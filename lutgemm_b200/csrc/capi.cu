@@ -1351,7 +1351,6 @@ int lutgemm_weight_reserve_batch(lutgemm_weight_t w, int m) {
     if (m >= 2 && ws->tc_rows < rows) {
         rc = grow_tc_rows(ws, rows, rows, batch_rows_for(w, kMaxBatch), nullptr);
         if (rc != LUTGEMM_OK) return rc;
-        LG_CUDA(cudaStreamSynchronize(nullptr));       // zeroed before a call on a stream that does not wait for this one
     }
     // transposed copies of the (output, nqW, input, n) overload
     rc = grow(&ws->t_in, &ws->t_in_bytes, (size_t)m * w->K * sizeof(__half), nullptr);
