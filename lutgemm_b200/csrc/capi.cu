@@ -48,6 +48,7 @@ struct lutgemm_workspace {
     void* t_in = nullptr;
     void* t_out = nullptr;
     size_t t_in_bytes = 0, t_out_bytes = 0;
+    lutgemm_retired_block* retired_copies = nullptr;   // earlier blocks of these
     std::atomic<int> ordered{-1};   // split-k mode of calls on this workspace: -1 = the process-wide setting, 0 / 1 = fixed
 };
 
@@ -251,11 +252,12 @@ void free_workspace_buffers(lutgemm_workspace* ws) {
     if (ws->tc_partial) cudaFree(ws->tc_partial);
     if (ws->t_in) cudaFree(ws->t_in);
     if (ws->t_out) cudaFree(ws->t_out);
-    while (lutgemm_retired_block* r = ws->retired) {
-        ws->retired = r->next;
-        cudaFree(r->ptr);
-        delete r;
-    }
+    for (lutgemm_retired_block** list : {&ws->retired, &ws->retired_copies})
+        while (lutgemm_retired_block* r = *list) {
+            *list = r->next;
+            cudaFree(r->ptr);
+            delete r;
+        }
     ws->partial = ws->partial2 = ws->tc_partial = nullptr;
     ws->counters = nullptr;
     ws->status = nullptr;
@@ -1119,14 +1121,32 @@ __global__ void host_done_kernel(unsigned* done_host, unsigned value) {
     *reinterpret_cast<volatile unsigned*>(done_host) = value;
 }
 
-int grow(void** buf, size_t* have, size_t need, cudaStream_t st) {
+// A buffer of at least `need` bytes.  As with grow_tc_rows the one that it replaces stays allocated (a captured graph may hold
+// it), and the size at least doubles where that can be had.
+int grow(void** buf, size_t* have, size_t need, lutgemm_retired_block** retired, cudaStream_t st) {
     if (*have >= need) return LUTGEMM_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone) return LUTGEMM_ERR_BATCH;
-    if (*buf) LG_CUDA(cudaFree(*buf));
-    *buf = nullptr; *have = 0;
-    LG_CUDA(cudaMalloc(buf, need));
-    *have = need;
+    size_t take = 2 * *have > need ? 2 * *have : need;
+    void* block = nullptr;
+    cudaError_t e = cudaMalloc(&block, take);
+    if (e != cudaSuccess && take > need) {
+        (void)cudaGetLastError();
+        take = need;
+        e = cudaMalloc(&block, take);
+    }
+    LG_CUDA(e);
+    if (*buf) {
+        lutgemm_retired_block* old = new (std::nothrow) lutgemm_retired_block;
+        if (!old) {
+            cudaFree(block);
+            return LUTGEMM_ERR_TOO_LARGE;
+        }
+        *old = {*buf, *have, *retired};
+        *retired = old;
+    }
+    *buf = block;
+    *have = take;
     return LUTGEMM_OK;
 }
 
@@ -1353,8 +1373,8 @@ int lutgemm_weight_reserve_batch(lutgemm_weight_t w, int m) {
         if (rc != LUTGEMM_OK) return rc;
     }
     // transposed copies of the (output, nqW, input, n) overload
-    rc = grow(&ws->t_in, &ws->t_in_bytes, (size_t)m * w->K * sizeof(__half), nullptr);
-    if (rc == LUTGEMM_OK) rc = grow(&ws->t_out, &ws->t_out_bytes, (size_t)m * w->N * sizeof(__half), nullptr);
+    rc = grow(&ws->t_in, &ws->t_in_bytes, (size_t)m * w->K * sizeof(__half), &ws->retired_copies, nullptr);
+    if (rc == LUTGEMM_OK) rc = grow(&ws->t_out, &ws->t_out_bytes, (size_t)m * w->N * sizeof(__half), &ws->retired_copies, nullptr);
     return rc;
 }
 
@@ -1375,8 +1395,8 @@ int lutgemm_matmul_wx(void* out, lutgemm_weight_t w, const void* in, int n, void
     if (((uintptr_t)in & 15) || ((uintptr_t)out & 15)) return LUTGEMM_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
     lutgemm_workspace* ws = &w->own;
-    int rc = grow(&ws->t_in, &ws->t_in_bytes, (size_t)n * w->K * sizeof(__half), st);
-    if (rc == LUTGEMM_OK) rc = grow(&ws->t_out, &ws->t_out_bytes, (size_t)n * w->N * sizeof(__half), st);
+    int rc = grow(&ws->t_in, &ws->t_in_bytes, (size_t)n * w->K * sizeof(__half), &ws->retired_copies, st);
+    if (rc == LUTGEMM_OK) rc = grow(&ws->t_out, &ws->t_out_bytes, (size_t)n * w->N * sizeof(__half), &ws->retired_copies, st);
     if (rc != LUTGEMM_OK) return rc;
     // input [K][n] -> [n][K]; X.W; output [n][N] -> [N][n]
     dim3 tb(32, 8);

@@ -185,3 +185,28 @@ def test_reserved_rows_are_enough_for_every_plan(q):
     assert split > 0
     plenty.close()
     w.close()
+
+
+def test_captured_wx_call_outlives_a_larger_one():
+    """The transposed copies of the (output, nqW, input, n) form: a larger call leaves those of a captured one in place."""
+    w, bW, alpha = _container()
+    w.reserve_batch(5)
+    x = synth.activations(5, K, seed=5)
+    xd = _device(np.ascontiguousarray(x.T))
+    y = torch.zeros((N, 5), dtype=torch.float16, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        L.matmul_wx(y, w, xd, 5)
+    for n in (6, 40):
+        xl = synth.activations(n, K, seed=n)
+        yl = torch.empty((N, n), dtype=torch.float16, device="cuda")
+        L.matmul_wx(yl, w, _device(np.ascontiguousarray(xl.T)), n)
+        _close(yl.cpu().numpy().T, xl, bW, alpha)
+        w.reserve_batch(2 * n)
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        _close(y.cpu().numpy().T, x, bW, alpha)
+    del graph
+    w.close()
