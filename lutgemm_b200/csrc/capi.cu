@@ -578,24 +578,30 @@ int batch_rows_for(const lutgemm_weight* w, int m) {
     return rows > tc_rows_for(m) ? rows : tc_rows_for(m);
 }
 
-// Split-k plan of a batched launch (256-column tiles x k-ranges of whole 128-k steps) and, when it splits, the fp32
-// reduction rows of the workspace: at least m, and `rows` where they have to be allocated anyway (for the kernels that ask
-// for this plan only to follow its rule on scratch).
-int tc_split(lutgemm_weight* w, lutgemm_workspace* ws, int m, int rows, cudaStream_t st, int* splitk_out, int* steps_per_cta_out) {
+// 128-k steps of a CTA of the plane kernel.  The split-k factor fills whole waves of one CTA per SM; among equally full choices
+// the smallest.
+int tc_steps_per_cta(const lutgemm_weight* w, bool ordered) {
     const int tiles = (w->N + lg::kTcTileN - 1) / lg::kTcTileN;
-    const int steps_total = (w->K + lg::kTcStepK - 1) / lg::kTcStepK;
-    // split-k factor: fill whole waves of one CTA per SM; among equally full choices take the smallest
-    const int sms = sm_count();
-    int splitk = 1, steps_per_cta = 0;
+    const int steps_total = (w->K + lg::kTcStepK - 1) / lg::kTcStepK, sms = sm_count();
+    int splitk = 1;
     double best = 0.0;
     for (int c = 1; c <= 8 && c <= steps_total; c++) {
         const int ctas = tiles * c;
         const double eff = (double)ctas / ((double)((ctas + sms - 1) / sms) * sms);
         if (eff > best + 0.02) { best = eff; splitk = c; }
     }
-    if (ordered_for(ws)) splitk = 1;             // bit-reproducible mode: no unordered reductions across k-ranges
-    steps_per_cta = (steps_total + splitk - 1) / splitk;
-    splitk = (steps_total + steps_per_cta - 1) / steps_per_cta;
+    if (ordered) splitk = 1;                     // bit-reproducible mode: no unordered reductions across k-ranges
+    return (steps_total + splitk - 1) / splitk;
+}
+
+// Split-k plan of a batched launch (256-column tiles x k-ranges of whole 128-k steps) and, when it splits, the fp32
+// reduction rows of the workspace: at least m, and `rows` where they have to be allocated anyway (for the kernels that ask
+// for this plan only to follow its rule on scratch).
+int tc_split(lutgemm_weight* w, lutgemm_workspace* ws, int m, int rows, cudaStream_t st, int* splitk_out, int* steps_per_cta_out) {
+    const int tiles = (w->N + lg::kTcTileN - 1) / lg::kTcTileN;
+    const int steps_total = (w->K + lg::kTcStepK - 1) / lg::kTcStepK;
+    const int steps_per_cta = tc_steps_per_cta(w, ordered_for(ws));
+    const int splitk = (steps_total + steps_per_cta - 1) / steps_per_cta;
     if (tiles > kMaxCounters) return LUTGEMM_ERR_TOO_LARGE;
     if (splitk > 1 && ws->tc_rows < m) {
         // Not reserved (lutgemm_weight_reserve_batch / lutgemm_workspace_create): only the container's own workspace
@@ -655,6 +661,15 @@ int gemm_tc_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 }
 
 // ---- split-operand kernel (gemm_hl.cuh): plan, launch ----
+// Longest chain of tensor-core accumulations (each cuts the fp32 sum off) between two drains: the plane kernel's, 8 per plane
+// and 128 k, less a sixteenth, so that an fp32 result is no further off than that kernel's.  An fp16 result has an error of 2.1e-4 of its own; a
+// chain of 1024 adds 1.8e-5 to that, 0.4 % of it, and costs no drain up to 8192 k.
+constexpr int kHlChain16 = 1024;
+int hl_chain(const lutgemm_weight* w, bool ordered, bool f32) {
+    const int plane = 8 * (w->q + (w->q_bias ? 1 : 0)) * tc_steps_per_cta(w, ordered);
+    return f32 ? plane - plane / 16 : plane > kHlChain16 ? plane : kHlChain16;
+}
+
 // One CTA per SM: an item is 128 columns x 256 rows, and an item may be cut into two halves of 128 rows or into k-ranges.
 // Cost model in cycles: a block of 64 k takes the tensor pipe and shared memory kHlRowCycles per row and pass, and the
 // expansion kHlExpCycles whatever the rows, more with more table entries; a CTA's start, first loads and epilogue add
@@ -666,8 +681,8 @@ int gemm_tc_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 // The plan with the smallest estimate is taken: whole items, halves, whole items
 // with a last partial wave of halves, each with 1 to 8 k-ranges.  Returns the estimate.
 constexpr double kHlRowCycles = 2.18, kHlExpCycles = 630, kHlEntryCycles = 8.5, kHlBiasCycles = 14.5;
-constexpr double kHlCtaCycles = 6300, kHlSplitCycles = 4400, kHlSplitRowCycles = 30;
-double hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) {
+constexpr double kHlCtaCycles = 6300, kHlSplitCycles = 4400, kHlSplitRowCycles = 30, kHlDrainRowCycles = 25;
+double hl_plan(const lutgemm_weight* w, int m, bool may_split, int chain, lg::HlParams* p) {
     const int sms = sm_count();
     const int T = (w->N + lg::kHlCols - 1) / lg::kHlCols, RT = (m + lg::kHlRows - 1) / lg::kHlRows;
     const long long items = (long long)T * RT;
@@ -681,6 +696,8 @@ double hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) 
     p->splits = 1;
     p->blocks_per_split = blocks;
     p->full_items = (int)items;
+    p->segment_lo = chain / 4 < 1 ? 1 : chain / 4;
+    p->segment = chain / 8 < 1 ? 1 : chain / 8;
     double best = 1e300;
     auto consider = [&](long long full, long long halves, int c) {
         const int bps = (blocks + c - 1) / c;
@@ -690,7 +707,10 @@ double hl_plan(const lutgemm_weight* w, int m, bool may_split, lg::HlParams* p) 
         auto waves = [&](long long n, int rows) {
             const double busy = (double)(n < sms ? n : sms) / sms;
             const double split = real > 1 ? kHlSplitCycles + kHlSplitRowCycles * rows * (1 + 1.8 / real) * (1 + 2 * busy) / 3 : 0.0;
-            return (double)((n + sms - 1) / sms) * (kHlCtaCycles + split + bps * block_cost(rows));
+            const int most = rows <= lg::kHlLoRows || per_row == kHlRowCycles ? p->segment_lo : p->segment;
+            const bool seg = 4 * bps * (per_row == kHlRowCycles ? 1 : 2) > chain;
+            const double drains = ((bps + most - 1) / most - 1) * kHlDrainRowCycles * rows;
+            return (double)((n + sms - 1) / sms) * (kHlCtaCycles + split + drains + bps * block_cost(rows) * (seg ? 1.12 : 1.0));
         };
         const double t = waves(nf, whole_rows) + waves(nh, half_rows);
         if (t < best * 0.98) {
@@ -719,7 +739,7 @@ int hl_split_rows_of(const lutgemm_weight* w) {
     const int cap = lg::kHlRows * ((sm_count() - 1) / T);
     lg::HlParams p = {};
     auto splits = [&](int m) {
-        hl_plan(w, m, true, &p);
+        hl_plan(w, m, true, kHlChain16, &p);
         return p.splits > 1;
     };
     int coarse = cap;
@@ -733,10 +753,15 @@ int hl_split_rows_of(const lutgemm_weight* w) {
 // From which row count the split-operand kernel is the faster one: it always takes two tensor-core passes, gemm_tc one
 // per plane and one for q_bias.  Measured, us (gemm_tc / split operand), g = 128: 2 passes, 8192 x 8192, 96 rows 33.3 / 33.8,
 // 128 rows 39.1 / 35.7; 3 passes, 8192 x 8192, 32 rows 31.6 / 32.0, 64 rows 36.7 / 32.4; 4 passes, 12288 x 4096, 32 rows
-// 28.0 / 30.0, 64 rows 33.7 / 31.0, 96 rows 40.5 / 32.3; 5 passes, 28672 x 8192, 4 rows 160 / 116.
-bool gemm_hl_ok(const lutgemm_weight* w, int m) {
+// 28.0 / 30.0, 64 rows 33.7 / 31.0, 96 rows 40.5 / 32.3; 5 passes, 28672 x 8192, 4 rows 160 / 116.  At and above these row
+// counts no call was slower than with gemm_tc by more than 2 % at 14 widths from 1024 to 28672 (672 calls, g = 128; 216 at g =
+// 32, 64, 256).
+// Where it has to drain its accumulators (fp32 results, very long k): 2 passes, 28672 x 8192, 128 rows, fp32 113 / 128, 11008 x
+// 4096 31 / 35, 8192 x 28672, fp16 96 / 108; more passes as above (3 passes, 28672 x 8192, 100 rows, fp32 141 / 132).
+bool gemm_hl_ok(const lutgemm_weight* w, int m, bool f32) {
     const int passes = w->q + (w->q_bias ? 1 : 0);
-    const int from = passes >= 5 ? 4 : passes >= 3 ? 64 : passes == 2 ? 97 : 129;
+    const bool drains = f32 || w->K > 16 * kHlChain16;            // (two k-ranges at the widths where that is not so)
+    const int from = passes >= 5 ? 4 : passes >= 3 ? 64 : passes == 2 && !drains ? 97 : 129;
     // with g = 32 every block builds two tables: up to 128 rows, where the expansion bounds it, that goes to gemm_tc
     return w->tc_ok && w->q <= 4 && m >= from && (m > 128 || w->g >= lg::kHlStepK);
 }
@@ -745,15 +770,17 @@ bool gemm_hl_ok(const lutgemm_weight* w, int m) {
 long long rows_there(const lutgemm_weight* w, const lutgemm_workspace* ws) { return (long long)ws->tc_rows * ws->n_cap / w->N; }
 
 template <int Q>
-int launch_gemm_hl_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::HlParams& p, dim3 grid, cudaStream_t st) {
-    static bool configured[64][2] = {};   // the attribute is per device
+int launch_gemm_hl_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::HlParams& p, bool seg, dim3 grid, cudaStream_t st) {
+    static bool configured[64][4] = {};   // the attribute is per device
     const bool bias = w->q_bias != nullptr;
-    auto kern = bias ? lg::gemm_hl_kernel<Q, true> : lg::gemm_hl_kernel<Q, false>;
+    auto kern = bias ? (seg ? lg::gemm_hl_kernel<Q, true, true> : lg::gemm_hl_kernel<Q, true, false>)
+                     : (seg ? lg::gemm_hl_kernel<Q, false, true> : lg::gemm_hl_kernel<Q, false, false>);
+    const int which = 2 * seg + bias;
     int dev = 0;
     LG_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64 || !configured[dev][bias]) {
+    if (dev >= 64 || !configured[dev][which]) {
         LG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lg::kSmemLimit));
-        if (dev < 64) configured[dev][bias] = true;
+        if (dev < 64) configured[dev][which] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -773,11 +800,13 @@ int launch_gemm_hl_q(const lutgemm_weight* w, const CUtensorMap& tmX, const lg::
 
 // Rows [0, m) through the split-operand kernel, one launch.
 int gemm_hl_launch(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __half* y16, float* y32, int m, bool may_split,
-                   cudaStream_t st) {
+                   int chain, cudaStream_t st) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return LUTGEMM_ERR_CUDA;
     lg::HlParams p = {};
-    hl_plan(w, m, may_split, &p);
+    hl_plan(w, m, may_split, chain, &p);
+    // one chain where it is short enough as it is: 4 accumulations per pass and block of 64 k
+    const bool seg = 4 * p.blocks_per_split * (w->q == 1 && !w->q_bias ? 1 : 2) > chain;
     p.box_rows = m < lg::kHlBoxRows ? (m + 15) / 16 * 16 : lg::kHlBoxRows;
     p.x_slot_bytes = (m <= lg::kHlBoxRows || p.full_items == 0 ? 1 : 2) * p.box_rows * 128;
     p.x_slots = lg::kHlXBudget / p.x_slot_bytes;
@@ -800,15 +829,15 @@ int gemm_hl_launch(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __
     const long long items = (long long)p.col_tiles * ((m + lg::kHlRows - 1) / lg::kHlRows);
     dim3 grid((unsigned)(p.full_items + 2 * (items - p.full_items)), p.splits);
     switch (w->q) {
-        case 1: return launch_gemm_hl_q<1>(w, tmX, p, grid, st);
-        case 2: return launch_gemm_hl_q<2>(w, tmX, p, grid, st);
-        case 3: return launch_gemm_hl_q<3>(w, tmX, p, grid, st);
-        case 4: return launch_gemm_hl_q<4>(w, tmX, p, grid, st);
+        case 1: return launch_gemm_hl_q<1>(w, tmX, p, seg, grid, st);
+        case 2: return launch_gemm_hl_q<2>(w, tmX, p, seg, grid, st);
+        case 3: return launch_gemm_hl_q<3>(w, tmX, p, seg, grid, st);
+        case 4: return launch_gemm_hl_q<4>(w, tmX, p, seg, grid, st);
     }
     return LUTGEMM_ERR_BITS;
 }
 
-// Rows [0, m), gemm_hl_ok(w, m) holds: one launch, which may split k when the workspace has fp32 rows for all of m.  When it
+// Rows [0, m), gemm_hl_ok holds: one launch, which may split k when the workspace has fp32 rows for all of m.  When it
 // has fewer (a captured call above the reserved batch, a small explicit workspace), either one launch without k-ranges or as
 // many rows at a time as there are; a piece that gemm_tc is the faster for goes there.  Pieces are taken where the model puts
 // them below 0.78 of the one launch: measured at 128 rows a piece, 1024 x 8192, q = 4 + q_bias, 300 rows 38.0 / 59.0 us, 4096 x
@@ -820,25 +849,26 @@ int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
     int rc = tc_split(w, ws, m < 128 ? m : 128, batch_rows_for(w, m), st, &unused_split, &unused_steps);
     if (rc != LUTGEMM_OK) return rc;
     const bool ordered = ordered_for(ws);
+    const int chain = hl_chain(w, ordered, y32 != nullptr);
     const long long there = rows_there(w, ws);
     const int piece = there < batch_rows_for(w, m) ? (int)(there / 128 * 128) : m;
     if (!ordered && piece >= 128 && piece < m) {
         lg::HlParams p = {};
-        double pieces = (m / piece) * hl_plan(w, piece, true, &p);
-        if (m % piece) pieces += hl_plan(w, m % piece, true, &p);
-        if (pieces < 0.78 * hl_plan(w, m, false, &p)) {
+        double pieces = (m / piece) * hl_plan(w, piece, true, chain, &p);
+        if (m % piece) pieces += hl_plan(w, m % piece, true, chain, &p);
+        if (pieces < 0.78 * hl_plan(w, m, false, chain, &p)) {
             for (int r0 = 0; r0 < m; r0 += piece) {
                 const int rows = m - r0 < piece ? m - r0 : piece;
                 const __half* xr = x + (size_t)r0 * w->K;
                 __half* y16r = y16 ? y16 + (size_t)r0 * w->N : nullptr;
                 float* y32r = y32 ? y32 + (size_t)r0 * w->N : nullptr;
-                rc = gemm_hl_ok(w, rows) ? gemm_hl_launch(w, ws, xr, y16r, y32r, rows, true, st) : gemm_tc_rows(w, ws, xr, y16r, y32r, rows, st);
+                rc = gemm_hl_ok(w, rows, y32 != nullptr) ? gemm_hl_launch(w, ws, xr, y16r, y32r, rows, true, chain, st) : gemm_tc_rows(w, ws, xr, y16r, y32r, rows, st);
                 if (rc != LUTGEMM_OK) return rc;
             }
             return LUTGEMM_OK;
         }
     }
-    return gemm_hl_launch(w, ws, x, y16, y32, m, !ordered && there >= m, st);
+    return gemm_hl_launch(w, ws, x, y16, y32, m, !ordered && there >= m, chain, st);
 }
 
 // ---- register-operand kernel (gemm_frag.cuh): plan, launch ----
@@ -1077,7 +1107,7 @@ int matmul_impl(__half* y16, float* y32, const void* in, lutgemm_weight_t w, int
         }
         return LUTGEMM_OK;
     }
-    if (gemm_hl_ok(w, m) && !gemm_i8_ok(w, m)) return gemm_hl_rows(w, ws, x, y16, y32, m, st);
+    if (gemm_hl_ok(w, m, y32 != nullptr) && !gemm_i8_ok(w, m)) return gemm_hl_rows(w, ws, x, y16, y32, m, st);
     // batched: 128 rows per tensor-core launch
     for (int r0 = 0; r0 < m; r0 += 128) {
         const int rows = (m - r0 < 128) ? (m - r0) : 128;

@@ -24,8 +24,8 @@
 //
 // Bound by instruction issue and its latencies: per plane and 4096 weights 64 LOP3, 20 shifts and 16 MT mma.sync, on 16 warps
 // that 128 registers a thread allow; plus some 10 us at 8192 x 8192 that do not grow with the planes (activations, column
-// sums, k-ranges).  Measured, 28672 x 8192, q = 4 + q_bias, 4 rows: 82.6 us = 1.65 TB/s (160 with gemm_tc, 116 with gemm_hl;
-// 121 with one shift per bit position and a plane at a time).
+// sums, k-ranges).  Measured, 28672 x 8192, q = 4 + q_bias, 4 rows: 81.4 us = 1.67 TB/s (160 with gemm_tc, 116 with gemm_hl;
+// 121 with one shift per bit position).
 #pragma once
 #include "gemv_tma.cuh"
 

@@ -21,6 +21,13 @@
 //   tcgen05.st as the A operand in tensor memory.
 //   One lane issues tcgen05.mma.kind::f16: M = 128 columns, N = rows, K = 16, A (hi, then lo) in tensor memory, the
 //   activations [rows][64 k] (TMA, 128-byte swizzle) in shared memory, one fp32 accumulator.
+//   Every accumulation of the tensor core cuts its fp32 sum off toward zero: measured, the error of a chain of n is 1.8e-8 n
+//   of the result, whoever's chain it is.  SEG, for fp32 results and long k: chains no longer than gemm_tc's, which its
+//   k-ranges cut.  Lo has an accumulator of its own up to 128 rows, and k is walked in segments: between two, the expansion
+//   warps add the accumulators to sums of their own (fp32, rounded to nearest; in local memory, 64 a thread) while the next
+//   blocks' operands wait.  Relative error of an fp32 result, gemm_tc / one chain / SEG: 28672 x 8192, q = 3, 100 rows 5.8e-6 /
+//   1.8e-5 / 4.9e-6 (141 / 111 / 132 us); 8192 x 28672, q = 1, 300 rows 8.4e-6 / 3.4e-5 / 8.4e-6.  SEG's expansion loop issues some 10 %
+//   more, which fp16 results, whose own rounding is 2.1e-4, do not pay.
 //
 // Tensor memory: 256 accumulator columns, then four operand stages of 64 columns (hi 32, lo 32), one per `sub`.
 //
@@ -43,6 +50,7 @@ constexpr int kHlThreads = (kHlFirstExpWarp + kHlExpWarps) * 32;      // 576
 constexpr int kHlStages = 4;                  // operand stages in tensor memory, one per `sub`
 constexpr uint32_t kHlACol = 256;             // first operand column
 constexpr int kHlMaxSlots = 8;                // activation ring
+constexpr int kHlLoRows = 128;                // up to so many rows lo has accumulators of its own, at this column
 constexpr int kHlTableBytes = kHlExpWarps * 16 * 128;                 // offset 0: [pair of warps][16 values][2 warps][32 lanes] x 4 B
 constexpr int kHlScaleOff = kHlTableBytes;                            // [128] largest |scale| (fp16 bits) per column
 constexpr int kHlBarOff = kHlScaleOff + kHlCols * 4;
@@ -64,6 +72,7 @@ struct HlParams {
     int full_items;          // items (column tile, 256 rows) that one CTA takes whole; the rest go as two halves of 128 rows
     int splits;              // k-ranges per item; a range is blocks_per_split blocks of 64 k
     int blocks_per_split;
+    int segment_lo, segment; // most blocks between two drains, with lo in its own accumulator and without
     int box_rows;            // rows of a TMA box: 128, or m rounded up to 16 when that is less
     int x_slot_bytes, x_slots;
 };
@@ -146,8 +155,26 @@ __device__ __noinline__ float hl_by_product(const HlParams& p, int row, int col,
     return sum;
 }
 
+// Adds this warp's part of the accumulators (16 rows of every 64, lane = column) to `sums`, or puts it there.  lo_col: column
+// of the accumulators of lo, 0 if there are none.
+__device__ __noinline__ void hl_drain(float* sums, uint32_t t_acc, uint32_t lo_col, int sub, int rows, bool add) {
+#pragma unroll 1
+    for (int c = sub, at = 0; 16 * c < rows; c += 4, at += 16) {
+        uint32_t r[16], l[16];
+        tmem_ld_x16(t_acc + 16u * (uint32_t)c, r);
+        if (lo_col) tmem_ld_x16(t_acc + lo_col + 16u * (uint32_t)c, l);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            float v = __uint_as_float(r[i]);
+            if (lo_col) v += __uint_as_float(l[i]);
+            sums[at + i] = add ? sums[at + i] + v : v;
+        }
+    }
+}
+
 // Q: number of bit planes (1..4); BIAS: container has q_bias.  tmX: 2-D map {K, m} of fp16, box {64, box_rows}, 128-byte swizzle.
-template <int Q, bool BIAS>
+template <int Q, bool BIAS, bool SEG>
 __global__ void __launch_bounds__(kHlThreads, 1)
 gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ HlParams p) {
     constexpr int NV = 1 << Q;
@@ -158,7 +185,8 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     const uint32_t bar_xempty = bar_xfull + 8 * kHlMaxSlots;
     const uint32_t bar_afull = bar_xempty + 8 * kHlMaxSlots;      // kHlStages each
     const uint32_t bar_aempty = bar_afull + 8 * kHlStages;
-    const uint32_t bar_acc = bar_aempty + 8 * kHlStages;
+    const uint32_t bar_acc = bar_aempty + 8 * kHlStages;          // a segment's accumulators are complete
+    const uint32_t bar_drained = bar_acc + 8;                     // ... and have been read
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + kHlBarOff + 16 * kHlMaxSlots + 16 * kHlStages + 16);
     int* s_flag = reinterpret_cast<int*>(s_tmem + 1);
     unsigned* s_max = reinterpret_cast<unsigned*>(smem + kHlScaleOff);
@@ -183,6 +211,9 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     const int blocks_total = (p.K + kHlStepK - 1) / kHlStepK;
     const int blk_begin = blockIdx.y * p.blocks_per_split;
     const int nblk = min(blocks_total, blk_begin + p.blocks_per_split) - blk_begin;      // >= 1 by the plan
+    const uint32_t lo_col = SEG && PASSES == 2 && rows <= kHlLoRows ? (uint32_t)kHlLoRows : 0u;
+    const int most = !SEG ? nblk : lo_col || PASSES == 1 ? p.segment_lo : p.segment;
+    const int segments = SEG ? (nblk + most - 1) / most : 1, seg_blocks = SEG ? (nblk + segments - 1) / segments : nblk;
 
     if (tid == 0) {
         for (int s = 0; s < kHlMaxSlots; s++) {
@@ -194,6 +225,7 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
             mbar_init(bar_aempty + 8 * s, 1);
         }
         mbar_init(bar_acc, 1);
+        mbar_init(bar_drained, kHlExpWarps);
         mbar_fence_init();
     }
     if (tid < kHlCols) s_max[tid] = 0u;
@@ -212,7 +244,9 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     const int lq = warp & 3;                                      // TMEM lane quarter this warp may access
     const int ew = warp - kHlFirstExpWarp, sub = ew >> 2;
     const int col_l = lq * 32 + lane, col = n0 + col_l;
+    const uint32_t t_acc = tmem_base + ((uint32_t)(lq * 32) << 16);
     float unscale = 1.f;
+    float sums[SEG ? kHlRows / 4 : 1];                            // of the segments that have been drained
     if (warp >= kHlFirstExpWarp) {
         // ---------------- expansion ----------------
         const size_t row_w = (size_t)Q * N;                       // words per k-word row, scales per group
@@ -299,8 +333,13 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         const uint32_t pair4 = (uint32_t)(ew >> 1) * 0x10101010u;
         unsigned char* tab = smem + (ew >> 1) * 4096 + bank;
         const uint32_t t_dst = tmem_base + ((uint32_t)(lq * 32) << 16) + kHlACol + (uint32_t)sub * 64u;
-        int round = 0;
-        for (int j = sub; j < nblk; j += kHlStages, round++) {
+        int round = 0, j = sub;
+        // segment by segment: this warp's blocks up to and with its first one beyond the segment, then the drain, during which
+        // those blocks wait for the tensor core (the stage of block j is free once block j - 4, of this segment, has been read)
+#pragma unroll 1
+        for (int seg = 0; seg < segments && !timed_out; seg++) {
+        const int upto = seg + 1 < segments ? min(nblk, (seg + 1) * seg_blocks + kHlStages) : nblk;
+        for (; j < upto; j += kHlStages, round++) {
             uint32_t cw[2][Q];
             float a[2][Q], qb[2] = {0.f, 0.f};
 #pragma unroll
@@ -398,6 +437,15 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_afull + 8 * sub);
         }
+        if (SEG && seg + 1 < segments && !timed_out) {
+            if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar_acc, seg & 1))) { timed_out = true; break; }
+            tc_fence_after_sync();
+            hl_drain(sums, t_acc, lo_col, sub, rows, seg > 0);
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_drained);
+        }
+        }
     } else if (warp == kHlTmaWarp) {
         // ---------------- TMA: activation blocks [rows][64 k] (the whole warp walks the loop, lane 0 issues) ----------------
         if (lane == 0) tma_prefetch_descriptor(&tmX);
@@ -426,8 +474,15 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         const uint32_t idesc = umma_idesc_f16_f32(n_mma);
         const uint64_t dx0 = umma_desc_k_sw128(smem_base + kHlXOff);
         const uint32_t elected = elect_one();
-        int xs = 0, xround = 0;
+        int xs = 0, xround = 0, seg = 0, left = 0;                // left: blocks of the segment that are to come
         for (int j = 0; j < nblk; j++) {
+            const bool first = SEG ? left == 0 : j == 0;
+            if (SEG && first) {
+                if (seg > 0 && !__all_sync(0xffffffffu, mbar_wait_bounded(bar_drained, (seg - 1) & 1))) { timed_out = true; break; }
+                left = seg_blocks;
+                seg++;
+            }
+            if (SEG) left--;
             const int st = j & (kHlStages - 1);
             const uint32_t ap = (uint32_t)(j / kHlStages) & 1u;
             if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar_xfull + 8 * xs, xround & 1) && mbar_wait_bounded(bar_afull + 8 * st, ap))) {
@@ -441,10 +496,11 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
             for (int ps = 0; ps < PASSES; ps++)
 #pragma unroll
                 for (int k16 = 0; k16 < 4; k16++)
-                    umma_f16_ts_if(elected, tmem_base, a_t + (uint32_t)(ps * 32 + k16 * 8), dx + (uint64_t)(k16 * 2), idesc,
-                                   (j | ps | k16) ? 1u : 0u);
+                    umma_f16_ts_if(elected, tmem_base + (ps ? lo_col : 0u), a_t + (uint32_t)(ps * 32 + k16 * 8), dx + (uint64_t)(k16 * 2),
+                                   idesc, k16 || !first || (ps && !lo_col) ? 1u : 0u);
             umma_commit_if(elected, bar_aempty + 8 * st);
             umma_commit_if(elected, bar_xempty + 8 * xs);
+            if (SEG && left == 0 && j + 1 < nblk) umma_commit_if(elected, bar_acc);
             if (++xs == p.x_slots) { xs = 0; xround++; }
         }
         umma_commit_if(elected, bar_acc);
@@ -456,10 +512,9 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     // ---------------- epilogue: TMEM lane = output column, TMEM column = activation row ----------------
     const bool split = p.splits > 1;
     if (warp >= kHlFirstExpWarp) {
-        const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar_acc, 0));
+        const bool ok = __all_sync(0xffffffffu, !timed_out && mbar_wait_bounded(bar_acc, (segments - 1) & 1));
         if (!ok) atomicExch(p.status, kStatusTcTimeout);
         tc_fence_after_sync();
-        const uint32_t t_src = tmem_base + ((uint32_t)(lq * 32) << 16);
         // the activation ring is idle: every load has been consumed when the accumulators are complete
         float* scratch = reinterpret_cast<float*>(smem + kHlXOff) + ew * (16 * 33);
         // columns that the split operand does not hold exactly (not finite: nothing to be exact about)
@@ -472,8 +527,19 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         const bool any_wide = __any_sync(0xffffffffu, wide);
         for (int c = sub; 16 * c < rows && ok; c += 4) {          // 16 activation rows per tcgen05.ld; warp-uniform
             uint32_t r[16];
-            tmem_ld_x16(t_src + 16u * (uint32_t)c, r);
+            tmem_ld_x16(t_acc + 16u * (uint32_t)c, r);
+            if (SEG && lo_col) {
+                uint32_t l[16];
+                tmem_ld_x16(t_acc + lo_col + 16u * (uint32_t)c, l);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(l[i]));
+            }
             tmem_ld_wait();
+            if (SEG && segments > 1) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) + sums[4 * (c - sub) + i]);
+            }
 #pragma unroll
             for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) * unscale);
             unsigned redo = wide ? 0xffffu : 0u;

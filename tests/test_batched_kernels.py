@@ -226,3 +226,21 @@ def test_plane_kernel_activations_not_finite():
                                             (36, 4128, 3, 96, True, 18), (264, 8192, 2, 512, False, 4)])
 def test_register_operand_kernel_activations_not_finite(N, K, q, g, bias, m):
     _not_finite(N, K, q, g, bias, m, "gemm_frag_kernel")
+
+
+@pytest.mark.parametrize("N,K,q,bias,m", [(1024, 8192, 1, False, 2048), (1024, 8192, 2, False, 2048), (264, 8192, 3, False, 64), (520, 4096, 4, True, 300)])
+def test_split_operand_kernel_sums_are_as_close_as_the_plane_kernels(N, K, q, bias, m):
+    """Every accumulation of the tensor core cuts its sum off: an fp32 result is no further off than the chains of the plane
+    kernel make it, 8 accumulations per plane and 128 k, over 8 k-ranges at these widths."""
+    bW, alpha, q_bias = synth.bcq_layer(N, K, q, 128, seed=N + m, with_bias=bias)
+    x = synth.activations(m, K, seed=m)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // 128, q_bias).reserve_batch(m)
+    y = torch.empty((m, N), dtype=torch.float32, device="cuda")
+    L.matmul_f32(y, torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16), w, m)
+    assert L.last_launch()[0] == "gemm_hl_kernel"
+    rows = np.arange(0, m, max(1, m // 32))
+    ref = oracle.bcq_matmul_f64(np.ascontiguousarray(x[rows]), bW, alpha.astype(np.float16), None if q_bias is None else q_bias.astype(np.float16), 128)
+    chain = 8 * (q + bias) * (K // 128) / 8
+    # 1.8e-8 per accumulation is what the tensor core was measured at; 1.2 for the spread, and the fp32 roundings of the rest
+    assert np.linalg.norm(y.cpu().numpy()[rows] - ref) <= (1.2 * 1.8e-8 * chain + 2.0 ** -22) * np.linalg.norm(ref)
+    w.close()
