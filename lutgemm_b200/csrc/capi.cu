@@ -663,8 +663,9 @@ int gemm_tc_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 // ---- split-operand kernel (gemm_hl.cuh): plan, launch ----
 // Longest chain of tensor-core accumulations (each cuts the fp32 sum off) between two drains: the plane kernel's, 8 per plane
 // and 128 k, less a sixteenth, so that an fp32 result is no further off than that kernel's.  An fp16 result has an error of 2.1e-4 of its own; a
-// chain of 1024 adds 1.8e-5 to that, 0.4 % of it, and costs no drain up to 8192 k.
-constexpr int kHlChain16 = 1024;
+// chain of 1536 adds 2.8e-5 to that, 0.9 % of it, and costs no drain up to 12288 k (12288 x 12288, q = 4 + q_bias, 1024 rows:
+// 427 us, 464 with one drain).
+constexpr int kHlChain16 = 1536;
 int hl_chain(const lutgemm_weight* w, bool ordered, bool f32) {
     const int plane = 8 * (w->q + (w->q_bias ? 1 : 0)) * tc_steps_per_cta(w, ordered);
     return f32 ? plane - plane / 16 : plane > kHlChain16 ? plane : kHlChain16;
@@ -760,7 +761,8 @@ int hl_split_rows_of(const lutgemm_weight* w) {
 // 4096 31 / 35, 8192 x 28672, fp16 96 / 108; more passes as above (3 passes, 28672 x 8192, 100 rows, fp32 141 / 132).
 bool gemm_hl_ok(const lutgemm_weight* w, int m, bool f32) {
     const int passes = w->q + (w->q_bias ? 1 : 0);
-    const bool drains = f32 || w->K > 16 * kHlChain16;            // (two k-ranges at the widths where that is not so)
+    const int T = (w->N + lg::kHlCols - 1) / lg::kHlCols, ranges = sm_count() / T < 1 ? 1 : sm_count() / T;
+    const bool drains = f32 || w->K / 8 > kHlChain16 * ranges;    // up to 128 rows: 8 accumulations per 64 k of a range
     const int from = passes >= 5 ? 4 : passes >= 3 ? 64 : passes == 2 && !drains ? 97 : 129;
     // with g = 32 every block builds two tables: up to 128 rows, where the expansion bounds it, that goes to gemm_tc
     return w->tc_ok && w->q <= 4 && m >= from && (m > 128 || w->g >= lg::kHlStepK);
