@@ -875,10 +875,13 @@ int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 
 // ---- register-operand kernel (gemm_frag.cuh): plan, launch ----
 // One CTA per SM and one wave: the slabs of k first (a slab is what the warps of a CTA hold activations for), then as many
-// column ranges as still fit.  Cost in units of 4096 weights: the longest warp's share, plus what a column tile's sum and a
-// slab's start cost.
+// column ranges as still fit.  Cost in units of 4096 weights per warp: half the longest warp's share and half the average one
+// (the SM's pipes are shared: 28672 x 8192, q = 4 + q_bias, 4 rows, where the longest share is the same, 2 / 4 / 8 slabs with 416 /
+// 400 / 400 units to the CTA 68.3 / 65.3 / 64.7 us), plus what a column tile's sum and a slab's start cost.
 bool frag_plan(const lutgemm_weight* w, int m, lg::FrParams* p, dim3* grid) {
     if (w->N % 4 != 0 || m > lg::kFrMaxRows) return false;
+    // the kernel's byte offsets and its division by g / 32 are 32 bits wide
+    if ((long long)(w->K / 32) * w->q * w->N * 4 >= 1ll << 32 || (long long)(w->K / 32 + 64) * (w->g / 32) >= 1ll << 32) return false;
     const int gw = w->g % 128 == 0 ? 4 : w->g % 64 == 0 ? 2 : 1;
     p->depth = lg::fr_depth(gw, m <= 8 ? 1 : 2, w->q, w->q_bias != nullptr);
     if (p->depth < 2) return false;
@@ -894,7 +897,8 @@ bool frag_plan(const lutgemm_weight* w, int m, lg::FrParams* p, dim3* grid) {
         ranges = (tiles + tpc - 1) / tpc;
         const int cw = lg::kFrWarps / kw, rounds = (tpc + cw - 1) / cw, wsteps = (sps + kw - 1) / kw;
         const double waves = (double)(((long long)slabs * ranges + sms - 1) / sms);
-        const double t = waves * (12.0 + rounds * (wsteps * P + 1.0)) + (slabs > 1 ? 8.0 : 0.0);
+        const double longest = rounds * (wsteps * P + 1.0), average = (double)tpc * sps * (P + 1.0) / lg::kFrWarps;
+        const double t = waves * (12.0 + 0.5 * (longest + average)) + (slabs > 1 ? 8.0 : 0.0);
         if (t < best) {
             best = t;
             p->kw = kw; p->steps_per_slab = sps; p->tiles_per_cta = tpc;
@@ -904,11 +908,11 @@ bool frag_plan(const lutgemm_weight* w, int m, lg::FrParams* p, dim3* grid) {
     return grid->y <= 65535;
 }
 
-template <int MT, int GW>
+template <int MT, int GW, int Q>
 int launch_gemm_frag(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, cudaStream_t st) {
     static bool configured[64][2] = {};   // the attribute is per device
     const bool bias = w->q_bias != nullptr;
-    auto kern = bias ? lg::gemm_frag_kernel<MT, GW, true> : lg::gemm_frag_kernel<MT, GW, false>;
+    auto kern = bias ? lg::gemm_frag_kernel<MT, GW, true, Q> : lg::gemm_frag_kernel<MT, GW, false, Q>;
     int dev = 0;
     LG_CUDA(cudaGetDevice(&dev));
     if (dev >= 64 || !configured[dev][bias]) {
@@ -931,6 +935,19 @@ int launch_gemm_frag(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, 
     return LUTGEMM_OK;
 }
 
+// Up to four planes of groups of 64 or more have a kernel each, their loops unrolled: 2048 x 2048, q = 4, 4 rows 5.2 us, 5.7 with
+// the kernel for any number of planes; 28672 x 8192, 64.9 and 67.2.
+template <int GW>
+int launch_gemm_frag_q(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, cudaStream_t st) {
+    switch (GW == 1 ? 0 : w->q) {
+        case 1: return launch_gemm_frag<1, GW, GW == 1 ? 0 : 1>(w, p, grid, st);
+        case 2: return launch_gemm_frag<1, GW, GW == 1 ? 0 : 2>(w, p, grid, st);
+        case 3: return launch_gemm_frag<1, GW, GW == 1 ? 0 : 3>(w, p, grid, st);
+        case 4: return launch_gemm_frag<1, GW, GW == 1 ? 0 : 4>(w, p, grid, st);
+        default: return launch_gemm_frag<1, GW, 0>(w, p, grid, st);
+    }
+}
+
 int gemm_frag_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, lg::FrParams p, dim3 grid, const __half* x, __half* y16,
                    float* y32, int m, cudaStream_t st) {
     p.bW = w->bW; p.alpha = w->alpha; p.q_bias = w->q_bias; p.x = x;
@@ -938,9 +955,10 @@ int gemm_frag_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, lg::FrP
     p.y16 = y16; p.y32 = y32;
     p.N = w->N; p.K = w->K; p.q = w->q; p.g = w->g; p.m = m;
     p.ones = 0x3c003c00u; p.twos = 0x40004000u; p.fours = 0x44004400u;
-    if (w->g % 128 == 0) return m <= 8 ? launch_gemm_frag<1, 4>(w, p, grid, st) : launch_gemm_frag<2, 4>(w, p, grid, st);
-    if (w->g % 64 == 0) return m <= 8 ? launch_gemm_frag<1, 2>(w, p, grid, st) : launch_gemm_frag<2, 2>(w, p, grid, st);
-    return m <= 8 ? launch_gemm_frag<1, 1>(w, p, grid, st) : launch_gemm_frag<2, 1>(w, p, grid, st);
+    p.group_magic = w->g == 32 ? 0u : (uint32_t)(((1ull << 32) + w->g / 32 - 1) / (w->g / 32));
+    if (w->g % 128 == 0) return m <= 8 ? launch_gemm_frag_q<4>(w, p, grid, st) : launch_gemm_frag<2, 4, 0>(w, p, grid, st);
+    if (w->g % 64 == 0) return m <= 8 ? launch_gemm_frag_q<2>(w, p, grid, st) : launch_gemm_frag<2, 2, 0>(w, p, grid, st);
+    return m <= 8 ? launch_gemm_frag_q<1>(w, p, grid, st) : launch_gemm_frag<2, 1, 0>(w, p, grid, st);
 }
 
 template <int Q>
@@ -1011,19 +1029,22 @@ int gemm_i8_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
     return LUTGEMM_ERR_BITS;
 }
 
-// Batches that the register-operand kernel is the fastest for.  Measured, us, register operand against what ran instead,
-// g = 128: 8192 x 8192, q = 2, 2 rows 17.6 / 13.1 (two-row LUT kernel), 3 rows 17.8 / 21.5 (that and one LUT row; on
-// larger weights these two are the faster: 256 / 207); q = 3, 4 rows
-// 22.2 / 28.7, 8 rows 23.8 / 28.9, 16 rows 32.9 / 29.8 (gemm_tc); q = 1, 8 rows 14.8 / 16.0; 12288 x 4096, q = 4, 8 rows
-// 20.1 / 25.7, 16 rows 34.4 / 26.3; 2048 x 2048, q = 4, 4 rows 4.7 / 8.1; 28672 x 8192, q = 4 + q_bias, 4 rows 82.6 / 116.5
-// (gemm_hl); g = 64, 28672 x 8192, q = 4, 4 rows 90.7 / 113.2, 8 rows 95.5 / 114.0; g = 32 (four scales to a unit) 8 rows
-// 118.9 / 114.1, which is why it stays with gemm_tc.  Containers that the tcgen05 kernels refuse (N % 8 != 0, or a group size that neither divides nor is a multiple
-// of 128) take it for every batch, 16 rows at a time: what is left for them is one matvec per row.
+// Batches that the register-operand kernel is the fastest for.  Measured, us, register operand against what ran instead, g = 128
+// unless stated.  Two rows (two-row LUT kernel): 2048 x 2048, q = 4, 4.4 / 7.4; 4096 x 4096, q = 3, 6.3 / 7.1; 8192 x 2048, q = 3 + q_bias,
+// 6.5 / 7.4; 8192 x 4096, q = 2, 7.5 / 8.2; 8192 x 8192, q = 2, 14.2 / 11.5, and with k in slabs 2048 x 8192, q = 3, 8.0 / 7.1: one slab and
+// up to kFragPairWeights weights of planes.  Three (that kernel and one LUT row): 4096 x 4096,
+// q = 3, 6.3 / 12.6; 12288 x 12288, q = 3, 35.6 / 40.6; 49152 x 12288, q = 3, 127 / 135; 28672 x 8192, q = 4 + q_bias, 65.0 / 78.0; g =
+// 64, 8192 x 8192, q = 3, 19.6 / 26.0, but g = 32 26.3 / 26.3.  More rows: q = 3, 8192 x 8192, 8 rows 20.5 / 28.9, 12 rows 29.2 / 28.7
+// (gemm_tc); 12288 x 4096, q = 4, 8 rows 17.0 / 25.7; 28672 x 8192, q = 4 + q_bias, 4 rows 64.8 / 116.5 (gemm_hl); g = 64, 28672 x
+// 8192, q = 4, 4 rows 72.7 / 113.2; g = 32 (four scales to a unit) 8 rows 106.7 / 112.3, but 8192 x 8192 with fewer planes
+// the other way, which is why it stays with gemm_tc.  Containers that the tcgen05 kernels refuse (N % 8 != 0, or a group size that
+// neither divides nor is a multiple of 128) take it for every batch, 16 rows at a time: what is left for them is one matvec per row.
+constexpr long long kFragPairWeights = 64ll << 20;
 bool frag_wanted(const lutgemm_weight* w, const lutgemm_workspace* ws, int m) {
     if (m < 2 || w->N % 4 != 0 || ordered_for(ws) || gemm_i8_ok(w, m)) return false;
     if (m < kBatchedFromRows && g_variant.load() != 0) return false;       // the caller asked for a matvec kernel by name
-    if (m == 2) return false;
-    if (m == 3) return !gemv_pair_ok(w, ws);
+    if (m == 2) return w->g % 64 == 0 && gemv_pair_ok(w, ws) && (long long)w->N * w->K * w->q <= kFragPairWeights;
+    if (m == 3) return w->g % 64 == 0 || !gemv_pair_ok(w, ws);
     return !w->tc_ok || (m <= 8 && w->g % 64 == 0);
 }
 
@@ -1036,6 +1057,7 @@ int frag_rows_if_ready(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x
     const int whole = m / lg::kFrMaxRows, rest = m % lg::kFrMaxRows;       // launches of 16 rows, and one of the rest
     if (whole && !frag_plan(w, lg::kFrMaxRows, &p[0], &grid[0])) return LUTGEMM_OK;
     if (rest && !frag_plan(w, rest, &p[1], &grid[1])) return LUTGEMM_OK;
+    if (m == 2 && grid[1].y > 1) return LUTGEMM_OK;
     if (m >= kBatchedFromRows && w->tc_ok) {
         // what a call without reserved scratch is told does not depend on the kernel: the plane kernel's rule
         int unused_split = 1, unused_steps = 0;

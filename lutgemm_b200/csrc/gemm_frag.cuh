@@ -22,10 +22,16 @@
 // than four, the four lanes t of a product share the words of one group (each takes NJ = 4 GW of the 16 bit positions).
 // MT: tiles of 8 activation rows (1 or 2).  KS: units along k that a warp keeps activations for (2 for 8 rows, 1 for 16).
 //
-// Bound by instruction issue and its latencies: per plane and 4096 weights 64 LOP3, 20 shifts and 16 MT mma.sync, on 16 warps
-// that 128 registers a thread allow; plus some 10 us at 8192 x 8192 that do not grow with the planes (activations, column
-// sums, k-ranges).  Measured, 28672 x 8192, q = 4 + q_bias, 4 rows: 81.4 us = 1.67 TB/s (160 with gemm_tc, 116 with gemm_hl;
-// 121 with one shift per bit position).
+// Bound by the operands' making and the products together: per plane and 4096 weights 64 LOP3 on a pipe that takes half a warp a
+// cycle (32 cycles per SM), 20 shifts as multiplications on the other, 16 MT mma.sync at 1024 multiply-adds a cycle (33 MT
+// cycles): 52 cycles at MT = 1 and 88 at MT = 2 on registers alone.  What a unit costs beside its planes is then the rest,
+// and is kept small: all planes' loops unrolled (Q), addresses as 32-bit offsets from the tensors' bases, pieces beyond an end
+// fetched as zeros rather than branched around, words in shared memory at places that 16-byte reads find without conflicts
+// (chunk XOR k-word), the accumulators' start as the first product's C operand (it was copied: 8 moves a plane).  156
+// instructions a plane instead of 192.  Measured, us, with this / before, 28672 x 8192, q = 4 + q_bias, 4 rows: 64.8 / 80.0 = 2.1
+// TB/s (160 with gemm_tc, 116 with gemm_hl); 49152 x 12288, q = 3, 4 rows: 126.7 / 149.6; 8192 x 8192, q = 2, 4 rows: 14.3 /
+// 17.2; 2048 x 2048, q = 4, 4 rows: 4.37 / 4.43.  Activations in shared memory and runs of units per warp instead of a k-range
+// per warp: 64.4, but 1 to 2 us more below 4096 x 4096.
 #pragma once
 #include "gemv_tma.cuh"
 
@@ -45,7 +51,7 @@ __host__ __device__ constexpr int fr_red_floats(int mt) { return 4 * mt * 8 * kF
 __host__ __device__ constexpr int fr_depth(int gw, int mt, int q, bool bias) {
     const int per_warp = (kFrSmemBytes - kFrTailBytes - 2 * kFrWarps * fr_red_floats(mt) * 4) / kFrWarps;
     const int d = per_warp / fr_unit_bytes(gw, q, bias);
-    return d > kFrMaxDepth ? kFrMaxDepth : d;
+    return d >= kFrMaxDepth ? kFrMaxDepth : d >= 3 ? 3 : d;       // a wait for each of these
 }
 
 struct FrParams {
@@ -64,13 +70,15 @@ struct FrParams {
     int depth;               // units of a warp's ring
     // fp16 pairs of 1, 2 and 4: as arguments they stay in registers; as literals the compiler made them anew for every LOP3
     uint32_t ones, twos, fours;
+    uint32_t group_magic;    // ceil(2^32 / (g / 32)), 0 for g = 32: k-word -> scale group
 };
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool live) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+// `size` bytes (all or none: then src is not read) and zeros behind them
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t size) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
 }
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, bool live) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(live ? 8 : 0) : "memory");
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, uint32_t size) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -81,6 +89,12 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// D = A B + C
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2], const float4& c) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(c.x), "f"(c.y), "f"(c.z), "f"(c.w));
 }
 // Where bit position pos of a half goes (shift left by fr_shift) and what it becomes there: class 0 the sign, 1 to 3 as above.
 __host__ __device__ constexpr int fr_shift(int pos) {
@@ -113,8 +127,8 @@ __device__ __forceinline__ uint32_t fr_operand(uint32_t word, uint32_t ones, uin
 }
 // One plane of one scale group: both operand tiles times MT x 8 rows.  Product S: positions FIRST + 2 S, FIRST + 2 S + 1.
 template <int S, int COUNT, int FIRST, int MT>
-__device__ __forceinline__ void fr_products(float (&d0)[MT][4], float (&d1)[MT][4], const uint32_t (&w)[4],
-                                            const uint32_t (&bx)[COUNT][MT][2], uint32_t ones, uint32_t twos, uint32_t fours) {
+__device__ __forceinline__ void fr_products(float (&d0)[MT][4], float (&d1)[MT][4], const uint32_t (&w)[4], const uint32_t (&bx)[COUNT][MT][2],
+                                            const float4 (&start)[MT], uint32_t ones, uint32_t twos, uint32_t fours) {
     if constexpr (S < COUNT) {
         constexpr int P0 = FIRST + 2 * S, P1 = P0 + 1;
         const uint32_t a0[4] = {fr_operand<P0>(w[0], ones, twos, fours), fr_operand<P0>(w[1], ones, twos, fours),
@@ -123,10 +137,15 @@ __device__ __forceinline__ void fr_products(float (&d0)[MT][4], float (&d1)[MT][
                                 fr_operand<P1>(w[2], ones, twos, fours), fr_operand<P1>(w[3], ones, twos, fours)};
 #pragma unroll
         for (int nt = 0; nt < MT; nt++) {
-            mma_16816(d0[nt], a0, bx[S][nt]);
-            mma_16816(d1[nt], a1, bx[S][nt]);
+            if constexpr (S == 0) {
+                mma_16816(d0[nt], a0, bx[S][nt], start[nt]);
+                mma_16816(d1[nt], a1, bx[S][nt], start[nt]);
+            } else {
+                mma_16816(d0[nt], a0, bx[S][nt]);
+                mma_16816(d1[nt], a1, bx[S][nt]);
+            }
         }
-        fr_products<S + 1, COUNT, FIRST, MT>(d0, d1, w, bx, ones, twos, fours);
+        fr_products<S + 1, COUNT, FIRST, MT>(d0, d1, w, bx, start, ones, twos, fours);
     }
 }
 // What those accumulators start from: the offsets' products.
@@ -191,7 +210,8 @@ __device__ __noinline__ void fr_by_product(const FrParams& p, unsigned rows, int
     }
 }
 
-template <int MT, int GW, bool BIAS>
+// Q: planes, 0 for any number.
+template <int MT, int GW, bool BIAS, int Q>
 __global__ void __launch_bounds__(kFrThreads, 1)
 gemm_frag_kernel(const __grid_constant__ FrParams p) {
     constexpr int KS = MT == 1 ? 2 : 1;
@@ -203,7 +223,7 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
     const int r = lane >> 2, t = lane & 3;
     const int kw_log = 31 - __clz(p.kw), kw_mask = p.kw - 1;
     const int wk = warp & kw_mask, wc = warp >> kw_log, cw = kFrWarps >> kw_log;
-    const int N = p.N, K = p.K, q = p.q;
+    const int N = p.N, K = p.K, q = Q ? Q : p.q;
     const uint32_t ones = p.ones, twos = p.twos, fours = p.fours;
     const int P = q + (BIAS ? 1 : 0);
     const int a_off = q * 512, ub = a_off + P * NG * 64;          // a unit: words of the planes, then scales [plane][group][32 columns]
@@ -223,47 +243,42 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
     const int tile0 = blockIdx.x * p.tiles_per_cta, tile1 = min(tiles, tile0 + p.tiles_per_cta);
 
     // ---- the warp's stream of units: (tile, step) ----
-    int ftile = nsteps ? tile0 + wc : tile1, fi = 0, fslot = 0;
-    const int nalpha = P * NG * 8;            // 8-byte pieces of scales
+    // Byte offsets are 32 bits wide (the plan refuses more); beyond the end of the stream, the columns or K zeros come instead.
+    const uint32_t row_b = (uint32_t)q * (uint32_t)N * 4u;       // bytes of a k-word row of words
+    const int f_kw = lane >> 3, f_chunk = lane & 7;
+    int fi = 0, fslot = 0, fcol = (tile0 + wc) * kFrCols + 4 * f_chunk;
+    const int fcol_end = nsteps ? min(N, tile1 * kFrCols) : 0;    // N % 4 == 0: whole quads
+    // this lane's 16 bytes of every plane: chunks of a k-word's 128 bytes at their number XOR the k-word (conflict-free reads below)
+    const uint32_t f_dst = ring_u + f_kw * 128 + (f_chunk ^ f_kw) * 16;
+    // and its 8 bytes of scales: four (of NG groups: 4 / NG) planes at a time
+    constexpr int PB = 4 / NG;
+    const int f_plane = f_kw / NG, f_group = f_kw % NG;
+    const uint32_t f_adst = ring_u + a_off + lane * 8;
     auto fetch = [&]() {
-        if (ftile < tile1) {
-            const int step = slab0 + wk + fi * p.kw;
-            const uint32_t dst = ring_u + fslot * ub;
-            {
-                const int kw = 4 * step + (lane >> 3), col = ftile * kFrCols + 4 * (lane & 7);
-                const bool ok = col < N && kw < words;            // N % 4 == 0: whole quads
-                const uint32_t* src = ok ? p.bW + (size_t)kw * q * N + col : p.bW;
-                const size_t inc = ok ? (size_t)N : 0;
-#pragma unroll 4
-                for (int b = 0; b < q; b++) {
-                    cp_async16(dst + b * 512 + lane * 16, src, ok);
-                    src += inc;
-                }
-            }
-            for (int at = lane; at < nalpha; at += 32) {
-                const int b = at / (NG * 8), gi = (at >> 3) % NG, col = ftile * kFrCols + 4 * (at & 7);
-                const int k = 128 * step + 32 * GW * gi;
-                const bool ok = col < N && k < K;
-                const size_t grp = ok ? (size_t)((unsigned)k / (unsigned)p.g) : 0;
-                const __half* src = (!BIAS || b < q) ? p.alpha + (grp * q + b) * N + col : p.q_bias + grp * N + col;
-                cp_async8(dst + a_off + at * 8, ok ? src : p.alpha, ok);
-            }
-            if (++fslot == p.depth) fslot = 0;
-            if (++fi == nsteps) {
-                fi = 0;
-                ftile += cw;
-            }
+        const int kw0 = 4 * (slab0 + wk + fi * p.kw), akw = kw0 + GW * f_group;
+        const int end = fcol < fcol_end ? words : 0;
+        const uint32_t size = kw0 + f_kw < end ? 16u : 0u, asize = akw < end ? 8u : 0u, at = fslot * ub;
+        const uint32_t off = (uint32_t)(kw0 + f_kw) * row_b + (uint32_t)fcol * 4u;
+#pragma unroll
+        for (int b = 0; b < (Q ? Q : 8); b++)
+            if (Q || b < q) cp_async16(f_dst + at + b * 512, reinterpret_cast<const unsigned char*>(p.bW) + (off + b * ((uint32_t)N * 4u)), size);
+        const uint32_t grp = GW == 1 && !p.group_magic ? (unsigned)akw : __umulhi((unsigned)akw, p.group_magic);
+        const uint32_t aoff = ((grp * q + f_plane) * (uint32_t)N + fcol) * 2u;
+#pragma unroll
+        for (int b = 0; b < (Q ? Q : 8); b += PB)
+            if (b + f_plane < q) cp_async8(f_adst + at + b * (NG * 64), reinterpret_cast<const unsigned char*>(p.alpha) + (aoff + b * ((uint32_t)N * 2u)), asize);
+        if (BIAS && f_plane == 0) cp_async8(f_adst + at + q * (NG * 64), reinterpret_cast<const unsigned char*>(p.q_bias) + (grp * (uint32_t)N + fcol) * 2u, asize);
+        if (++fslot == p.depth) fslot = 0;
+        if (++fi == nsteps) {
+            fi = 0;
+            fcol += cw * kFrCols;
         }
-        cp_async_commit();                    // one group per unit, empty ones at the end: the wait below counts groups
+        cp_async_commit();                    // one group per unit: the wait below counts groups
     };
     auto wait_unit = [&]() {                  // all but the last depth - 2 groups
-        switch (p.depth) {
-            case 2: cp_async_wait<0>(); break;
-            case 3: cp_async_wait<1>(); break;
-            case 4: cp_async_wait<2>(); break;
-            case 5: cp_async_wait<3>(); break;
-            default: cp_async_wait<4>(); break;
-        }
+        if (p.depth == 2) cp_async_wait<0>();
+        else if (p.depth == 3) cp_async_wait<1>();
+        else cp_async_wait<kFrMaxDepth - 2>();
         __syncwarp();                         // every lane's copies of this unit have landed, every lane has read the previous one
     };
     // packed words and scales are never written by a kernel: the stream starts while the previous kernel drains
@@ -274,7 +289,7 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
 
     // ---- activations of this warp's k-range, in operand order ----
     uint32_t bx[KS][NG][NJ / 2][MT][2];
-    float start[KS][NG][MT][2];               // what the accumulators of rows 8 nt + 2 t, + 1 start from
+    float4 start[KS][NG][MT];                 // what the accumulators start from: rows 8 nt + 2 t, + 1, the same of the tile's other half
     float sx[KS][NG][MT][2];                  // BIAS: sums of the group's activations for those rows
     unsigned open = 0u;                       // rows with an activation that is not finite: nor is, then, what they start from
 #pragma unroll
@@ -314,8 +329,7 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
             fr_start<0, NJ / 2, FIRST, MT>(d, bx[i][gi]);
 #pragma unroll
             for (int nt = 0; nt < MT; nt++) {
-                start[i][gi][nt][0] = d[nt][0];
-                start[i][gi][nt][1] = d[nt][1];
+                start[i][gi][nt] = make_float4(d[nt][0], d[nt][1], d[nt][0], d[nt][1]);
 #pragma unroll
                 for (int e = 0; e < 2; e++) open |= fabsf(d[nt][e]) <= 3.402823466e38f ? 0u : 1u << (8 * nt + 2 * t + e);
                 if (BIAS) {
@@ -335,6 +349,7 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
 
     // ---- columns ----
     const int my_tiles = (tile1 - tile0 + cw - 1) >> (4 - kw_log);      // every warp of the CTA walks as many: the barriers match
+    const int quad = (r >> 1) + 4 * (r & 1);  // this lane's columns of a tile: two lanes r of a quarter warp are four chunks apart
     int slot = 0, parity = 0;
 #pragma unroll 1
     for (int ti = 0; ti < my_tiles; ti++) {
@@ -352,24 +367,20 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
                 fetch();
                 const unsigned char* u = ring + slot * ub;
                 if (++slot == p.depth) slot = 0;
-#pragma unroll 1
-                for (int b = 0; b < q; b++) {
+                auto plane = [&](int b) {
 #pragma unroll
                     for (int gi = 0; gi < NG; gi++) {
-                        const uint2 av = *reinterpret_cast<const uint2*>(u + a_off + (b * NG + gi) * 64 + r * 8);
+                        const int kw = gi * GW + ((t * GW) >> 2);
+                        const uint2 av = *reinterpret_cast<const uint2*>(u + a_off + (b * NG + gi) * 64 + quad * 8);
+                        const uint4 wv = *reinterpret_cast<const uint4*>(u + b * 512 + kw * 128 + (quad ^ kw) * 16);
                         const float2 a01 = half2_bits_to_float2(av.x), a23 = half2_bits_to_float2(av.y);
-                        const uint4 wv = *reinterpret_cast<const uint4*>(u + b * 512 + (gi * GW + ((t * GW) >> 2)) * 128 + r * 16);
                         uint32_t w[4] = {wv.x, wv.y, wv.z, wv.w};
                         if (GW < 4) {         // this lane's NJ positions to the top of each half
 #pragma unroll
                             for (int c = 0; c < 4; c++) w[c] <<= FIRST - (t * GW % 4) * 4;
                         }
                         float d0[MT][4], d1[MT][4];
-#pragma unroll
-                        for (int nt = 0; nt < MT; nt++)
-#pragma unroll
-                            for (int e = 0; e < 4; e++) d0[nt][e] = d1[nt][e] = start[i][gi][nt][e & 1];
-                        fr_products<0, NJ / 2, FIRST, MT>(d0, d1, w, bx[i][gi], ones, twos, fours);
+                        fr_products<0, NJ / 2, FIRST, MT>(d0, d1, w, bx[i][gi], start[i][gi], ones, twos, fours);
 #pragma unroll
                         for (int nt = 0; nt < MT; nt++)
 #pragma unroll
@@ -380,11 +391,18 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
                                 acc[3][nt][e] = fmaf(a23.y, d1[nt][2 + e], acc[3][nt][e]);
                             }
                     }
+                };
+                if constexpr (Q != 0) {
+#pragma unroll
+                    for (int b = 0; b < Q; b++) plane(b);
+                } else {
+#pragma unroll 1
+                    for (int b = 0; b < q; b++) plane(b);
                 }
                 if (BIAS) {
 #pragma unroll
                     for (int gi = 0; gi < NG; gi++) {
-                        const uint2 av = *reinterpret_cast<const uint2*>(u + a_off + (q * NG + gi) * 64 + r * 8);
+                        const uint2 av = *reinterpret_cast<const uint2*>(u + a_off + (q * NG + gi) * 64 + quad * 8);
                         const float2 a01 = half2_bits_to_float2(av.x), a23 = half2_bits_to_float2(av.y);
 #pragma unroll
                         for (int nt = 0; nt < MT; nt++)
@@ -408,7 +426,7 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
                 for (int nt = 0; nt < MT; nt++)
 #pragma unroll
                     for (int e = 0; e < 2; e++)
-                        mine[((c * MT + nt) * 8 + 2 * t + e) * kFrRedStride + r] = acc[c][nt][e];
+                        mine[((c * MT + nt) * 8 + 2 * t + e) * kFrRedStride + quad] = acc[c][nt][e];
             asm volatile("bar.sync %0, %1;" ::"r"(1 + wc), "r"(p.kw * 32) : "memory");
             // 64 MT (row, column quad) sums by two warps per 8 rows, other warps each time
             const int turn = (wk - ti * 2 * MT) & kw_mask;

@@ -94,6 +94,21 @@ def test_register_operand_kernel(N, K, q, g, bias, m):
     _run("gemm_frag_kernel", N, K, q, g, bias, m)
 
 
+# one to four planes have kernels of their own: a last tile of one quad, a last step of two words, several tiles and steps to a warp
+@pytest.mark.parametrize("q", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K,g,bias,m", [(68, 192, 64, True, 4), (5220, 1152, 64, False, 8), (68, 128, 128, False, 5), (9508, 768, 384, True, 4)])
+def test_register_operand_kernel_per_plane_count(N, K, q, g, bias, m):
+    _run("gemm_frag_kernel", N, K, q, g, bias, m)
+
+
+# two and three rows: the register operand up to 64 Mi weights of planes and where one slab of k is enough, else the LUT kernels
+@pytest.mark.parametrize("N,K,q,g,bias,m,kernel", [
+    (72, 128, 1, 64, True, 2, "gemm_frag_kernel"), (4096, 4096, 4, 128, False, 2, "gemm_frag_kernel"), (4104, 4096, 4, 128, False, 2, "gemv_tma2_kernel"),
+    (72, 8192, 1, 128, False, 2, "gemv_tma2_kernel"), (72, 192, 2, 32, True, 2, "gemv_tma2_kernel"), (72, 8192, 1, 128, True, 3, "gemm_frag_kernel")])
+def test_two_and_three_rows(N, K, q, g, bias, m, kernel):
+    _run(kernel, N, K, q, g, bias, m)
+
+
 @pytest.mark.parametrize("q,g,bias,m", [(4, 128, True, 8), (3, 64, False, 4), (2, 32, True, 5)])
 def test_register_operand_kernel_scales_far_apart(q, g, bias, m):
     _run("gemm_frag_kernel", 260, 1024, q, g, bias, m, column_scales=True)
