@@ -451,15 +451,10 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
     if (gridDim.y == 1) return;
 
     // ---- slabs: the last CTA of the column range converts the reduced sums and zeroes the workspace ----
-    __threadfence();
     __syncthreads();
-    if (tid == 0) {
-        const unsigned prev = atomicAdd(p.counters + blockIdx.x, 1u);
-        *s_flag = (prev == gridDim.y - 1u);
-    }
+    if (tid == 0) *s_flag = arrive_acq_rel(p.counters + blockIdx.x) == gridDim.y - 1u;
     __syncthreads();
     if (!*s_flag) return;
-    __threadfence();
     const int c0 = tile0 * kFrCols, quads = (min(N, tile1 * kFrCols) - c0) / 4;
     for (int idx = tid; idx < quads * p.m; idx += kFrThreads) {
         const size_t off = (size_t)(idx / quads) * N + c0 + 4 * (idx % quads);

@@ -564,7 +564,6 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         }
         tc_fence_before_sync();
     }
-    if (split) __threadfence();
     __syncthreads();
     if (warp == kHlMmaWarp) {
         tc_fence_after_sync();
@@ -573,13 +572,9 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     if (!split) return;
 
     // ---------------- split-k: the last CTA of the tile converts the reduced sums and zeroes the workspace ----------------
-    if (tid == 0) {
-        const unsigned prev = atomicAdd(p.counters + blockIdx.x, 1u);
-        *s_flag = (prev == (unsigned)p.splits - 1u);
-    }
+    if (tid == 0) *s_flag = arrive_acq_rel(p.counters + blockIdx.x) == (unsigned)p.splits - 1u;
     __syncthreads();
     if (!*s_flag) return;
-    __threadfence();
     const int nvec = rows * (kHlCols / 4);
     for (int base = tid; base < nvec; base += 4 * kHlThreads) {
         float4 v[4];

@@ -432,7 +432,6 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         tc_store_block(scratch, v, lane, 0, n0 + hN * 128 + lq * 32, p.m, N, split, p.partial, p.y16, p.y32);
     }
     tc_fence_before_sync();
-    __threadfence();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after_sync();

@@ -214,18 +214,14 @@ __device__ __forceinline__ void tc_store_block(float* scratch, const uint32_t (&
     __syncwarp();
 }
 
-// Split-k finish, called by every thread of the CTA after its reductions (and a __threadfence + __syncthreads): the last
+// Split-k finish, called by every thread of the CTA after its reductions (and a __syncthreads): the last
 // CTA of this column tile converts the reduced sums and zeroes the workspace.
 __device__ __forceinline__ void tc_splitk_finish(float* partial, unsigned* counters, __half* y16, float* y32, int m, int N,
                                                  int n0, int* s_flag, int nthreads) {
     const int tid = threadIdx.x;
-    if (tid == 0) {
-        const unsigned prev = atomicAdd(counters + blockIdx.x, 1u);
-        *s_flag = (prev == gridDim.y - 1u);
-    }
+    if (tid == 0) *s_flag = arrive_acq_rel(counters + blockIdx.x) == gridDim.y - 1u;
     __syncthreads();
     if (!*s_flag) return;
-    __threadfence();
     // whole float4 groups, several loads in flight per thread
     const int nvec = m * (kTcTileN / 4);
     for (int base = tid; base < nvec; base += 4 * nthreads) {
@@ -540,7 +536,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         }
         tc_fence_before_sync();
     }
-    __threadfence();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after_sync();

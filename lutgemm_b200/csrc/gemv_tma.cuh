@@ -243,41 +243,17 @@ __device__ __forceinline__ void build_lut2(unsigned char* lut, const __half* x, 
 // out.  The last CTA of the column tile [n_begin, n_end) either adds the slabs in slab order or reads the row
 // of L2-reduced sums and zeroes it again for the next launch; one fp16 rounding either way; then the
 // tensor-parallel output links, if any.
+// Everybody waits for the last CTA, so its reads are all under way before the first is used (8192 columns one read after the other
+// took it some 7000 cycles: 49152 x 12288, q = 4: 64.0 -> 62.8 us with arrive_acq_rel).
 template <int THREADS>
 __device__ __forceinline__ void splitk_finish(const Gemv2Params& p, int tid, int n_begin, int n_end, int* s_flag) {
     const size_t rowN = (size_t)p.N;
-    __threadfence();
     __syncthreads();
-    if (tid == 0) {
-        const unsigned prev = atomicAdd(p.counters + blockIdx.x, 1u);
-        *s_flag = (prev == (unsigned)p.nslabs - 1u);
-    }
+    if (tid == 0) *s_flag = arrive_acq_rel(p.counters + blockIdx.x) == (unsigned)p.nslabs - 1u;
     __syncthreads();
     if (!*s_flag) return;
-    __threadfence();
-    for (int c = n_begin + 4 * tid; c < n_end; c += 4 * THREADS) {
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float* src = p.partial + c;
-        int sl = 0;
-        if (!p.ordered) {
-            s = __ldcg(reinterpret_cast<const float4*>(src));
-            __stcg(reinterpret_cast<float4*>(p.partial + c), make_float4(0.f, 0.f, 0.f, 0.f));
-            sl = p.nslabs;
-        }
-        for (; sl + 8 <= p.nslabs; sl += 8) {
-            float4 v[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(sl + i) * rowN));
-#pragma unroll
-            for (int i = 0; i < 8; i++) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
-        }
-        for (; sl < p.nslabs; sl++) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(src + (size_t)sl * rowN));
-            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-        }
-        // Row 0 is also the L2 reduction row of the default mode, which expects to find it zero: leave it so, so
-        // that the mode may be switched between calls on one workspace.
-        if (p.ordered) __stcg(reinterpret_cast<float4*>(p.partial + c), make_float4(0.f, 0.f, 0.f, 0.f));
+    auto emit = [&](int c, float4 s) {
+        __stcg(reinterpret_cast<float4*>(p.partial + c), make_float4(0.f, 0.f, 0.f, 0.f));
         __half2 lo = __floats2half2_rn(s.x, s.y), hi = __floats2half2_rn(s.z, s.w);
         uint2 o;
         o.x = *reinterpret_cast<uint32_t*>(&lo);
@@ -289,6 +265,38 @@ __device__ __forceinline__ void splitk_finish(const Gemv2Params& p, int tid, int
             for (int r = 0; r < p.tp.world; r++) *reinterpret_cast<uint2*>(p.tp.out16[r] + p.tp.out_off + c) = o;   // peer stores
         } else {
             for (int r = 0; r < p.tp.world; r++) *reinterpret_cast<float4*>(p.tp.out32[r] + c) = s;                  // peer stores
+        }
+    };
+    if (!p.ordered) {
+        constexpr int kBatch = 4;
+        for (int c = n_begin + 4 * tid; c < n_end; c += kBatch * 4 * THREADS) {
+            float4 s[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; i++)
+                s[i] = c + i * 4 * THREADS < n_end ? __ldcg(reinterpret_cast<const float4*>(p.partial + c + i * 4 * THREADS)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < kBatch; i++)
+                if (c + i * 4 * THREADS < n_end) emit(c + i * 4 * THREADS, s[i]);
+        }
+    } else {
+        for (int c = n_begin + 4 * tid; c < n_end; c += 4 * THREADS) {
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float* src = p.partial + c;
+            int sl = 0;
+            for (; sl + 8 <= p.nslabs; sl += 8) {
+                float4 v[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[i] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(sl + i) * rowN));
+#pragma unroll
+                for (int i = 0; i < 8; i++) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
+            }
+            for (; sl < p.nslabs; sl++) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(src + (size_t)sl * rowN));
+                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+            }
+            // Row 0 is also the L2 reduction row of the default mode, which expects to find it zero: emit leaves it so, so
+            // that the mode may be switched between calls on one workspace.
+            emit(c, s);
         }
     }
     if (p.tp.out_mode != 0) {

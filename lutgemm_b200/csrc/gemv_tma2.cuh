@@ -254,32 +254,39 @@ gemv_tma2_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     }
 
     // ---- split-k finish: the last CTA of the column tile converts both reduction rows and leaves them zeroed ----
-    __threadfence();
     __syncthreads();
-    if (tid == 0) {
-        const unsigned prev = atomicAdd(p.counters + blockIdx.x, 1u);
-        *s_flag = (prev == (unsigned)p.nslabs - 1u);
-    }
+    if (tid == 0) *s_flag = arrive_acq_rel(p.counters + blockIdx.x) == (unsigned)p.nslabs - 1u;
     __syncthreads();
     if (!*s_flag) return;
-    __threadfence();
-    for (int c = n_begin + 4 * tid; c < n_end; c += 4 * kGemv2Threads) {
+    constexpr int kBatch = 4;                     // as in splitk_finish: the reads first
+    for (int c0 = n_begin + 4 * tid; c0 < n_end; c0 += kBatch * 4 * kGemv2Threads) {
+        float4 v[kBatch][kRows2];
 #pragma unroll
-        for (int r = 0; r < kRows2; r++) {
-            float* src = (r == 0 ? p.partial : pp.partial1) + c;
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(src));
-            __stcg(reinterpret_cast<float4*>(src), make_float4(0.f, 0.f, 0.f, 0.f));
-            float* y32 = r == 0 ? p.y32 : pp.y32_1;
-            __half* y16 = r == 0 ? p.y16 : pp.y16_1;
-            if (y32) *reinterpret_cast<float4*>(y32 + c) = v;
-            if (y16) {
-                __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
-                uint2 o;
-                o.x = *reinterpret_cast<uint32_t*>(&lo);
-                o.y = *reinterpret_cast<uint32_t*>(&hi);
-                *reinterpret_cast<uint2*>(y16 + c) = o;
+        for (int i = 0; i < kBatch; i++)
+#pragma unroll
+            for (int r = 0; r < kRows2; r++) {
+                const int c = c0 + i * 4 * kGemv2Threads;
+                if (c < n_end) v[i][r] = __ldcg(reinterpret_cast<const float4*>((r == 0 ? p.partial : pp.partial1) + c));
             }
-        }
+#pragma unroll
+        for (int i = 0; i < kBatch; i++)
+#pragma unroll
+            for (int r = 0; r < kRows2; r++) {
+                const int c = c0 + i * 4 * kGemv2Threads;
+                if (c >= n_end) continue;
+                const float4 f = v[i][r];
+                __stcg(reinterpret_cast<float4*>((r == 0 ? p.partial : pp.partial1) + c), make_float4(0.f, 0.f, 0.f, 0.f));
+                float* y32 = r == 0 ? p.y32 : pp.y32_1;
+                __half* y16 = r == 0 ? p.y16 : pp.y16_1;
+                if (y32) *reinterpret_cast<float4*>(y32 + c) = f;
+                if (y16) {
+                    __half2 lo = __floats2half2_rn(f.x, f.y), hi = __floats2half2_rn(f.z, f.w);
+                    uint2 o;
+                    o.x = *reinterpret_cast<uint32_t*>(&lo);
+                    o.y = *reinterpret_cast<uint32_t*>(&hi);
+                    *reinterpret_cast<uint2*>(y16 + c) = o;
+                }
+            }
     }
     if (tid == 0) p.counters[blockIdx.x] = 0u;   // ready for the next launch on this stream
 }
