@@ -17,6 +17,7 @@
 #include "gemv_tma.cuh"
 #include "gemv_reg.cuh"
 #include "gemv_tma2.cuh"
+#include "gemv_flat.cuh"
 #include "gemv_seq.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_hl.cuh"
@@ -453,6 +454,57 @@ void gemv_tma_geometry(const lutgemm_weight* w, int* nslabs, int* n_tile, int* t
     *tiles = (w->N + *n_tile - 1) / *n_tile;
 }
 
+// Whether a matvec goes to gemv_flat_kernel: the stages of the longest run there, 4 % slower, against those of a CTA of
+// gemv_tma_kernel, whose every wave starts anew (some four stages); a table costs one and a half.  Predicted and measured
+// ratio: 8192 x 28672, q = 4 + q_bias, 0.91 / 0.88; 8192 x 20480, q = 3, 0.86 / 0.88; 12288 x 49152, q = 3, 0.99 / 0.98; 8192 x 8192, q = 3,
+// 1.12 / 1.05; 4096 x 4096, q = 3, 1.2 / 1.06.
+bool gemv_flat_better(const lutgemm_weight* w, int nslabs, int n_tile, int tiles) {
+    const int sms = sm_count(), groups = (w->N + lg::kStageCols - 1) / lg::kStageCols;
+    const long long total = (long long)nslabs * groups * w->q, run = (total + sms - 1) / sms;
+    if (sms > lg::kFlatMaxCtas || total < sms || total >= 1ll << 31 || groups > kMaxCounters || run / w->q + 2 > lg::kFlatMaxPieces) return false;
+    const long long waves = ((long long)tiles * nslabs + sms - 1) / sms;
+    const double flat = 1.04 * (double)run + 4.0 + 1.5 * (double)((run + (long long)groups * w->q - 1) / ((long long)groups * w->q));
+    return flat < 0.96 * (double)waves * ((double)(n_tile / lg::kStageCols) * w->q + 4.0);
+}
+
+template <int WPG>
+int launch_gemv_flat(const lutgemm_weight* w, const lg::Gemv2Params& p, bool bias, cudaStream_t st) {
+    static bool configured[64][2] = {};   // the attribute is per device
+    auto kern = bias ? lg::gemv_flat_kernel<WPG, true> : lg::gemv_flat_kernel<WPG, false>;
+    int dev = 0;
+    LG_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !configured[dev][bias]) {
+        LG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lg::kSmemLimit));
+        if (dev < 64) configured[dev][bias] = true;
+    }
+    const dim3 grid(sm_count());
+    lg::FlatRuns runs;
+    const int groups = (p.N + lg::kStageCols - 1) / lg::kStageCols;
+    const int total = p.nslabs * groups * p.q, n = (int)grid.x, base = total / n, longer = total % n;
+    int unit = 0, plane = 0;                 // run i begins at stage i * base + min(i, longer)
+    for (int i = 0; i < n; i++) {
+        const int stages = base + (i < longer ? 1 : 0);
+        runs.run[i] = {stages, plane, unit % groups, unit / groups};
+        plane += stages;
+        unit += plane / p.q;
+        plane %= p.q;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(lg::kGemv2Threads);
+    cfg.dynamicSmemBytes = (size_t)lg::gemv2_smem_bytes(p.a_rows);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_pdl.load() ? 1 : 0;
+    LG_CUDA(cudaLaunchKernelEx(&cfg, kern, w->tmW, w->tmA, p, runs));
+    note_launch("gemv_flat_kernel", grid);
+    LG_CUDA(cudaGetLastError());
+    return LUTGEMM_OK;
+}
+
 int launch_gemv_tma_any(const lutgemm_weight* w, const lutgemm_workspace* ws, const __half* x, __half* y16, float* y32,
                         const lg::TpLink* link, cudaStream_t st) {
     lg::Gemv2Params p2 = {};
@@ -466,6 +518,8 @@ int launch_gemv_tma_any(const lutgemm_weight* w, const lutgemm_workspace* ws, co
     if (link) p2.tp = *link;
     dim3 grid2(tiles, p2.nslabs);
     const bool bias2 = w->q_bias != nullptr;
+    if (!link && !p2.ordered && !g_ntile_override.load() && gemv_flat_better(w, p2.nslabs, p2.n_tile, tiles))
+        return w->g % 128 == 0 ? launch_gemv_flat<2>(w, p2, bias2, st) : launch_gemv_flat<1>(w, p2, bias2, st);
     if (w->g % 128 == 0) return launch_gemv_tma<2>(w, p2, grid2, bias2, st);
     return launch_gemv_tma<1>(w, p2, grid2, bias2, st);
 }

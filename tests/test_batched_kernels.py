@@ -101,6 +101,15 @@ def test_register_operand_kernel_per_plane_count(N, K, q, g, bias, m):
     _run("gemm_frag_kernel", N, K, q, g, bias, m)
 
 
+# one row where the slabs do not share out evenly: runs of stages that begin and end between planes, cross into one or several
+# slabs, hold a column group twice; ragged last groups and slabs; both alpha forms; a run of one stage
+@pytest.mark.parametrize("N,K,q,g,bias", [
+    (520, 8224, 5, 32, True), (4096, 28672, 3, 256, False), (20488, 1024, 5, 1024, True), (2048, 30720, 7, 64, True),
+    (8192, 20480, 1, 128, True), (256, 153088, 1, 512, True), (1032, 40480, 2, 32, False)])
+def test_matvec_in_runs(N, K, q, g, bias):
+    _run("gemv_flat_kernel", N, K, q, g, bias, 1)
+
+
 # two and three rows: the register operand up to 64 Mi weights of planes and where one slab of k is enough, else the LUT kernels
 @pytest.mark.parametrize("N,K,q,g,bias,m,kernel", [
     (72, 128, 1, 64, True, 2, "gemm_frag_kernel"), (4096, 4096, 4, 128, False, 2, "gemm_frag_kernel"), (4104, 4096, 4, 128, False, 2, "gemv_tma2_kernel"),
