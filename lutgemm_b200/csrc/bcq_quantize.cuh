@@ -17,6 +17,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace lg {
 
 constexpr int kBqMaxQ = 8;
@@ -239,7 +241,8 @@ bcq_quantize_kernel(const BqParams p) {
 // pairs to a word.  A weight then costs its q comparisons, one table read, q multiply-adds (B^T w) and one integer add
 // (B^T B) per word of pairs, and the sums of the next round are complete when the weights of this one are placed.
 // Bound by instruction issue, not by memory: the weights are read once.  Measured, N = K = 4096, q = 3, g = 128, 15
-// rounds: 406 us; bcq_quantize_kernel, which gives every group a whole warp, takes 3291 us.
+// rounds: 406 us; bcq_quantize_kernel, which gives every group a whole warp, takes 3291 us.  Layers of 4 Mi weights or more take
+// bcq_quantize_lane_kernel (below) instead.
 // Sums are added in the order of bcq_quantize_kernel, whose lane L holds weights L, L + 32, ...: a lane here stands for
 // NJ = 32 / LG of those lanes (lane, lane + LG, ...), keeps their partial sums apart and adds them first, which is that
 // kernel's shuffle over distances 16 .. LG.  So both give the same bits, and which one a group takes does not show.
@@ -268,6 +271,56 @@ __device__ __forceinline__ float tile_sum_f(float (&v)[32 / LG]) {
 #pragma unroll
         for (int j = 0; j < d; j++) v[j] += v[j + d];
     return group_sum_f<LG>(v[0]);
+}
+
+// The scales of a group from B^T B and B^T w: Q steps of conjugate gradient from the current ones, |alpha| in descending order.
+template <int Q>
+__device__ __forceinline__ void bq_solve(const float (&A)[Q][Q], const float (&btw)[Q], float (&alpha)[Q]) {
+    float x[Q], r[Q], pp[Q], Ap[Q];
+    float rtr_new = 0.f;
+#pragma unroll
+    for (int i = 0; i < Q; i++) {
+        x[i] = alpha[i];
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < Q; j++) s += A[i][j] * alpha[j];
+        r[i] = btw[i] - s;
+        pp[i] = r[i];
+        rtr_new += r[i] * r[i];
+    }
+#pragma unroll
+    for (int it = 0; it < Q; it++) {
+        const float rtr = rtr_new;
+        float pAp = 0.f;
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < Q; j++) s += A[i][j] * pp[j];
+            Ap[i] = s;
+            pAp += pp[i] * s;
+        }
+        const float a = rtr / (pAp + 1e-6f);
+        rtr_new = 0.f;
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            x[i] += a * pp[i];
+            r[i] -= a * Ap[i];
+            rtr_new += r[i] * r[i];
+        }
+        const float beta = rtr_new / (rtr + 1e-6f);
+#pragma unroll
+        for (int i = 0; i < Q; i++) pp[i] = r[i] + beta * pp[i];
+    }
+    // insertion sort
+#pragma unroll
+    for (int i = 0; i < Q; i++) alpha[i] = fabsf(x[i]);
+#pragma unroll
+    for (int i = 1; i < Q; i++) {
+#pragma unroll
+        for (int j = i; j > 0; j--)
+            if (alpha[j] > alpha[j - 1]) { const float t = alpha[j]; alpha[j] = alpha[j - 1]; alpha[j - 1] = t; }
+    }
 }
 
 template <int LG, int Q>
@@ -346,54 +399,7 @@ bcq_quantize_tile_kernel(const BqParams p) {
     // ---- alternating refinement ----
     const uint32_t pad = (uint32_t)(E - __popc(valid));
     for (int round = 0; Q > 1 && round < p.rounds; round++) {
-        // Q steps of conjugate gradient from the current alpha
-        {
-            float x[Q], r[Q], pp[Q], Ap[Q];
-            float rtr_new = 0.f;
-#pragma unroll
-            for (int i = 0; i < Q; i++) {
-                x[i] = alpha[i];
-                float s = 0.f;
-#pragma unroll
-                for (int j = 0; j < Q; j++) s += A[i][j] * alpha[j];
-                r[i] = btw[i] - s;
-                pp[i] = r[i];
-                rtr_new += r[i] * r[i];
-            }
-#pragma unroll
-            for (int it = 0; it < Q; it++) {
-                const float rtr = rtr_new;
-                float pAp = 0.f;
-#pragma unroll
-                for (int i = 0; i < Q; i++) {
-                    float s = 0.f;
-#pragma unroll
-                    for (int j = 0; j < Q; j++) s += A[i][j] * pp[j];
-                    Ap[i] = s;
-                    pAp += pp[i] * s;
-                }
-                const float a = rtr / (pAp + 1e-6f);
-                rtr_new = 0.f;
-#pragma unroll
-                for (int i = 0; i < Q; i++) {
-                    x[i] += a * pp[i];
-                    r[i] -= a * Ap[i];
-                    rtr_new += r[i] * r[i];
-                }
-                const float beta = rtr_new / (rtr + 1e-6f);
-#pragma unroll
-                for (int i = 0; i < Q; i++) pp[i] = r[i] + beta * pp[i];
-            }
-            // |alpha| descending (insertion sort)
-#pragma unroll
-            for (int i = 0; i < Q; i++) alpha[i] = fabsf(x[i]);
-#pragma unroll
-            for (int i = 1; i < Q; i++) {
-#pragma unroll
-                for (int j = i; j > 0; j--)
-                    if (alpha[j] > alpha[j - 1]) { const float t = alpha[j]; alpha[j] = alpha[j - 1]; alpha[j - 1] = t; }
-            }
-        }
+        bq_solve<Q>(A, btw, alpha);
         // the levels, in ascending order, ties by index: level c has sign -1 on plane i iff bit Q-1-i of c is set
         constexpr int LPL = (NLEV + LG - 1) / LG;          // levels per lane
         float lv[LPL];
@@ -536,6 +542,364 @@ bcq_quantize_tile_kernel(const BqParams p) {
                 for (int o = LG / 2; o > 0; o >>= 1) word |= __shfl_xor_sync(0xffffffffu, word, o);
                 if (live && l == kw % LG && kw * 32 < g) p.bW[((size_t)(gi * (g / 32) + kw) * Q + b) * p.N + n] = word;
             }
+    }
+}
+
+// ---- the same, a group to a lane: two to four planes, refined at least once ----
+// The levels come in pairs +-v, so the midpoints do too and the middle one is 0: a weight's level is decided by |w| among the
+// 2^(Q-1) levels of the upper half and by its sign, and sign times weight by the level's signs and |w|.  A plane's sign is a step
+// function of |w|: one multiply-add per midpoint with the comparison's 1 or 0 and the step's height (0 or +-2, of this group's
+// levels).  Nothing is searched or looked up: at Q = 3 a weight and round is 3 comparisons, 6 multiply-adds for the signs, 3
+// for B^T w and 3 for B^T B.  A lane does that for a group of its own, so there is nothing to reduce, and the solve costs the
+// warp once for 32 groups instead of once for 32 / LG.  The weights lie in shared memory, four of a group to 16 bytes, at
+// places that reading (a lane per group) and filling (a row of the matrix at a time) both find without bank conflicts.
+// `w < mid goes left` is strict on both sides: a negative weight leaves the inner level only if |w| > midpoint.  Those compare with
+// the float below |w|: w plus the smallest float, cut off toward zero, which leaves the others as they are.
+// Sums are added in the order of the other kernels: per residue of 32 the weights in turn, then residues 16, 8, 4, 2 and 1 apart.  So
+// all give the same bits.
+//
+// Bound by issue and its latencies on 14 warps to an SM: an ALU instruction (a comparison) keeps a scheduler for two cycles, an
+// fp32 one for one, some 20 cycles a weight and round at Q = 3.  Measured, us, this / tiled kernel, 15 rounds, 4096 x 4096: q = 3, g = 128,
+// 256 / 409, g = 256 276 / 422, g = 512 421 / 462; q = 2, g = 64, 184 / 257, g = 128 123 / 231; q = 4, g = 128, 616 / 842.  A round takes
+// 14 us of the 256; reading, greedy start and packing 50.
+// Sums of |w| per midpoint, two packed instructions for two weights, are a third faster (171 us) but round otherwise: then a
+// weight in a million takes another level.
+constexpr int kBqLaneWarps = 7;               // 16 KB a warp at g = 128: two CTAs of 7 warps to an SM
+constexpr int kBqLaneMaxG = 512;
+__host__ __device__ constexpr int bq_lane_warp_bytes(int g) { return (g + 31) / 32 * 4096; }
+__host__ __device__ constexpr int bq_lane_warps(int g) {
+    return 232448 / bq_lane_warp_bytes(g) < kBqLaneWarps ? 232448 / bq_lane_warp_bytes(g) : kBqLaneWarps;
+}
+
+// What a weight is compared with: |w|, or for a negative one the float below (the sum with the smallest float, cut off toward zero).
+__device__ __forceinline__ float bq_key(float w) { return fabsf(__fadd_rz(w, 1.401298464324817e-45f)); }
+// 1 where key >= mid, else 0
+__device__ __forceinline__ float bq_from(float key, float mid) {
+    float f;
+    asm("set.ge.f32.f32 %0, %1, %2;" : "=f"(f) : "f"(key), "f"(mid));
+    return f;
+}
+__device__ __forceinline__ float4 bq_add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+template <int Q>
+__global__ void __launch_bounds__(kBqLaneWarps * 32, 2)
+bcq_quantize_lane_kernel(const BqParams p) {
+    constexpr int NH = 1 << (Q - 1);                       // levels of the upper half
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int G = p.K / p.g, g = p.g, words = (g + 31) / 32;
+    const long long groups = (long long)p.N * G;
+    const long long first = ((long long)blockIdx.x * (blockDim.x >> 5) + wib) * 32;
+    if (first >= groups) return;                           // whole warps leave together
+    // groups of consecutive rows share a warp: their packed words are neighbours
+    const bool live = first + lane < groups;               // a group beyond the end repeats the warp's first one
+    const long long grp = live ? first + lane : first;
+    const int gi = (int)(grp / p.N), n = (int)(grp % p.N);
+    const float* wg = p.w + (size_t)n * p.K + (size_t)gi * g;
+    unsigned char* mine = smem + (size_t)wib * bq_lane_warp_bytes(g);
+    // quad j + 8 e of row r: weights 32 e + 4 j .. + 3
+    auto place = [&](int j, int e, int row) { return mine + e * 4096 + (j * 32 + (row ^ j)) * 16; };
+
+    // ---- the weights, zeros up to whole words of 32: the whole warp takes one group after the other ----
+    const bool wide = g % 4 == 0 && ((uintptr_t)p.w & 15) == 0;      // then every group begins on 16 bytes
+#pragma unroll 16
+    for (int r = 0; r < 32; r++) {
+        const float* src = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, (unsigned long long)wg, r));
+        if (wide) {
+            for (int k4 = lane; k4 < words * 8; k4 += 32)
+                *reinterpret_cast<float4*>(place(k4 & 7, k4 >> 3, r)) = 4 * k4 < g ? __ldg(reinterpret_cast<const float4*>(src) + k4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+            for (int k = lane; k < words * 32; k += 32)
+                reinterpret_cast<float*>(place((k >> 2) & 7, k >> 5, r))[k & 3] = k < g ? __ldg(src + k) : 0.f;
+        }
+    }
+    __syncwarp();
+
+    // Sums over the group's weights, COUNT at a time: f(w, part) adds what a weight contributes to part[0 .. COUNT-1].
+    auto sums = [&](auto& out, auto&& f) {
+        constexpr int COUNT = sizeof(out) / sizeof(float), UNROLL = Q == 4 ? 1 : 2;       // twice as much: 261 and, Q = 4, 671 us
+        float4 even[COUNT], acc[COUNT];                    // residues 4 j .. 4 j + 3 for j = 0, 4, 2, 6, and then 1, 5, 3, 7
+#pragma unroll 1
+        for (int jj = 0; jj < 4; jj++) {
+            const int j = (jj & 1) << 1 | jj >> 1;
+            const unsigned char *at0 = place(j, 0, lane), *at1 = place(j + 4, 0, lane);
+            float part[2][4][COUNT] = {};
+#pragma unroll UNROLL
+            for (int e = 0; e < words; e++) {
+                const float4 v = *reinterpret_cast<const float4*>(at0 + e * 4096), u = *reinterpret_cast<const float4*>(at1 + e * 4096);
+                f(v.x, part[0][0]); f(v.y, part[0][1]); f(v.z, part[0][2]); f(v.w, part[0][3]);
+                f(u.x, part[1][0]); f(u.y, part[1][1]); f(u.z, part[1][2]); f(u.w, part[1][3]);
+            }
+#pragma unroll
+            for (int i = 0; i < COUNT; i++) {
+                const float4 both = make_float4(part[0][0][i] + part[1][0][i], part[0][1][i] + part[1][1][i],
+                                                part[0][2][i] + part[1][2][i], part[0][3][i] + part[1][3][i]);
+                acc[i] = jj & 1 ? bq_add4(acc[i], both) : both;
+                if (jj == 1) even[i] = acc[i];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < COUNT; i++) {
+            const float4 all = bq_add4(even[i], acc[i]);
+            out[i] = (all.x + all.z) + (all.y + all.w);
+        }
+    };
+
+    // ---- greedy ----
+    float alpha[Q], btw[Q];
+    float A[Q][Q];                                         // B^T B
+    auto scale = [&](float sum) {
+        const float a = sum / (float)g;
+        return a != a ? 0.f : a;
+    };
+    // By signs relative to the weight's own: plane 0 is +, r = |w| - alpha_0 decides plane 1, and so on.  A residual that is 0 (a
+    // weight that is 0, to begin with) has no sign: a warp that meets one does it over below.
+    auto toward0 = [](float r, float a) { return r - copysignf(a, r); };
+    float whole;                                           // sum of |w|
+    float least = __int_as_float(0x7f800000);              // of the |residuals| whose signs were used
+    {
+        float s[1];
+        sums(s, [&](float w, float (&part)[1]) {
+            least = fminf(least, fabsf(w));
+            part[0] += fabsf(w);
+        });
+        whole = btw[0] = s[0];
+        alpha[0] = scale(s[0]);
+    }
+#pragma unroll
+    for (int i = 1; i < Q; i++) {
+        float s[1];
+        sums(s, [&](float w, float (&part)[1]) {
+            float r = fabsf(w) - alpha[0];
+#pragma unroll
+            for (int j = 1; j < i; j++) r = toward0(r, alpha[j]);
+            least = fminf(least, fabsf(r));
+            part[0] += fabsf(r);
+        });
+        alpha[i] = scale(s[0]);
+    }
+    {
+        float t[Q - 1];
+        float both[Q][Q] = {};                             // [j][i], j < i: sum of the products of the signs
+        sums(t, [&](float w, float (&part)[Q - 1]) {
+            float r[Q];
+            r[1] = fabsf(w) - alpha[0];
+#pragma unroll
+            for (int i = 2; i < Q; i++) r[i] = toward0(r[i - 1], alpha[i - 1]);
+#pragma unroll
+            for (int i = 1; i < Q; i++) {
+                part[i - 1] += copysignf(w, r[i]);
+                both[0][i] += copysignf(1.f, r[i]);
+#pragma unroll
+                for (int j = 1; j < i; j++) both[j][i] += copysignf(1.f, __uint_as_float(__float_as_uint(r[i]) ^ __float_as_uint(r[j])));
+            }
+        });
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            if (i) btw[i] = t[i ? i - 1 : 0];
+            A[i][i] = (float)g;
+#pragma unroll
+            for (int j = 0; j < i; j++) A[j][i] = A[i][j] = both[j][i];
+        }
+    }
+    if (__any_sync(0xffffffffu, !(least > 0.f))) {         // (so do the zeros behind a group's end)
+        auto take = [&](float r, float a) { return r != 0.f ? toward0(r, a) : r; };
+#pragma unroll
+        for (int i = 1; i < Q; i++) {
+            float s[1];
+            sums(s, [&](float w, float (&part)[1]) {
+                float r = w;
+#pragma unroll
+                for (int j = 0; j < i; j++) r = take(r, alpha[j]);
+                part[0] += fabsf(r);
+            });
+            alpha[i] = scale(s[0]);
+        }
+        float both[Q][Q] = {};
+        sums(btw, [&](float w, float (&part)[Q]) {
+            float r = w, b[Q];
+#pragma unroll
+            for (int i = 0; i < Q; i++) {
+                b[i] = r > 0.f ? 1.f : (r < 0.f ? -1.f : 0.f);
+                r = take(r, alpha[i]);
+                part[i] = fmaf(b[i], w, part[i]);
+#pragma unroll
+                for (int j = 0; j <= i; j++) both[j][i] = fmaf(b[j], b[i], both[j][i]);
+            }
+        });
+#pragma unroll
+        for (int i = 0; i < Q; i++)
+#pragma unroll
+            for (int j = 0; j <= i; j++) A[j][i] = A[i][j] = both[j][i];
+    }
+
+    // ---- alternating refinement ----
+    float mid[NH];                                         // [1 ..]: between the upper half's levels
+    uint32_t code[NH];                                     // bit Q - 1 - i set: plane i is -1 in this level
+    const float pad = (float)(words * 32 - g);
+#pragma unroll 1
+    for (int round = 0;; round++) {
+        bq_solve<Q>(A, btw, alpha);
+        // the upper half's levels in ascending order, ties by index: of c and its complement the one above 0, the larger one at 0
+        float v[NH];
+#pragma unroll
+        for (int c = 0; c < NH; c++) {
+            float x = 0.f;
+#pragma unroll
+            for (int i = 0; i < Q; i++) x += ((c >> (Q - 1 - i)) & 1) ? -alpha[i] : alpha[i];
+            v[c] = fabsf(x);
+            code[c] = x > 0.f ? c : 2 * NH - 1 - c;
+        }
+#pragma unroll
+        for (int c = 1; c < NH; c++)
+#pragma unroll
+            for (int d = c; d > 0; d--)
+                if (v[d] < v[d - 1] || (v[d] == v[d - 1] && code[d] < code[d - 1])) {
+                    const float t = v[d]; v[d] = v[d - 1]; v[d - 1] = t;
+                    const uint32_t u = code[d]; code[d] = code[d - 1]; code[d - 1] = u;
+                }
+#pragma unroll
+        for (int c = 1; c < NH; c++) mid[c] = (v[c - 1] + v[c]) / 2.f;
+        if (round + 1 == p.rounds) break;
+        // a plane's sign: in the lowest level, and the steps at the midpoints
+        float step[Q][NH];
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            float last = 0.f;
+#pragma unroll
+            for (int c = 0; c < NH; c++) {
+                const float sign = ((code[c] >> (Q - 1 - i)) & 1u) ? -1.f : 1.f;
+                step[i][c] = sign - last;
+                last = sign;
+            }
+        }
+        float both[Q][Q] = {};
+        // KIND 1, Q = 3: above the lowest level the codes are 1, 2, ... from the top, as they are without ties, and steps are known.
+        // 2, Q = 2: the codes are 0 and 1, and plane 0 is + throughout.
+        auto refine = [&](auto kind) {
+            constexpr int KIND = decltype(kind)::value;
+            auto signs = [&](float key, float (&sg)[Q]) {
+                float from[NH];
+#pragma unroll
+                for (int c = 1; c < NH; c++) from[c] = bq_from(key, mid[c]);
+#pragma unroll
+                for (int i = 0; i < Q; i++) {
+                    if (KIND == 2) {
+                        // plane 1 rises at 2; plane 2 rises at 1, falls at 2, rises at 3
+                        sg[i] = i ? -1.f : 1.f;
+                        if (i == 1) sg[i] = fmaf(2.f, from[NH / 2], sg[i]);
+                        if (i == 2)
+#pragma unroll
+                            for (int c = 1; c < NH; c++) sg[i] = fmaf(c & 1 ? 2.f : -2.f, from[c], sg[i]);
+                    } else {
+                        sg[i] = step[i][0];
+#pragma unroll
+                        for (int c = 1; c < NH; c++) {
+                            if (KIND == 1 && c >= 2) {
+                                if (i == 1 && c == 2 || i == 2 && c == 3) sg[i] = fmaf(2.f, from[c], sg[i]);
+                                if (i == 2 && c == 2) sg[i] = fmaf(-2.f, from[c], sg[i]);
+                            } else {
+                                sg[i] = fmaf(step[i][c], from[c], sg[i]);
+                            }
+                        }
+                    }
+                }
+            };
+            constexpr int FROM = KIND == 2 ? 1 : 0;       // first plane whose sum changes
+            float t[Q - FROM];
+            sums(t, [&](float w, float (&part)[Q - FROM]) {
+                float sg[Q];
+                signs(bq_key(w), sg);
+#pragma unroll
+                for (int i = 0; i < Q; i++) {
+                    if (i >= FROM) part[i >= FROM ? i - FROM : 0] = fmaf(sg[i], fabsf(w), part[i >= FROM ? i - FROM : 0]);
+#pragma unroll
+                    for (int j = 0; j < i; j++) both[j][i] = fmaf(sg[j], sg[i], both[j][i]);
+                }
+            });
+            if (FROM) btw[0] = whole;
+#pragma unroll
+            for (int i = FROM; i < Q; i++) btw[i] = t[i - FROM];
+            if (pad != 0.f) {                              // the zeros behind the group's end were counted
+                float sg[Q];
+                signs(bq_key(0.f), sg);
+#pragma unroll
+                for (int i = 0; i < Q; i++)
+#pragma unroll
+                    for (int j = 0; j < i; j++) both[j][i] -= pad * (sg[i] * sg[j]);
+            }
+        };
+        if constexpr (Q == 3) {
+            if (__all_sync(0xffffffffu, code[3] == 0u && code[2] == 1u && code[1] == 2u)) refine(std::integral_constant<int, 1>{});
+            else refine(std::integral_constant<int, 0>{});
+        } else if constexpr (Q == 2) {
+            if (__all_sync(0xffffffffu, code[1] == 0u && code[0] == 1u)) refine(std::integral_constant<int, 2>{});
+            else refine(std::integral_constant<int, 0>{});
+        } else {
+            refine(std::integral_constant<int, 0>{});
+        }
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            A[i][i] = (float)g;
+#pragma unroll
+            for (int j = 0; j < i; j++) A[j][i] = A[i][j] = both[j][i];
+        }
+    }
+
+    // ---- outputs ----
+    if (live) {
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            if (p.alpha_py) p.alpha_py[((size_t)n * G + gi) * Q + i] = alpha[i];
+            if (p.alpha_k) p.alpha_k[((size_t)gi * Q + i) * p.N + n] = __float2half_rn(alpha[i]);
+        }
+    }
+    if (!p.bW && !p.binary_py) return;
+    // 32 weights at a time: a bit per weight of every plane, 1 for +1
+    for (int kw = 0; kw < words; kw++) {
+        uint32_t from[NH] = {}, neg = 0u;                  // [1 ..]: from mid on
+        auto mark = [&](float w, int e) {
+            const float key = bq_key(w);
+            neg |= w < 0.f ? 1u << e : 0u;
+#pragma unroll
+            for (int c = 1; c < NH; c++) from[c] |= key >= mid[c] ? 1u << e : 0u;
+        };
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const float4 v = *reinterpret_cast<const float4*>(place(j, kw, lane));
+            mark(v.x, 4 * j); mark(v.y, 4 * j + 1); mark(v.z, 4 * j + 2); mark(v.w, 4 * j + 3);
+        }
+        from[0] = 0xffffffffu;
+        uint32_t plus[Q] = {};
+#pragma unroll
+        for (int c = 0; c < NH; c++) {
+            const uint32_t here = c + 1 < NH ? from[c] & ~from[c + 1] : from[c];
+#pragma unroll
+            for (int i = 0; i < Q; i++) plus[i] |= ((code[c] >> (Q - 1 - i)) & 1u) ? 0u : here;
+        }
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            plus[i] ^= neg;
+            if (p.bW && live) p.bW[((size_t)(gi * (g / 32) + kw) * Q + i) * p.N + n] = plus[i];      // g % 32 == 0: whole words
+        }
+        if (p.binary_py) {
+            // a row after the other, by the whole warp: consecutive bytes of it
+            const int count = min(32, g - 32 * kw);
+            for (int r = 0; r < 32; r++) {
+                const bool there = __shfl_sync(0xffffffffu, live ? 1 : 0, r);
+                signed char* dst = p.binary_py + ((size_t)__shfl_sync(0xffffffffu, n, r) * G + __shfl_sync(0xffffffffu, gi, r)) * g * Q + (size_t)32 * kw * Q;
+                uint32_t row[Q];
+#pragma unroll
+                for (int i = 0; i < Q; i++) row[i] = __shfl_sync(0xffffffffu, plus[i], r);
+                for (int at = lane; there && at < count * Q; at += 32) {
+                    const int e = at / Q, i = at % Q;
+                    uint32_t bits = row[0];
+#pragma unroll
+                    for (int j = 1; j < Q; j++) bits = i == j ? row[j] : bits;
+                    dst[at] = (bits >> e) & 1u ? 1 : -1;
+                }
+            }
+        }
     }
 }
 

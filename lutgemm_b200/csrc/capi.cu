@@ -1288,6 +1288,29 @@ void launch_bcq_tile(const lg::BqParams& p, long long groups, cudaStream_t st) {
     else lg::bcq_quantize_tile_kernel<32, Q><<<ctas, block, 0, st>>>(p);
 }
 
+// Whether the kernel with a group to a lane is the faster one: a warp of it takes some 60 us whatever the layer is, more with wider
+// groups, of which fewer fit an SM; the tiled kernel 14 to 50 us per million weights.  Measured, us, this / tiled, 15 rounds: 1024 x
+// 1024, q = 3, g = 128, 62 / 38; 2048 x 2048, q = 3, 88 / 110, q = 2, g = 64, 57 / 77, q = 2, g = 256, 75 / 69; 1024 x 8192, q = 3, g = 256, 157 /
+// 216; 2048 x 4096, q = 3, g = 512, 287 / 238; 4096 x 4096, g = 512, 421 / 462.
+bool bq_lane_better(long long groups, int g) { return groups * g >= (4ll << 20) * (g > 256 ? 4 : g > 128 ? 2 : 1); }
+
+template <int Q>
+int launch_bcq_lane(const lg::BqParams& p, long long groups, cudaStream_t st) {
+    static bool configured[64] = {};      // the attribute is per device
+    int dev = 0;
+    LG_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !configured[dev]) {
+        LG_CUDA(cudaFuncSetAttribute(lg::bcq_quantize_lane_kernel<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, lg::kSmemLimit));
+        if (dev < 64) configured[dev] = true;
+    }
+    // few groups are spread over the SMs
+    const long long warps_all = (groups + 31) / 32, per_sm = (warps_all + sm_count() - 1) / sm_count();
+    const int most = lg::bq_lane_warps(p.g), warps = per_sm < most ? (int)per_sm : most;
+    const long long ctas = (warps_all + warps - 1) / warps;
+    lg::bcq_quantize_lane_kernel<Q><<<(unsigned)ctas, warps * 32, (size_t)warps * lg::bq_lane_warp_bytes(p.g), st>>>(p);
+    return LUTGEMM_OK;
+}
+
 template <int WPG, bool BIAS>
 int launch_sequence(lutgemm_sequence* s, cudaStream_t st) {
     static bool configured[64] = {};
@@ -2226,8 +2249,13 @@ int lutgemm_bcq_quantize_device(const float* d_w, int N, int K, int q, int group
     const long long ctas = (groups + lg::kBqWarps - 1) / lg::kBqWarps;
     if (ctas > 0x7fffffffLL) return LUTGEMM_ERR_TOO_LARGE;
     cudaStream_t st = (cudaStream_t)stream;
-    // The tiled kernel is 7 to 8 times as fast wherever it was measured (406 / 3292 us at q = 3, g = 128); more planes or wider groups take a warp or a CTA per group.
-    if (q <= lg::kBqTileMaxQ && g <= lg::kBqTileMaxG) {
+    // Up to four planes and 512 weights to a group: a group to a lane, or, for small layers, one plane or no refinement, several to a
+    // warp (406 us at 4096 x 4096, q = 3, g = 128, where a group to a warp takes 3292); the rest take a warp or a CTA per group.
+    if (q >= 2 && q <= lg::kBqTileMaxQ && g <= lg::kBqLaneMaxG && rounds >= 1 && bq_lane_better(groups, g)) {
+        const int rc = q == 2 ? launch_bcq_lane<2>(p, groups, st) : q == 3 ? launch_bcq_lane<3>(p, groups, st) : launch_bcq_lane<4>(p, groups, st);
+        if (rc != LUTGEMM_OK) return rc;
+    }
+    else if (q <= lg::kBqTileMaxQ && g <= lg::kBqTileMaxG) {
         if (q == 1) launch_bcq_tile<1>(p, groups, st);
         else if (q == 2) launch_bcq_tile<2>(p, groups, st);
         else if (q == 3) launch_bcq_tile<3>(p, groups, st);

@@ -93,6 +93,34 @@ def test_device_quantiser_several_groups_per_warp(N, K, g, q, rounds):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,K,g,q,rounds,zeros", [
+    # layers large enough for a group to go to a lane: whole and ragged words, quads and columns, one round, residuals that are
+    # 0, a group count that is no multiple of a warp's
+    (5, 192, 64, 3, 4, False), (7, 96, 32, 2, 3, True), (3, 512, 512, 4, 5, False), (9, 400, 400, 3, 3, True), (13, 129, 43, 4, 2, False),
+    (6, 384, 192, 2, 15, False), (16, 1024, 128, 3, 15, False), (4, 256, 256, 3, 1, True), (11, 200, 50, 3, 3, False)])
+def test_device_quantiser_group_per_lane(N, K, g, q, rounds, zeros):
+    import torch
+    import lutgemm_b200 as L
+    rng = np.random.default_rng(N * K + q)
+    w = (rng.normal(0, 0.02, (N, K))).astype(np.float32)
+    if zeros:
+        w[:, ::17] = 0.0
+    times = (4 << 20) * (4 if g > 256 else 2 if g > 128 else 1) // w.size + 1
+    _, B_ref, alpha_ref = bq.quantize(w, q, rounds, g)
+    _, B, alpha = L.bcq_quantize(np.tile(w, (times, 1)), q, rounds, g)
+    B, alpha = B.reshape((times, N) + B.shape[1:]), alpha.reshape((times, N) + alpha.shape[1:])
+    assert (B == B[0]).all() and (alpha == alpha[0]).all()           # the same rows again, in other lanes and warps
+    _, B_small, alpha_small = L.bcq_quantize(w, q, rounds, g)        # the tiled kernel: the same bits
+    assert (B_small.reshape(B[0].shape) == B[0]).all() and (alpha_small.reshape(alpha[0].shape) == alpha[0]).all()
+    _compare(alpha[0], B[0], alpha_ref, B_ref.astype(np.int8), w)
+    if g % 32 == 0:
+        bW, alpha_k = L.bcq_quantize_device(torch.from_numpy(np.tile(w, (times, 1))).cuda(), q, rounds=rounds, group_size=g)
+        bits = ((B[0].reshape(N, K // 32, 32, q) > 0).astype(np.uint64) << np.arange(32, dtype=np.uint64)[:, None]).sum(2).astype(np.uint32)
+        assert (bW.cpu().numpy().view(np.uint32).transpose(2, 0, 1).reshape(times, N, K // 32, q) == bits).all()
+        assert (alpha_k.cpu().numpy().transpose(2, 0, 1).reshape(times, N, K // g, q) == alpha[0].astype(np.float16)).all()
+
+
+@pytest.mark.gpu
 def test_device_quantiser_feeds_the_matmul():
     """Quantise on the device straight into the container layout, multiply, compare with x W_hat^T from the oracle."""
     import torch
