@@ -428,13 +428,13 @@ int launch_gemv_reg(const lg::Gemv2Params& p, dim3 grid, bool bias, cudaStream_t
     int dev = 0;
     LG_CUDA(cudaGetDevice(&dev));
     if (dev >= 64 || !configured[dev][bias]) {
-        LG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lg::kRegSmemBytes));
+        LG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lg::kSmemLimit));
         if (dev < 64) configured[dev][bias] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(lg::kRegThreads);
-    cfg.dynamicSmemBytes = (size_t)lg::kRegSmemBytes;
+    cfg.dynamicSmemBytes = (size_t)lg::gemv2_smem_bytes(p.a_rows);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -574,12 +574,18 @@ bool gemv_pair_ok(const lutgemm_weight* w, const lutgemm_workspace* ws) {
            lg::gemv22_num_stages(w->a_rows) >= 2;
 }
 
+// Most scale groups of g that a slab of 512 k touches: slabs and groups begin on multiples of 32.
+int reg_scale_rows(int g) {
+    if (g >= lg::kSlab2) return g % lg::kSlab2 == 0 ? 1 : 2;
+    return lg::kSlab2 % g == 0 ? lg::kSlab2 / g : (lg::kSlab2 - 32) / g + 2;
+}
+
 // One matvec row: y (fp16 and/or fp32) = x . W
 int gemv_row(const lutgemm_weight* w, const lutgemm_workspace* ws, const __half* x, __half* y16, float* y32, cudaStream_t st) {
     const bool use_tma = (g_variant.load() == 0) && w->tma_ok;
     if (use_tma) return launch_gemv_tma_any(w, ws, x, y16, y32, nullptr, st);
     if (w->N % 4 == 0) {
-        // register-fed kernel: any group size that is a multiple of 32
+        // fed by regular copies: any group size that is a multiple of 32
         lg::Gemv2Params p = {};
         p.bW = w->bW; p.alpha = w->alpha; p.q_bias = w->q_bias; p.x = x;
         p.partial = ws->partial; p.counters = ws->counters; p.status = ws->status; p.y16 = y16; p.y32 = y32;
@@ -587,6 +593,7 @@ int gemv_row(const lutgemm_weight* w, const lutgemm_workspace* ws, const __half*
         p.nslabs = (w->K + lg::kSlab2 - 1) / lg::kSlab2;
         p.n_tile = choose_ntile(w->N, p.nslabs, 1, lg::kStageCols);
         p.ordered = ordered_for(ws);
+        p.a_rows = reg_scale_rows(w->g);
         dim3 grid((w->N + p.n_tile - 1) / p.n_tile, p.nslabs);
         const bool bias = w->q_bias != nullptr;
         if (w->g % 128 == 0) return launch_gemv_reg<2>(p, grid, bias, st);

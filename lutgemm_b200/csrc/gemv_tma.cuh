@@ -41,6 +41,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "sm100_async.cuh"
 
 namespace lg {
@@ -308,14 +310,43 @@ __device__ __forceinline__ void splitk_finish(const Gemv2Params& p, int tid, int
     if (tid == 0) p.counters[blockIdx.x] = 0u;   // ready for the next launch on this stream
 }
 
+// One lane of the 17th warp, two TMA loads per stage.  tmW: 3-D map {N, q, K/32} of uint32, box {256, 1, 16}; tmA: 3-D map {N, q, G} of
+// fp16, box {256, 1, a_rows}.
+struct FeedTma {
+    static constexpr int kArrivals = 1;
+    const CUtensorMap *tmW, *tmA;
+    __device__ __forceinline__ void operator()(const Gemv2Params& p, unsigned char* smem, uint32_t bar_full, uint32_t bar_empty, int n_begin, int,
+                                               int total_stages) const {
+        if ((threadIdx.x & 31) != 0) return;
+        const int q = p.q, stage_bytes = gemv2_stage_bytes(p.a_rows), nstages = gemv2_num_stages(p.a_rows);
+        const int kw0 = blockIdx.y * kSlabWords;
+        tma_prefetch_descriptor(tmW);
+        tma_prefetch_descriptor(tmA);
+        const int grp0 = blockIdx.y * kSlab2 / p.g;
+        const uint32_t tx = (uint32_t)stage_bytes;           // out-of-range parts are zero-filled and counted
+        int slot = 0, round = 0;
+        for (int t = 0; t < total_stages; t++) {
+            const int cg = t / q, b = t - cg * q;
+            if (round > 0) {
+                if (!mbar_wait_bounded(bar_empty + 8 * slot, (round - 1) & 1)) {
+                    atomicExch(p.status, kStatusProducerTimeout);
+                    break;
+                }
+            }
+            const int col0 = n_begin + cg * kStageCols;
+            const uint32_t dst = smem_u32(smem + kStage0Off + slot * stage_bytes);
+            mbar_arrive_expect_tx(bar_full + 8 * slot, tx);
+            tma_load_3d(dst, tmW, col0, b, kw0, bar_full + 8 * slot);
+            tma_load_3d(dst + kWStageBytes, tmA, col0, b, grp0, bar_full + 8 * slot);
+            if (++slot == nstages) { slot = 0; round++; }
+        }
+    }
+};
+
 // WPG: packed words per alpha group among a lane's two words of a stage (2: g % 128 == 0, else 1).
-// BIAS: container has q_bias.  tmW: 3-D map {N, q, K/32} of uint32, box {256, 1, 16};
-// tmA: 3-D map {N, q, G} of fp16, box {256, 1, a_rows}.
-template <int WPG, bool BIAS>
-__global__ void __launch_bounds__(kGemv2Threads, 1)
-gemv_tma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,
-                const Gemv2Params p) {
-    extern __shared__ __align__(1024) unsigned char smem[];
+// BIAS: container has q_bias.  FEED: what the warps behind the consumers do, a functor that brings stage after stage; THREADS: all warps.
+template <int WPG, bool BIAS, int THREADS, class FEED>
+__device__ __forceinline__ void gemv_body(const Gemv2Params& p, unsigned char* smem, FEED&& feed) {
     unsigned char* lut = smem;
     const int stage_bytes = gemv2_stage_bytes(p.a_rows);
     const int nstages = gemv2_num_stages(p.a_rows);
@@ -336,7 +367,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 
     if (tid == 0) {
         for (int s = 0; s < nstages; s++) {
-            mbar_init(bar_full + 8 * s, 1);
+            mbar_init(bar_full + 8 * s, std::remove_reference_t<FEED>::kArrivals);
             mbar_init(bar_empty + 8 * s, kConsWarps);
         }
         mbar_fence_init();
@@ -344,31 +375,10 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     __syncthreads();
     pdl_launch_dependents();
 
-    if (warp == kConsWarps) {
-        // ---------------- producer: one lane, two TMA loads per stage.  Weights and scales are never
-        // written by a kernel, so the stream may start before the previous kernel has finished. -------
-        if (lane == 0) {
-            tma_prefetch_descriptor(&tmW);
-            tma_prefetch_descriptor(&tmA);
-            const int grp0 = k0 / p.g;
-            const uint32_t tx = (uint32_t)stage_bytes;           // out-of-range parts are zero-filled and counted
-            int slot = 0, round = 0;
-            for (int t = 0; t < total_stages; t++) {
-                const int cg = t / q, b = t - cg * q;
-                if (round > 0) {
-                    if (!mbar_wait_bounded(bar_empty + 8 * slot, (round - 1) & 1)) {
-                        atomicExch(p.status, kStatusProducerTimeout);
-                        break;
-                    }
-                }
-                const int col0 = n_begin + cg * kStageCols;
-                const uint32_t dst = smem_u32(smem + kStage0Off + slot * stage_bytes);
-                mbar_arrive_expect_tx(bar_full + 8 * slot, tx);
-                tma_load_3d(dst, &tmW, col0, b, kw0, bar_full + 8 * slot);
-                tma_load_3d(dst + kWStageBytes, &tmA, col0, b, grp0, bar_full + 8 * slot);
-                if (++slot == nstages) { slot = 0; round++; }
-            }
-        }
+    if (warp >= kConsWarps) {
+        // ---------------- producers.  Weights and scales are never written by a kernel, so the stream may start before the
+        // previous kernel has finished. -------
+        feed(p, smem, bar_full, bar_empty, n_begin, n_end, total_stages);
         pdl_wait_prior_grids();
     } else {
         // ---------------- consumers ----------------
@@ -514,7 +524,14 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
     }
 
-    splitk_finish<kGemv2Threads>(p, tid, n_begin, n_end, s_flag);
+    splitk_finish<THREADS>(p, tid, n_begin, n_end, s_flag);
+}
+
+template <int WPG, bool BIAS>
+__global__ void __launch_bounds__(kGemv2Threads, 1)
+gemv_tma_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA, const Gemv2Params p) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    gemv_body<WPG, BIAS, kGemv2Threads>(p, smem, FeedTma{&tmW, &tmA});
 }
 
 // Last consumer of a tensor-parallel chain: waits for the ranks' fp32 rows, adds them in rank order and writes

@@ -101,6 +101,16 @@ def test_register_operand_kernel_per_plane_count(N, K, q, g, bias, m):
     _run("gemm_frag_kernel", N, K, q, g, bias, m)
 
 
+# one row of containers that tensor maps cannot describe: columns and K that end inside a stage, groups that begin anywhere in
+# a slab, wide ones and several to a lane's words, more stages than the ring holds, one nearly empty slab
+@pytest.mark.parametrize("N,K,q,g,bias", [
+    (4, 32, 1, 32, True), (260, 544, 3, 32, False), (1020, 1056, 4, 96, True), (516, 2080, 2, 160, False), (1284, 1536, 8, 128, True),
+    (9000, 1824, 5, 608, False), (132, 3328, 3, 416, True), (2052, 4128, 2, 1376, False), (20484, 576, 7, 64, True)])
+def test_matvec_by_copies(N, K, q, g, bias):
+    _run("gemv_reg_kernel", N, K, q, g, bias, 1)
+    _run("gemv_reg_kernel", N, K, q, g, bias, 1, ordered=True)
+
+
 # one row where the slabs do not share out evenly: runs of stages that begin and end between planes, cross into one or several
 # slabs, hold a column group twice; ragged last groups and slabs; both alpha forms; a run of one stage
 @pytest.mark.parametrize("N,K,q,g,bias", [
