@@ -69,14 +69,54 @@ pack_planes_kernel(const int8_t* __restrict__ planes, uint32_t* __restrict__ bW,
     bW[(size_t)kw * q * N + col] = s;
 }
 
+// Four planes, from b on, of eight rows x 32 codes that eight lanes hold (lane l8 codes 4 l8 .. + 3 of every row, the low bytes
+// of code u in byte u of t): lane l8 gets row l8's four words.
+__device__ __forceinline__ void u2b_words(const uint32_t (&t)[8], int b, int l8, uint32_t (&w)[4]) {
+    // per row 16 bits, the four codes' bits of a plane side by side (a 4 x 4 transpose); two rows to a register
+    uint32_t r[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t u0 = (t[2 * i] >> b) & 0x0f0f0f0fu, u1 = (t[2 * i + 1] >> b) & 0x0f0f0f0fu;
+        uint32_t x = __byte_perm(u0 | (u0 >> 4), u1 | (u1 >> 4), 0x6420), y;
+        y = (x ^ (x >> 3)) & 0x0a0a0a0au;
+        x ^= y ^ (y << 3);
+        y = (x ^ (x >> 6)) & 0x00cc00ccu;
+        r[i] = x ^ y ^ (y << 6);
+    }
+    // rows 4 .. 7 for the same of the lane four on, then rows 2, 3 of each four with the lane two on: sources in the order of lanes
+    const bool up4 = l8 & 4, up2 = l8 & 2, up1 = l8 & 1;
+    uint32_t s[4];
+    {
+        const uint32_t v0 = __shfl_xor_sync(0xffffffffu, up4 ? r[0] : r[2], 4), v1 = __shfl_xor_sync(0xffffffffu, up4 ? r[1] : r[3], 4);
+        const uint32_t a0 = up4 ? v0 : r[0], a1 = up4 ? v1 : r[1], c0 = up4 ? r[2] : v0, c1 = up4 ? r[3] : v1;
+        const uint32_t x0 = __shfl_xor_sync(0xffffffffu, up2 ? a0 : a1, 2), x1 = __shfl_xor_sync(0xffffffffu, up2 ? c0 : c1, 2);
+        s[0] = up2 ? x0 : a0;
+        s[1] = up2 ? a1 : x0;
+        s[2] = up2 ? x1 : c0;
+        s[3] = up2 ? c1 : x1;
+    }
+    // a row of the pair for the other of the neighbour
+    const uint32_t mine = up1 ? 0x7632u : 0x5410u, other = up1 ? 0x5410u : 0x7632u;
+    const uint32_t x0 = __shfl_xor_sync(0xffffffffu, __byte_perm(s[0], s[1], other), 1), x1 = __shfl_xor_sync(0xffffffffu, __byte_perm(s[2], s[3], other), 1);
+    const uint32_t o0 = __byte_perm(s[0], s[1], mine), o1 = __byte_perm(s[2], s[3], mine);
+    const uint32_t even0 = up1 ? x0 : o0, odd0 = up1 ? o0 : x0, even1 = up1 ? x1 : o1, odd1 = up1 ? o1 : x1;
+    // nibbles of lanes 2 i and 2 i + 1 to byte i of their plane's word
+    const uint32_t p0 = (even0 & 0x0f0f0f0fu) | ((odd0 << 4) & 0xf0f0f0f0u), p1 = (even1 & 0x0f0f0f0fu) | ((odd1 << 4) & 0xf0f0f0f0u);
+    const uint32_t q0 = ((even0 >> 4) & 0x0f0f0f0fu) | (odd0 & 0xf0f0f0f0u), q1 = ((even1 >> 4) & 0x0f0f0f0fu) | (odd1 & 0xf0f0f0f0u);
+    w[0] = __byte_perm(p0, p1, 0x6420);
+    w[2] = __byte_perm(p0, p1, 0x7531);
+    w[1] = __byte_perm(q0, q1, 0x6420);
+    w[3] = __byte_perm(q0, q1, 0x7531);
+}
+
 // Uniform (scale, zero, code) -> kernel-layout BCQ with offset, following
 // RTNParameter.convert_bcq_format (examples/rtn_parameter.py:77-96):
 //   alpha_b = scale/2 * 2^b, plane b = bit b of the code, q_bias = sum_b alpha_b - scale*zero (fp32),
-// then rounded to the container's fp16.  A warp takes 32 rows x 128 k (four k-words), one row at a time: a lane reads four
-// codes (128 bits, the warp 512 contiguous bytes), packs bit b of them into a nibble with one multiply, and three shuffles
-// OR the nibbles of eight lanes into a packed word, which the lane whose number in the eight is the row's keeps: the
-// stores are whole 32-byte sectors.  Bound by HBM (4 bytes read per code).  Measured, N = K = 8192, q = 4, g = 128:
-// 61.5 us (5.1 TB/s); one thread per word and row, as before, takes 250 us (every lane on another row's line).
+// then rounded to the container's fp16.  A warp takes 32 rows x 128 k (four k-words), eight rows at a time: a lane reads four
+// codes of each (128 bits, the warp 512 contiguous bytes), lays its codes' bits of a plane side by side, and eight lanes exchange
+// their eight rows (u2b_words) until each has one row's words: the stores are whole 32-byte sectors.  Bound by HBM (4 bytes read
+// per code).  Measured, N = K = 8192, q = 4, g = 128: 53.4 us (5.8 TB/s); 61.5 with three shuffles per row and plane (the issue slots 69 %
+// taken); one thread per word and row takes 250 us (every lane on another row's line).
 constexpr int kU2bWarps = 8;
 template <int Q>
 __global__ void __launch_bounds__(kU2bWarps * 32)
@@ -90,32 +130,34 @@ uniform_to_bcq_kernel(const float* __restrict__ scale, const float* __restrict__
     const size_t k = k0 + 4 * lane;                          // this lane's four codes; K % 32 == 0: whole octets of lanes
     const bool k_ok = k < K;
     const bool vec = (reinterpret_cast<uintptr_t>(code) & 15) == 0;
-    const int32_t* c = code + (size_t)n0 * K + k;
-    const int rows = min(32, N - n0);
+    // beyond the last row or K the last row's or first codes are read: their words are not stored
+    const int32_t* c = code + (size_t)n0 * K + (k_ok ? k : 0);
+    const int last = min(32, N - n0) - 1;
     uint32_t words[4][Q];                                    // rows l8, l8 + 8, ... of k-word k0 / 32 + lane / 8
 #pragma unroll
     for (int rb = 0; rb < 4; rb++) {
         int4 v[8];
+        if (vec) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            v[i] = make_int4(0, 0, 0, 0);
-            if (k_ok && 8 * rb + i < rows) {
-                const int32_t* src = c + (size_t)(8 * rb + i) * K;
-                if (vec) v[i] = __ldcs(reinterpret_cast<const int4*>(src));
-                else v[i] = make_int4(src[0], src[1], src[2], src[3]);
+            for (int i = 0; i < 8; i++) v[i] = __ldcs(reinterpret_cast<const int4*>(c + (size_t)min(8 * rb + i, last) * K));
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int32_t* src = c + (size_t)min(8 * rb + i, last) * K;
+                v[i] = make_int4(src[0], src[1], src[2], src[3]);
             }
         }
+        // the low byte of each code (planes 0..7), code t in byte t
+        uint32_t t[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            // the low byte of each code (planes 0..7), code t in byte t
-            const uint32_t t = __byte_perm(__byte_perm(v[i].x, v[i].y, 0x0040), __byte_perm(v[i].z, v[i].w, 0x0040), 0x5410);
+        for (int i = 0; i < 8; i++) t[i] = __byte_perm(__byte_perm(v[i].x, v[i].y, 0x0040), __byte_perm(v[i].z, v[i].w, 0x0040), 0x5410);
 #pragma unroll
-            for (int b = 0; b < Q; b++) {
-                uint32_t w = ((((t >> b) & 0x01010101u) * 0x01020408u) >> 24) << (4 * l8);      // bits 24..27 of the product
+        for (int b = 0; b < Q; b += 4) {
+            uint32_t w[4];
+            u2b_words(t, b, l8, w);
 #pragma unroll
-                for (int o = 4; o > 0; o >>= 1) w |= __shfl_xor_sync(0xffffffffu, w, o);
-                if (l8 == i) words[rb][b] = w;
-            }
+            for (int i = 0; i < 4; i++)
+                if (b + i < Q) words[rb][b + i] = w[i];
         }
     }
 #pragma unroll
