@@ -734,7 +734,7 @@ int hl_chain(const lutgemm_weight* w, bool ordered, bool f32) {
 
 // One CTA per SM: an item is 128 columns x 256 rows, and an item may be cut into two halves of 128 rows or into k-ranges.
 // Cost model in cycles: a block of 64 k takes the tensor pipe and shared memory kHlRowCycles per row and pass, and the
-// expansion kHlExpCycles whatever the rows, more with more table entries; a CTA's start, first loads and epilogue add
+// expansion kHlExpCycles whatever the rows, more with more table entries (kHlExpRegCycles up to two planes, which have no table); a CTA's start, first loads and epilogue add
 // kHlCtaCycles; a split adds kHlSplitCycles and, per row, the reductions in L2 and the last arriver's pass (shared among the
 // k-ranges), which a part-filled wave does faster.  Fitted to 804 timed calls (1024 x 8192 to 28672 x 4096, q = 1 to 4, 16 to
 // 2048 rows, split and not; the estimate's spread is 7 %).  A split that cost 4000 cycles whatever its rows gave 8192 x 2048,
@@ -742,7 +742,7 @@ int hl_chain(const lutgemm_weight* w, bool ordered, bool f32) {
 // at 14 widths 214 got faster by more than 3 % and 17 slower, the most 5120 x 5120, q = 2, 400 rows: 51.7 (46.4).
 // The plan with the smallest estimate is taken: whole items, halves, whole items
 // with a last partial wave of halves, each with 1 to 8 k-ranges.  Returns the estimate.
-constexpr double kHlRowCycles = 2.18, kHlExpCycles = 630, kHlEntryCycles = 8.5, kHlBiasCycles = 14.5;
+constexpr double kHlRowCycles = 2.18, kHlExpCycles = 630, kHlEntryCycles = 8.5, kHlBiasCycles = 14.5, kHlExpRegCycles = 510;
 constexpr double kHlCtaCycles = 6300, kHlSplitCycles = 4400, kHlSplitRowCycles = 30, kHlDrainRowCycles = 25;
 double hl_plan(const lutgemm_weight* w, int m, bool may_split, int chain, lg::HlParams* p) {
     const int sms = sm_count();
@@ -750,7 +750,7 @@ double hl_plan(const lutgemm_weight* w, int m, bool may_split, int chain, lg::Hl
     const long long items = (long long)T * RT;
     const int blocks = (w->K + lg::kHlStepK - 1) / lg::kHlStepK;
     const double per_row = (w->q == 1 && !w->q_bias ? 1 : 2) * kHlRowCycles;
-    const double expansion = kHlExpCycles + kHlEntryCycles * ((1 << w->q) - 2) + (w->q_bias ? kHlBiasCycles : 0);
+    const double expansion = w->q <= 2 ? kHlExpRegCycles : kHlExpCycles + kHlEntryCycles * ((1 << w->q) - 2) + (w->q_bias ? kHlBiasCycles : 0);
     auto block_cost = [&](int rows) { const double t = per_row * ((rows + 15) / 16 * 16); return t > expansion ? t : expansion; };
     const int whole_rows = m < lg::kHlRows ? m : lg::kHlRows, half_rows = m < 128 ? m : 128;
     const long long units = m <= 128 ? items : (long long)T * ((m + 127) / 128);       // halves that have rows
@@ -813,18 +813,21 @@ int hl_split_rows_of(const lutgemm_weight* w) {
 }
 
 // From which row count the split-operand kernel is the faster one: it always takes two tensor-core passes, gemm_tc one
-// per plane and one for q_bias.  Measured, us (gemm_tc / split operand), g = 128: 2 passes, 8192 x 8192, 96 rows 33.3 / 33.8,
-// 128 rows 39.1 / 35.7; 3 passes, 8192 x 8192, 32 rows 31.6 / 32.0, 64 rows 36.7 / 32.4; 4 passes, 12288 x 4096, 32 rows
-// 28.0 / 30.0, 64 rows 33.7 / 31.0, 96 rows 40.5 / 32.3; 5 passes, 28672 x 8192, 4 rows 160 / 116.  At and above these row
-// counts no call was slower than with gemm_tc by more than 2 % at 14 widths from 1024 to 28672 (672 calls, g = 128; 216 at g =
-// 32, 64, 256).
+// per plane and one for q_bias.  Measured, us (gemm_tc / split operand), g = 128, fp16 results: one plane, 8192 x 8192, 64 rows 22.2 /
+// 20.3, 96 rows 21.4 / 22.9, 128 rows 24.6 / 24.3; 2 passes, 8192 x 8192, 32 rows 23.1 / 23.0, 64 rows 27.4 / 24.1, 12288 x 4096, 48 rows 18.6 / 21.1, 64
+// rows 21.5 / 21.4; 2 planes + q_bias, 8192 x 8192, 9 rows 31.7 / 22.7, 12288 x 4096, 22.6 / 20.5, 28672 x 8192, 107 / 82; 3 planes,
+// 8192 x 8192, 32 rows 31.6 / 32.0, 64 rows 36.7 / 32.4; 4 planes, 12288 x 4096, 32 rows 28.0 / 30.0, 64 rows 33.7 / 31.0; 5 passes, 28672 x 8192,
+// 4 rows 160 / 116.  Up to 2048 columns gemm_tc's 256-column tiles and 8 k-ranges leave half of the SMs idle: 2048 x 8192, 9 rows, q = 2 12.4 /
+// 8.4, q = 4 18.6 / 10.4; 2048 x 2048, q = 3 6.3 / 5.7; 1024 x 4096, q = 4 10.9 / 5.4.
 // Where it has to drain its accumulators (fp32 results, very long k): 2 passes, 28672 x 8192, 128 rows, fp32 113 / 128, 11008 x
-// 4096 31 / 35, 8192 x 28672, fp16 96 / 108; more passes as above (3 passes, 28672 x 8192, 100 rows, fp32 141 / 132).
+// 4096 31 / 35, 8192 x 28672, 64 rows, fp16 75 / 84; more passes as above (3 passes, 28672 x 8192, 100 rows, fp32 141 / 132).
 bool gemm_hl_ok(const lutgemm_weight* w, int m, bool f32) {
     const int passes = w->q + (w->q_bias ? 1 : 0);
     const int T = (w->N + lg::kHlCols - 1) / lg::kHlCols, ranges = sm_count() / T < 1 ? 1 : sm_count() / T;
     const bool drains = f32 || w->K / 8 > kHlChain16 * ranges;    // up to 128 rows: 8 accumulations per 64 k of a range
-    const int from = passes >= 5 ? 4 : passes >= 3 ? 64 : passes == 2 && !drains ? 97 : 129;
+    int from = passes >= 5 ? 4 : passes >= 3 || (passes == 2 && !drains) ? 64 : 129;
+    if (!drains && w->N <= 8 * lg::kTcTileN) from = 4;
+    else if (!drains && w->q == 2 && w->q_bias) from = 9;
     // with g = 32 every block builds two tables: up to 128 rows, where the expansion bounds it, that goes to gemm_tc
     return w->tc_ok && w->q <= 4 && m >= from && (m > 128 || w->g >= lg::kHlStepK);
 }

@@ -19,6 +19,8 @@
 //   them: no synchronisation, no bank conflicts), turns the q words into one code per byte (a bit transpose of shifts
 //   and LOP3s), looks 64 weights up (one PRMT makes a code byte and the lane's bank an address) and stores them with
 //   tcgen05.st as the A operand in tensor memory.
+//   Up to two planes the values (four at most) stay in registers and a PRMT picks two weights' halves at a time: no table, no
+//   reads of shared memory.  8192 x 8192, q = 2, 128 rows 31.4 us (32.9 with the table), q = 2 + q_bias, 64 rows 24.4 (27.4).
 //   One lane issues tcgen05.mma.kind::f16: M = 128 columns, N = rows, K = 16, A (hi, then lo) in tensor memory, the
 //   activations [rows][64 k] (TMA, 128-byte swizzle) in shared memory, one fp32 accumulator.
 //   Every accumulation of the tensor core cuts its fp32 sum off toward zero: measured, the error of a chain of n is 1.8e-8 n
@@ -179,6 +181,7 @@ __global__ void __launch_bounds__(kHlThreads, 1)
 gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ HlParams p) {
     constexpr int NV = 1 << Q;
     constexpr int PASSES = (Q == 1 && !BIAS) ? 1 : 2;
+    constexpr bool IN_REGS = Q <= 2;          // up to four values: a PRMT picks them out of two registers
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t smem_base = smem_u32(smem);
     const uint32_t bar_xfull = smem_base + kHlBarOff;             // kHlMaxSlots each
@@ -250,6 +253,7 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     if (warp >= kHlFirstExpWarp) {
         // ---------------- expansion ----------------
         const size_t row_w = (size_t)Q * N;                       // words per k-word row, scales per group
+        // one block ahead: with two or three a call of 16 to 128 rows took 1 to 2 us more (registers, moves)
         uint32_t w[2][Q];
         unsigned short av[2][Q], bv[2];
         // This warp's next block: its words, its group (advanced by 4 blocks = 256 k without a division).  Loads are not
@@ -334,6 +338,7 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         unsigned char* tab = smem + (ew >> 1) * 4096 + bank;
         const uint32_t t_dst = tmem_base + ((uint32_t)(lq * 32) << 16) + kHlACol + (uint32_t)sub * 64u;
         int round = 0, j = sub;
+        uint32_t t_hi[NV / 2] = {}, t_lo[NV / 2] = {};           // IN_REGS: the values' halves, two to a register
         // segment by segment: this warp's blocks up to and with its first one beyond the segment, then the drain, during which
         // those blocks wait for the tensor core (the stage of block j is free once block j - 4, of this segment, has been read)
 #pragma unroll 1
@@ -373,22 +378,42 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
                             v[c + (1 << b)] = s + a[u][b];
                         }
                     }
+                    if constexpr (IN_REGS) {
 #pragma unroll
-                    for (int c = 0; c < NC; c += 2) {
-                        uint32_t e0, e1;
-                        hl_pack_pair(v[c], v[c + 1], e0, e1);
-                        *reinterpret_cast<uint32_t*>(tab + c * 256) = e0;
-                        *reinterpret_cast<uint32_t*>(tab + (c + 1) * 256) = e1;
-                        if (NC < NV) {
-                            *reinterpret_cast<uint32_t*>(tab + (NV - 1 - c) * 256) = e0 ^ 0x80008000u;
-                            *reinterpret_cast<uint32_t*>(tab + (NV - 2 - c) * 256) = e1 ^ 0x80008000u;
+                        for (int c = 0; c < NV; c += 2) {
+                            // without q_bias the upper half of four values are the lower's negatives, the other way round
+                            const float v0 = c < NC ? v[c < NC ? c : 0] : -v[c < NC ? 0 : NV - 1 - c], v1 = c < NC ? v[c < NC ? c + 1 : 0] : -v[c < NC ? 0 : NV - 2 - c];
+                            const __half2 h = __floats2half2_rn(v0, v1);
+                            const float2 f = __half22float2(h);
+                            const __half2 l = __floats2half2_rn(v0 - f.x, v1 - f.y);
+                            t_hi[c / 2] = *reinterpret_cast<const uint32_t*>(&h);
+                            t_lo[c / 2] = *reinterpret_cast<const uint32_t*>(&l);
                         }
-                    }
-                    if (!(bound <= 65504.f)) {                    // an infinite or NaN scale: the value itself, lo = 0
+                        if (!(bound <= 65504.f)) {                // an infinite or NaN scale: the value itself, lo = 0
+#pragma unroll
+                            for (int c = 0; c < NV / 2; c++) {
+                                if ((t_hi[c] & 0x7c00u) == 0x7c00u) t_lo[c] &= 0xffff0000u;
+                                if ((t_hi[c] & 0x7c000000u) == 0x7c000000u) t_lo[c] &= 0xffffu;
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < NC; c += 2) {
+                            uint32_t e0, e1;
+                            hl_pack_pair(v[c], v[c + 1], e0, e1);
+                            *reinterpret_cast<uint32_t*>(tab + c * 256) = e0;
+                            *reinterpret_cast<uint32_t*>(tab + (c + 1) * 256) = e1;
+                            if (NC < NV) {
+                                *reinterpret_cast<uint32_t*>(tab + (NV - 1 - c) * 256) = e0 ^ 0x80008000u;
+                                *reinterpret_cast<uint32_t*>(tab + (NV - 2 - c) * 256) = e1 ^ 0x80008000u;
+                            }
+                        }
+                        if (!(bound <= 65504.f)) {                    // an infinite or NaN scale: the value itself, lo = 0
 #pragma unroll 1
-                        for (int c = 0; c < NV; c++) {
-                            uint32_t* e = reinterpret_cast<uint32_t*>(tab + c * 256);
-                            if ((*e & 0x7c00u) == 0x7c00u) *e &= 0xffffu;
+                            for (int c = 0; c < NV; c++) {
+                                uint32_t* e = reinterpret_cast<uint32_t*>(tab + c * 256);
+                                if ((*e & 0x7c00u) == 0x7c00u) *e &= 0xffffu;
+                            }
                         }
                     }
                 }
@@ -406,22 +431,36 @@ gemm_hl_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
                     n[3] = ((o01 >> 2) & 0x33333333u) | (o23 & 0xccccccccu);
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
-                        lo4[r] = (n[r] & 0x0f0f0f0fu) | pair4;
-                        hi4[r] = ((n[r] >> 4) & 0x0f0f0f0fu) | pair4;
+                        lo4[r] = n[r] & 0x0f0f0f0fu;
+                        hi4[r] = (n[r] >> 4) & 0x0f0f0f0fu;
+                        // code c to the selectors of a value's two bytes, 2 c and 2 c + 1; or to its place in the table
+                        lo4[r] = IN_REGS ? lo4[r] * 0x22u + 0x10101010u : lo4[r] | pair4;
+                        hi4[r] = IN_REGS ? hi4[r] * 0x22u + 0x10101010u : hi4[r] | pair4;
                     }
                 }
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
-                    uint32_t e[4];
+                    if constexpr (IN_REGS) {
 #pragma unroll
-                    for (int r = 0; r < 4; r++)
-                        e[r] = *reinterpret_cast<const uint32_t*>(smem + prmt_b32((i & 1) ? hi4[r] : lo4[r], bank, 0x6504u | (uint32_t)((i >> 1) << 4)));
-                    hi[2 * i] = prmt_b32(e[0], e[1], 0x5410u);
-                    hi[2 * i + 1] = prmt_b32(e[2], e[3], 0x5410u);
-                    if (PASSES == 2) {
-                        lo[2 * i] = prmt_b32(e[0], e[1], 0x7632u);
-                        lo[2 * i + 1] = prmt_b32(e[2], e[3], 0x7632u);
+                        for (int r = 0; r < 4; r += 2) {
+                            // two weights at a time: a byte of selectors from each of two words
+                            const uint32_t pick = (uint32_t)(i >> 1) | (uint32_t)(4 + (i >> 1)) << 4;
+                            const uint32_t at = (i & 1) ? prmt_b32(hi4[r], hi4[r + 1], pick) : prmt_b32(lo4[r], lo4[r + 1], pick);
+                            hi[2 * i + r / 2] = prmt_b32(t_hi[0], t_hi[NV / 2 - 1], at);
+                            if (PASSES == 2) lo[2 * i + r / 2] = prmt_b32(t_lo[0], t_lo[NV / 2 - 1], at);
+                        }
+                    } else {
+                        uint32_t e[4];
+#pragma unroll
+                        for (int r = 0; r < 4; r++)
+                            e[r] = *reinterpret_cast<const uint32_t*>(smem + prmt_b32((i & 1) ? hi4[r] : lo4[r], bank, 0x6504u | (uint32_t)((i >> 1) << 4)));
+                        hi[2 * i] = prmt_b32(e[0], e[1], 0x5410u);
+                        hi[2 * i + 1] = prmt_b32(e[2], e[3], 0x5410u);
+                        if (PASSES == 2) {
+                            lo[2 * i] = prmt_b32(e[0], e[1], 0x7632u);
+                            lo[2 * i + 1] = prmt_b32(e[2], e[3], 0x7632u);
+                        }
                     }
                 }
                 if (u == 0 && round > 0) {                        // the stage is touched only here: the work above overlaps its last MMAs

@@ -69,6 +69,30 @@ def test_split_operand_kernel(N, K, q, g, bias, m):
     _run("gemm_hl_kernel", N, K, q, g, bias, m)
 
 
+# fp16 results of few rows: narrow weights of any plane count, and two planes with q_bias; values in registers (up to two planes)
+# and in the table, ragged last columns and blocks, one and two scale groups to a block
+@pytest.mark.parametrize("N,K,q,g,bias,m", [
+    (8, 64, 1, 64, False, 9), (136, 576, 1, 64, True, 12), (264, 2048, 2, 64, False, 16), (2048, 1152, 3, 128, False, 11),
+    (520, 4096, 4, 128, False, 33), (2056, 320, 2, 64, True, 9), (4104, 1024, 2, 128, True, 31), (4104, 192, 2, 64, False, 64), (24, 128, 2, 128, True, 63)])
+def test_split_operand_kernel_few_rows(N, K, q, g, bias, m):
+    bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + K + m, with_bias=bias)
+    x = synth.activations(m, K, seed=m)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g, q_bias).reserve_batch(m)
+    xd = torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
+    y = torch.empty((m, N), dtype=torch.float16, device="cuda")
+    a16, b16 = alpha.astype(np.float16), None if q_bias is None else q_bias.astype(np.float16)
+    ref = oracle.bcq_matmul_f64(x, bW, a16, b16, g)
+    # as in _run: K / 16 additions per pass, a weight off by up to 2^-22 of it, one rounding to fp16
+    mag = np.abs(a16.astype(np.float64)).sum(1) + (0 if b16 is None else np.abs(b16.astype(np.float64)))
+    size = np.abs(x.astype(np.float64)).reshape(m, K // g, g).sum(2) @ mag
+    lim = ((2 * K / 16 + 64) * 2.0 ** -23 + 2.0 ** -22) * size + np.maximum(np.abs(ref) * 2.0 ** -11, 2.0 ** -25)
+    for _ in range(2):
+        L.matmul(y, xd, w, m)
+        assert L.last_launch()[0] == "gemm_hl_kernel"
+        assert (np.abs(y.cpu().numpy().astype(np.float64) - ref) <= lim * 1.0001).all()
+    w.close()
+
+
 @pytest.mark.parametrize("q,bias,m", [(4, True, 40), (2, False, 150), (1, False, 200), (3, True, 256)])
 def test_split_operand_kernel_scales_far_apart(q, bias, m):
     _run("gemm_hl_kernel", 264, 1024, q, 128, bias, m, column_scales=True)
