@@ -382,7 +382,7 @@ unsigned long long lutgemm_kernel_launch_count(void);
 const char* lutgemm_last_launch(int* grid_x, int* grid_y);
 /* Tuning knob: columns per CTA of the LUT matvec (0 = automatic).  Process-wide. */
 int lutgemm_set_gemv_ntile(int columns);
-/* Tuning knob: 0 = bulk-copy (TMA) fed matvec kernel (default), 1 = register-streaming kernel.
+/* Tuning knob: 0 = bulk-copy (TMA) fed matvec kernel (default), 1 = the same kernel fed by regular copies.
  * Process-wide; both compute the same function. */
 int lutgemm_set_gemv_variant(int variant);
 /* 0 (default): the TMA-fed matvec adds its k-slabs with fp32 reductions in L2, whose order is not
