@@ -154,10 +154,11 @@ gemv_flat_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 const int nb = min(q - b0, left);
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
                 uint2 bv[NG];
+                const bool first = b0 == 0;      // the piece with the group's first plane adds the offset term: 0 times an infinite sum is NaN
                 if (BIAS) {
 #pragma unroll
                     for (int gi = 0; gi < NG; gi++)
-                        bv[gi] = (col_ok && b0 == 0 && bias[gi]) ? ldg_nc_v2(bias[gi] + cg * kStageCols) : make_uint2(0u, 0u);
+                        bv[gi] = (col_ok && first && bias[gi]) ? ldg_nc_v2(bias[gi] + cg * kStageCols) : make_uint2(0u, 0u);
                 }
                 for (int b = 0; b < nb && !aborted; b++) {
                     if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar_full + 8 * slot, round & 1))) {
@@ -197,7 +198,7 @@ gemv_flat_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                         acc[3] = fmaf(s2[3].x + s2[3].y, a23.y, acc[3]);
                     }
                 }
-                if (BIAS) {
+                if (BIAS && first) {
 #pragma unroll
                     for (int gi = 0; gi < NG; gi++) {
                         const float2 b01 = half2_bits_to_float2(bv[gi].x), b23 = half2_bits_to_float2(bv[gi].y);

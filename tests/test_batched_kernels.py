@@ -144,6 +144,33 @@ def test_matvec_in_runs(N, K, q, g, bias):
     _run("gemv_flat_kernel", N, K, q, g, bias, 1)
 
 
+# An infinite activation among the last three of its eight, whose sign a table entry has no sum of both signs of: an infinity where
+# the planes (and the offset) agree in sign, else NaN, wherever a run begins and ends.
+@pytest.mark.parametrize("kernel,N,K,q,g,bias", [
+    ("gemv_flat_kernel", 4096, 28672, 3, 256, True), ("gemv_flat_kernel", 1032, 40480, 2, 32, True), ("gemv_flat_kernel", 8192, 20480, 2, 128, False),
+    ("gemv_tma_kernel", 1032, 4096, 3, 128, True), ("gemv_reg_kernel", 1028, 4128, 2, 96, True)])
+def test_matvec_activations_not_finite(kernel, N, K, q, g, bias):
+    bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + K, with_bias=bias)
+    alpha = np.maximum(alpha, 2.0 ** -10)                 # 0 * inf would be NaN in every column
+    x = synth.activations(1, K, seed=K)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g, q_bias)
+    y = torch.empty((1, N), dtype=torch.float32, device="cuda")
+    for k, value in ((K // 2 // 8 * 8 + 6, np.inf), (K - 8 + 5, -np.inf), (7, np.inf)):
+        xi = x.copy()
+        xi[0, k] = value
+        bits = (bW[k // 32] >> np.uint32(k % 32)) & np.uint32(1)                                      # [q, N]
+        terms = np.where(bits == 1, 1.0, -1.0) * alpha[k // g].astype(np.float16).astype(np.float64)
+        if bias:
+            terms = np.concatenate([terms, q_bias[k // g].astype(np.float16).astype(np.float64)[None]])
+        with np.errstate(invalid="ignore"):
+            ref = (terms * np.float64(value)).sum(0)
+        assert 0 < np.isinf(ref).sum() < N
+        L.matmul_f32(y, torch.from_numpy(xi.view(np.int16)).cuda().view(torch.float16), w, 1)
+        assert L.last_launch()[0] == kernel
+        assert np.array_equal(y.cpu().numpy()[0], ref.astype(np.float32), equal_nan=True), k
+    w.close()
+
+
 # two and three rows: the register operand up to 64 Mi weights of planes and where one slab of k is enough, else the LUT kernels
 @pytest.mark.parametrize("N,K,q,g,bias,m,kernel", [
     (72, 128, 1, 64, True, 2, "gemm_frag_kernel"), (4096, 4096, 4, 128, False, 2, "gemm_frag_kernel"), (4104, 4096, 4, 128, False, 2, "gemv_tma2_kernel"),
