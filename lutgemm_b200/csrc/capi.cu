@@ -479,16 +479,7 @@ int launch_gemv_flat(const lutgemm_weight* w, const lg::Gemv2Params& p, bool bia
     }
     const dim3 grid(sm_count());
     lg::FlatRuns runs;
-    const int groups = (p.N + lg::kStageCols - 1) / lg::kStageCols;
-    const int total = p.nslabs * groups * p.q, n = (int)grid.x, base = total / n, longer = total % n;
-    int unit = 0, plane = 0;                 // run i begins at stage i * base + min(i, longer)
-    for (int i = 0; i < n; i++) {
-        const int stages = base + (i < longer ? 1 : 0);
-        runs.run[i] = {stages, plane, unit % groups, unit / groups};
-        plane += stages;
-        unit += plane / p.q;
-        plane %= p.q;
-    }
+    lg::flat_plan(runs, p.nslabs, (p.N + lg::kStageCols - 1) / lg::kStageCols, p.q, (int)grid.x);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(lg::kGemv2Threads);

@@ -17,6 +17,10 @@
 
 namespace lg {
 
+// The lookups have the table's address in their instructions (lookup_word_seq) where dynamic shared memory begins at BASE, as it
+// does for a kernel without static shared memory; elsewhere, as under a tool that takes some for itself, the same loop adds the address
+// in a register, which is 2 to 7 % slower (8192 x 28672, q = 4, 31.0 and 32.3 us).
+//
 // The runs travel as a parameter: read at blockIdx.x they are in uniform registers and so are the loops' bounds.  (Worked out from
 // blockIdx.x in the kernel, by divisions, they were not, and every loop reconverged its warp, as it does where
 // one lane's failed wait may end it: hence the vote.  49152 x 12288, q = 4, 67.6 us without either, 64.8 with both.)
@@ -30,7 +34,20 @@ struct FlatRuns {
 };
 constexpr int kFlatMaxPieces = kConsWarps * 16;             // column groups of a CTA's run: their list lies in the exchange area
 
-template <int WPG, bool BIAS>
+// Stages (slab, group, plane) cut into `ctas` runs that differ by one stage at most.
+inline void flat_plan(FlatRuns& runs, int nslabs, int groups, int q, int ctas) {
+    const int total = nslabs * groups * q, base = total / ctas, longer = total % ctas;
+    int unit = 0, plane = 0;                 // run i begins at stage i * base + min(i, longer)
+    for (int i = 0; i < ctas; i++) {
+        const int stages = base + (i < longer ? 1 : 0);
+        runs.run[i] = {stages, plane, unit % groups, unit / groups};
+        plane += stages;
+        unit += plane / q;
+        plane %= q;
+    }
+}
+
+template <int WPG, bool BIAS, uint32_t BASE = kSeqSmemBase>
 __global__ void __launch_bounds__(kGemv2Threads, 1)
 gemv_flat_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA, const Gemv2Params p,
                  const __grid_constant__ FlatRuns runs) {
@@ -47,10 +64,6 @@ gemv_flat_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     const int groups = (N + kStageCols - 1) / kStageCols;
     const FlatRun run = runs.run[blockIdx.x];
     const int plane0 = run.plane, slab0 = run.slab, group0 = run.group;
-    if (smem_u32(smem) != kSeqSmemBase) {                        // the lookups have the table's address in their instructions
-        if (tid == 0) atomicExch(p.status, kStatusLayout);
-        return;
-    }
 
     if (tid == 0) {
         for (int s = 0; s < nstages; s++) {
@@ -121,6 +134,8 @@ gemv_flat_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         int slot = 0, round = 0;
         int left = run.stages, b0 = plane0, cg = group0;
         pdl_wait_prior_grids();                  // the activations may come from the previous kernel
+        auto consume = [&](auto known_base) {
+        constexpr bool KNOWN = decltype(known_base)::value;
 #pragma unroll 1
         for (int slab = slab0; left > 0; slab++, cg = 0) {
             const int k0 = slab * kSlab2;
@@ -187,7 +202,9 @@ gemv_flat_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                             const uint32_t ww[4] = {wv[u].x, wv[u].y, wv[u].z, wv[u].w};
 #pragma unroll
                             for (int c = 0; c < 4; c++) {
-                                const float2 v = (u == 0) ? lookup_word_seq<0>(ww[c], cs, sel) : lookup_word_seq<128>(ww[c], cs, sel);
+                                float2 v;
+                                if constexpr (KNOWN) v = (u == 0) ? lookup_word_seq<0>(ww[c], cs, sel) : lookup_word_seq<128>(ww[c], cs, sel);
+                                else v = (u == 0) ? lookup_word<0>(lut, ww[c], cs, sel) : lookup_word<128>(lut, ww[c], cs, sel);
                                 s2[c] = (jj == 0) ? v : add_f32x2(s2[c], v);
                             }
                         }
@@ -225,6 +242,9 @@ gemv_flat_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                 b0 = 0;
             }
         }
+        };
+        if (smem_u32(smem) == BASE) consume(std::true_type{});
+        else consume(std::false_type{});
     }
 
     // ---- finish: the column groups that this CTA's planes complete ----

@@ -1,9 +1,12 @@
 """The batched kernels that fold planes or keep operands in registers, at the edges of their tiles, against 64-bit sums."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
 import lutgemm_b200 as L
-from lutgemm_b200 import synth
+from lutgemm_b200 import _build, synth
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -169,6 +172,16 @@ def test_matvec_activations_not_finite(kernel, N, K, q, g, bias):
         assert L.last_launch()[0] == kernel
         assert np.array_equal(y.cpu().numpy()[0], ref.astype(np.float32), equal_nan=True), k
     w.close()
+
+
+def test_matvec_in_runs_wherever_shared_memory_begins(tmp_path):
+    """The lookups' fixed address is where dynamic shared memory begins; instantiated for another one, the kernel still gives the
+    result (tests/cpp/flat_any_base.cu compares both with 64-bit sums)."""
+    src, exe = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cpp", "flat_any_base.cu"), str(tmp_path / "flat_any_base")
+    subprocess.check_call([_build.NVCC, "-std=c++17", "-O2", "-gencode", "arch=compute_100a,code=sm_100a", src, "-o", exe],
+                          stdout=subprocess.DEVNULL, stderr=subprocess.DEVNULL)
+    out = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0 and "flat ok" in out.stdout, out.stdout + out.stderr
 
 
 # two and three rows: the register operand up to 64 Mi weights of planes and where one slab of k is enough, else the LUT kernels
