@@ -713,14 +713,26 @@ int gemm_tc_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 }
 
 // ---- split-operand kernel (gemm_hl.cuh): plan, launch ----
-// Longest chain of tensor-core accumulations (each cuts the fp32 sum off) between two drains: the plane kernel's, 8 per plane
-// and 128 k, less a sixteenth, so that an fp32 result is no further off than that kernel's.  An fp16 result has an error of 2.1e-4 of its own; a
-// chain of 1536 adds 2.8e-5 to that, 0.9 % of it, and costs no drain up to 12288 k (12288 x 12288, q = 4 + q_bias, 1024 rows:
-// 427 us, 464 with one drain).
+// Rows from which the split-operand kernel is the faster one whatever the columns (figures at gemm_hl_ok).
 constexpr int kHlChain16 = 1536;
-int hl_chain(const lutgemm_weight* w, bool ordered, bool f32) {
+int hl_many_rows(const lutgemm_weight* w, bool f32) {
+    const int passes = w->q + (w->q_bias ? 1 : 0);
+    const int T = (w->N + lg::kHlCols - 1) / lg::kHlCols, ranges = sm_count() / T < 1 ? 1 : sm_count() / T;
+    const bool drains = f32 || w->K / 8 > kHlChain16 * ranges;    // up to 128 rows: 8 accumulations per 64 k of a range
+    return passes >= 5 ? 4 : passes >= 3 ? 64 : passes == 2 && !drains ? 97 : 129;
+}
+
+// Longest chain of tensor-core accumulations (each cuts the fp32 sum off) between two drains.  fp32 results: the plane kernel's, 8 per
+// plane and 128 k, less a sixteenth, so that they are no further off than that kernel's.  fp16 results of many rows have an error of
+// 2.1e-4 of their own; a chain of 1536 adds 2.8e-5 to that, 0.9 % of it, and costs no drain up to 12288 k (12288 x 12288, q = 4 + q_bias,
+// 1024 rows: 427 us, 464 with one drain).  fp16 results of fewer rows, for which this kernel stands in where the plane kernel is merely
+// the slower one: the plane kernel's, so that as many sums fall on the right side of a rounding.  Measured, sums that do not, plane
+// kernel / this one / this one in a single chain, %: 28672 x 1024, q = 2, 80 rows 0.28 / 0.28 / 0.81; 12288 x 4096, q = 2 + q_bias, 24 rows
+// 1.2 / 1.2 / 1.5; 2560 x 1024, q = 1 + q_bias, 80 rows 0.15 / 0.12 / 0.41; 8192 x 8192, q = 2 + q_bias, 24 rows 2.4 / 1.7 / 2.2.
+int hl_chain(const lutgemm_weight* w, int m, bool ordered, bool f32) {
     const int plane = 8 * (w->q + (w->q_bias ? 1 : 0)) * tc_steps_per_cta(w, ordered);
-    return f32 ? plane - plane / 16 : plane > kHlChain16 ? plane : kHlChain16;
+    if (f32) return plane - plane / 16;
+    return m < hl_many_rows(w, false) || plane > kHlChain16 ? plane : kHlChain16;
 }
 
 // One CTA per SM: an item is 128 columns x 256 rows, and an item may be cut into two halves of 128 rows or into k-ranges.
@@ -803,22 +815,27 @@ int hl_split_rows_of(const lutgemm_weight* w) {
     return rows;
 }
 
-// From which row count the split-operand kernel is the faster one: it always takes two tensor-core passes, gemm_tc one
-// per plane and one for q_bias.  Measured, us (gemm_tc / split operand), g = 128, fp16 results: one plane, 8192 x 8192, 64 rows 22.2 /
-// 20.3, 96 rows 21.4 / 22.9, 128 rows 24.6 / 24.3; 2 passes, 8192 x 8192, 32 rows 23.1 / 23.0, 64 rows 27.4 / 24.1, 12288 x 4096, 48 rows 18.6 / 21.1, 64
-// rows 21.5 / 21.4; 2 planes + q_bias, 8192 x 8192, 9 rows 31.7 / 22.7, 12288 x 4096, 22.6 / 20.5, 28672 x 8192, 107 / 82; 3 planes,
-// 8192 x 8192, 32 rows 31.6 / 32.0, 64 rows 36.7 / 32.4; 4 planes, 12288 x 4096, 32 rows 28.0 / 30.0, 64 rows 33.7 / 31.0; 5 passes, 28672 x 8192,
-// 4 rows 160 / 116.  Up to 2048 columns gemm_tc's 256-column tiles and 8 k-ranges leave half of the SMs idle: 2048 x 8192, 9 rows, q = 2 12.4 /
-// 8.4, q = 4 18.6 / 10.4; 2048 x 2048, q = 3 6.3 / 5.7; 1024 x 4096, q = 4 10.9 / 5.4.
-// Where it has to drain its accumulators (fp32 results, very long k): 2 passes, 28672 x 8192, 128 rows, fp32 113 / 128, 11008 x
-// 4096 31 / 35, 8192 x 28672, 64 rows, fp16 75 / 84; more passes as above (3 passes, 28672 x 8192, 100 rows, fp32 141 / 132).
+// Which batches the split-operand kernel is the faster one for: it always takes two tensor-core passes, gemm_tc one per plane and
+// one for q_bias.  Measured, us (gemm_tc / split operand), g = 128 unless stated.  Many rows, any columns: 2 passes, 8192 x 8192, 128 rows
+// 39.1 / 34.3; 3 passes, 8192 x 8192, 32 rows 31.6 / 32.0, 64 rows 36.7 / 32.4; 4 passes, 12288 x 4096, 32 rows 28.0 / 30.0, 64 rows 33.7 /
+// 31.0; 5 passes, 28672 x 8192, 4 rows 160 / 116.  Where it has to drain its accumulators (fp32 results, very long k): 2 passes, 28672 x
+// 8192, 128 rows, fp32 113 / 128, 11008 x 4096 31 / 35, 8192 x 28672, 64 rows, fp16 75 / 84; more passes as above.
+// fp16 results of fewer rows, with the drains that the plane kernel's chain asks for (hl_chain).  Up to 2048 columns gemm_tc's 256-column
+// tiles and 8 k-ranges leave half of the SMs idle: 2048 x 8192, 9 rows, q = 2 12.4 / 8.4, q = 4 18.6 / 10.4; 2048 x 1024, q = 3, 9 rows 5.4 / 5.0.
+// Two planes + q_bias from 9 rows: 4096 x 12288, 9 rows 25.2 / 20.2; 8192 x 8192, 9 rows 32.7 / 26.5, 63 rows 38.3 / 29.8; 12288 x 4096, 9 rows
+// 23.7 / 23.0; 28672 x 1024, 24 rows 32.2 / 19.7; of 345 calls 4096 x 1024 alone was slower, 9 rows 5.7 / 6.2, 16 rows 6.3 / 6.5.  Two
+// passes from 64 rows, up to 4096 columns or 2048 k: 2560 x 8192, 80 rows 20.0 / 13.7; 4096 x 12288, 25.0 / 25.1; 8192 x 2048, 96 rows 0.94 of it;
+// beyond both 8192 x 8192, 80 rows 30.6 / 31.8, 12288 x 4096, 24.3 / 28.9; and with more column tiles than SMs from 1024 k on: 28672 x 512, 80 rows
+// 1.32 of it, 28672 x 1024 37.2 / 23.6.
 bool gemm_hl_ok(const lutgemm_weight* w, int m, bool f32) {
     const int passes = w->q + (w->q_bias ? 1 : 0);
-    const int T = (w->N + lg::kHlCols - 1) / lg::kHlCols, ranges = sm_count() / T < 1 ? 1 : sm_count() / T;
-    const bool drains = f32 || w->K / 8 > kHlChain16 * ranges;    // up to 128 rows: 8 accumulations per 64 k of a range
-    int from = passes >= 5 ? 4 : passes >= 3 || (passes == 2 && !drains) ? 64 : 129;
-    if (!drains && w->N <= 8 * lg::kTcTileN) from = 4;
-    else if (!drains && w->q == 2 && w->q_bias) from = 9;
+    int from = hl_many_rows(w, f32);
+    if (!f32) {
+        if (w->N <= 8 * lg::kTcTileN) from = 4;
+        else if (w->q == 2 && w->q_bias) from = 9;
+        else if (passes == 2 && from > 64 && (w->N <= 16 * lg::kTcTileN || w->K <= 2048) &&
+                 (w->K >= 1024 || (w->N + lg::kHlCols - 1) / lg::kHlCols <= sm_count())) from = 64;
+    }
     // with g = 32 every block builds two tables: up to 128 rows, where the expansion bounds it, that goes to gemm_tc
     return w->tc_ok && w->q <= 4 && m >= from && (m > 128 || w->g >= lg::kHlStepK);
 }
@@ -906,20 +923,21 @@ int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
     int rc = tc_split(w, ws, m < 128 ? m : 128, batch_rows_for(w, m), st, &unused_split, &unused_steps);
     if (rc != LUTGEMM_OK) return rc;
     const bool ordered = ordered_for(ws);
-    const int chain = hl_chain(w, ordered, y32 != nullptr);
+    const int chain = hl_chain(w, m, ordered, y32 != nullptr);
     const long long there = rows_there(w, ws);
     const int piece = there < batch_rows_for(w, m) ? (int)(there / 128 * 128) : m;
     if (!ordered && piece >= 128 && piece < m) {
         lg::HlParams p = {};
         double pieces = (m / piece) * hl_plan(w, piece, true, chain, &p);
-        if (m % piece) pieces += hl_plan(w, m % piece, true, chain, &p);
+        if (m % piece) pieces += hl_plan(w, m % piece, true, hl_chain(w, m % piece, ordered, y32 != nullptr), &p);
         if (pieces < 0.78 * hl_plan(w, m, false, chain, &p)) {
             for (int r0 = 0; r0 < m; r0 += piece) {
                 const int rows = m - r0 < piece ? m - r0 : piece;
                 const __half* xr = x + (size_t)r0 * w->K;
                 __half* y16r = y16 ? y16 + (size_t)r0 * w->N : nullptr;
                 float* y32r = y32 ? y32 + (size_t)r0 * w->N : nullptr;
-                rc = gemm_hl_ok(w, rows, y32 != nullptr) ? gemm_hl_launch(w, ws, xr, y16r, y32r, rows, true, chain, st) : gemm_tc_rows(w, ws, xr, y16r, y32r, rows, st);
+                rc = gemm_hl_ok(w, rows, y32 != nullptr) ? gemm_hl_launch(w, ws, xr, y16r, y32r, rows, true, hl_chain(w, rows, ordered, y32 != nullptr), st)
+                                                     : gemm_tc_rows(w, ws, xr, y16r, y32r, rows, st);
                 if (rc != LUTGEMM_OK) return rc;
             }
             return LUTGEMM_OK;

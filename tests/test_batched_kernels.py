@@ -96,6 +96,27 @@ def test_split_operand_kernel_few_rows(N, K, q, g, bias, m):
     w.close()
 
 
+@pytest.mark.parametrize("N,K,q,g,bias,m", [(28672, 1024, 2, 64, True, 16), (12288, 1024, 2, 128, False, 64), (4096, 1024, 1, 64, True, 80),
+                                            (11008, 4096, 2, 64, True, 40), (2048, 4096, 2, 128, False, 24)])
+def test_split_operand_kernel_few_rows_are_rounded_as_the_plane_kernels(N, K, q, g, bias, m):
+    """fp16 results of few rows come from sums as good as the plane kernel's: no more of them, beyond the spread of such a count,
+    lie on the wrong side of a rounding than of that kernel's sums, which matmul_f32 gives."""
+    bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + m, with_bias=bias)
+    x = synth.activations(m, K, seed=m)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g, q_bias).reserve_batch(m)
+    xd = torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
+    y16, y32 = (torch.empty((m, N), dtype=t, device="cuda") for t in (torch.float16, torch.float32))
+    L.matmul(y16, xd, w, m)
+    assert L.last_launch()[0] == "gemm_hl_kernel"
+    L.matmul_f32(y32, xd, w, m)
+    assert L.last_launch()[0] == "gemm_tc_kernel"
+    ref = oracle.bcq_matmul_f64(x, bW, alpha.astype(np.float16), None if q_bias is None else q_bias.astype(np.float16), g).astype(np.float16)
+    off, off_plane = (y16.cpu().numpy() != ref).sum(), (y32.cpu().numpy().astype(np.float16) != ref).sum()
+    assert off_plane > 50
+    assert off <= off_plane + 4 * np.sqrt(off_plane)
+    w.close()
+
+
 @pytest.mark.parametrize("q,bias,m", [(4, True, 40), (2, False, 150), (1, False, 200), (3, True, 256)])
 def test_split_operand_kernel_scales_far_apart(q, bias, m):
     _run("gemm_hl_kernel", 264, 1024, q, 128, bias, m, column_scales=True)
