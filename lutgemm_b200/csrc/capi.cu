@@ -1112,12 +1112,15 @@ int gemm_i8_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 // 8192, q = 4, 4 rows 72.7 / 113.2; g = 32 (four scales to a unit) 8 rows 106.7 / 112.3, but 8192 x 8192 with fewer planes
 // the other way, which is why it stays with gemm_tc.  Containers that the tcgen05 kernels refuse (N % 8 != 0, or a group size that
 // neither divides nor is a multiple of 128) take it for every batch, 16 rows at a time: what is left for them is one matvec per row.
+// fp32 results of two and three rows stay with the LUT kernels where those can run: their sums are rounded to nearest, this kernel's
+// are cut off and carry the offsets of its operands.  Against 64 bits, 8192 x 1024, q = 5 + q_bias, 3 rows: 6.3e-8 / 1.3e-7; 12288 x 2048,
+// q = 4, 7.4e-8 / 3.5e-7.  fp16 results are as far off with either (2.1e-4).
 constexpr long long kFragPairWeights = 64ll << 20;
-bool frag_wanted(const lutgemm_weight* w, const lutgemm_workspace* ws, int m) {
+bool frag_wanted(const lutgemm_weight* w, const lutgemm_workspace* ws, int m, bool f32) {
     if (m < 2 || w->N % 4 != 0 || ordered_for(ws) || gemm_i8_ok(w, m)) return false;
     if (m < kBatchedFromRows && g_variant.load() != 0) return false;       // the caller asked for a matvec kernel by name
-    if (m == 2) return w->g % 64 == 0 && gemv_pair_ok(w, ws) && (long long)w->N * w->K * w->q <= kFragPairWeights;
-    if (m == 3) return w->g % 64 == 0 || !gemv_pair_ok(w, ws);
+    if (m == 2) return !f32 && w->g % 64 == 0 && gemv_pair_ok(w, ws) && (long long)w->N * w->K * w->q <= kFragPairWeights;
+    if (m == 3) return (!f32 && w->g % 64 == 0) || !gemv_pair_ok(w, ws);
     return !w->tc_ok || (m <= 8 && w->g % 64 == 0);
 }
 
@@ -1183,7 +1186,7 @@ int matmul_impl(__half* y16, float* y32, const void* in, lutgemm_weight_t w, int
     cudaStream_t st = (cudaStream_t)stream;
     const __half* x = (const __half*)in;
     const int batched_mode = g_batched.load();
-    if (batched_mode != 0 && frag_wanted(w, ws, m)) {
+    if (batched_mode != 0 && frag_wanted(w, ws, m, y32 != nullptr)) {
         bool taken = false;
         const int rc = frag_rows_if_ready(w, ws, x, y16, y32, m, st, &taken);
         if (taken || rc != LUTGEMM_OK) return rc;

@@ -13,8 +13,8 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-def _run(kernel, N, K, q, g, bias, m, column_scales=False, ordered=False):
-    """Two calls against 64-bit sums; `kernel` is the one that has to have run them."""
+def _run(kernel, N, K, q, g, bias, m, column_scales=False, ordered=False, kernel32=None):
+    """Two calls against 64-bit sums; `kernel` is the one that has to have run them, `kernel32` where fp32 results take another."""
     bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + K + m, with_bias=bias)
     if column_scales:
         # columns whose scales lie far apart, down to fp16's subnormals and up to its largest values
@@ -31,7 +31,7 @@ def _run(kernel, N, K, q, g, bias, m, column_scales=False, ordered=False):
     first = None
     for _ in range(2):                                    # the second call finds the workspace as the first one left it
         L.matmul_f32(y32, xd, w, m)
-        assert L.last_launch()[0] == kernel
+        assert L.last_launch()[0] == (kernel32 or kernel)
         L.matmul(y16, xd, w, m)
         assert L.last_launch()[0] == kernel
         if ordered:
@@ -42,8 +42,9 @@ def _run(kernel, N, K, q, g, bias, m, column_scales=False, ordered=False):
     # Products are exact, sums are fp32: every addition errs by at most 2^-23 of the largest partial sum, which is at most
     # |x| |scale| summed; 11 times that with the register operand (up to 6, and its offset of up to 5, for a sign).  K / 16
     # additions per pass.  The split operand's weight is off by up to 2^-22 of it.
-    grow = 11 if kernel == "gemm_frag_kernel" else 1
-    unit = grow * (2 * K / 16 + 64) * 2.0 ** -23 + 2.0 ** -22
+    per_add = (2 * K / 16 + 64) * 2.0 ** -23
+    grow = {True: 11, False: 1}
+    unit = grow[(kernel32 or kernel) == "gemm_frag_kernel"] * per_add + 2.0 ** -22
     mag = np.abs(a16.astype(np.float64)).sum(1) + (0 if b16 is None else np.abs(b16.astype(np.float64)))       # [G, N]
     size = np.abs(x.astype(np.float64)).reshape(m, K // g, g).sum(2) @ mag
     bound = unit * size + 1e-30
@@ -55,7 +56,7 @@ def _run(kernel, N, K, q, g, bias, m, column_scales=False, ordered=False):
         assert (np.linalg.norm(err, axis=0) <= 1.5 * unit * np.linalg.norm(ref, axis=0)).all()
     # one rounding to fp16 on top: half a unit in the last place, at least half the subnormal step
     with np.errstate(over="ignore"):
-        lim = bound + np.maximum(np.abs(ref) * 2.0 ** -11, 2.0 ** -25)
+        lim = (grow[kernel == "gemm_frag_kernel"] * per_add + 2.0 ** -22) * size + 1e-30 + np.maximum(np.abs(ref) * 2.0 ** -11, 2.0 ** -25)
     got = y16.cpu().numpy().astype(np.float64)
     finite = np.abs(ref) + lim < 65504
     assert (np.abs(got - ref)[finite] <= lim[finite] * 1.0001).all()
@@ -205,12 +206,29 @@ def test_matvec_in_runs_wherever_shared_memory_begins(tmp_path):
     assert out.returncode == 0 and "flat ok" in out.stdout, out.stdout + out.stderr
 
 
-# two and three rows: the register operand up to 64 Mi weights of planes and where one slab of k is enough, else the LUT kernels
+# two and three rows: fp16 results by the register operand, two up to 64 Mi weights of planes and where one slab of k is enough, else
+# by the LUT kernels, as fp32 results are
 @pytest.mark.parametrize("N,K,q,g,bias,m,kernel", [
     (72, 128, 1, 64, True, 2, "gemm_frag_kernel"), (4096, 4096, 4, 128, False, 2, "gemm_frag_kernel"), (4104, 4096, 4, 128, False, 2, "gemv_tma2_kernel"),
-    (72, 8192, 1, 128, False, 2, "gemv_tma2_kernel"), (72, 192, 2, 32, True, 2, "gemv_tma2_kernel"), (72, 8192, 1, 128, True, 3, "gemm_frag_kernel")])
+    (72, 8192, 1, 128, False, 2, "gemv_tma2_kernel"), (72, 192, 2, 32, True, 2, "gemv_tma2_kernel"), (72, 8192, 1, 128, True, 3, "gemm_frag_kernel"),
+    (72, 192, 2, 32, True, 3, "gemv_tma_kernel")])
 def test_two_and_three_rows(N, K, q, g, bias, m, kernel):
-    _run(kernel, N, K, q, g, bias, m)
+    _run(kernel, N, K, q, g, bias, m, kernel32="gemv_tma2_kernel" if m == 2 else "gemv_tma_kernel")
+
+
+@pytest.mark.parametrize("N,K,q,bias,m", [(4096, 2048, 4, True, 2), (12288, 2048, 4, False, 3)])
+def test_fp32_results_of_two_and_three_rows(N, K, q, bias, m):
+    """Sums rounded to nearest.  Table entries, of eight fp16 activations, are all but exact; from there a result goes through 7 + q
+    additions of a slab and K / 512 slabs, each off by up to half a unit, 2^-24 of a partial sum no larger than the whole, either
+    way: 2^-24 / sqrt(3) in the 2-norm, and the root of their number for all."""
+    bW, alpha, q_bias = synth.bcq_layer(N, K, q, 128, seed=N + m, with_bias=bias)
+    x = synth.activations(m, K, seed=m)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // 128, q_bias).reserve_batch(m)
+    y = torch.empty((m, N), dtype=torch.float32, device="cuda")
+    L.matmul_f32(y, torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16), w, m)
+    ref = oracle.bcq_matmul_f64(x, bW, alpha.astype(np.float16), None if q_bias is None else q_bias.astype(np.float16), 128)
+    assert np.linalg.norm(y.cpu().numpy() - ref) <= np.sqrt((7 + q + K / 512) / 3) * 2.0 ** -24 * np.linalg.norm(ref)
+    w.close()
 
 
 @pytest.mark.parametrize("q,g,bias,m", [(4, 128, True, 8), (3, 64, False, 4), (2, 32, True, 5)])
