@@ -392,14 +392,15 @@ int lutgemm_set_gemv_variant(int variant);
  * Switch only while no matmul is in flight; a workspace may be used in either mode from call to call.  (The reference's half2 atomicAdd accumulation,
  * lutGEMM/src/cuda/kernels/mv_fp16.hpp:95, has no ordered mode.) */
 int lutgemm_set_ordered_reduction(int enabled);
-/* 1 (default): rows that go through the LUT matvec (m = 2, 3; any m with lutgemm_set_batched_path(0)) are taken
+/* 1 (default): rows that go through the LUT matvec (some of m = 2, 3, see below; any m with lutgemm_set_batched_path(0)) are taken
  * two at a time by a two-table kernel that reads the weights once for both; 0: one row per launch.  The pair
  * kernel is used only with the default reductions (not in ordered mode) and the default matvec variant. */
 int lutgemm_set_row_pairs(int enabled);
 /* 1 (default): m >= 4 runs a tensor-core kernel (mma.sync with the weights in registers up to 8 rows; beyond, tcgen05 plane
  * by plane, 128 rows per launch, or with the planes folded into one split operand, whichever is faster for the row and
  * plane count), batches (m >= 3) on containers that the tcgen05 kernels do not take the mma.sync kernel where scratch is
- * reserved for them, smaller ones the LUT matvec; 0: always one LUT matvec per row; 2: tensor-core kernel from m = 2.  All
+ * reserved for them, fp16 results of m = 3, and of m = 2 on smaller weights, with groups of a multiple of 64 the mma.sync
+ * kernel without any scratch to reserve, smaller batches otherwise and fp32 results of m = 2 and 3 the LUT matvec; 0: always one LUT matvec per row; 2: tensor-core kernel from m = 2.  All
  * compute the same function. */
 int lutgemm_set_batched_path(int mode);
 /* 0 (default): every batch on the tensor-core path takes the fp16 kernel (operand = +-alpha in fp16, exact products).

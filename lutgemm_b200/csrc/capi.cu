@@ -38,7 +38,7 @@ struct lutgemm_retired_block {
 // default; lutgemm_workspace_create makes more, so that several streams can use one container at a time.
 struct lutgemm_workspace {
     float* partial = nullptr;    // partial sums [slabs][n_cap] fp32 (ordered mode) / row 0 = zeroed L2 reduction row
-    float* partial2 = nullptr;   // second zeroed reduction row [n_cap] of the two-row matvec
+    float* few = nullptr;        // zeroed reduction rows [kFewRows][n_cap]: the first is the second of the two-row matvec
     unsigned* counters = nullptr;   // per-tile arrival counters, zero between launches
     int* status = nullptr;       // device word set by a kernel whose bounded wait ran out
     float* tc_partial = nullptr; // fp32 split-k rows of the batched (tensor-core) path, [tc_rows][n_cap], kept zeroed
@@ -136,6 +136,7 @@ inline void note_launch(const char* kernel, dim3 grid) {
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 constexpr int kBatchedFromRows = 4;      // m >= 4 goes to the tensor-core kernel
+constexpr int kFewRows = 3;              // batches below that find reduction rows in every workspace
 
 #define LG_CUDA(call)                                  \
     do {                                               \
@@ -247,7 +248,7 @@ void make_tensor_maps(lutgemm_weight* w, bool with_batched = true) {
 
 void free_workspace_buffers(lutgemm_workspace* ws) {
     if (ws->partial) cudaFree(ws->partial);
-    if (ws->partial2) cudaFree(ws->partial2);
+    if (ws->few) cudaFree(ws->few);
     if (ws->counters) cudaFree(ws->counters);
     if (ws->status) cudaFree(ws->status);
     if (ws->tc_partial) cudaFree(ws->tc_partial);
@@ -259,7 +260,7 @@ void free_workspace_buffers(lutgemm_workspace* ws) {
             cudaFree(r->ptr);
             delete r;
         }
-    ws->partial = ws->partial2 = ws->tc_partial = nullptr;
+    ws->partial = ws->few = ws->tc_partial = nullptr;
     ws->counters = nullptr;
     ws->status = nullptr;
     ws->t_in = ws->t_out = nullptr;
@@ -329,8 +330,8 @@ int fill_workspace(lutgemm_workspace* ws, int N, int K, int batch_rows) {
     ws->n_cap = N; ws->slabs = (int)nslabs;
     LG_CUDA(cudaMalloc(&ws->partial, nslabs * (size_t)N * sizeof(float)));
     LG_CUDA(cudaMemset(ws->partial, 0, nslabs * (size_t)N * sizeof(float)));   // row 0 doubles as the reduction row
-    LG_CUDA(cudaMalloc(&ws->partial2, (size_t)N * sizeof(float)));
-    LG_CUDA(cudaMemset(ws->partial2, 0, (size_t)N * sizeof(float)));
+    LG_CUDA(cudaMalloc(&ws->few, kFewRows * (size_t)N * sizeof(float)));
+    LG_CUDA(cudaMemset(ws->few, 0, kFewRows * (size_t)N * sizeof(float)));
     LG_CUDA(cudaMalloc(&ws->counters, kMaxCounters * sizeof(unsigned)));
     LG_CUDA(cudaMemset(ws->counters, 0, kMaxCounters * sizeof(unsigned)));
     LG_CUDA(cudaMalloc(&ws->status, sizeof(int)));
@@ -554,14 +555,14 @@ int gemv_pair(const lutgemm_weight* w, const lutgemm_workspace* ws, const __half
     p.x1 = x + w->K;
     p.y16_1 = y16 ? y16 + w->N : nullptr;
     p.y32_1 = y32 ? y32 + w->N : nullptr;
-    p.partial1 = ws->partial2;
+    p.partial1 = ws->few;
     dim3 grid(tiles, b.nslabs);
     const bool bias = w->q_bias != nullptr;
     if (w->g % 128 == 0) return launch_gemv_tma2<2>(w, p, grid, bias, st);
     return launch_gemv_tma2<1>(w, p, grid, bias, st);
 }
 bool gemv_pair_ok(const lutgemm_weight* w, const lutgemm_workspace* ws) {
-    return g_variant.load() == 0 && w->tma_ok && ws->partial2 && !ordered_for(ws) && g_pairs.load() &&
+    return g_variant.load() == 0 && w->tma_ok && ws->few && !ordered_for(ws) && g_pairs.load() &&
            lg::gemv22_num_stages(w->a_rows) >= 2;
 }
 
@@ -1021,10 +1022,10 @@ int launch_gemm_frag_q(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid
     }
 }
 
-int gemm_frag_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, lg::FrParams p, dim3 grid, const __half* x, __half* y16,
-                   float* y32, int m, cudaStream_t st) {
+int gemm_frag_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, float* partial, lg::FrParams p, dim3 grid, const __half* x,
+                   __half* y16, float* y32, int m, cudaStream_t st) {
     p.bW = w->bW; p.alpha = w->alpha; p.q_bias = w->q_bias; p.x = x;
-    p.partial = ws->tc_partial; p.counters = ws->counters;
+    p.partial = partial; p.counters = ws->counters;
     p.y16 = y16; p.y32 = y32;
     p.N = w->N; p.K = w->K; p.q = w->q; p.g = w->g; p.m = m;
     p.ones = 0x3c003c00u; p.twos = 0x40004000u; p.fours = 0x44004400u;
@@ -1140,11 +1141,14 @@ int frag_rows_if_ready(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x
         const int rc = tc_split(w, ws, m < 128 ? m : 128, m, st, &unused_split, &unused_steps);
         if (rc != LUTGEMM_OK) return rc;
     }
-    if (((whole && grid[0].y > 1) || (rest && grid[1].y > 1)) && rows_there(w, ws) < (whole ? lg::kFrMaxRows : m)) return LUTGEMM_OK;
+    // Three rows in place of the LUT kernels reduce into rows that every workspace has: the same kernel whatever was reserved or
+    // called before, and nothing allocated.  Where the LUT kernels take a row at a time it needs scratch as more rows do.
+    const bool few = m == kFewRows && gemv_pair_ok(w, ws);
+    if (!few && ((whole && grid[0].y > 1) || (rest && grid[1].y > 1)) && rows_there(w, ws) < (whole ? lg::kFrMaxRows : m)) return LUTGEMM_OK;
     *taken = true;
     for (int r0 = 0; r0 < m; r0 += lg::kFrMaxRows) {
         const int rows = m - r0 < lg::kFrMaxRows ? m - r0 : lg::kFrMaxRows, i = rows == lg::kFrMaxRows ? 0 : 1;
-        const int rc = gemm_frag_rows(w, ws, p[i], grid[i], x + (size_t)r0 * w->K, y16 ? y16 + (size_t)r0 * w->N : nullptr,
+        const int rc = gemm_frag_rows(w, ws, few ? ws->few : ws->tc_partial, p[i], grid[i], x + (size_t)r0 * w->K, y16 ? y16 + (size_t)r0 * w->N : nullptr,
                                       y32 ? y32 + (size_t)r0 * w->N : nullptr, rows, st);
         if (rc != LUTGEMM_OK) return rc;
     }
@@ -1191,9 +1195,9 @@ int matmul_impl(__half* y16, float* y32, const void* in, lutgemm_weight_t w, int
         const int rc = frag_rows_if_ready(w, ws, x, y16, y32, m, st, &taken);
         if (taken || rc != LUTGEMM_OK) return rc;
     }
-    // Up to three rows one LUT matvec per row is cheaper than the tensor-core kernel, whose cost is nearly
-    // independent of m up to 64 rows (measured: 8192^2, q = 2: m x 10.2 us against 29 us; 12288^2, q = 3:
-    // m x 17.6 us against 64 us).
+    // One row, and two or three that the register-operand kernel did not take (frag_wanted): one or two to a LUT matvec are cheaper
+    // than a tcgen05 kernel, whose cost is nearly independent of m up to 64 rows (measured: 8192^2, q = 2: 10.2 us a row, 22 us;
+    // 12288^2, q = 3: 17.0 us a row, 64 us).
     if (m == 1 || batched_mode == 0 || (batched_mode == 1 && m < kBatchedFromRows) || !w->tc_ok) {
         const bool pairs = gemv_pair_ok(w, ws);
         for (int r = 0; r < m;) {

@@ -263,6 +263,50 @@ def test_three_rows_without_reserved_scratch_inside_a_capture():
     w.close()
 
 
+def test_three_rows_take_the_same_kernel_whatever_was_called_before():
+    """Several k-ranges reduce into rows that the container has from the start: a first call, one in a capture, calls after a larger
+    batch and in an explicit workspace run the same launch."""
+    N, K, q, g = 264, 8192, 2, 128
+    bW, alpha, _ = synth.bcq_layer(N, K, q, g, seed=8)
+    x = synth.activations(8, K, seed=9)
+    xd = torch.from_numpy(x.view(np.int16)).cuda().view(torch.float16)
+    ref = oracle.bcq_matmul_f64(x, bW, alpha.astype(np.float16), None, g)
+    w, captured = (L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g) for _ in range(2))
+    seen = []
+
+    def three(w, **workspace):
+        y = torch.empty((3, N), dtype=torch.float16, device="cuda")
+        L.matmul(y, xd, w, 3, **workspace)
+        seen.append(L.last_launch())
+        return y
+
+    def right(y, rows=3):
+        assert np.linalg.norm(y.cpu().numpy() - ref[:rows]) <= 8e-4 * np.linalg.norm(ref[:rows])
+
+    right(three(w))
+    assert w.scratch() == (0, 0, 0) and seen[0][0] == "gemm_frag_kernel" and seen[0][2] > 1
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        y = three(captured)
+    graph.replay()
+    torch.cuda.synchronize()
+    right(y)
+    for m, dtype, f in ((8, torch.float16, L.matmul), (2, torch.float32, L.matmul_f32)):
+        y = torch.empty((m, N), dtype=dtype, device="cuda")
+        f(y, xd, w, m)
+        right(y, m)
+        right(three(w))
+    ws = L.Workspace(2 * N, K)
+    right(three(w, workspace=ws))
+    right(three(w, workspace=ws))
+    assert len(set(seen)) == 1, seen
+    ws.close()
+    del graph
+    w.close()
+    captured.close()
+
+
 def _far_apart_in_a_column(N, K, q, g, bias, m):
     """Scales whose exponents differ from group to group of one column from one end of fp16 to the other; activations are zero
     wherever some column's scales are large, so that what the outputs consist of are the products with the small ones."""
