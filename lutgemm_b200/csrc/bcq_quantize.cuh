@@ -241,7 +241,7 @@ bcq_quantize_kernel(const BqParams p) {
 // pairs to a word.  A weight then costs its q comparisons, one table read, q multiply-adds (B^T w) and one integer add
 // (B^T B) per word of pairs, and the sums of the next round are complete when the weights of this one are placed.
 // Bound by instruction issue, not by memory: the weights are read once.  Measured, N = K = 4096, q = 3, g = 128, 15
-// rounds: 406 us; bcq_quantize_kernel, which gives every group a whole warp, takes 3291 us.  Layers of 4 Mi weights or more take
+// rounds: 406 us; bcq_quantize_kernel, which gives every group a whole warp, takes 3291 us.  Large layers of two to four planes take
 // bcq_quantize_lane_kernel (below) instead.
 // Sums are added in the order of bcq_quantize_kernel, whose lane L holds weights L, L + 32, ...: a lane here stands for
 // NJ = 32 / LG of those lanes (lane, lane + LG, ...), keeps their partial sums apart and adds them first, which is that

@@ -1314,11 +1314,21 @@ void launch_bcq_tile(const lg::BqParams& p, long long groups, cudaStream_t st) {
     else lg::bcq_quantize_tile_kernel<32, Q><<<ctas, block, 0, st>>>(p);
 }
 
-// Whether the kernel with a group to a lane is the faster one: a warp of it takes some 60 us whatever the layer is, more with wider
+// Whether the kernel with a group to a lane is the faster one.  A warp of it takes some 60 us whatever the layer is, more with wider
 // groups, of which fewer fit an SM; the tiled kernel 14 to 50 us per million weights.  Measured, us, this / tiled, 15 rounds: 1024 x
 // 1024, q = 3, g = 128, 62 / 38; 2048 x 2048, q = 3, 88 / 110, q = 2, g = 64, 57 / 77, q = 2, g = 256, 75 / 69; 1024 x 8192, q = 3, g = 256, 157 /
 // 216; 2048 x 4096, q = 3, g = 512, 287 / 238; 4096 x 4096, g = 512, 421 / 462.
-bool bq_lane_better(long long groups, int g) { return groups * g >= (4ll << 20) * (g > 256 ? 4 : g > 128 ? 2 : 1); }
+// Reading and greedy start cost it more where groups are narrow, or wide and the layer large, and its rounds have to win that back:
+// fewest rounds per plane count, group and size, the measured ratio to the tiled kernel at them and below.  q = 2, g = 64, 16 Mi weights
+// 0.96 (3 rounds) 1.07 (2), 32 Mi 0.95 (8) 1.09 (5); g = 384, 32 Mi 0.96 (8) 1.09 (5); q = 3, g = 64, 16 Mi 1.01 (2) 1.07 (1), 32 Mi
+// 0.97 (5) 1.05 (3); g = 192, 32 Mi 0.89 (3) 1.06 (1).  Four planes of groups of 512 are the other way round: 0.86 (3) 1.03 (5) 1.41 (15).
+bool bq_lane_better(long long groups, int g, int q, int rounds) {
+    if (groups * g < (4ll << 20) * (g > 256 ? 4 : g > 128 ? 2 : 1)) return false;
+    const bool narrow = g <= 64, wide = g > 128 && g <= 384, large = groups * g > 24ll << 20;
+    if (q == 2) return rounds >= (narrow ? (large ? 8 : 3) : wide && large ? 8 : 1);
+    if (q == 3) return rounds >= (narrow ? (large ? 5 : 2) : wide && g <= 256 && large ? 2 : 1);
+    return g <= 384 || rounds <= 4;
+}
 
 template <int Q>
 int launch_bcq_lane(const lg::BqParams& p, long long groups, cudaStream_t st) {
@@ -2275,9 +2285,9 @@ int lutgemm_bcq_quantize_device(const float* d_w, int N, int K, int q, int group
     const long long ctas = (groups + lg::kBqWarps - 1) / lg::kBqWarps;
     if (ctas > 0x7fffffffLL) return LUTGEMM_ERR_TOO_LARGE;
     cudaStream_t st = (cudaStream_t)stream;
-    // Up to four planes and 512 weights to a group: a group to a lane, or, for small layers, one plane or no refinement, several to a
+    // Up to four planes and 512 weights to a group: a group to a lane, or, for small layers, one plane or little refinement, several to a
     // warp (406 us at 4096 x 4096, q = 3, g = 128, where a group to a warp takes 3292); the rest take a warp or a CTA per group.
-    if (q >= 2 && q <= lg::kBqTileMaxQ && g <= lg::kBqLaneMaxG && rounds >= 1 && bq_lane_better(groups, g)) {
+    if (q >= 2 && q <= lg::kBqTileMaxQ && g <= lg::kBqLaneMaxG && rounds >= 1 && bq_lane_better(groups, g, q, rounds)) {
         const int rc = q == 2 ? launch_bcq_lane<2>(p, groups, st) : q == 3 ? launch_bcq_lane<3>(p, groups, st) : launch_bcq_lane<4>(p, groups, st);
         if (rc != LUTGEMM_OK) return rc;
     }
