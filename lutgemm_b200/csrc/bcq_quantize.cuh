@@ -554,7 +554,8 @@ bcq_quantize_tile_kernel(const BqParams p) {
 // warp once for 32 groups instead of once for 32 / LG.  The weights lie in shared memory, four of a group to 16 bytes, at
 // places that reading (a lane per group) and filling (a row of the matrix at a time) both find without bank conflicts.
 // `w < mid goes left` is strict on both sides: a negative weight leaves the inner level only if |w| > midpoint.  Those compare with
-// the float below |w|: w plus the smallest float, cut off toward zero, which leaves the others as they are.
+// the float below |w|: w plus the smallest float, cut off toward zero, which leaves the others as they are from 2^-125 on; a group with a
+// midpoint no larger than that compares everything times 2^60.
 // Sums are added in the order of the other kernels: per residue of 32 the weights in turn, then residues 16, 8, 4, 2 and 1 apart.  So
 // all give the same bits.
 //
@@ -571,8 +572,8 @@ __host__ __device__ constexpr int bq_lane_warps(int g) {
     return 232448 / bq_lane_warp_bytes(g) < kBqLaneWarps ? 232448 / bq_lane_warp_bytes(g) : kBqLaneWarps;
 }
 
-// What a weight is compared with: |w|, or for a negative one the float below (the sum with the smallest float, cut off toward zero).
-__device__ __forceinline__ float bq_key(float w) { return fabsf(__fadd_rz(w, 1.401298464324817e-45f)); }
+// What a weight is compared with: |w|, or for a negative one the float below (the sum with the smallest float, cut off toward zero); times unit.
+__device__ __forceinline__ float bq_key(float w, float unit) { return fabsf(__fmaf_rz(w, unit, 1.401298464324817e-45f)); }
 // 1 where key >= mid, else 0
 __device__ __forceinline__ float bq_from(float key, float mid) {
     float f;
@@ -734,7 +735,8 @@ bcq_quantize_lane_kernel(const BqParams p) {
     }
 
     // ---- alternating refinement ----
-    float mid[NH];                                         // [1 ..]: between the upper half's levels
+    float mid[NH];                                         // [1 ..]: between the upper half's levels, times unit
+    float unit;                                            // 1, or 2^60 where a midpoint is so low that bq_key would move positive weights
     uint32_t code[NH];                                     // bit Q - 1 - i set: plane i is -1 in this level
     const float pad = (float)(words * 32 - g);
 #pragma unroll 1
@@ -760,6 +762,11 @@ bcq_quantize_lane_kernel(const BqParams p) {
                 }
 #pragma unroll
         for (int c = 1; c < NH; c++) mid[c] = (v[c - 1] + v[c]) / 2.f;
+        unit = 1.f;
+#pragma unroll
+        for (int c = 1; c < NH; c++) unit = mid[c] > 0.f && mid[c] <= 2.350988701644575e-38f ? 1.152921504606846976e18f : unit;
+#pragma unroll
+        for (int c = 1; c < NH; c++) mid[c] *= unit;
         if (round + 1 == p.rounds) break;
         // a plane's sign: in the lowest level, and the steps at the midpoints
         float step[Q][NH];
@@ -809,7 +816,7 @@ bcq_quantize_lane_kernel(const BqParams p) {
             float t[Q - FROM];
             sums(t, [&](float w, float (&part)[Q - FROM]) {
                 float sg[Q];
-                signs(bq_key(w), sg);
+                signs(bq_key(w, unit), sg);
 #pragma unroll
                 for (int i = 0; i < Q; i++) {
                     if (i >= FROM) part[i >= FROM ? i - FROM : 0] = fmaf(sg[i], fabsf(w), part[i >= FROM ? i - FROM : 0]);
@@ -822,7 +829,7 @@ bcq_quantize_lane_kernel(const BqParams p) {
             for (int i = FROM; i < Q; i++) btw[i] = t[i - FROM];
             if (pad != 0.f) {                              // the zeros behind the group's end were counted
                 float sg[Q];
-                signs(bq_key(0.f), sg);
+                signs(bq_key(0.f, unit), sg);
 #pragma unroll
                 for (int i = 0; i < Q; i++)
 #pragma unroll
@@ -859,7 +866,7 @@ bcq_quantize_lane_kernel(const BqParams p) {
     for (int kw = 0; kw < words; kw++) {
         uint32_t from[NH] = {}, neg = 0u;                  // [1 ..]: from mid on
         auto mark = [&](float w, int e) {
-            const float key = bq_key(w);
+            const float key = bq_key(w, unit);
             neg |= w < 0.f ? 1u << e : 0u;
 #pragma unroll
             for (int c = 1; c < NH; c++) from[c] |= key >= mid[c] ? 1u << e : 0u;

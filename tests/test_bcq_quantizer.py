@@ -121,6 +121,39 @@ def test_device_quantiser_group_per_lane(N, K, g, q, rounds, zeros):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("g,q,rounds", [(64, 2, 4), (128, 3, 3), (96, 4, 3)])
+def test_device_quantiser_group_per_lane_of_the_smallest_weights(g, q, rounds):
+    """Weights of a few times the smallest float, where the float below a weight is no rounding of a sum: large layers, a group to
+    a lane, and small ones, several to a warp, get the same bits."""
+    import lutgemm_b200 as L
+    rng = np.random.default_rng(g + q)
+    w = (rng.integers(-40, 41, (33, 4 * g)) * 2.0 ** -149).astype(np.float32)
+    times = (4 << 20) // w.size + 1
+    _, B, alpha = L.bcq_quantize(np.tile(w, (times, 1)), q, rounds, g)
+    _, B_small, alpha_small = L.bcq_quantize(w, q, rounds, g)
+    B, alpha = B.reshape((times,) + B_small.shape), alpha.reshape((times,) + alpha_small.shape)
+    assert (alpha_small > 0).any()
+    assert (alpha == alpha_small).all() and (B == B_small).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("g,q,rounds", [(64, 2, 4), (128, 3, 3), (96, 4, 3)])
+def test_device_quantiser_group_per_lane_weights_not_finite(g, q, rounds):
+    """A group with an infinite or NaN weight has no scales (NaN), and its neighbours keep their bits."""
+    import lutgemm_b200 as L
+    rng = np.random.default_rng(g + q)
+    w = rng.normal(0, 0.02, ((4 << 20) // (4 * g) + 1, 4 * g)).astype(np.float32)
+    _, B, alpha = L.bcq_quantize(w, q, rounds, g)
+    bad = np.zeros(alpha.shape[:2], dtype=bool)
+    for i, value in enumerate((np.inf, -np.inf, np.nan)):
+        w[5 + 40 * i, g + 3] = value
+        bad[5 + 40 * i, 1] = True
+    _, B_bad, alpha_bad = L.bcq_quantize(w, q, rounds, g)
+    assert np.isnan(alpha_bad[bad]).all()
+    assert (alpha_bad[~bad] == alpha[~bad]).all() and (B_bad[~bad] == B[~bad]).all()
+
+
+@pytest.mark.gpu
 def test_device_quantiser_feeds_the_matmul():
     """Quantise on the device straight into the container layout, multiply, compare with x W_hat^T from the oracle."""
     import torch
