@@ -951,7 +951,9 @@ int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 // One CTA per SM and one wave: the slabs of k first (a slab is what the warps of a CTA hold activations for), then as many
 // column ranges as still fit.  Cost in units of 4096 weights per warp: half the longest warp's share and half the average one
 // (the SM's pipes are shared: 28672 x 8192, q = 4 + q_bias, 4 rows, where the longest share is the same, 2 / 4 / 8 slabs with 416 /
-// 400 / 400 units to the CTA 68.3 / 65.3 / 64.7 us), plus what a column tile's sum and a slab's start cost.
+// 400 / 400 units to the CTA 68.3 / 65.3 / 64.7 us), plus what a column tile's sum and a slab's start cost, and the slabs' reductions in
+// L2 at 2.5 MB a unit.  Without those many slabs won by a hair where there is little else to do: 12292 x 4096, q = 1, 16 rows, 2 / 16 slabs
+// 18.0 / 21.2 us, 4100 x 4096, q = 4 + q_bias 15.2 / 16.1; at 1.1 MB a unit too few did: 49152 x 11008, q = 3, 4 rows, 3 / 11 slabs 126 / 119.
 bool frag_plan(const lutgemm_weight* w, int m, lg::FrParams* p, dim3* grid) {
     if (w->N % 4 != 0 || m > lg::kFrMaxRows) return false;
     // the kernel's byte offsets and its division by g / 32 are 32 bits wide
@@ -972,7 +974,7 @@ bool frag_plan(const lutgemm_weight* w, int m, lg::FrParams* p, dim3* grid) {
         const int cw = lg::kFrWarps / kw, rounds = (tpc + cw - 1) / cw, wsteps = (sps + kw - 1) / kw;
         const double waves = (double)(((long long)slabs * ranges + sms - 1) / sms);
         const double longest = rounds * (wsteps * P + 1.0), average = (double)tpc * sps * (P + 1.0) / lg::kFrWarps;
-        const double t = waves * (12.0 + 0.5 * (longest + average)) + (slabs > 1 ? 8.0 : 0.0);
+        const double t = waves * (12.0 + 0.5 * (longest + average)) + (slabs > 1 ? 8.0 + (double)slabs * w->N * m * 4.0 / 2.5e6 : 0.0);
         if (t < best) {
             best = t;
             p->kw = kw; p->steps_per_slab = sps; p->tiles_per_cta = tpc;

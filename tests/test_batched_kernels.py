@@ -231,6 +231,21 @@ def test_fp32_results_of_two_and_three_rows(N, K, q, bias, m):
     w.close()
 
 
+# k-ranges cost reductions: no more of them where the longest share stays what it is
+@pytest.mark.parametrize("N,K,q,g,bias,m,ranges", [(4100, 4096, 2, 64, True, 16, 2), (12292, 4096, 1, 128, False, 16, 2), (12288, 8192, 3, 64, False, 4, 2)])
+def test_register_operand_kernel_k_ranges(N, K, q, g, bias, m, ranges):
+    bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + m, with_bias=bias)
+    w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g, q_bias).reserve_batch(m)
+    x, y = torch.zeros((m, K), dtype=torch.float16, device="cuda"), torch.empty((m, N), dtype=torch.float16, device="cuda")
+    L.matmul(y, x, w, m)
+    name, _, gy = L.last_launch()
+    assert name == "gemm_frag_kernel"
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert gy == ranges
+    assert not y.any()
+    w.close()
+
+
 @pytest.mark.parametrize("q,g,bias,m", [(4, 128, True, 8), (3, 64, False, 4), (2, 32, True, 5)])
 def test_register_operand_kernel_scales_far_apart(q, g, bias, m):
     _run("gemm_frag_kernel", 260, 1024, q, g, bias, m, column_scales=True)
