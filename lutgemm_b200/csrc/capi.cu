@@ -1011,15 +1011,15 @@ int launch_gemm_frag(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, 
     return LUTGEMM_OK;
 }
 
-// Up to four planes of groups of 64 or more have a kernel each, their loops unrolled: 2048 x 2048, q = 4, 4 rows 5.2 us, 5.7 with
-// the kernel for any number of planes; 28672 x 8192, 64.9 and 67.2.
+// Up to four planes have a kernel each, their loops unrolled: 2048 x 2048, q = 4, 4 rows 5.2 us, 5.7 with the kernel for any number of
+// planes; 28672 x 8192, 64.9 and 67.2; 4100 x 4096, q = 1, g = 32, 8 rows 6.3 and 7.6.
 template <int GW>
 int launch_gemm_frag_q(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, cudaStream_t st) {
-    switch (GW == 1 ? 0 : w->q) {
-        case 1: return launch_gemm_frag<1, GW, GW == 1 ? 0 : 1>(w, p, grid, st);
-        case 2: return launch_gemm_frag<1, GW, GW == 1 ? 0 : 2>(w, p, grid, st);
-        case 3: return launch_gemm_frag<1, GW, GW == 1 ? 0 : 3>(w, p, grid, st);
-        case 4: return launch_gemm_frag<1, GW, GW == 1 ? 0 : 4>(w, p, grid, st);
+    switch (w->q) {
+        case 1: return launch_gemm_frag<1, GW, 1>(w, p, grid, st);
+        case 2: return launch_gemm_frag<1, GW, 2>(w, p, grid, st);
+        case 3: return launch_gemm_frag<1, GW, 3>(w, p, grid, st);
+        case 4: return launch_gemm_frag<1, GW, 4>(w, p, grid, st);
         default: return launch_gemm_frag<1, GW, 0>(w, p, grid, st);
     }
 }

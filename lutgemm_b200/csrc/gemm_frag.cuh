@@ -259,13 +259,14 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
         const int end = fcol < fcol_end ? words : 0;
         const uint32_t size = kw0 + f_kw < end ? 16u : 0u, asize = akw < end ? 8u : 0u, at = fslot * ub;
         const uint32_t off = (uint32_t)(kw0 + f_kw) * row_b + (uint32_t)fcol * 4u;
-#pragma unroll
-        for (int b = 0; b < (Q ? Q : 8); b++)
-            if (Q || b < q) cp_async16(f_dst + at + b * 512, reinterpret_cast<const unsigned char*>(p.bW) + (off + b * ((uint32_t)N * 4u)), size);
+        const int pu = Q ? Q : GW == 1 ? q : 8;      // GW = 1 copies scales as often as words: planes that are not there cost too much
+#pragma unroll (Q ? Q : GW == 1 ? 4 : 8)
+        for (int b = 0; b < pu; b++)
+            if (Q || GW == 1 || b < q) cp_async16(f_dst + at + b * 512, reinterpret_cast<const unsigned char*>(p.bW) + (off + b * ((uint32_t)N * 4u)), size);
         const uint32_t grp = GW == 1 && !p.group_magic ? (unsigned)akw : __umulhi((unsigned)akw, p.group_magic);
         const uint32_t aoff = ((grp * q + f_plane) * (uint32_t)N + fcol) * 2u;
-#pragma unroll
-        for (int b = 0; b < (Q ? Q : 8); b += PB)
+#pragma unroll (Q ? Q : GW == 1 ? 2 : 8)
+        for (int b = 0; b < pu; b += PB)
             if (b + f_plane < q) cp_async8(f_adst + at + b * (NG * 64), reinterpret_cast<const unsigned char*>(p.alpha) + (aoff + b * ((uint32_t)N * 2u)), asize);
         if (BIAS && f_plane == 0) cp_async8(f_adst + at + q * (NG * 64), reinterpret_cast<const unsigned char*>(p.q_bias) + (grp * (uint32_t)N + fcol) * 2u, asize);
         if (++fslot == p.depth) fslot = 0;
