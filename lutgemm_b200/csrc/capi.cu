@@ -956,8 +956,6 @@ int gemm_hl_rows(lutgemm_weight* w, lutgemm_workspace* ws, const __half* x, __ha
 // 18.0 / 21.2 us, 4100 x 4096, q = 4 + q_bias 15.2 / 16.1; at 1.1 MB a unit too few did: 49152 x 11008, q = 3, 4 rows, 3 / 11 slabs 126 / 119.
 bool frag_plan(const lutgemm_weight* w, int m, lg::FrParams* p, dim3* grid) {
     if (w->N % 4 != 0 || m > lg::kFrMaxRows) return false;
-    // the kernel's byte offsets and its division by g / 32 are 32 bits wide
-    if ((long long)(w->K / 32) * w->q * w->N * 4 >= 1ll << 32 || (long long)(w->K / 32 + 64) * (w->g / 32) >= 1ll << 32) return false;
     const int gw = w->g % 128 == 0 ? 4 : w->g % 64 == 0 ? 2 : 1;
     p->depth = lg::fr_depth(gw, m <= 8 ? 1 : 2, w->q, w->q_bias != nullptr);
     if (p->depth < 2) return false;
@@ -981,14 +979,21 @@ bool frag_plan(const lutgemm_weight* w, int m, lg::FrParams* p, dim3* grid) {
             *grid = dim3(ranges, slabs);
         }
     }
-    return grid->y <= 65535;
+    // the kernel's byte offsets within a slab are 32 bits wide
+    const long long words = w->K / 32, slab_words = 4ll * p->steps_per_slab;
+    return grid->y <= 65535 && (words < slab_words ? words : slab_words) * w->q * w->N * 4 < 1ll << 32;
 }
 
-template <int MT, int GW, int Q>
+// Whether byte offsets from the tensors' bases, or the division by g / 32 without a shift, take more than 32 bits.
+bool frag_wide(const lutgemm_weight* w) {
+    return (long long)(w->K / 32) * w->q * w->N * 4 >= 1ll << 32 || (long long)(w->K / 32 + 64) * (w->g / 32) >= 1ll << 32;
+}
+
+template <int MT, int GW, int Q, bool WIDE = false>
 int launch_gemm_frag(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, cudaStream_t st) {
     static bool configured[64][2] = {};   // the attribute is per device
     const bool bias = w->q_bias != nullptr;
-    auto kern = bias ? lg::gemm_frag_kernel<MT, GW, true, Q> : lg::gemm_frag_kernel<MT, GW, false, Q>;
+    auto kern = bias ? lg::gemm_frag_kernel<MT, GW, true, Q, WIDE> : lg::gemm_frag_kernel<MT, GW, false, Q, WIDE>;
     int dev = 0;
     LG_CUDA(cudaGetDevice(&dev));
     if (dev >= 64 || !configured[dev][bias]) {
@@ -1015,6 +1020,7 @@ int launch_gemm_frag(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, 
 // planes; 28672 x 8192, 64.9 and 67.2; 4100 x 4096, q = 1, g = 32, 8 rows 6.3 and 7.6.
 template <int GW>
 int launch_gemm_frag_q(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, cudaStream_t st) {
+    if (frag_wide(w)) return launch_gemm_frag<1, GW, 0, true>(w, p, grid, st);
     switch (w->q) {
         case 1: return launch_gemm_frag<1, GW, 1>(w, p, grid, st);
         case 2: return launch_gemm_frag<1, GW, 2>(w, p, grid, st);
@@ -1024,6 +1030,11 @@ int launch_gemm_frag_q(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid
     }
 }
 
+template <int GW>
+int launch_gemm_frag_16(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, cudaStream_t st) {
+    return frag_wide(w) ? launch_gemm_frag<2, GW, 0, true>(w, p, grid, st) : launch_gemm_frag<2, GW, 0>(w, p, grid, st);
+}
+
 int gemm_frag_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, float* partial, lg::FrParams p, dim3 grid, const __half* x,
                    __half* y16, float* y32, int m, cudaStream_t st) {
     p.bW = w->bW; p.alpha = w->alpha; p.q_bias = w->q_bias; p.x = x;
@@ -1031,10 +1042,14 @@ int gemm_frag_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, float* 
     p.y16 = y16; p.y32 = y32;
     p.N = w->N; p.K = w->K; p.q = w->q; p.g = w->g; p.m = m;
     p.ones = 0x3c003c00u; p.twos = 0x40004000u; p.fours = 0x44004400u;
-    p.group_magic = w->g == 32 ? 0u : (uint32_t)(((1ull << 32) + w->g / 32 - 1) / (w->g / 32));
-    if (w->g % 128 == 0) return m <= 8 ? launch_gemm_frag_q<4>(w, p, grid, st) : launch_gemm_frag<2, 4, 0>(w, p, grid, st);
-    if (w->g % 64 == 0) return m <= 8 ? launch_gemm_frag_q<2>(w, p, grid, st) : launch_gemm_frag<2, 2, 0>(w, p, grid, st);
-    return m <= 8 ? launch_gemm_frag_q<1>(w, p, grid, st) : launch_gemm_frag<2, 1, 0>(w, p, grid, st);
+    const unsigned d = w->g / 32;
+    p.group_shift = 0;
+    if (frag_wide(w))
+        while (2u << p.group_shift < d) p.group_shift++;
+    p.group_magic = d == 1 ? 0u : (uint32_t)(((1ull << (32 + p.group_shift)) + d - 1) / d);
+    if (w->g % 128 == 0) return m <= 8 ? launch_gemm_frag_q<4>(w, p, grid, st) : launch_gemm_frag_16<4>(w, p, grid, st);
+    if (w->g % 64 == 0) return m <= 8 ? launch_gemm_frag_q<2>(w, p, grid, st) : launch_gemm_frag_16<2>(w, p, grid, st);
+    return m <= 8 ? launch_gemm_frag_q<1>(w, p, grid, st) : launch_gemm_frag_16<1>(w, p, grid, st);
 }
 
 template <int Q>

@@ -70,7 +70,10 @@ struct FrParams {
     int depth;               // units of a warp's ring
     // fp16 pairs of 1, 2 and 4: as arguments they stay in registers; as literals the compiler made them anew for every LOP3
     uint32_t ones, twos, fours;
-    uint32_t group_magic;    // ceil(2^32 / (g / 32)), 0 for g = 32: k-word -> scale group
+    // k-word -> scale group: ceil(2^(32 + shift) / (g / 32)), 0 for g = 32.  shift: 0, or where WIDE the most that is less than g / 32,
+    // which is exact for every k-word below 2^31
+    uint32_t group_magic;
+    int group_shift;
 };
 
 // `size` bytes (all or none: then src is not read) and zeros behind them
@@ -210,8 +213,9 @@ __device__ __noinline__ void fr_by_product(const FrParams& p, unsigned rows, int
     }
 }
 
-// Q: planes, 0 for any number.
-template <int MT, int GW, bool BIAS, int Q>
+// Q: planes, 0 for any number.  WIDE: byte offsets count from the slab's first k-word and group, not from the tensors' bases, so that
+// those may be 4 GiB long or more (3 % slower).
+template <int MT, int GW, bool BIAS, int Q, bool WIDE = false>
 __global__ void __launch_bounds__(kFrThreads, 1)
 gemm_frag_kernel(const __grid_constant__ FrParams p) {
     constexpr int KS = MT == 1 ? 2 : 1;
@@ -243,7 +247,7 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
     const int tile0 = blockIdx.x * p.tiles_per_cta, tile1 = min(tiles, tile0 + p.tiles_per_cta);
 
     // ---- the warp's stream of units: (tile, step) ----
-    // Byte offsets are 32 bits wide (the plan refuses more); beyond the end of the stream, the columns or K zeros come instead.
+    // Byte offsets are 32 bits wide; beyond the end of the stream, the columns or K zeros come instead.
     const uint32_t row_b = (uint32_t)q * (uint32_t)N * 4u;       // bytes of a k-word row of words
     const int f_kw = lane >> 3, f_chunk = lane & 7;
     int fi = 0, fslot = 0, fcol = (tile0 + wc) * kFrCols + 4 * f_chunk;
@@ -254,21 +258,31 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
     constexpr int PB = 4 / NG;
     const int f_plane = f_kw / NG, f_group = f_kw % NG;
     const uint32_t f_adst = ring_u + a_off + lane * 8;
+    auto group_of = [&](int kw) {
+        if (GW == 1 && !p.group_magic) return (uint32_t)kw;
+        const uint32_t at = __umulhi((uint32_t)kw, p.group_magic);
+        return WIDE ? at >> p.group_shift : at;
+    };
+    const int word0 = WIDE ? 4 * slab0 : 0;
+    const uint32_t grp0 = WIDE ? group_of(word0) : 0u;
+    const unsigned char* const bW0 = reinterpret_cast<const unsigned char*>(p.bW) + (WIDE ? (size_t)word0 * q * N * 4 : 0);
+    const unsigned char* const alpha0 = reinterpret_cast<const unsigned char*>(p.alpha) + (WIDE ? (size_t)grp0 * q * N * 2 : 0);
+    const unsigned char* const q_bias0 = reinterpret_cast<const unsigned char*>(p.q_bias) + (WIDE ? (size_t)grp0 * N * 2 : 0);
     auto fetch = [&]() {
         const int kw0 = 4 * (slab0 + wk + fi * p.kw), akw = kw0 + GW * f_group;
         const int end = fcol < fcol_end ? words : 0;
         const uint32_t size = kw0 + f_kw < end ? 16u : 0u, asize = akw < end ? 8u : 0u, at = fslot * ub;
-        const uint32_t off = (uint32_t)(kw0 + f_kw) * row_b + (uint32_t)fcol * 4u;
+        const uint32_t off = (uint32_t)(kw0 - word0 + f_kw) * row_b + (uint32_t)fcol * 4u;
         const int pu = Q ? Q : GW == 1 ? q : 8;      // GW = 1 copies scales as often as words: planes that are not there cost too much
 #pragma unroll (Q ? Q : GW == 1 ? 4 : 8)
         for (int b = 0; b < pu; b++)
-            if (Q || GW == 1 || b < q) cp_async16(f_dst + at + b * 512, reinterpret_cast<const unsigned char*>(p.bW) + (off + b * ((uint32_t)N * 4u)), size);
-        const uint32_t grp = GW == 1 && !p.group_magic ? (unsigned)akw : __umulhi((unsigned)akw, p.group_magic);
+            if (Q || GW == 1 || b < q) cp_async16(f_dst + at + b * 512, bW0 + (off + b * ((uint32_t)N * 4u)), size);
+        const uint32_t grp = group_of(akw) - grp0;
         const uint32_t aoff = ((grp * q + f_plane) * (uint32_t)N + fcol) * 2u;
 #pragma unroll (Q ? Q : GW == 1 ? 2 : 8)
         for (int b = 0; b < pu; b += PB)
-            if (b + f_plane < q) cp_async8(f_adst + at + b * (NG * 64), reinterpret_cast<const unsigned char*>(p.alpha) + (aoff + b * ((uint32_t)N * 2u)), asize);
-        if (BIAS && f_plane == 0) cp_async8(f_adst + at + q * (NG * 64), reinterpret_cast<const unsigned char*>(p.q_bias) + (grp * (uint32_t)N + fcol) * 2u, asize);
+            if (b + f_plane < q) cp_async8(f_adst + at + b * (NG * 64), alpha0 + (aoff + b * ((uint32_t)N * 2u)), asize);
+        if (BIAS && f_plane == 0) cp_async8(f_adst + at + q * (NG * 64), q_bias0 + (grp * (uint32_t)N + fcol) * 2u, asize);
         if (++fslot == p.depth) fslot = 0;
         if (++fi == nsteps) {
             fi = 0;

@@ -232,8 +232,36 @@ def test_fp32_results_of_two_and_three_rows(N, K, q, bias, m):
     w.close()
 
 
+# planes of 4 GiB, and a k and groups so long that their product has more than 32 bits; a word or a scale from the wrong place is an
+# error of the size of the result
+@pytest.mark.parametrize("N,K,q,g,bias,rows", [(65540, 131200, 4, 320, False, (4, 16)), (36, 6291456, 1, 3145728, True, (5, 11)), (36, 6291488, 2, 32, True, (8, 9))])
+def test_register_operand_kernel_of_wide_containers(N, K, q, g, bias, rows):
+    gen = torch.Generator(device="cuda").manual_seed(N + q)
+    bW = torch.randint(-2 ** 31, 2 ** 31, (K // 32, q, N), dtype=torch.int32, device="cuda", generator=gen)
+    alpha = torch.rand((K // g, q, N), dtype=torch.float16, device="cuda", generator=gen) * 0.02
+    q_bias = torch.rand((K // g, N), dtype=torch.float16, device="cuda", generator=gen) * 0.02 if bias else None
+    x = torch.rand((max(rows), K), dtype=torch.float16, device="cuda", generator=gen) - 0.5
+    w = L.nQWeight_fp16.from_device(bW, alpha, q_bias, K, N, q, False, K // g).reserve_batch(max(rows))
+    cols = torch.tensor([0, 3, 17, N // 2, N - 5, N - 1], device="cuda")
+    ref = torch.zeros((max(rows), len(cols)), dtype=torch.float64, device="cuda")
+    for i, c in enumerate(cols):
+        for b in range(q):
+            bits = (bW[:, b, c, None] >> torch.arange(32, device="cuda")) & 1
+            ref[:, i] += ((bits.reshape(-1) * 2 - 1) * x.double()).reshape(-1, K // g, g).sum(2) @ alpha[:, b, c].double()
+        if bias:
+            ref[:, i] += x.double().reshape(-1, K // g, g).sum(2) @ q_bias[:, c].double()
+    for m in rows:
+        y = torch.full((m, N), float("nan"), device="cuda")
+        for _ in range(2):
+            L.matmul_f32(y, x, w, m)
+            assert L.last_launch()[0] == "gemm_frag_kernel"
+            assert torch.linalg.norm(y[:, cols].double() - ref[:m]) <= 1e-3 * torch.linalg.norm(ref[:m])
+            assert torch.isfinite(y).all()
+    w.close()
+
+
 # k-ranges cost reductions: no more of them where the longest share stays what it is
-@pytest.mark.parametrize("N,K,q,g,bias,m,ranges", [(4100, 4096, 2, 64, True, 16, 2), (12292, 4096, 1, 128, False, 16, 2), (12288, 8192, 3, 64, False, 4, 2)])
+@pytest.mark.parametrize("N,K,q,g,bias,m,ranges", [(4100, 4096, 2, 64, True, 16, 2), (12292, 4096, 1, 128, False, 16, 2), (12288, 8192, 3, 64, False, 4, 4)])
 def test_register_operand_kernel_k_ranges(N, K, q, g, bias, m, ranges):
     bW, alpha, q_bias = synth.bcq_layer(N, K, q, g, seed=N + m, with_bias=bias)
     w = L.nQWeight_fp16(bW, alpha, K, N, q, False, K // g, q_bias).reserve_batch(m)
