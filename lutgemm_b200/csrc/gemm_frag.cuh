@@ -259,30 +259,26 @@ gemm_frag_kernel(const __grid_constant__ FrParams p) {
     const int f_plane = f_kw / NG, f_group = f_kw % NG;
     const uint32_t f_adst = ring_u + a_off + lane * 8;
     auto group_of = [&](int kw) {
-        if (GW == 1 && !p.group_magic) return (uint32_t)kw;
-        const uint32_t at = __umulhi((uint32_t)kw, p.group_magic);
-        return WIDE ? at >> p.group_shift : at;
+        if (WIDE) return (p.group_magic ? __umulhi((unsigned)kw, p.group_magic) : (unsigned)kw) >> p.group_shift;
+        return GW == 1 && !p.group_magic ? (unsigned)kw : __umulhi((unsigned)kw, p.group_magic);
     };
-    const int word0 = WIDE ? 4 * slab0 : 0;
-    const uint32_t grp0 = WIDE ? group_of(word0) : 0u;
-    const unsigned char* const bW0 = reinterpret_cast<const unsigned char*>(p.bW) + (WIDE ? (size_t)word0 * q * N * 4 : 0);
-    const unsigned char* const alpha0 = reinterpret_cast<const unsigned char*>(p.alpha) + (WIDE ? (size_t)grp0 * q * N * 2 : 0);
-    const unsigned char* const q_bias0 = reinterpret_cast<const unsigned char*>(p.q_bias) + (WIDE ? (size_t)grp0 * N * 2 : 0);
+    const uint32_t grp0 = WIDE ? group_of(4 * slab0) : 0u;
+    auto base = [&](const void* tensor, size_t offset) { return reinterpret_cast<const unsigned char*>(tensor) + (WIDE ? offset : 0); };
     auto fetch = [&]() {
         const int kw0 = 4 * (slab0 + wk + fi * p.kw), akw = kw0 + GW * f_group;
         const int end = fcol < fcol_end ? words : 0;
         const uint32_t size = kw0 + f_kw < end ? 16u : 0u, asize = akw < end ? 8u : 0u, at = fslot * ub;
-        const uint32_t off = (uint32_t)(kw0 - word0 + f_kw) * row_b + (uint32_t)fcol * 4u;
+        const uint32_t off = (uint32_t)(kw0 + f_kw - (WIDE ? 4 * slab0 : 0)) * row_b + (uint32_t)fcol * 4u;
         const int pu = Q ? Q : GW == 1 ? q : 8;      // GW = 1 copies scales as often as words: planes that are not there cost too much
 #pragma unroll (Q ? Q : GW == 1 ? 4 : 8)
         for (int b = 0; b < pu; b++)
-            if (Q || GW == 1 || b < q) cp_async16(f_dst + at + b * 512, bW0 + (off + b * ((uint32_t)N * 4u)), size);
-        const uint32_t grp = group_of(akw) - grp0;
+            if (Q || GW == 1 || b < q) cp_async16(f_dst + at + b * 512, base(p.bW, (size_t)(4 * slab0) * q * N * 4) + (off + b * ((uint32_t)N * 4u)), size);
+        const uint32_t grp = WIDE ? group_of(akw) - grp0 : group_of(akw);
         const uint32_t aoff = ((grp * q + f_plane) * (uint32_t)N + fcol) * 2u;
 #pragma unroll (Q ? Q : GW == 1 ? 2 : 8)
         for (int b = 0; b < pu; b += PB)
-            if (b + f_plane < q) cp_async8(f_adst + at + b * (NG * 64), alpha0 + (aoff + b * ((uint32_t)N * 2u)), asize);
-        if (BIAS && f_plane == 0) cp_async8(f_adst + at + q * (NG * 64), q_bias0 + (grp * (uint32_t)N + fcol) * 2u, asize);
+            if (b + f_plane < q) cp_async8(f_adst + at + b * (NG * 64), base(p.alpha, (size_t)grp0 * q * N * 2) + (aoff + b * ((uint32_t)N * 2u)), asize);
+        if (BIAS && f_plane == 0) cp_async8(f_adst + at + q * (NG * 64), base(p.q_bias, (size_t)grp0 * N * 2) + (grp * (uint32_t)N + fcol) * 2u, asize);
         if (++fslot == p.depth) fslot = 0;
         if (++fi == nsteps) {
             fi = 0;
