@@ -566,11 +566,6 @@ bool gemv_pair_ok(const lutgemm_weight* w, const lutgemm_workspace* ws) {
            lg::gemv22_num_stages(w->a_rows) >= 2;
 }
 
-// Most scale groups of g that a slab of 512 k touches: slabs and groups begin on multiples of 32.
-int reg_scale_rows(int g) {
-    if (g >= lg::kSlab2) return g % lg::kSlab2 == 0 ? 1 : 2;
-    return lg::kSlab2 % g == 0 ? lg::kSlab2 / g : (lg::kSlab2 - 32) / g + 2;
-}
 
 // One matvec row: y (fp16 and/or fp32) = x . W
 int gemv_row(const lutgemm_weight* w, const lutgemm_workspace* ws, const __half* x, __half* y16, float* y32, cudaStream_t st) {
@@ -585,7 +580,7 @@ int gemv_row(const lutgemm_weight* w, const lutgemm_workspace* ws, const __half*
         p.nslabs = (w->K + lg::kSlab2 - 1) / lg::kSlab2;
         p.n_tile = choose_ntile(w->N, p.nslabs, 1, lg::kStageCols);
         p.ordered = ordered_for(ws);
-        p.a_rows = reg_scale_rows(w->g);
+        p.a_rows = lg::reg_scale_rows(w->g);
         dim3 grid((w->N + p.n_tile - 1) / p.n_tile, p.nslabs);
         const bool bias = w->q_bias != nullptr;
         if (w->g % 128 == 0) return launch_gemv_reg<2>(p, grid, bias, st);

@@ -17,6 +17,25 @@ namespace lg {
 constexpr int kRegFeedWarps = 4;
 constexpr int kRegThreads = (kConsWarps + kRegFeedWarps) * 32;
 
+// Most scale groups of g that a slab of 512 k touches: it begins at a multiple of the largest power of two in g (up to 512) into one,
+// the last of those at most, and its last word 480 further.
+constexpr int reg_scale_rows(int g) {
+    const int step = (g & -g) < kSlab2 ? g & -g : kSlab2;
+    return (g - step + kSlab2 - 32) / g + 1;
+}
+constexpr bool reg_scale_rows_exact() {
+    for (int g = 32; g <= 2 * kSlab2 + 32; g += 32) {
+        int most = 0;
+        for (int slab = 0; slab < g / 32; slab++) {               // 512 slab runs through all its remainders
+            const int touched = (slab * kSlab2 + kSlab2 - 32) / g - slab * kSlab2 / g + 1;
+            if (touched > most) most = touched;
+        }
+        if (most != reg_scale_rows(g)) return false;
+    }
+    return true;
+}
+static_assert(reg_scale_rows_exact(), "rows of scales for every slab, and none too many");
+
 struct FeedCopies {
     static constexpr int kArrivals = kRegFeedWarps * 32;
     __device__ __forceinline__ void operator()(const Gemv2Params& p, unsigned char* smem, uint32_t bar_full, uint32_t bar_empty, int n_begin, int,
