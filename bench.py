@@ -74,7 +74,7 @@ def parse():
     ap.add_argument("--m", type=int, default=1, help="activation rows per matmul (1 = the headline matvec)")
     ap.add_argument("--rot", type=int, default=8, help="distinct weight sets cycled per step")
     ap.add_argument("--ntile", type=int, default=0, help="columns per CTA of the matvec (0 = automatic)")
-    ap.add_argument("--variant", type=int, default=0, help="0 = bulk-copy fed matvec kernel, 1 = register-streaming kernel")
+    ap.add_argument("--variant", type=int, default=0, help="0 = bulk-copy fed matvec kernel, 1 = the same fed by regular copies")
     ap.add_argument("--ordered", action="store_true", help="bit-reproducible split-k (slabs added in order)")
     ap.add_argument("--int8", action="store_true", help="batches of up to 16 rows: the integer tensor-core kernel instead of the fp16 one")
     ap.add_argument("--no-pdl", action="store_true", help="plain launches instead of programmatic dependent launch")

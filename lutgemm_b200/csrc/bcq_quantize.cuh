@@ -586,7 +586,7 @@ template <int Q>
 __global__ void __launch_bounds__(kBqLaneWarps * 32, 2)
 bcq_quantize_lane_kernel(const BqParams p) {
     constexpr int NH = 1 << (Q - 1);                       // levels of the upper half
-    extern __shared__ __align__(16) unsigned char smem[];
+    extern __shared__ __align__(1024) unsigned char smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int G = p.K / p.g, g = p.g, words = (g + 31) / 32;
     const long long groups = (long long)p.N * G;
@@ -792,12 +792,7 @@ bcq_quantize_lane_kernel(const BqParams p) {
 #pragma unroll
                 for (int i = 0; i < Q; i++) {
                     if (KIND == 2) {
-                        // plane 1 rises at 2; plane 2 rises at 1, falls at 2, rises at 3
-                        sg[i] = i ? -1.f : 1.f;
-                        if (i == 1) sg[i] = fmaf(2.f, from[NH / 2], sg[i]);
-                        if (i == 2)
-#pragma unroll
-                            for (int c = 1; c < NH; c++) sg[i] = fmaf(c & 1 ? 2.f : -2.f, from[c], sg[i]);
+                        sg[i] = i ? fmaf(2.f, from[1], -1.f) : 1.f;
                     } else {
                         sg[i] = step[i][0];
 #pragma unroll

@@ -125,7 +125,7 @@ std::atomic<int> g_ordered{0};
 std::atomic<int> g_pairs{1};     // 1: rows that go through the LUT matvec are taken two at a time where possible
 std::atomic<int> g_batched{1};   // 0: one matvec per row; 1: tensor-core kernel from kBatchedFromRows rows; 2: from 2 rows
 std::atomic<int> g_int8{0};      // 1: batches of up to 16 rows take the integer tensor-core kernel (measured slower: off)
-std::atomic<int> g_variant{0};   // 0: bulk-copy fed kernel (default); 1: register-streaming kernel
+std::atomic<int> g_variant{0};   // 0: bulk-copy fed kernel (default); 1: the same fed by regular copies
 // Split-k mode of a call on this workspace (read once per call).
 inline int ordered_for(const lutgemm_workspace* ws);
 constexpr int kMaxCounters = 4096;

@@ -51,7 +51,8 @@ __host__ __device__ constexpr int fr_red_floats(int mt) { return 4 * mt * 8 * kF
 __host__ __device__ constexpr int fr_depth(int gw, int mt, int q, bool bias) {
     const int per_warp = (kFrSmemBytes - kFrTailBytes - 2 * kFrWarps * fr_red_floats(mt) * 4) / kFrWarps;
     const int d = per_warp / fr_unit_bytes(gw, q, bias);
-    return d >= kFrMaxDepth ? kFrMaxDepth : d >= 3 ? 3 : d;       // a wait for each of these
+    // a wait for each of these; 4 and 5 units are no faster than 3: 8196 x 8192, g = 64, q = 3, 8 rows 22.9 / 21.5 us, q = 2 + q_bias, 16 rows 29.9 / 29.0
+    return d >= kFrMaxDepth ? kFrMaxDepth : d >= 3 ? 3 : d;
 }
 
 struct FrParams {
@@ -76,13 +77,6 @@ struct FrParams {
     int group_shift;
 };
 
-// `size` bytes (all or none: then src is not read) and zeros behind them
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t size) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
-}
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, uint32_t size) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }

@@ -38,7 +38,7 @@ static_assert(reg_scale_rows_exact(), "rows of scales for every slab, and none t
 
 struct FeedCopies {
     static constexpr int kArrivals = kRegFeedWarps * 32;
-    __device__ __forceinline__ void operator()(const Gemv2Params& p, unsigned char* smem, uint32_t bar_full, uint32_t bar_empty, int n_begin, int,
+    __device__ __forceinline__ void operator()(const Gemv2Params& p, unsigned char* smem, uint32_t bar_full, uint32_t bar_empty, int n_begin,
                                                int total_stages) const {
         const int tid = threadIdx.x - kConsWarps * 32;
         const int q = p.q, N = p.N, G = p.K / p.g, stage_bytes = gemv2_stage_bytes(p.a_rows), nstages = gemv2_num_stages(p.a_rows);
@@ -61,8 +61,8 @@ struct FeedCopies {
             const __half* asrc = p.alpha + ((size_t)grp0 * q + b) * N + col;
             const uint32_t dst = dst0 + slot * stage_bytes, adst = adst0 + slot * stage_bytes;
 #pragma unroll
-            for (int i = 0; i < kSlabWords / 2; i++) reg_copy16(dst + i * 2 * kRowPitch, src + i * step, ok && i < words ? 16u : 0u);
-            for (int i = 0; 2 * i + row0 < p.a_rows; i++) reg_copy8(adst + i * 2 * kARowPitch, asrc + i * step, ok && i < scales ? 8u : 0u);
+            for (int i = 0; i < kSlabWords / 2; i++) cp_async16(dst + i * 2 * kRowPitch, src + i * step, ok && i < words ? 16u : 0u);
+            for (int i = 0; 2 * i + row0 < p.a_rows; i++) cp_async8(adst + i * 2 * kARowPitch, asrc + i * step, ok && i < scales ? 8u : 0u);
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar_full + 8 * slot) : "memory");
             if (++slot == nstages) { slot = 0; round++; }
             if (++b == q) {
@@ -70,13 +70,6 @@ struct FeedCopies {
                 col += kStageCols;
             }
         }
-    }
-    // `size` bytes (all or none: then src is not read) and zeros behind them
-    static __device__ __forceinline__ void reg_copy16(uint32_t dst, const void* src, uint32_t size) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
-    }
-    static __device__ __forceinline__ void reg_copy8(uint32_t dst, const void* src, uint32_t size) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
     }
 };
 

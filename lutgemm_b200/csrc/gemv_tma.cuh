@@ -315,7 +315,7 @@ __device__ __forceinline__ void splitk_finish(const Gemv2Params& p, int tid, int
 struct FeedTma {
     static constexpr int kArrivals = 1;
     const CUtensorMap *tmW, *tmA;
-    __device__ __forceinline__ void operator()(const Gemv2Params& p, unsigned char* smem, uint32_t bar_full, uint32_t bar_empty, int n_begin, int,
+    __device__ __forceinline__ void operator()(const Gemv2Params& p, unsigned char* smem, uint32_t bar_full, uint32_t bar_empty, int n_begin,
                                                int total_stages) const {
         if ((threadIdx.x & 31) != 0) return;
         const int q = p.q, stage_bytes = gemv2_stage_bytes(p.a_rows), nstages = gemv2_num_stages(p.a_rows);
@@ -358,7 +358,6 @@ __device__ __forceinline__ void gemv_body(const Gemv2Params& p, unsigned char* s
     const int N = p.N, q = p.q;
     const int slab = blockIdx.y;
     const int k0 = slab * kSlab2;
-    const int kw0 = slab * kSlabWords;
     const int n_begin = blockIdx.x * p.n_tile;
     const int n_end = min(N, n_begin + p.n_tile);
     const int ncg = (n_end - n_begin + kStageCols - 1) / kStageCols;
@@ -378,7 +377,7 @@ __device__ __forceinline__ void gemv_body(const Gemv2Params& p, unsigned char* s
     if (warp >= kConsWarps) {
         // ---------------- producers.  Weights and scales are never written by a kernel, so the stream may start before the
         // previous kernel has finished. -------
-        feed(p, smem, bar_full, bar_empty, n_begin, n_end, total_stages);
+        feed(p, smem, bar_full, bar_empty, n_begin, total_stages);
         pdl_wait_prior_grids();
     } else {
         // ---------------- consumers ----------------

@@ -62,6 +62,14 @@ __device__ __forceinline__ void tma_prefetch_descriptor(const void* tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 
+// `size` bytes (all or none: then src is not read) and zeros behind them
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t size) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, uint32_t size) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(size) : "memory");
+}
+
 // Arrival of a CTA at a counter in global memory, by one thread behind a barrier: orders what the whole CTA wrote before that
 // barrier against what the last arriver's CTA reads behind the barrier that follows.  With this
 // instead of a fence by every thread, and one more by every thread of the last CTA: 4096 x 4096, q = 3, one row 5.53 -> 4.92 us, 12288
