@@ -115,8 +115,8 @@ __device__ __forceinline__ void u2b_words(const uint32_t (&t)[8], int b, int l8,
 // then rounded to the container's fp16.  A warp takes 32 rows x 128 k (four k-words), eight rows at a time: a lane reads four
 // codes of each (128 bits, the warp 512 contiguous bytes), lays its codes' bits of a plane side by side, and eight lanes exchange
 // their eight rows (u2b_words) until each has one row's words: the stores are whole 32-byte sectors.  Bound by HBM (4 bytes read
-// per code).  Measured, N = K = 8192, q = 4, g = 128: 53.4 us (5.8 TB/s); 61.5 with three shuffles per row and plane (the issue slots 69 %
-// taken); one thread per word and row takes 250 us (every lane on another row's line).
+// per code).  Measured, N = K = 8192, q = 4, g = 128: 53.4 us (5.8 TB/s); 61.5 with three shuffles per row and plane; now memory
+// holds it (issue slots 41 % taken); one thread per word and row takes 250 us (every lane on another row's line).
 constexpr int kU2bWarps = 8;
 template <int Q>
 __global__ void __launch_bounds__(kU2bWarps * 32)

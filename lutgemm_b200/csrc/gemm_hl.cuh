@@ -20,7 +20,8 @@
 //   and LOP3s), looks 64 weights up (one PRMT makes a code byte and the lane's bank an address) and stores them with
 //   tcgen05.st as the A operand in tensor memory.
 //   Up to two planes the values (four at most) stay in registers and a PRMT picks two weights' halves at a time: no table, no
-//   reads of shared memory.  8192 x 8192, q = 2, 128 rows 31.4 us (32.9 with the table), q = 2 + q_bias, 64 rows 24.4 (27.4).
+//   reads of shared memory.  Calls back to back on one weight, 8192 x 8192, q = 2, 128 rows 31.4 us (32.9 with the
+//   table), q = 2 + q_bias, 64 rows 24.4 (27.4); on weights in turn that L2 does not hold 34.3.
 //   One lane issues tcgen05.mma.kind::f16: M = 128 columns, N = rows, K = 16, A (hi, then lo) in tensor memory, the
 //   activations [rows][64 k] (TMA, 128-byte swizzle) in shared memory, one fp32 accumulator.
 //   Every accumulation of the tensor core cuts its fp32 sum off toward zero: measured, the error of a chain of n is 1.8e-8 n

@@ -11,7 +11,7 @@
 //
 // Bound like gemv_tma_kernel by lookups and staging in shared memory (some 860 cycles a stage; its loop takes 3.5 % more here).
 // Measured, us, one row, this / gemv_tma_kernel: 8192 x 28672, q = 4 + q_bias, 30.4 / 34.4; 4096 x 28672, q = 3, 16.3 / 28.7; 8192 x
-// 20480, q = 3, 19.8 / 22.5; where the shares are even 49152 x 12288, q = 4, 64.8 / 62.6.
+// 20480, q = 3, 19.8 / 22.5; where the shares are even 49152 x 12288, q = 4, on one weight 64.8 / 62.6.
 #pragma once
 #include "gemv_seq.cuh"
 

@@ -72,7 +72,7 @@ __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, uint32_
 
 // Arrival of a CTA at a counter in global memory, by one thread behind a barrier: orders what the whole CTA wrote before that
 // barrier against what the last arriver's CTA reads behind the barrier that follows.  With this
-// instead of a fence by every thread, and one more by every thread of the last CTA: 4096 x 4096, q = 3, one row 5.53 -> 4.92 us, 12288
+// instead of a fence by every thread, and one more by every thread of the last CTA, calls back to back on one weight: 4096 x 4096, q = 3, one row 5.53 -> 4.92 us, 12288
 // x 12288 17.56 -> 16.95, two rows of 8192 x 8192, q = 2 11.6 -> 10.3, 16 rows (gemm_tc) 22.4 -> 21.8, 128 rows (gemm_hl) 33.0 -> 31.8.
 __device__ __forceinline__ unsigned arrive_acq_rel(unsigned* counter) {
     unsigned prev;
