@@ -1012,7 +1012,8 @@ int launch_gemm_frag(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, 
 }
 
 // Up to four planes have a kernel each, their loops unrolled: 2048 x 2048, q = 4, 4 rows 5.2 us, 5.7 with the kernel for any number of
-// planes; 28672 x 8192, 64.9 and 67.2; 4100 x 4096, q = 1, g = 32, 8 rows 6.3 and 7.6.
+// planes; 28672 x 8192, 64.9 and 67.2; 4100 x 4096, q = 1, g = 32, 8 rows 6.3 and 7.6; 16 rows, in the mean of 15 to 30 calls of up to 2048 k
+// against the loops that ended with the planes, q = 1 0.94 and 1.06, q = 2 0.95 and 1.02, q = 3 0.96 and 1.00, q = 4 0.97 and 1.00.
 template <int GW>
 int launch_gemm_frag_q(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, cudaStream_t st) {
     if (frag_wide(w)) return launch_gemm_frag<1, GW, 0, true>(w, p, grid, st);
@@ -1027,7 +1028,14 @@ int launch_gemm_frag_q(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid
 
 template <int GW>
 int launch_gemm_frag_16(const lutgemm_weight* w, const lg::FrParams& p, dim3 grid, cudaStream_t st) {
-    return frag_wide(w) ? launch_gemm_frag<2, GW, 0, true>(w, p, grid, st) : launch_gemm_frag<2, GW, 0>(w, p, grid, st);
+    if (frag_wide(w)) return launch_gemm_frag<2, GW, 0, true>(w, p, grid, st);
+    switch (w->q) {
+        case 1: return launch_gemm_frag<2, GW, 1>(w, p, grid, st);
+        case 2: return launch_gemm_frag<2, GW, 2>(w, p, grid, st);
+        case 3: return launch_gemm_frag<2, GW, 3>(w, p, grid, st);
+        case 4: return launch_gemm_frag<2, GW, 4>(w, p, grid, st);
+        default: return launch_gemm_frag<2, GW, 0>(w, p, grid, st);
+    }
 }
 
 int gemm_frag_rows(const lutgemm_weight* w, const lutgemm_workspace* ws, float* partial, lg::FrParams p, dim3 grid, const __half* x,

@@ -146,7 +146,9 @@ def test_register_operand_kernel(N, K, q, g, bias, m):
 # one to four planes have kernels of their own: a last tile of one quad, a last step of two words, several tiles and steps to a warp
 @pytest.mark.parametrize("q", [1, 2, 3, 4])
 @pytest.mark.parametrize("N,K,g,bias,m", [(68, 192, 64, True, 4), (5220, 1152, 64, False, 8), (68, 128, 128, False, 5), (9508, 768, 384, True, 4),
-                                           (68, 160, 32, True, 8), (5220, 1152, 96, False, 4)])
+                                           (68, 160, 32, True, 8), (5220, 1152, 96, False, 4),
+                                           (68, 192, 64, True, 9), (5220, 1152, 64, False, 16), (68, 160, 32, True, 16), (1044, 4128, 96, False, 12),
+                                           (132, 128, 128, False, 12), (9508, 2304, 384, True, 16)])
 def test_register_operand_kernel_per_plane_count(N, K, q, g, bias, m):
     _run("gemm_frag_kernel", N, K, q, g, bias, m)
 
